@@ -9,13 +9,17 @@
 // a = x (.) s_g exist nowhere in memory: a CTA owns one group (64 output features), up to 64 activation rows and a range of K,
 // and its converter warps make them from x and s_g stage by stage.
 //
-// Arithmetic.  q = round(a * 2^e) with |q| < 2^31, e chosen per (row, group) from a bound on |a| over the WHOLE row (so that
-// partial sums of different K ranges are integers of one unit, and their order does not matter).  q + 2^31 is four unsigned
-// bytes: four planes of the A operand, no digit carries to work out; sum_k (q + 2^31) u is exact in int32 per plane
-// (255 * 255 * K < 2^31 for K <= 32768) and int64 together, and 2^31 * sum_k u[n,k], a property of the weight row, is taken off
-// once at the end.  The bound is max over 64-wide chunks of K of max|x| * max|s|: at most a factor of the spread inside a
-// chunk above max|a|, so a keeps 30 bits below the bound (28 below the largest |a| with a chunk 4x off).  The bias term is an
-// f32 sum per lane over at most 16 stages (64 terms), added up in double.
+// Arithmetic.  q = round(a * 2^e) with |q| < 2^31, e chosen per (row, group) so that the largest |a| of the WHOLE row times 2^e
+// lies in [2^30, 2^31) (partial sums of different K ranges are then integers of one unit, and their order does not matter).
+// q + 2^31 is four unsigned bytes: four planes of the A operand, no digit carries to work out; sum_k (q + 2^31) u is exact in
+// int32 per plane (255 * 255 * K < 2^31 for K <= 32768) and int64 together, and 2^31 * sum_k u[n,k], a property of the weight
+// row, is taken off once at the end.  The largest |a| has to be the true one: max|x| max|s| over a stretch of k is far above it
+// where an outlier of x meets a small scale, and every factor of two of that is a bit of all other activations (an outlier of
+// 10^6 on a scale of 10^-6 cost 1e-3 of the result).  Up to eight rows every CTA multiplies x and s_g once more for it.  Larger
+// batches know the largest |x| of a stage (128 k), its place and the second largest: the product at that place is one of the
+// row's, and second largest times the stage's largest |s| bounds the others; all products of a stage are taken only where
+// that bound has a larger exponent than the largest product so far (hardly ever for weights and activations of one scale).
+// The bias term is an f32 sum per lane over BSUM stages (16 terms), added up in double.
 //
 // Roles: warp 0 brings weights, scales and biases by TMA into a ring of stages (128 k each), starting before
 // griddepcontrol.wait; warp 1 issues the MMAs (M = 128: 32 rows x 4 planes, row 4m + p; N = 64 output features; K = 32); eight
@@ -46,7 +50,6 @@ constexpr int CW = 8;                          // converter / epilogue warps
 constexpr int GC_THREADS = 32 * (2 + CW);
 constexpr int W_BYTES = GN * SK;               // weight bytes of a stage
 constexpr int STAGE_BYTES = W_BYTES + 2 * SK * 4;   // + scales + biases (9 KiB: every stage starts on 1 KiB)
-constexpr int CHUNK = 64;                      // k per entry of the bound tables
 constexpr int BSUM = 4;                        // stages a lane's f32 bias sum runs (from multiples of four stages on)
 constexpr int MAX_STAGES = 8;
 // The A operand of a stage, 128 rows of 128 bytes per row block.  A CTA of few rows fills the first 32 RPW rows only, and its
@@ -60,11 +63,11 @@ constexpr int A_BUFS = RB == 2 ? 2 : 8 / RPW;
 struct GcParams {
     const float* scales;         // [N/64][K]
     const float* biases;         // [N/64][K]
-    const float* smax;           // [N/64][K/64]: largest |scale| of a chunk
+    const float* smax;           // [N/64][K/128]: largest |scale| of a stage
     const int* rowsum;           // [N]: sum of a weight row's bytes
     const void* x;               // the caller's rows; RPW > 1: gc_prepare_kernel's copy [K/128][Mp][128]
     size_t xstep;                // elements from a stage to the next: 128, or 128 Mp
-    const uint32_t* xmax;        // [M][K/64]: |x| maxima (as bits) made by gc_prepare_kernel; null: the converter warps work them out
+    const uint2* xtop;           // RPW > 1: [M][K/128], a stage's largest |x|s, made by gc_prepare_kernel
     void* y;
     const void* residual;        // null, or added to every output
     int M, N, K;
@@ -77,7 +80,12 @@ struct GcParams {
     long long peer_delta[PEER_MAX_RANKS];
 };
 
+// Magnitudes are compared as bits: a NaN or an infinity is above every number.
 __device__ __forceinline__ uint32_t abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ uint32_t abs_max(const float4& v) { return max(max(abs_bits(v.x), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w))); }
+__device__ __forceinline__ uint32_t abs_max(const float4& x, const float4& s) {   // of the products, rounded as the converters round them
+    return abs_max(make_float4(__fmul_rn(x.x, s.x), __fmul_rn(x.y, s.y), __fmul_rn(x.z, s.z), __fmul_rn(x.w, s.w)));
+}
 
 template <typename XT>
 __device__ __forceinline__ float4 ldg_x4(const XT* p) {
@@ -96,12 +104,9 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 }
 __device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 
-// Bound (as float bits) -> exponent e of the row's unit 2^-e: bound * 2^e in [2^29, 2^30).  Very small bounds stop at 2^126.
+// Largest |a| (as float bits) -> exponent e of the row's unit 2^-e: |a| * 2^e in [2^30, 2^31).  Very small ones stop at 2^127.
 __device__ __forceinline__ int unit_exponent(uint32_t bits) {
-    if (bits == 0u) return 0;
-    const int eb = (int)(bits >> 23) - 127;   // subnormal: -127
-    const int e = 29 - eb;
-    return e > 126 ? 126 : e;
+    return min(157 - (int)(bits >> 23), 127);
 }
 
 // XT: type of the caller's x (RPW = 1 reads it as it is).  RB: row blocks of 32 (1 or 2); RPW: rows per converter warp (1, 2, 4 or 8; RB = 2 has 8)
@@ -119,9 +124,9 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
     uint64_t* d_full = a_empty + MAX_STAGES;
     double* s_bias = reinterpret_cast<double*>(d_full + 1);          // [RB * 32]: this K range's bias term of a row
     int* s_exp = reinterpret_cast<int*>(s_bias + RB * 32);           // [RB * 32]: e of a row, or INT_MIN: poisoned
-    uint32_t* s_bnd = reinterpret_cast<uint32_t*>(s_exp + RB * 32);  // [RB * 32]: bound of a row's |a| (bits)
-    float* s_smax = reinterpret_cast<float*>(s_bnd + RB * 32);       // [K / 64]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_smax + p.K / CHUNK);
+    uint32_t* s_top = reinterpret_cast<uint32_t*>(s_exp + RB * 32);  // [RB * 32]: largest |a| of a row (bits, its exponent at least)
+    float* s_smax = reinterpret_cast<float*>(s_top + RB * 32);       // [K / 128]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_smax + p.nst);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = warp_id(), lane = threadIdx.x & 31;
@@ -133,6 +138,21 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
     const int st0 = nb * way / p.ways * BSUM, st1 = min(p.nst, nb * (way + 1) / p.ways * BSUM);
     const int active = min(CW, rows);          // converter warps that arrive on a stage
     pdl_launch_dependents();
+    // The scales are needed before the first weights are: asked for ahead of the ring's 70 KB, up to eight rows the first ones
+    // into registers.
+    constexpr int AHEAD = 4;          // stages whose scales a converter warp holds while the rows go by (RPW = 1)
+    const float* gs = p.scales + (size_t)g * p.K + lane * 4;
+    float4 sv[AHEAD];
+    auto fetch_scales = [&](int st) {
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u)
+            if (st + u * CW < p.nst) sv[u] = ldg_x4(gs + (st + u * CW) * SK);
+    };
+    if (warp >= 2) {
+        if constexpr (RPW == 1) fetch_scales(warp - 2);
+        for (int k = (RPW == 1 ? AHEAD * CW * SK : 0) + ((int)threadIdx.x - 64) * 32; k < p.K; k += 32 * CW * 32)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.scales + (size_t)g * p.K + k));
+    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
             mbar_init(&in_full[s], 1);
@@ -147,7 +167,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
         fence_barrier_init();
     }
     if (threadIdx.x >= 64 && threadIdx.x < 64 + RB * 32) {
-        s_bnd[threadIdx.x - 64] = 0u;
+        s_top[threadIdx.x - 64] = 0u;
         s_bias[threadIdx.x - 64] = 0.0;
     }
     if (warp == 1) tmem_alloc(tmem_slot, RB * GN);
@@ -211,62 +231,94 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
     } else {
         // ------------------------------ converters ----------------------------
         const int cw = warp - 2, ct = threadIdx.x - 64;
-        const int nch = p.K / CHUNK;
-        for (int c = ct; c < nch; c += 32 * CW) s_smax[c] = __ldg(p.smax + (size_t)g * nch + c);   // the weight's own: before the wait
-        pdl_wait();   // x (and xmax) may come from the previous kernel
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * CW) : "memory");
+        if constexpr (RPW > 1)      // the weight's own: before the wait
+            for (int st = ct; st < p.nst; st += 32 * CW) s_smax[st] = __ldg(p.smax + (size_t)g * p.nst + st);
+        pdl_wait();   // x (and xtop) may come from the previous kernel
+        if constexpr (RPW > 1) asm volatile("bar.sync 1, %0;" ::"n"(32 * CW) : "memory");
         // Up to four rows: two warps a row, every other BSUM stages each (a ring of 8 stages and 8 A buffers: a warp meets the
         // same slots again and again, one phase further each time).
         const bool shared_rows = RPW == 1 && rows <= 4;
         const int row_w = shared_rows ? cw & 3 : cw;                    // this warp's first row; further ones 8 apart
         const int sub = shared_rows ? cw >> 2 : 0;
         const int nr = row_w < rows ? (rows - row_w + 7) / 8 : 0;       // rows of this warp
-        // bounds: NaN or infinity anywhere shows as a bound above every number
-        auto bound_of = [&](uint32_t xb, uint32_t sb) {
-            const uint32_t prod = __float_as_uint(fminf(__uint_as_float(xb) * __uint_as_float(sb), 3.0e38f));
-            return (xb > 0x7f7fffffu || sb > 0x7f7fffffu) ? 0xffffffffu : prod;
-        };
-        if (p.xmax) {
-            for (int i = 0; i < nr; ++i) {
-                const uint32_t* xm = p.xmax + (size_t)(m0 + row_w + 8 * i) * nch;
-                uint32_t bnd = 0u;
-                for (int c = lane; c < nch; c += 32) bnd = max(bnd, bound_of(__ldg(xm + c), __float_as_uint(s_smax[c])));
-                bnd = __reduce_max_sync(0xffffffffu, bnd);
-                if (lane == 0) s_bnd[row_w + 8 * i] = bnd;
-            }
-            __syncwarp();
-        } else {
+        if constexpr (RPW == 1) {
             // every warp takes an eighth of K of every row
             const XT* xr = reinterpret_cast<const XT*>(p.x) + (size_t)m0 * p.K + lane * 4;
-            for (int m = 0; m < rows; ++m, xr += p.K) {
-                uint32_t bnd = 0u;
-                for (int kb = cw; kb < p.nst; kb += 4 * CW) {
-                    float4 v[4];
+            for (int kb = cw; kb < p.nst; kb += AHEAD * CW) {
+                if (kb != cw) fetch_scales(kb);
+                for (int m = 0; m < rows; ++m) {
+                    float4 v[AHEAD];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (kb + u * CW < p.nst) v[u] = ldg_x4<XT>(xr + (kb + u * CW) * SK);
+                    for (int u = 0; u < AHEAD; ++u)
+                        if (kb + u * CW < p.nst) v[u] = ldg_x4<XT>(xr + (size_t)m * p.K + (kb + u * CW) * SK);
+                    uint32_t top = 0u;
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (kb + u * CW < p.nst) {
-                            const uint32_t xb = max(max(abs_bits(v[u].x), abs_bits(v[u].y)), max(abs_bits(v[u].z), abs_bits(v[u].w)));
-                            bnd = max(bnd, bound_of(xb, __float_as_uint(s_smax[(kb + u * CW) * 2 + (lane >> 4)])));
-                        }
+                    for (int u = 0; u < AHEAD; ++u)
+                        if (kb + u * CW < p.nst) top = max(top, abs_max(v[u], sv[u]));
+                    top = __reduce_max_sync(0xffffffffu, top);
+                    if (lane == 0) atomicMax(s_top + m, top);
                 }
-                bnd = __reduce_max_sync(0xffffffffu, bnd);
-                if (lane == 0) atomicMax(s_bnd + m, bnd);
             }
             asm volatile("bar.sync 1, %0;" ::"n"(32 * CW) : "memory");
+        } else {
+            // (the unit depends on the exponent alone, and that is the true one here as well: a row has the same in any batch)
+            const uint2* xt = p.xtop + (size_t)(m0 + row_w) * p.nst;
+            const float* xr = reinterpret_cast<const float*>(p.x) + (size_t)(m0 + row_w) * SK + lane * 4;
+            auto rest_bound = [&](uint2 v, int st) { return abs_bits(__fmul_rn(__uint_as_float(v.y & 0xffff0000u), s_smax[st])); };
+            uint32_t top[RPW], rest[RPW];
+#pragma unroll
+            for (int i = 0; i < RPW; ++i) top[i] = rest[i] = 0u;
+            for (int st = lane; st < p.nst; st += 32) {
+                uint2 v[RPW];
+                float s1[RPW];
+#pragma unroll
+                for (int i = 0; i < RPW; ++i)
+                    if (i < nr) v[i] = __ldg(xt + (size_t)(8 * i) * p.nst + st);
+#pragma unroll
+                for (int i = 0; i < RPW; ++i)
+                    if (i < nr) s1[i] = __ldg(p.scales + (size_t)g * p.K + st * SK + (v[i].y & 0xffffu));
+#pragma unroll
+                for (int i = 0; i < RPW; ++i)
+                    if (i < nr) {
+                        top[i] = max(top[i], abs_bits(__fmul_rn(__uint_as_float(v[i].x), s1[i])));
+                        rest[i] = max(rest[i], rest_bound(v[i], st));
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < RPW; ++i)
+                if (i < nr) {
+                    top[i] = __reduce_max_sync(0xffffffffu, top[i]);
+                    if (__any_sync(0xffffffffu, rest[i] >> 23 > top[i] >> 23)) {
+                        for (int base = 0; base < p.nst; base += 32) {
+                            const int st = base + lane;
+                            const uint32_t b = st < p.nst ? rest_bound(__ldg(xt + (size_t)(8 * i) * p.nst + st), st) >> 23 : 0u;
+                            uint32_t todo = __ballot_sync(0xffffffffu, b > top[i] >> 23);
+                            auto stage_max = [&](int s) { return abs_max(ldg_x4(xr + (size_t)s * p.xstep + i * (8 * SK)), ldg_x4(gs + s * SK)); };
+                            while (todo) {     // two stages at a time
+                                const int sa = base + __ffs(todo) - 1;
+                                todo &= todo - 1;
+                                const int sb = todo ? base + __ffs(todo) - 1 : sa;
+                                todo &= todo - 1;
+                                top[i] = max(top[i], __reduce_max_sync(0xffffffffu, max(stage_max(sa), stage_max(sb))));
+                                todo &= __ballot_sync(0xffffffffu, b > top[i] >> 23);
+                            }
+                        }
+                    }
+                    if (lane == 0) s_top[row_w + 8 * i] = top[i];
+                }
+            __syncwarp();
         }
         float scale[RPW];
 #pragma unroll
         for (int i = 0; i < RPW; ++i) {
             scale[i] = 0.0f;
             if (i < nr) {
-                const uint32_t bnd = s_bnd[row_w + 8 * i];
-                const int e = unit_exponent(bnd);
-                // 2^e: between 2^-98 (bounds near the largest float) and 2^126, always a normal number
-                scale[i] = bnd == 0xffffffffu ? 0.0f : __uint_as_float((uint32_t)(127 + e) << 23);
-                if (lane == 0) s_exp[row_w + 8 * i] = bnd == 0xffffffffu ? INT_MIN : e;
+                const uint32_t top = s_top[row_w + 8 * i];
+                const bool finite = top < 0x7f800000u;
+                const int e = unit_exponent(top);
+                // 2^e: between 2^-97 (products near the largest float) and 2^127, always a normal number
+                scale[i] = finite ? __uint_as_float((uint32_t)(127 + e) << 23) : 0.0f;
+                if (lane == 0) s_exp[row_w + 8 * i] = finite ? e : INT_MIN;
             }
         }
         if (nr > 0) {
@@ -505,34 +557,44 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
     if (p.ways > 1) cl.sync();   // the others have read this CTA's sums
 }
 
-// For batches of more than 8 rows, once instead of in every CTA: xmax[m][c] = max |x| over 64 k (as bits: a NaN is above every
-// number), and x as f32 in the order the converters read it, [K/128][Mp][128]: a warp's rows of a stage then lie at constant
-// offsets, and rows M .. Mp and k beyond K (zeros) need no checks.  One block a row.  K % 4 == 0.
+// For batches of more than 8 rows, once instead of in every CTA: xtop[m][st] = (largest |x| of 128 k; the next largest, rounded
+// up to 16 bits, above the place of the largest), as bits: a NaN is above every number; and x as f32 in the order the
+// converters read it, [K/128][Mp][128]: a warp's rows of a stage then lie at constant offsets, and rows M .. Mp and k beyond K
+// (zeros) need no checks.  A block takes 1024 k of a row.  K % 4 == 0.
 template <typename XT>
-__global__ void __launch_bounds__(256) gc_prepare_kernel(const XT* __restrict__ x, float* __restrict__ xs, uint32_t* __restrict__ xmax, int M, int Mp,
+__global__ void __launch_bounds__(256) gc_prepare_kernel(const XT* __restrict__ x, float* __restrict__ xs, uint2* __restrict__ xtop, int M, int Mp,
                                                          int K) {
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31, m = blockIdx.x;
     const XT* row = x + (size_t)m * K;
     const int Kp = (K + SK - 1) / SK * SK;
-    for (int k = threadIdx.x * 4; k < Kp; k += 1024) {   // (a warp is inside or outside)
+    const int k = (blockIdx.y * 256 + threadIdx.x) * 4;
+    if (k < Kp) {                                        // (a warp is inside or outside)
         const float4 v = m < M && k < K ? ldg_x4<XT>(row + k) : make_float4(0.f, 0.f, 0.f, 0.f);
         *reinterpret_cast<float4*>(xs + ((size_t)(k / SK) * Mp + m) * SK + (k & (SK - 1))) = v;
-        uint32_t b = max(max(abs_bits(v.x), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w)));
+        const uint32_t c[4] = {abs_bits(v.x), abs_bits(v.y), abs_bits(v.z), abs_bits(v.w)};
+        uint32_t best = c[0], next = 0u, at = 0u;
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
-        if ((lane & 15) == 0 && m < M) xmax[(size_t)m * (Kp / CHUNK) + k / CHUNK] = b;
+        for (uint32_t i = 1; i < 4; ++i) {
+            const bool more = c[i] > best;
+            next = max(next, more ? best : c[i]);
+            if (more) best = c[i], at = i;
+        }
+        const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+        const int who = __ffs(__ballot_sync(0xffffffffu, best == top)) - 1;
+        next = __reduce_max_sync(0xffffffffu, lane == who ? next : best);
+        next = min((next >> 16) + ((next & 0xffffu) != 0u), 0x7fffu);
+        if (lane == who && m < M) xtop[(size_t)m * (Kp / SK) + k / SK] = make_uint2(top, next << 16 | (lane * 4 + at));
     }
 }
 
-// The weight's own tables, once at create: largest |scale| of every 64 k of a group (a NaN or infinite scale shows as such),
+// The weight's own tables, once at create: largest |scale| of every 128 k of a group (a NaN or infinite scale shows as such),
 // and the byte sum of every row.
-__global__ void __launch_bounds__(256) gc_smax_kernel(const float* __restrict__ s, float* __restrict__ smax, size_t chunks) {
-    for (size_t c = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); c < chunks; c += (size_t)gridDim.x * 8) {
-        const float* p = s + c * CHUNK;
+__global__ void __launch_bounds__(256) gc_smax_kernel(const float* __restrict__ s, float* __restrict__ smax, size_t entries) {
+    for (size_t c = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); c < entries; c += (size_t)gridDim.x * 8) {
         const int lane = threadIdx.x & 31;
-        uint32_t b = __reduce_max_sync(0xffffffffu, max(abs_bits(p[lane]), abs_bits(p[lane + 32])));
+        const uint32_t b = __reduce_max_sync(0xffffffffu, abs_max(ldg_x4(s + c * SK + lane * 4)));
         if (lane == 0) smax[c] = __uint_as_float(b);
     }
 }
@@ -567,16 +629,16 @@ bool gc_tc_supported(const rusty_cuda_ctx* ctx, uint32_t N, uint32_t K) {
     return ctx->tc_ws && encode_tiled_fn() && K % 4 == 0 && K <= 32768u && N % GN == 0 && N / GN <= 65535u;
 }
 uint32_t gc_padded(uint32_t K) { return (K + SK - 1) / SK * SK; }
-size_t gc_tables_bytes(uint32_t N, uint32_t K) { return (size_t)(N / GN) * (gc_padded(K) / CHUNK) * 4 + (size_t)N * 4; }
+size_t gc_tables_bytes(uint32_t N, uint32_t K) { return (size_t)(N / GN) * (gc_padded(K) / SK) * 4 + (size_t)N * 4; }
 int launch_gc_tables(rusty_cuda_ctx* ctx, const uint8_t* w, const float* scales, void* tables, uint32_t N, uint32_t K) {
     K = gc_padded(K);
-    const size_t chunks = (size_t)(N / GN) * (K / CHUNK);
+    const size_t entries = (size_t)(N / GN) * (K / SK);
     float* smax = (float*)tables;
-    const size_t blocks = (chunks + 7) / 8, cap = (size_t)ctx->sm_count * 8;
-    gc_smax_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, ctx->stream>>>(scales, smax, chunks);
+    const size_t blocks = (entries + 7) / 8, cap = (size_t)ctx->sm_count * 8;
+    gc_smax_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, ctx->stream>>>(scales, smax, entries);
     int rc = after_launch(ctx, "gc_smax");
     if (rc) return rc;
-    gc_rowsum_kernel<<<(N + 7) / 8, 256, 0, ctx->stream>>>(w, (int*)(smax + chunks), (int)N, (int)K);
+    gc_rowsum_kernel<<<(N + 7) / 8, 256, 0, ctx->stream>>>(w, (int*)(smax + entries), (int)N, (int)K);
     return after_launch(ctx, "gc_rowsum");
 }
 
@@ -587,7 +649,7 @@ int launch_gc_tc(rusty_cuda_ctx* ctx, const QLinearArgs& a) {
     p.smax = (const float*)a.gc_tables;
     p.N = (int)a.N;
     p.K = (int)gc_padded(a.K);   // the weight's rows, scales and biases are that long, zeros behind a.K
-    p.rowsum = (const int*)(p.smax + (size_t)(p.N / GN) * (p.K / CHUNK));
+    p.rowsum = (const int*)(p.smax + (size_t)(p.N / GN) * (p.K / SK));
     p.nst = p.K / SK;
     p.ldy = (int)a.ldy;
     p.y_col0 = (int)a.y_col0;
@@ -600,8 +662,8 @@ int launch_gc_tc(rusty_cuda_ctx* ctx, const QLinearArgs& a) {
     if (!make_map_u8(&map_w, a.w, a.N, (uint32_t)p.K, GN)) return fail(ctx, RUSTY_CUDA_ERR_KERNEL_EXECUTION, "gc_tc: cuTensorMapEncodeTiled failed");
     const bool xb = a.x_dtype == RUSTY_CUDA_BF16;
     const size_t xs = xb ? 2 : 4, ys = p.y_bf16 ? 2 : 4;
-    // the digit region of the workspace: x rearranged (Mp rows), then the maxima
-    const size_t row_bytes = (size_t)p.K * 4 + (size_t)(p.K / CHUNK) * 4;
+    // the digit region of the workspace: x rearranged (Mp rows), then its largest values
+    const size_t row_bytes = (size_t)p.K * 4 + (size_t)p.nst * 8;
     const uint32_t per_pass = (uint32_t)(tc_workspace_xq_bytes() / row_bytes) & ~63u;
     for (uint32_t m0 = 0; m0 < a.M; m0 += per_pass) {
         p.M = (int)(a.M - m0 < per_pass ? a.M - m0 : per_pass);
@@ -613,18 +675,19 @@ int launch_gc_tc(rusty_cuda_ctx* ctx, const QLinearArgs& a) {
         const int rpw = p.M <= 8 && p.K == (int)a.K ? 1 : p.M <= 16 ? 2 : p.M <= 32 ? 4 : 8;
         const int rb = rpw == 8 ? 2 : 1, tile = rpw == 8 ? 64 : 8 * rpw, tiles = (p.M + tile - 1) / tile;
         p.xstep = SK;
-        p.xmax = nullptr;
+        p.xtop = nullptr;
         if (rpw > 1) {
             const int Mp = tiles * tile;
             float* xbuf = (float*)ctx->tc_ws;
-            uint32_t* xmax = (uint32_t*)(xbuf + (size_t)Mp * p.K);
-            cudaError_t e = xb ? launch_pdl(gc_prepare_kernel<__nv_bfloat16>, dim3((unsigned)Mp), dim3(256), 0, ctx->stream, (const __nv_bfloat16*)p.x, xbuf, xmax, p.M, Mp, (int)a.K)
-                               : launch_pdl(gc_prepare_kernel<float>, dim3((unsigned)Mp), dim3(256), 0, ctx->stream, (const float*)p.x, xbuf, xmax, p.M, Mp, (int)a.K);
+            uint2* xtop = (uint2*)(xbuf + (size_t)Mp * p.K);
+            const dim3 pg((unsigned)Mp, (unsigned)(p.K + 1023) / 1024);
+            cudaError_t e = xb ? launch_pdl(gc_prepare_kernel<__nv_bfloat16>, pg, dim3(256), 0, ctx->stream, (const __nv_bfloat16*)p.x, xbuf, xtop, p.M, Mp, (int)a.K)
+                               : launch_pdl(gc_prepare_kernel<float>, pg, dim3(256), 0, ctx->stream, (const float*)p.x, xbuf, xtop, p.M, Mp, (int)a.K);
             if (e != cudaSuccess) return check_cuda(ctx, e, "gc_prepare");
             int rc = after_launch(ctx, "gc_prepare");
             if (rc) return rc;
             p.x = xbuf;
-            p.xmax = xmax;
+            p.xtop = xtop;
             p.xstep = (size_t)Mp * SK;
         }
         const int groups = p.N / GN;
@@ -632,7 +695,7 @@ int launch_gc_tc(rusty_cuda_ctx* ctx, const QLinearArgs& a) {
         // suffice, and the start and the end of a CTA cost as much as ten stages.
         p.ways = 1;
         while (tiles == 1 && p.ways < 4 && groups * p.ways * 2 <= 2 * ctx->sm_count && p.nst / (p.ways * 2) >= 4) p.ways *= 2;
-        const size_t fixed = 1024 + (size_t)rb * A_BYTES + (4 * MAX_STAGES + 1) * 8 + (size_t)rb * 32 * 16 + (size_t)(p.K / CHUNK) * 4 + 64;
+        const size_t fixed = 1024 + (size_t)rb * A_BYTES + (4 * MAX_STAGES + 1) * 8 + (size_t)rb * 32 * 16 + (size_t)p.nst * 4 + 64;
         const size_t budget = (ctx->smem_optin + 1024) / 2 - 1024;   // half an SM, less the 1 KiB every block pays
         int stages = budget > fixed ? (int)((budget - fixed) / STAGE_BYTES) : 0;
         if (stages > MAX_STAGES) stages = MAX_STAGES;

@@ -526,6 +526,28 @@ def test_native_affine_batches(ctx, engine, oracle, M, K, N):
     assert np.isnan(got[0]).all() and np.isfinite(got[1:]).all()
 
 
+@pytest.mark.parametrize("M,K,N", [(1, 4096, 64), (4, 11008, 64), (8, 4352, 128), (9, 4096, 64), (13, 8192, 128), (32, 4100, 64), (64, 4096, 192), (65, 4096, 64), (150, 2112, 128)])
+@pytest.mark.parametrize("outliers", ["one", "per_stage"])
+def test_native_affine_outliers_on_small_scales(ctx, engine, M, K, N, outliers):
+    """Input features a million times the others whose scales are as much smaller: what an activation keeps depends on the
+    largest product x * scale, not on the largest of each.  One such feature, or one in every 128 (no stage of a row can be told
+    from its neighbours by its largest value and largest scale).  1e-6 as for the ordinary distributions above; a unit taken from
+    the separate maxima is off by 1e-3."""
+    rng = np.random.default_rng(M + K + N)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    sg = rng.uniform(0.001, 0.02, size=(K, N // 64)).astype(np.float32)
+    at = rng.integers(0, K, size=1) if outliers == "one" else np.arange(0, K, 128) + rng.integers(0, 64, size=(K + 127) // 128)
+    at = at[at < K]
+    x[:, at] *= np.float32(1e6)
+    sg[at] *= np.float32(1e-6)
+    ukn = rng.integers(0, 256, size=(K, N), dtype=np.uint8)
+    bg = (-128.0 * sg * rng.uniform(0.9, 1.1, size=sg.shape)).astype(np.float32)
+    got = _forward(ctx, engine, QLinear.from_host(ctx, ukn, sg, bg, layout=capi.LAYOUT_KN), x)
+    wf = ukn.astype(np.float64) * np.repeat(sg.astype(np.float64), 64, axis=1) + np.repeat(bg.astype(np.float64), 64, axis=1)
+    assert rel_err_rows(got, x.astype(np.float64) @ wf) <= 1e-6
+    assert_bits_equal(got[M - 1:], _forward(ctx, engine, QLinear.from_host(ctx, ukn, sg, bg, layout=capi.LAYOUT_KN), x[M - 1:]))
+
+
 @pytest.mark.parametrize("M,K,N", [(65, 256, 128), (130, 400, 257), (391, 1024, 4100), (1030, 128, 300), (600, 28672, 128)])
 def test_f32_prompts_in_row_blocks(ctx, engine, M, K, N):
     """More than 64 f32 rows run as several row blocks of one launch pair: every row as if its block were alone, with the
