@@ -199,7 +199,7 @@ RUSTY_CUDA_API int rusty_cuda_linear_lora_f32(rusty_cuda_ctx* ctx, const rusty_c
  * (the reference's own quantised format: one scale and bias per 64
  * consecutive OUTPUT features of an input row) with K % 4 == 0 and K <= 32768
  * is re-laid-out the same way, bytes to [out,in] and scales / biases to
- * [N/64][K], rows padded to a multiple of 128 (N*K*9/8 more bytes; none of the
+ * [N/64][K], rows padded to a multiple of 128 (N*K*19/16 more bytes; none of the
  * caller's three buffers is kept): its forwards run on the int8 tensor cores
  * with the group's scales folded into the activations (f32 activations: 1e-5
  * of the reference's arithmetic) and, with bf16 activations, M >= 65 and

@@ -19,17 +19,23 @@
 // batches know the largest |x| of a stage (128 k), its place and the second largest: the product at that place is one of the
 // row's, and second largest times the stage's largest |s| bounds the others; all products of a stage are taken only where
 // that bound has a larger exponent than the largest product so far (hardly ever for weights and activations of one scale).
-// The bias term is an f32 sum per lane over BSUM stages (16 terms), added up in double.
+// The bias term is as large as the integer part and of the other sign for weights around zero, so it is summed as exactly: with
+// b = r s it is sum_k a[m,k] r[k], and r, at create, becomes 32 bits below the group's largest |r|, four more "weight rows" of
+// unsigned bytes per group (and a row of ones, for the sum of q that takes the offset off again).  An output is then
+// sum_k a (u + r) with nothing rounded but a.  (Summed in f32 beside the conversion, 16 terms at a time and those in double, the
+// bias alone cost 1.0e-7 of an output and everything else 0.6e-7; in double, 24 % of the time of a 512-row layer.)  A group with
+// a b of more than 4096 scales has no such r: its bias term is summed in double after the last stage.
 //
-// Roles: warp 0 brings weights, scales and biases by TMA into a ring of stages (128 k each), starting before
-// griddepcontrol.wait; warp 1 issues the MMAs (M = 128: 32 rows x 4 planes, row 4m + p; N = 64 output features; K = 32); eight
-// converter warps take rows cw, cw + 8, ..., 128 k of a row at a time (a lane's four neighbours: one 16-byte load of x, one
-// 4-byte store per plane, no bank conflicts under the 128-byte swizzle), and are the epilogue in the end.  Two CTAs fit an SM.
+// Roles: warp 0 brings weights, bytes of r and scales by TMA into a ring of stages (128 k each), starting before
+// griddepcontrol.wait; warp 1 issues the MMAs (M = 128: 32 rows x 4 planes, row 4m + p; N = 64 output features, 5 columns for the
+// bias and 11 nobody reads; K = 32); eight converter warps take rows cw, cw + 8, ..., 128 k of a row at a time (a lane's four
+// neighbours: one 16-byte load of x, one 4-byte store per plane, no bank conflicts under the 128-byte swizzle), and are the
+// epilogue in the end.  Two CTAs fit an SM.
 // A K range per CTA of a cluster (1, 2 or 4) where there are too few groups; their int64 sums meet in distributed shared memory.
 //
 // What bounds it: few rows, the weight stream (one pass; 4096 x 4096 x 13 rows took 80 us when every pair of rows walked the
-// weights again, converting activations per pair and CTA); from about 24 rows on the conversion, ~36 issue slots per row and
-// 128 k and group: 512 rows of a Llama-7B layer 415 us of issue time at the least.  Measured, 4096 x 4096 weights, device time:
+// weights again, converting activations per pair and CTA); from about 24 rows on the conversion, ~32 issue slots per row and
+// 128 k and group.  Measured, 4096 x 4096 weights, device time:
 // 4 rows 13.2 -> 9.8 us, 32 rows 58.6 -> 20 us (before: a kernel for one or two rows, a pair of rows per CTA).  12288 x 2112,
 // whose last stage is half empty (rows padded at create): 1 row 15.5 -> 11.6 us, 64 rows 600 -> 40 us (before: CUDA cores).
 #include <cooperative_groups.h>
@@ -48,9 +54,15 @@ constexpr int GN = 64;                         // output features per CTA = one 
 constexpr int SK = 128;                        // k per stage
 constexpr int CW = 8;                          // converter / epilogue warps
 constexpr int GC_THREADS = 32 * (2 + CW);
+constexpr int NC = 80;                         // columns of the MMA: GN, RD of r's bytes, one of ones (a multiple of 16)
+constexpr int RD = 4;
 constexpr int W_BYTES = GN * SK;               // weight bytes of a stage
-constexpr int STAGE_BYTES = W_BYTES + 2 * SK * 4;   // + scales + biases (9 KiB: every stage starts on 1 KiB)
-constexpr int BSUM = 4;                        // stages a lane's f32 bias sum runs (from multiples of four stages on)
+// + eight rows for r and ones (9 KiB: every stage starts on 1 KiB; what lies behind a stage multiplies into columns nobody reads)
+constexpr int STAGE_BYTES = W_BYTES + 8 * SK;
+constexpr int S_BYTES = SK * 4;                // scales of a stage, in a ring of their own behind it
+constexpr int TX_BYTES = W_BYTES + RD * SK + S_BYTES;
+constexpr int R_MAX = 4096;                    // largest |b / s| that goes to the tensor core
+constexpr int BSUM = 4;                        // K ranges start at multiples of this many stages
 constexpr int MAX_STAGES = 8;
 // The A operand of a stage, 128 rows of 128 bytes per row block.  A CTA of few rows fills the first 32 RPW rows only, and its
 // buffers lie that close together: the MMA then multiplies what follows (other buffers, the ring) into rows nobody reads.
@@ -63,6 +75,8 @@ constexpr int A_BUFS = RB == 2 ? 2 : 8 / RPW;
 struct GcParams {
     const float* scales;         // [N/64][K]
     const float* biases;         // [N/64][K]
+    const uint8_t* rbytes;       // [N/64][K/128][RD * 128]: r's rows of a stage, swizzled as they lie in shared memory
+    const int* rinfo;            // [N/64][8]: byte sums of r's four rows; r's unit is 2^-rinfo[4] (INT_MIN: a group without r)
     const float* smax;           // [N/64][K/128]: largest |scale| of a stage
     const int* rowsum;           // [N]: sum of a weight row's bytes
     const void* x;               // the caller's rows; RPW > 1: gc_prepare_kernel's copy [K/128][Mp][128]
@@ -114,15 +128,16 @@ template <typename XT, int RB, int RPW>
 __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ GcParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    constexpr int PITCH = A_PITCH<RB, RPW>, BUFS = A_BUFS<RB, RPW>;
+    constexpr int PITCH = A_PITCH<RB, RPW>, BUFS = A_BUFS<RB, RPW>, TCOLS = RB == 2 ? 256 : 128;
     uint8_t* sA = smem;                                              // [BUFS] x PITCH
     uint8_t* sIn = smem + RB * A_BYTES;                              // [stages][STAGE_BYTES]
-    uint64_t* in_full = reinterpret_cast<uint64_t*>(sIn + (size_t)p.stages * STAGE_BYTES);
+    uint8_t* sSc = sIn + (size_t)p.stages * STAGE_BYTES;             // [stages][S_BYTES]
+    uint64_t* in_full = reinterpret_cast<uint64_t*>(sSc + (size_t)p.stages * S_BYTES);
     uint64_t* in_empty = in_full + MAX_STAGES;
     uint64_t* a_full = in_empty + MAX_STAGES;
     uint64_t* a_empty = a_full + MAX_STAGES;
     uint64_t* d_full = a_empty + MAX_STAGES;
-    double* s_bias = reinterpret_cast<double*>(d_full + 1);          // [RB * 32]: this K range's bias term of a row
+    double2* s_bias = reinterpret_cast<double2*>(d_full + 2);        // [RB * 32]: a group without r: this K range's bias term, in two parts
     int* s_exp = reinterpret_cast<int*>(s_bias + RB * 32);           // [RB * 32]: e of a row, or INT_MIN: poisoned
     uint32_t* s_top = reinterpret_cast<uint32_t*>(s_exp + RB * 32);  // [RB * 32]: largest |a| of a row (bits, its exponent at least)
     float* s_smax = reinterpret_cast<float*>(s_top + RB * 32);       // [K / 128]
@@ -168,31 +183,37 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
     }
     if (threadIdx.x >= 64 && threadIdx.x < 64 + RB * 32) {
         s_top[threadIdx.x - 64] = 0u;
-        s_bias[threadIdx.x - 64] = 0.0;
+        s_bias[threadIdx.x - 64] = make_double2(0.0, 0.0);
     }
-    if (warp == 1) tmem_alloc(tmem_slot, RB * GN);
+    if (warp == 1) {
+        // the rows of ones (by a warp without loads in flight: the fence would wait for them)
+        for (int s = 0; s < p.stages; ++s) sts32(smem_u32(sIn + (size_t)s * STAGE_BYTES + W_BYTES + RD * SK) + lane * 4, 0x01010101u);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        tmem_alloc(tmem_slot, TCOLS);
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const int rowsum_n = warp >= 2 ? __ldg(p.rowsum + g * GN + ((threadIdx.x - 64) & (GN - 1))) : 0;   // for the very end
+    // (both for the very end)
+    const int4 rsum = warp >= 2 ? __ldg(reinterpret_cast<const int4*>(p.rinfo) + 2 * g) : make_int4(0, 0, 0, 0);
+    const int runit = warp >= 2 ? __ldg(p.rinfo + 8 * g + 4) : 0;
+    const int rowsum_n = warp >= 2 ? __ldg(p.rowsum + g * GN + ((threadIdx.x - 64) & (GN - 1))) : 0;
 
     if (warp == 0) {
         // ------------------------------ producer ------------------------------
         // several row tiles read the weights again (from L2); one tile: a single pass
         const uint64_t pol = p.M > RB * 32 ? policy_evict_last() : policy_evict_first();
-        const float* gs = p.scales + (size_t)g * p.K;
-        const float* gb = p.biases + (size_t)g * p.K;
         int s = 0, issued = 0;
         uint32_t ph = 0;
         for (int st = st0; st < st1; ++st, ++issued) {
             if (!mbar_wait(&in_empty[s], ph ^ 1u, abort_flag, p.status, 41)) break;
             uint8_t* dst = sIn + (size_t)s * STAGE_BYTES;
             if (elect_one()) {
-                mbar_expect_tx(&in_full[s], (uint32_t)STAGE_BYTES);
+                mbar_expect_tx(&in_full[s], (uint32_t)TX_BYTES);
                 tma_load_2d(dst, &map_w, st * SK, g * GN, &in_full[s], pol);
-                bulk_load(dst + W_BYTES, gs + st * SK, SK * 4, &in_full[s]);
-                bulk_load(dst + W_BYTES + SK * 4, gb + st * SK, SK * 4, &in_full[s]);
+                bulk_load(dst + W_BYTES, p.rbytes + ((size_t)g * p.nst + st) * (RD * SK), RD * SK, &in_full[s]);
+                bulk_load(sSc + (size_t)s * S_BYTES, p.scales + (size_t)g * p.K + st * SK, S_BYTES, &in_full[s]);
             }
             __syncwarp();
             if (++s == p.stages) { s = 0; ph ^= 1u; }
@@ -205,7 +226,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ----------------------------
         // u8 x u8 -> s32, both K-major: c_format = S32 (2) @4, a_format = b_format = U8 (0), N >> 3 @17, M >> 4 @24
-        constexpr uint32_t idesc = (2u << 4) | ((uint32_t)(GN >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        constexpr uint32_t idesc = (2u << 4) | ((uint32_t)(NC >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
         int s = 0, ab = 0;
         uint32_t ph = 0, aph = 0;
         for (int st = st0; st < st1; ++st) {
@@ -218,7 +239,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
                     const uint64_t da = make_smem_desc(smem_u32(sA + (size_t)ab * PITCH + (size_t)rb * 16384));
 #pragma unroll
                     for (int k4 = 0; k4 < SK / 32; ++k4)
-                        umma_i8(tmem_base + (uint32_t)(rb * GN), da + (uint64_t)(2 * k4), db + (uint64_t)(2 * k4), idesc, (st > st0 || k4 > 0) ? 1u : 0u);
+                        umma_i8(tmem_base + (uint32_t)(rb * NC), da + (uint64_t)(2 * k4), db + (uint64_t)(2 * k4), idesc, (st > st0 || k4 > 0) ? 1u : 0u);
                 }
                 umma_commit(&in_empty[s]);
                 umma_commit(&a_empty[ab]);
@@ -334,13 +355,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
 #pragma unroll
             for (int pl = 0; pl < 4; ++pl)
                 off[pl] = smem_u32(sA) + (uint32_t)(row_w * 512 + pl * 128 + ((((lane >> 2) ^ pl) << 4) ^ ((row_w & 1) << 6)) + (lane & 3) * 4);
-            const uint32_t sv0 = smem_u32(sIn) + W_BYTES + lane * 16;
-            float bacc[RPW];
-            double btot[RPW == 8 ? 1 : RPW];
-#pragma unroll
-            for (int i = 0; i < RPW; ++i) bacc[i] = 0.0f;
-#pragma unroll
-            for (int i = 0; i < (RPW == 8 ? 1 : RPW); ++i) btot[i] = 0.0;
+            const uint32_t sv0 = smem_u32(sSc) + lane * 16;
             bool ok = true;
             // (RPW > 1: the copy's rows are 512 bytes, and there are rows enough for the whole tile: no checks, constant offsets)
             const XT* xw = reinterpret_cast<const XT*>(p.x) + (RPW == 1 ? (size_t)(m0 + row_w) * p.K : (size_t)(m0 + row_w) * SK) + lane * 4 + st0 * p.xstep;
@@ -351,7 +366,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
 #pragma unroll
                         for (int i = 0; i < GR; ++i) v[i * GS + h] = ldg_x4<XT>(q + h * p.xstep + (half * GR + i) * (8 * SK));
             };
-            uint4 sq, bq;
+            uint4 sq;
             int slot = 0, ab = 0;
             uint32_t ph = 0, aph = 0, at[4];
             // waits for stage idx's scales and biases and for its A buffer
@@ -363,8 +378,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
                     aph = ((uint32_t)idx / BUFS) & 1u;
                 }
                 if (!mbar_wait(&in_full[slot], ph, abort_flag, p.status, 44)) return false;
-                sq = lds128(sv0 + (uint32_t)slot * STAGE_BYTES);
-                bq = lds128(sv0 + (uint32_t)slot * STAGE_BYTES + SK * 4);
+                sq = lds128(sv0 + (uint32_t)slot * S_BYTES);
                 if (!mbar_wait(&a_empty[ab], aph ^ 1u, abort_flag, p.status, 45)) return false;
 #pragma unroll
                 for (int pl = 0; pl < 4; ++pl) at[pl] = off[pl] + (uint32_t)ab * PITCH;
@@ -382,41 +396,15 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
                 sts32(at[1] + (uint32_t)(r * 4096), __byte_perm(t2, t3, 0x5410));
                 sts32(at[2] + (uint32_t)(r * 4096), __byte_perm(t0, t1, 0x7632));
                 sts32(at[3] + (uint32_t)(r * 4096), __byte_perm(t0, t1, 0x5410));
-                bacc[r] = fmaf(x4.x, __uint_as_float(bq.x), bacc[r]);
-                bacc[r] = fmaf(x4.y, __uint_as_float(bq.y), bacc[r]);
-                bacc[r] = fmaf(x4.z, __uint_as_float(bq.z), bacc[r]);
-                bacc[r] = fmaf(x4.w, __uint_as_float(bq.w), bacc[r]);
             };
-            // hands the stage's rows to the MMA; a lane's bias sums move on to double every BSUM stages
-            auto leave = [&](int idx, bool last) {
+            // hands the stage's rows to the MMA
+            auto leave = [&] {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMA reads through the async proxy
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&a_full[ab]);
                 if constexpr (RB == 2) {
                     if (++slot == p.stages) { slot = 0; ph ^= 1u; }
                     if (++ab == BUFS) { ab = 0; aph ^= 1u; }
-                }
-                if ((idx & (BSUM - 1)) == BSUM - 1 || last) {
-                    if constexpr (RPW == 8) {
-                        // lanes 4r .. 4r + 3 keep row r's sum: halve the rows a lane holds three times, adding as they go
-                        double d[8];
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) d[i] = (double)bacc[i];
-#pragma unroll
-                        for (int w = 4, o = 16; w >= 1; w >>= 1, o >>= 1)
-#pragma unroll
-                            for (int i = 0; i < w; ++i) {
-                                const bool up = (lane & o) != 0;
-                                const double give = up ? d[i] : d[i + w], keep = up ? d[i + w] : d[i];
-                                d[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-                            }
-                        btot[0] += d[0];
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < RPW; ++i) btot[i] += (double)bacc[i];
-                    }
-#pragma unroll
-                    for (int i = 0; i < RPW; ++i) bacc[i] = 0.0f;
                 }
             };
             float4 xa[4], xb[4];
@@ -433,7 +421,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
                     if (both)
 #pragma unroll
                         for (int i = 0; i < GR; ++i) item(xb[i], GR + i);
-                    leave(st - st0, st == st1 - 1);
+                    leave();
                 }
             } else {
                 auto convert = [&](const float4 (&v)[4], int st) {
@@ -443,7 +431,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
                         if (!enter(st + h - st0)) { ok = false; return; }
 #pragma unroll
                         for (int i = 0; i < GR; ++i) item(v[i * GS + h], i);
-                        leave(st + h - st0, st + h == st1 - 1);
+                        leave();
                     }
                 };
                 int st = st0 + sub * BSUM;
@@ -458,19 +446,26 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
                     convert(xb, st + step);
                 }
             }
-            if constexpr (RPW == 8) {
-                double b = btot[0];
-                b += __shfl_xor_sync(0xffffffffu, b, 2);
-                b += __shfl_xor_sync(0xffffffffu, b, 1);
-                const int r = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
-                if ((lane & 3) == 0 && r < nr) s_bias[row_w + 8 * r] = b;
-            } else {
+            if (runit == INT_MIN && sub == 0) {
+                // A group without r: x . b in double.  Upper 24 bits and the rest of every four terms are added up apart: exact
+                // sums, whatever the K ranges.
+                const XT* xb = reinterpret_cast<const XT*>(p.x) + (RPW == 1 ? (size_t)(m0 + row_w) * p.K : (size_t)(m0 + row_w) * SK) + lane * 4;
+                const float* gb = p.biases + (size_t)g * p.K + lane * 4;
+                for (int i = 0; i < nr; ++i) {
+                    double hi = 0.0, lo = 0.0;
+                    for (int st = st0; st < st1; ++st) {
+                        const float4 x4 = ldg_x4<XT>(xb + (size_t)st * p.xstep + i * (RPW == 1 ? 8 * p.K : 8 * SK)), b4 = ldg_x4(gb + st * SK);
+                        const double d = fma((double)x4.x, (double)b4.x, fma((double)x4.y, (double)b4.y, fma((double)x4.z, (double)b4.z, (double)x4.w * (double)b4.w)));
+                        const double u = __hiloint2double(__double2hiint(d), __double2loint(d) & (int)0xe0000000);
+                        hi += u;
+                        lo += d - u;
+                    }
 #pragma unroll
-                for (int i = 0; i < RPW; ++i) {
-                    double b = btot[i];
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
-                    if (lane == 0 && i < nr) atomicAdd(s_bias + row_w + 8 * i, b);   // (two warps a row: two sums, either order)
+                    for (int o = 16; o > 0; o >>= 1) {
+                        hi += __shfl_xor_sync(0xffffffffu, hi, o);
+                        lo += __shfl_xor_sync(0xffffffffu, lo, o);
+                    }
+                    if (lane == 0) s_bias[row_w + 8 * i] = make_double2(hi, lo);
                 }
             }
         }
@@ -485,9 +480,10 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    constexpr int LDW = 33;                                            // words between rows of a warp's corner: no bank conflicts
-    uint32_t* s_raw = reinterpret_cast<uint32_t*>(smem);               // [CW][32][LDW] (33 KiB)
-    long long* s_sum = reinterpret_cast<long long*>(smem + 36 * 1024); // [RB * 32][GN]
+    constexpr int LDW = RB == 1 ? 37 : 33;                             // words between rows of a warp's corner: no bank conflicts
+    uint32_t* s_raw = reinterpret_cast<uint32_t*>(smem);               // [CW][32][LDW]
+    long long* s_sum = reinterpret_cast<long long*>(smem + 40 * 1024); // [RB * 32][GN]
+    long long* s_ext = s_sum + RB * 32 * GN;                           // [RB * 32][RD + 1]: the bias columns
     const bool failed = *abort_flag != 0;
     if (warp >= 2 && !failed) {
         const int cw = warp - 2, q = warp & 3, half = cw >> 2;         // lane quarter of tensor memory, half of the columns
@@ -495,20 +491,42 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
 #pragma unroll
         for (int rb = 0; rb < RB; ++rb) {
             if (rb * 32 + q * 8 < rows) {
+                const uint32_t from = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(rb * NC);
+                uint32_t v[2][16], ext[16];
 #pragma unroll
-                for (int c = 0; c < 32; c += 16) {
-                    uint32_t v[16];
-                    tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(rb * GN + half * 32 + c), v);
-                    tmem_ld_wait();
+                for (int c = 0; c < 2; ++c) tmem_ld16(from + half * 32 + c * 16, v[c]);
+                if (half == 1) tmem_ld16(from + GN, ext);
+                tmem_ld_wait();
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) mine[lane * LDW + c + e] = v[e];
-                }
+                for (int c = 0; c < 2; ++c)
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) mine[lane * LDW + c * 16 + e] = v[c][e];
+                if (RB == 1 && half == 1)
+#pragma unroll
+                    for (int e = 0; e <= RD; ++e) mine[lane * LDW + 32 + e] = ext[e];
                 __syncwarp();
+                auto sum_at = [&](int m, int c) {
+                    const uint32_t* r = mine + (4 * m) * LDW + c;
+                    return ((((long long)r[0] * 256 + r[LDW]) * 256 + r[2 * LDW]) * 256) + r[3 * LDW];
+                };
+                const int row0 = rb * 32 + q * 8;
+                if constexpr (RB == 1) {
+                    // a loop over the rows there are and not its copies: code that runs once waits for its instructions
+#pragma unroll 1
+                    for (int m = 0; m < min(8, rows - row0); ++m) {
+                        s_sum[(size_t)(row0 + m) * GN + half * 32 + lane] = sum_at(m, lane);
+                        if (half == 1 && lane <= RD) s_ext[(size_t)(row0 + m) * (RD + 1) + lane] = sum_at(m, 32 + lane);
+                    }
+                } else {
 #pragma unroll
-                for (int m = 0; m < 8; ++m) {
-                    const uint32_t* r = mine + (4 * m) * LDW + lane;
-                    const long long t = ((((long long)r[0] * 256 + r[LDW]) * 256 + r[2 * LDW]) * 256) + r[3 * LDW];
-                    s_sum[(size_t)(rb * 32 + q * 8 + m) * GN + half * 32 + lane] = t;
+                    for (int m = 0; m < 8; ++m) s_sum[(size_t)(row0 + m) * GN + half * 32 + lane] = sum_at(m, lane);
+                    if (half == 1) {
+                        __syncwarp();
+#pragma unroll
+                        for (int e = 0; e <= RD; ++e) mine[lane * LDW + e] = ext[e];
+                        __syncwarp();
+                        for (int i = lane; i < 8 * (RD + 1); i += 32) s_ext[(size_t)row0 * (RD + 1) + i] = sum_at(i / (RD + 1), i % (RD + 1));
+                    }
                 }
                 __syncwarp();
             }
@@ -520,23 +538,37 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
     else __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, RB * GN);
+        tmem_dealloc(tmem_base, TCOLS);
     }
     if (warp >= 2 && !failed) {
         const int t = threadIdx.x - 64, n = t & (GN - 1);              // 256 threads: 64 columns, every fourth row
         const int col = g * GN + n;
         const long long rs = (long long)rowsum_n << 31;
         for (int j = (t >> 6) + 4 * way; j < rows; j += 4 * p.ways) {
-            long long sum = 0;
-            double bias = 0.0;
+            long long sum = 0, ext[RD + 1] = {0, 0, 0, 0, 0};
             for (int w = 0; w < p.ways; ++w) {
                 sum += p.ways > 1 ? cl.map_shared_rank(s_sum, w)[(size_t)j * GN + n] : s_sum[(size_t)j * GN + n];
-                bias += p.ways > 1 ? cl.map_shared_rank(s_bias, w)[j] : s_bias[j];
+                const long long* se = (p.ways > 1 ? cl.map_shared_rank(s_ext, w) : s_ext) + (size_t)j * (RD + 1);
+#pragma unroll
+                for (int i = 0; i <= RD; ++i) ext[i] += se[i];
             }
+            double bhi = 0.0, blo = 0.0;
+            if (runit == INT_MIN)
+                for (int w = 0; w < p.ways; ++w) {
+                    const double2 b = p.ways > 1 ? cl.map_shared_rank(s_bias, w)[j] : s_bias[j];
+                    bhi += b.x;
+                    blo += b.y;
+                }
+            // sum_k q r: the offsets off the planes, then r's own 2^31 off its top byte
+            const long long sq = ext[RD] - ((long long)p.K << 31);
+            const double top = (double)(ext[0] - ((long long)rsum.x << 31) - 128 * sq);
+            const double rest = (double)(ext[1] - ((long long)rsum.y << 31)) * 65536.0 + (double)(ext[2] - ((long long)rsum.z << 31)) * 256.0 +
+                                (double)(ext[3] - ((long long)rsum.w << 31));
+            const double r_unit = runit == INT_MIN ? 0.0 : __longlong_as_double((long long)(1023 - runit) << 52);
             const int e = s_exp[j];
             // 2^-e as a double from its exponent field; the sum is exact up to here
             const double unit = e == INT_MIN ? (double)__int_as_float(0x7fc00000) : __longlong_as_double((long long)(1023 - e) << 52);
-            float f = __double2float_rn((double)(sum - rs) * unit + bias);
+            float f = __double2float_rn(((double)(sum - rs) + (top * 16777216.0 + rest) * r_unit) * unit + (bhi + blo));
             const size_t at = (size_t)(m0 + j) * p.ldy + p.y_col0 + col;
             auto put = [&](auto* y0, auto value) {
                 auto* dst = y0 + at;
@@ -614,6 +646,49 @@ __global__ void __launch_bounds__(256) gc_rowsum_kernel(const uint8_t* __restric
     if (lane == 0) rowsum[n] = (int)sum;
 }
 
+// r = b / s of a group (one block each) as 32-bit integers below its largest |r|: four rows of bytes, offset 2^31, top byte first, in
+// the order of the 128-byte swizzle (16-byte chunk c of row i at c ^ i).
+__global__ void __launch_bounds__(256) gc_ratio_kernel(const float* __restrict__ scales, const float* __restrict__ biases, uint8_t* __restrict__ rows,
+                                                       int* __restrict__ info, int K) {
+    __shared__ double s_max[8];
+    __shared__ int s_sum[RD];
+    const int g = blockIdx.x, lane = threadIdx.x & 31;
+    const float *s = scales + (size_t)g * K, *b = biases + (size_t)g * K;
+    auto ratio = [&](int k) { return b[k] == 0.0f ? 0.0 : (double)b[k] / (double)s[k]; };
+    double most = 0.0;
+    for (int k = threadIdx.x; k < K; k += 256) {
+        const double r = fabs(ratio(k));
+        most = r <= (double)R_MAX ? fmax(most, r) : 2.0 * R_MAX;   // (a NaN lands there as well)
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) most = fmax(most, __shfl_xor_sync(0xffffffffu, most, o));
+    if (lane == 0) s_max[threadIdx.x >> 5] = most;
+    if (threadIdx.x < RD) s_sum[threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) most = fmax(most, s_max[w]);
+    const bool fits = most <= (double)R_MAX;
+    const int unit = fits ? (most > 0x1p-30 ? 30 - ilogb(most) : 60) : INT_MIN;
+    int sum[RD] = {0, 0, 0, 0};
+    for (int k = threadIdx.x; k < K; k += 256) {
+        const long long q = fits ? llrint(ldexp(ratio(k), unit)) : 0;
+        const uint32_t v = (uint32_t)((q > 0x7fffffffll ? 0x7fffffffll : q < -0x80000000ll ? -0x80000000ll : q) + 0x80000000ll);
+#pragma unroll
+        for (int i = 0; i < RD; ++i) {
+            const uint32_t byte = v >> (24 - 8 * i) & 255u;
+            rows[((size_t)g * (K / SK) + k / SK) * (RD * SK) + i * SK + ((k % SK) ^ (i << 4))] = (uint8_t)byte;
+            sum[i] += (int)byte;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < RD; ++i) {
+        sum[i] = __reduce_add_sync(0xffffffffu, sum[i]);
+        if (lane == 0) atomicAdd(&s_sum[i], sum[i]);
+    }
+    __syncthreads();
+    if (threadIdx.x < 8) info[8 * g + threadIdx.x] = threadIdx.x < RD ? s_sum[threadIdx.x] : threadIdx.x == 4 ? unit : 0;
+}
+
 template <typename XT, int RB, int RPW>
 cudaError_t launch_gc(rusty_cuda_ctx* ctx, const CUtensorMap& map_w, const GcParams& p, dim3 grid, size_t smem) {
     auto kern = qlinear_gc_tc_kernel<XT, RB, RPW>;
@@ -629,14 +704,23 @@ bool gc_tc_supported(const rusty_cuda_ctx* ctx, uint32_t N, uint32_t K) {
     return ctx->tc_ws && encode_tiled_fn() && K % 4 == 0 && K <= 32768u && N % GN == 0 && N / GN <= 65535u;
 }
 uint32_t gc_padded(uint32_t K) { return (K + SK - 1) / SK * SK; }
-size_t gc_tables_bytes(uint32_t N, uint32_t K) { return (size_t)(N / GN) * (gc_padded(K) / SK) * 4 + (size_t)N * 4; }
-int launch_gc_tables(rusty_cuda_ctx* ctx, const uint8_t* w, const float* scales, void* tables, uint32_t N, uint32_t K) {
+// r's rows (they start on 512 bytes) | r's sums and units | largest scales | byte sums
+static size_t gc_r_bytes(uint32_t N, uint32_t Kp) { return (size_t)(N / GN) * RD * Kp; }
+size_t gc_tables_bytes(uint32_t N, uint32_t K) {
+    const uint32_t Kp = gc_padded(K);
+    return gc_r_bytes(N, Kp) + (size_t)(N / GN) * (8 + Kp / SK) * 4 + (size_t)N * 4;
+}
+int launch_gc_tables(rusty_cuda_ctx* ctx, const uint8_t* w, const float* scales, const float* biases, void* tables, uint32_t N, uint32_t K) {
     K = gc_padded(K);
     const size_t entries = (size_t)(N / GN) * (K / SK);
-    float* smax = (float*)tables;
+    int* info = (int*)((char*)tables + gc_r_bytes(N, K));
+    float* smax = (float*)(info + (size_t)(N / GN) * 8);
     const size_t blocks = (entries + 7) / 8, cap = (size_t)ctx->sm_count * 8;
+    gc_ratio_kernel<<<N / GN, 256, 0, ctx->stream>>>(scales, biases, (uint8_t*)tables, info, (int)K);
+    int rc = after_launch(ctx, "gc_ratio");
+    if (rc) return rc;
     gc_smax_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, ctx->stream>>>(scales, smax, entries);
-    int rc = after_launch(ctx, "gc_smax");
+    rc = after_launch(ctx, "gc_smax");
     if (rc) return rc;
     gc_rowsum_kernel<<<(N + 7) / 8, 256, 0, ctx->stream>>>(w, (int*)(smax + entries), (int)N, (int)K);
     return after_launch(ctx, "gc_rowsum");
@@ -646,9 +730,11 @@ int launch_gc_tc(rusty_cuda_ctx* ctx, const QLinearArgs& a) {
     GcParams p{};
     p.scales = a.scales;
     p.biases = a.biases;
-    p.smax = (const float*)a.gc_tables;
     p.N = (int)a.N;
     p.K = (int)gc_padded(a.K);   // the weight's rows, scales and biases are that long, zeros behind a.K
+    p.rbytes = (const uint8_t*)a.gc_tables;
+    p.rinfo = (const int*)((const char*)a.gc_tables + gc_r_bytes(a.N, (uint32_t)p.K));
+    p.smax = (const float*)(p.rinfo + (size_t)(p.N / GN) * 8);
     p.rowsum = (const int*)(p.smax + (size_t)(p.N / GN) * (p.K / SK));
     p.nst = p.K / SK;
     p.ldy = (int)a.ldy;
@@ -695,13 +781,13 @@ int launch_gc_tc(rusty_cuda_ctx* ctx, const QLinearArgs& a) {
         // suffice, and the start and the end of a CTA cost as much as ten stages.
         p.ways = 1;
         while (tiles == 1 && p.ways < 4 && groups * p.ways * 2 <= 2 * ctx->sm_count && p.nst / (p.ways * 2) >= 4) p.ways *= 2;
-        const size_t fixed = 1024 + (size_t)rb * A_BYTES + (4 * MAX_STAGES + 1) * 8 + (size_t)rb * 32 * 16 + (size_t)p.nst * 4 + 64;
+        const size_t fixed = 1024 + (size_t)rb * A_BYTES + (4 * MAX_STAGES + 2) * 8 + (size_t)rb * 32 * 24 + (size_t)p.nst * 4 + 64;
         const size_t budget = (ctx->smem_optin + 1024) / 2 - 1024;   // half an SM, less the 1 KiB every block pays
-        int stages = budget > fixed ? (int)((budget - fixed) / STAGE_BYTES) : 0;
+        int stages = budget > fixed ? (int)((budget - fixed) / (STAGE_BYTES + S_BYTES)) : 0;
         if (stages > MAX_STAGES) stages = MAX_STAGES;
         if (stages < (rb == 1 ? MAX_STAGES : 4)) return fail(ctx, RUSTY_CUDA_ERR_UNSUPPORTED, "gc_tc: the ring does not fit shared memory");
         p.stages = stages;
-        const size_t smem = fixed + (size_t)stages * STAGE_BYTES;
+        const size_t smem = fixed + (size_t)stages * (STAGE_BYTES + S_BYTES);
         const dim3 grid((unsigned)(tiles * p.ways), (unsigned)groups);
         cudaError_t e = rpw == 8   ? launch_gc<float, 2, 8>(ctx, map_w, p, grid, smem)
                         : rpw == 4 ? launch_gc<float, 1, 4>(ctx, map_w, p, grid, smem)

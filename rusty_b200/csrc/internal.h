@@ -201,7 +201,7 @@ constexpr int QMODE_AFFINE_GC = 64;
 bool gc_tc_supported(const rusty_cuda_ctx* ctx, uint32_t N, uint32_t K);
 uint32_t gc_padded(uint32_t K);   // length of the re-laid-out rows
 size_t gc_tables_bytes(uint32_t N, uint32_t K);
-int launch_gc_tables(rusty_cuda_ctx* ctx, const uint8_t* w, const float* scales, void* tables, uint32_t N, uint32_t K);
+int launch_gc_tables(rusty_cuda_ctx* ctx, const uint8_t* w, const float* scales, const float* biases, void* tables, uint32_t N, uint32_t K);
 int launch_gc_tc(rusty_cuda_ctx* ctx, const struct QLinearArgs& a);
 size_t tc_workspace_xq_bytes();
 int launch_residual_add(rusty_cuda_ctx* ctx, const void* a, const void* b, void* out, size_t n, int y_dtype);

@@ -244,7 +244,7 @@ int rusty_cuda_qlinear_create(rusty_cuda_ctx* ctx, rusty_cuda_buf* weight, rusty
             rc = launch_transpose_u8(ctx, (const uint8_t*)weight->ptr, (uint8_t*)own->ptr, K, N, Kp);
             if (!rc) rc = launch_transpose_f32(ctx, (const float*)scales->ptr, (float*)q->scales->ptr, K, N / 64, Kp);
             if (!rc) rc = launch_transpose_f32(ctx, (const float*)biases->ptr, (float*)q->biases->ptr, K, N / 64, Kp);
-            if (!rc) rc = launch_gc_tables(ctx, (const uint8_t*)own->ptr, (const float*)q->scales->ptr, (void*)q->gc_tables, N, K);
+            if (!rc) rc = launch_gc_tables(ctx, (const uint8_t*)own->ptr, (const float*)q->scales->ptr, (const float*)q->biases->ptr, (void*)q->gc_tables, N, K);
             if (!rc) rc = check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "qlinear_create: re-layout");
         }
         if (rc) {

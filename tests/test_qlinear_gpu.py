@@ -548,6 +548,52 @@ def test_native_affine_outliers_on_small_scales(ctx, engine, M, K, N, outliers):
     assert_bits_equal(got[M - 1:], _forward(ctx, engine, QLinear.from_host(ctx, ukn, sg, bg, layout=capi.LAYOUT_KN), x[M - 1:]))
 
 
+@pytest.mark.parametrize("M,K,N", [(1, 4096, 512), (4, 11008, 256), (8, 640, 192), (9, 4096, 256), (13, 1152, 128), (32, 4100, 192), (64, 4096, 192), (150, 2112, 128)])
+@pytest.mark.parametrize("act", ["f32", "bf16"])
+def test_native_affine_sums_are_rounded_twice_only(ctx, engine, M, K, N, act):
+    """Of an output, x * scale is rounded once per term and the sum once: a relative error uniform within 2^-24 each at the
+    most, 2^-24 / sqrt(3) in the mean square, together 4.9e-8 of the outputs in the 2-norm.  The bias term, as large as the
+    other and cancelling it, adds nothing.  (bf16 activations from 65 rows on take the bf16 kernel.)"""
+    if act == "bf16" and M > 64:
+        pytest.skip("the bf16 kernel's")
+    rng = np.random.default_rng(M + K)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    dt = DType.FP32
+    if act == "bf16":
+        dt, x = DType.BF16, bf16_bits_to_f32(f32_to_bf16_bits(x)).reshape(M, K)
+    sg = rng.uniform(0.001, 0.02, size=(K, N // 64)).astype(np.float32)
+    bg = (-128.0 * sg * rng.uniform(0.8, 1.2, size=sg.shape)).astype(np.float32)
+    ukn = rng.integers(0, 256, size=(K, N), dtype=np.uint8)
+    got = _forward(ctx, engine, QLinear.from_host(ctx, ukn, sg, bg, layout=capi.LAYOUT_KN), x, x_dtype=dt, y_dtype=DType.FP32)
+    exact = x.astype(np.float64) @ (ukn * np.repeat(sg.astype(np.float64), 64, axis=1) + np.repeat(bg.astype(np.float64), 64, axis=1))
+    assert np.linalg.norm(got - exact) / np.linalg.norm(exact) <= 2.0 ** 0.5 * 2.0 ** -24 / 3.0 ** 0.5
+
+
+@pytest.mark.parametrize("M,K", [(1, 4096), (4, 1152), (8, 640), (9, 4096), (32, 4100), (64, 2048), (70, 2112)])
+def test_native_affine_groups_with_large_biases(ctx, engine, M, K):
+    """Groups side by side whose biases are of the scales' size, 4096 scales and a little more (either side of what goes to the
+    tensor core), and without any scale to measure them by (constant groups: scale zero).  The last are plain sums of x * bias,
+    half a unit in the last place from the exact ones."""
+    rng = np.random.default_rng(M + K)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    ratio = np.array([128.0, 4095.5, 4097.0, 1e6, 0.0, 128.0])
+    N = 64 * len(ratio)
+    sg = rng.uniform(0.001, 0.02, size=(K, len(ratio))).astype(np.float32)
+    bg = (-ratio * sg * rng.uniform(0.5, 1.0, size=sg.shape)).astype(np.float32)
+    bg[K // 2] = (-ratio * sg[K // 2]).astype(np.float32)
+    sg[:, 4] = 0.0
+    bg[:, 4] = rng.standard_normal(K).astype(np.float32)
+    sg[K // 3, 5], bg[K // 3, 5] = 0.0, 1.0          # one constant group in the midst of others
+    ukn = rng.integers(0, 256, size=(K, N), dtype=np.uint8)
+    got = _forward(ctx, engine, QLinear.from_host(ctx, ukn, sg, bg, layout=capi.LAYOUT_KN), x)
+    wf = ukn * np.repeat(sg.astype(np.float64), 64, axis=1) + np.repeat(bg.astype(np.float64), 64, axis=1)
+    exact = x.astype(np.float64) @ wf
+    for i in range(len(ratio)):
+        assert rel_err_rows(got[:, 64 * i:64 * i + 64], exact[:, 64 * i:64 * i + 64]) <= 1e-6, i
+    plain = np.repeat(x.astype(np.longdouble) @ bg[:, 4:5].astype(np.longdouble), 64, axis=1)
+    assert np.all(np.abs(got[:, 256:320] - plain) <= np.abs(plain) * 2.0 ** -24 * (1 + 1e-6))
+
+
 @pytest.mark.parametrize("M,K,N", [(65, 256, 128), (130, 400, 257), (391, 1024, 4100), (1030, 128, 300), (600, 28672, 128)])
 def test_f32_prompts_in_row_blocks(ctx, engine, M, K, N):
     """More than 64 f32 rows run as several row blocks of one launch pair: every row as if its block were alone, with the
