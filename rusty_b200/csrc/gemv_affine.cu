@@ -5,7 +5,9 @@
 // Arithmetic.  Scales change every 64 k along the contraction, so the integer sums are taken per 64 k: the activations of such a
 // chunk become four balanced signed bytes below a power-of-two scale of THEIR row and chunk (30 bits below the chunk's
 // largest), two mma.sync.m16n8k32 (u8 x s8) give the exact dot products of 16 weight rows with the four digit planes of two
-// activation rows, and the chunk's share of an output is dot * s + sum(x) * b in f32: two roundings per 64 products.  A lane
+// activation rows, and the chunk's share of an output is dot * s + sum(x) * b in f32, rounded before it joins the sum: for weights
+// around zero both terms are larger than their sum, and are never gathered apart.  sum(x) is exact, its upper part with the
+// upper planes, the rest with the lower ones; ranges, and runs of RUN chunks, are added up in double.  A lane
 // holds two neighbouring planes of a sum (columns 4m + 2h, 4m + 2h + 1): they fit one int32, the other two planes are the
 // neighbour lane's, and the two halves meet after the last chunk.
 //
@@ -24,6 +26,7 @@
 #include <cooperative_groups.h>
 
 #include <climits>
+#include <type_traits>
 
 #include "tc_common.cuh"
 
@@ -36,13 +39,14 @@ constexpr int AG = 64;             // k per scale
 constexpr int AF_WARPS = 8;
 constexpr int AF_THREADS = 32 * AF_WARPS;
 constexpr int AF_ROWS = 32;        // weight rows of a warp: two MMA tiles
+constexpr int RUN = 16;            // chunks of an f32 sum (a power of two)
 
 struct AfParams {
     const uint8_t* W;
     const float* scales;     // [N][K/64]
     const float* biases;
     const uint4* digits;     // [K/64][tiles][32 lanes] x 16 bytes
-    const float2* aux;       // [K/64][tiles][4]: (unit of the two planes, sum of x or 0)
+    const float2* aux;       // [K/64][tiles][4]: (unit of the two planes, upper or lower part of the sum of x)
     void* y;
     int M, N, K;
     int tiles, tpp;          // pairs of activation rows: all, and per pass (blockIdx.y)
@@ -96,15 +100,15 @@ __global__ void __launch_bounds__(256) affine_prepare_kernel(const XT* __restric
     uint32_t top = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) top = max(top, __float_as_uint(v[i]) & 0x7fffffffu);
-    float sum = (v[0] + v[1]) + (v[2] + v[3]);
+    double sum = ((double)v[0] + (double)v[1]) + ((double)v[2] + (double)v[3]);
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) {
         top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
         sum += __shfl_xor_sync(0xffffffffu, sum, o);
     }
     if (k >= K) return;
-    // |x| < 2^e, e >= -90 so that the units below stay normal numbers
-    const int e = max((int)(top >> 23) - 126, -90);
+    // |x| < 2^e, e >= -119 so that the units below are numbers, denormal ones below 2^-126
+    const int e = max((int)(top >> 23) - 126, -119);
     const float up = __uint_as_float((uint32_t)(133 - e) << 23);      // 2^(6 - e)
     uint32_t q[4];
 #pragma unroll
@@ -118,14 +122,19 @@ __global__ void __launch_bounds__(256) affine_prepare_kernel(const XT* __restric
     for (int i = 0; i < 4; ++i) digits[(at * 32 + ((m & 1) * 4 + i) * 4 + kk / 16) * 4 + (kk % 16) / 4] = plane[i];
     if (kk == 0) {
         const bool finite = top < 0x7f800000u;
-        const float unit = finite ? __uint_as_float((uint32_t)(97 + e) << 23) : __uint_as_float(0x7fc00000u);   // 2^(e - 30)
-        *reinterpret_cast<float4*>(aux + at * 4 + (m & 1) * 2) = make_float4(unit, sum, unit * 65536.0f, 0.0f);
+        const float unit = finite ? __uint_as_float(e > -97 ? (uint32_t)(97 + e) << 23 : 1u << (119 + e)) : __uint_as_float(0x7fc00000u);   // 2^(e - 30)
+        const float upper = (float)sum;   // (may be infinite where the largest x is not far from it: no rest then)
+        *reinterpret_cast<float4*>(aux + at * 4 + (m & 1) * 2) =
+            make_float4(unit, fabsf(upper) < 3.0e38f ? (float)(sum - (double)upper) : 0.0f, unit * 65536.0f, upper);
     }
 }
 
-template <int NT>
+// LONG: ranges of more than RUN chunks, whose f32 sums move on to doubles every RUN chunks: a longer chain rounds at the size of
+// what it has gathered.  (In one kernel for both, 16 rows x 4096 x 4096, four chunks a range, took 15.7 us instead of 14.3.)
+template <int NT, bool LONG>
 __global__ void __launch_bounds__(AF_THREADS, NT <= 8 ? 2 : 1) gemv_affine_kernel(const AfParams p) {
-    __shared__ float red[AF_WARPS * 2 * NT * AF_ROWS];   // [warp][activation row][weight row]
+    using Sum = std::conditional_t<LONG, double, float>;
+    __shared__ Sum red[AF_WARPS * 2 * NT * AF_ROWS];      // [warp][activation row][weight row]
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
     const int rank = blockIdx.x % p.ways, block = blockIdx.x / p.ways, wks = AF_WARPS / p.wr;
@@ -151,10 +160,14 @@ __global__ void __launch_bounds__(AF_THREADS, NT <= 8 ? 2 : 1) gemv_affine_kerne
         }
     };
     float acc[NT][4];
+    Sum* mine = red + (warp * 2 * NT + (tig >> 1)) * AF_ROWS + gid;   // (the even lane of a pair holds the pair's sums)
 #pragma unroll
     for (int t = 0; t < NT; ++t)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[t][i] = 0.0f;
+        for (int i = 0; i < 4; ++i) {
+            acc[t][i] = 0.0f;
+            if (LONG && (tig & 1) == 0) mine[2 * t * AF_ROWS + 8 * i] = 0.0;
+        }
     // digits of the next PF tiles, across the chunks: from L2 they take as long as several tiles' arithmetic
     constexpr int PF = NT < 2 ? 1 : NT <= 8 ? 2 : 4;
     static_assert(NT % PF == 0, "a tile's digits lie in the same registers in every chunk");
@@ -180,10 +193,10 @@ __global__ void __launch_bounds__(AF_THREADS, NT <= 8 ? 2 : 1) gemv_affine_kerne
                 mma_u8s8(lo, c.w[0].z, c.w[1].z, c.w[0].w, c.w[1].w, d.z, d.w);
                 mma_u8s8(hi, c.w[2].z, c.w[3].z, c.w[2].w, c.w[3].w, d.z, d.w);
                 // |sum| <= 64 * 255 * 128 per plane: both planes together stay below 2^30
-                acc[t][0] = fmaf((float)(lo[1] * 256 + lo[0]) * a.x, c.s[0], fmaf(a.y, c.b[0], acc[t][0]));
-                acc[t][1] = fmaf((float)(lo[3] * 256 + lo[2]) * a.x, c.s[1], fmaf(a.y, c.b[1], acc[t][1]));
-                acc[t][2] = fmaf((float)(hi[1] * 256 + hi[0]) * a.x, c.s[2], fmaf(a.y, c.b[2], acc[t][2]));
-                acc[t][3] = fmaf((float)(hi[3] * 256 + hi[2]) * a.x, c.s[3], fmaf(a.y, c.b[3], acc[t][3]));
+                acc[t][0] += fmaf((float)(lo[1] * 256 + lo[0]) * a.x, c.s[0], a.y * c.b[0]);
+                acc[t][1] += fmaf((float)(lo[3] * 256 + lo[2]) * a.x, c.s[1], a.y * c.b[1]);
+                acc[t][2] += fmaf((float)(hi[1] * 256 + hi[0]) * a.x, c.s[2], a.y * c.b[2]);
+                acc[t][3] += fmaf((float)(hi[3] * 256 + hi[2]) * a.x, c.s[3], a.y * c.b[3]);
             }
         }
     };
@@ -193,19 +206,24 @@ __global__ void __launch_bounds__(AF_THREADS, NT <= 8 ? 2 : 1) gemv_affine_kerne
     pdl_wait();
 #pragma unroll
     for (int t = 0; t < PF; ++t) fetch(g0, t, t);
+    auto move_on = [&] {
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float v = acc[t][i] + __shfl_xor_sync(0xffffffffu, acc[t][i], 1);
+                acc[t][i] = 0.0f;
+                if ((tig & 1) == 0) mine[2 * t * AF_ROWS + 8 * i] = (LONG ? mine[2 * t * AF_ROWS + 8 * i] : (Sum)0) + (Sum)v;
+            }
+    };
     for (int g = g0; g < g1; g += 2) {
         add(g, c0);
         load(g + 2, c0);
         if (g + 1 < g1) add(g + 1, c1);
         load(g + 3, c1);
+        if (LONG && ((g - g0) & (RUN - 1)) == RUN - 2) move_on();
     }
-#pragma unroll
-    for (int t = 0; t < NT; ++t)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float v = acc[t][i] + __shfl_xor_sync(0xffffffffu, acc[t][i], 1);
-            if ((tig & 1) == 0) red[(warp * 2 * NT + 2 * t + (tig >> 1)) * AF_ROWS + gid + 8 * i] = v;
-        }
+    move_on();
     cg::cluster_group cl = cg::this_cluster();
     if (p.ways > 1)
         cl.sync();
@@ -215,11 +233,12 @@ __global__ void __launch_bounds__(AF_THREADS, NT <= 8 ? 2 : 1) gemv_affine_kerne
     for (int i = rank * AF_THREADS + threadIdx.x; i < rows * 2 * nt; i += p.ways * AF_THREADS) {
         const int r = i % rows, m = i / rows, n = block * rows + r, mg = 2 * tile0 + m;
         if (n >= p.N || mg >= p.M) continue;
-        float v = 0.0f;
+        double sum = 0.0;   // of up to 64 ranges
         for (int c = 0; c < p.ways; ++c) {
-            const float* src = p.ways > 1 ? cl.map_shared_rank(red, c) : red;
-            for (int k = 0; k < wks; ++k) v += src[((k * p.wr + r / AF_ROWS) * 2 * NT + m) * AF_ROWS + r % AF_ROWS];
+            const Sum* src = p.ways > 1 ? cl.map_shared_rank(red, c) : red;
+            for (int k = 0; k < wks; ++k) sum += (double)src[((k * p.wr + r / AF_ROWS) * 2 * NT + m) * AF_ROWS + r % AF_ROWS];
         }
+        const float v = (float)sum;
         const size_t at = (size_t)mg * p.ldy + p.y_col0 + n;
         if (p.y_bf16)
             reinterpret_cast<__nv_bfloat16*>(p.y)[at] = __float2bfloat16_rn(v);
@@ -284,7 +303,16 @@ int launch_gemv_affine(rusty_cuda_ctx* ctx, const QLinearArgs& a) {
         p.wr = AF_WARPS / wks;
         p.ways = slices / wks;
         const dim3 grid((unsigned)((row_groups + p.wr - 1) / p.wr * p.ways), (unsigned)passes);
-        auto kern = p.tpp <= 1 ? gemv_affine_kernel<1> : p.tpp <= 2 ? gemv_affine_kernel<2> : p.tpp <= 4 ? gemv_affine_kernel<4> : p.tpp <= 8 ? gemv_affine_kernel<8> : gemv_affine_kernel<12>;
+        const bool run_on = (groups + slices - 1) / slices > RUN;
+        auto of = [&](auto nt) {
+            constexpr int NT = decltype(nt)::value;
+            return run_on ? gemv_affine_kernel<NT, true> : gemv_affine_kernel<NT, false>;
+        };
+        auto kern = p.tpp <= 1   ? of(std::integral_constant<int, 1>{})
+                    : p.tpp <= 2 ? of(std::integral_constant<int, 2>{})
+                    : p.tpp <= 4 ? of(std::integral_constant<int, 4>{})
+                    : p.tpp <= 8 ? of(std::integral_constant<int, 8>{})
+                                 : of(std::integral_constant<int, 12>{});
         e = launch_pdl_cluster(kern, grid, dim3(AF_THREADS), (unsigned)p.ways, 0, ctx->stream, p);
         if (e != cudaSuccess) return check_cuda(ctx, e, "gemv_affine");
         rc = after_launch(ctx, "gemv_affine");

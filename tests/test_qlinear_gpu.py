@@ -667,3 +667,28 @@ def test_affine_batches_in_out_in_storage(ctx, engine, M, K, N, act):
     x[0, K - 1] = np.nan
     got = _forward(ctx, engine, ql, x, x_dtype=dt, y_dtype=DType.FP32)
     assert np.isnan(got[0]).all() and np.isfinite(got[1:]).all()
+
+
+@pytest.mark.parametrize("M,K,N,act", [(1, 4096, 512, "f32"), (2, 28672, 8192, "f32"), (5, 2112, 300, "bf16"), (7, 28672, 8192, "bf16"), (13, 14336, 640, "f32"),
+                                       (24, 4096, 512, "bf16"), (32, 2112, 12288, "f32"), (64, 14336, 640, "bf16"), (64, 4096, 16384, "f32"), (130, 4096, 512, "f32")])
+def test_affine_out_in_sums(ctx, engine, M, K, N, act):
+    """Short and long ranges of chunks.  Around zero a chunk's share of an output has a mean square of 64 (x s 74)^2, rounded at
+    the size of its two terms, 64 (x s 148)^2 and 64 (x s 128)^2, and its own; a chain of up to 16 shares once per share at the
+    size of what it has gathered, half of 16 shares in the mean; the output once.  With 2^-24 / sqrt(3), the most a rounding has
+    in the mean square, that is 2^-24 (4 + 3 + 1 + 8 + 1)^(1/2) / 3^(1/2) of the outputs in the 2-norm."""
+    rng = np.random.default_rng(M + K + N)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    dt = DType.FP32
+    if act == "bf16":
+        dt, x = DType.BF16, bf16_bits_to_f32(f32_to_bf16_bits(x)).reshape(M, K)
+    u = rng.integers(0, 256, size=(N, K), dtype=np.uint8)
+    sg = rng.uniform(0.001, 0.02, size=(N, K // 64)).astype(np.float32)
+    bg = (-128.0 * sg * rng.uniform(0.9, 1.1, size=sg.shape)).astype(np.float32)
+    got = _forward(ctx, engine, QLinear.from_host(ctx, u, sg.reshape(-1), bg.reshape(-1)), x, x_dtype=dt, y_dtype=DType.FP32)
+    cols = _sampled_weight_rows(N, rng)
+    wf = u[cols] * np.repeat(sg[cols].astype(np.float64), 64, axis=1) + np.repeat(bg[cols].astype(np.float64), 64, axis=1)
+    exact = x.astype(np.float64) @ wf.T
+    assert np.linalg.norm(got[:, cols] - exact) / np.linalg.norm(exact) <= 2.0 ** -24 * (17.0 / 3.0) ** 0.5
+    x[M - 1] *= np.float32(2.0 ** -100)          # the scaled rows of a chunk keep their bits however small they are
+    tiny = _forward(ctx, engine, QLinear.from_host(ctx, u, sg.reshape(-1), bg.reshape(-1)), x, x_dtype=dt, y_dtype=DType.FP32)[M - 1]
+    assert np.linalg.norm(tiny[cols] - exact[M - 1] * 2.0 ** -100) / np.linalg.norm(exact[M - 1] * 2.0 ** -100) <= 2.0 ** -24 * (17.0 / 3.0) ** 0.5 * 1.25   # (one row's sample)
