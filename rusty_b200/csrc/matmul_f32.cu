@@ -265,11 +265,11 @@ int launch_matmul(rusty_cuda_ctx* ctx, const float* a, const float* b, float* ou
 constexpr int LD_THREADS = 256;
 template <int MT>
 __global__ void __launch_bounds__(LD_THREADS) lora_down_kernel(const float* __restrict__ x, const float* __restrict__ A, float* __restrict__ t,
-                                                               uint32_t M, uint32_t K, uint32_t r, uint32_t r4) {
+                                                               uint32_t M, uint32_t K, uint32_t r, uint32_t r4, uint32_t col0) {
     __shared__ float red[LD_THREADS / 32][MT * 4];
     pdl_wait();
     pdl_launch_dependents();   // after the wait: the matmul that follows may read x and W at once
-    const uint32_t m0 = blockIdx.x * MT, c0 = blockIdx.y * 4;
+    const uint32_t m0 = blockIdx.x * MT, c0 = col0 + blockIdx.y * 4;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     float acc[MT][4];
 #pragma unroll
@@ -343,15 +343,12 @@ int launch_lora_down(rusty_cuda_ctx* ctx, const float* x, const float* A, float*
     // columns that the blocks fill the chip twice over, the chain of the matmul is shorter than the re-reading
     const uint32_t cols = r4 / 4;
     const uint64_t want = 2ull * (unsigned)(ctx->sm_count > 0 ? ctx->sm_count : 1);
-    cudaError_t e;
-    if ((uint64_t)M * cols <= want)
-        e = launch_pdl(lora_down_kernel<1>, dim3(M, cols), dim3(LD_THREADS), 0, ctx->stream, x, A, t, M, K, r, r4);
-    else if ((uint64_t)(M / 4) * cols <= want)
-        e = launch_pdl(lora_down_kernel<4>, dim3((M + 3) / 4, cols), dim3(LD_THREADS), 0, ctx->stream, x, A, t, M, K, r, r4);
-    else if (r == r4 && (uint64_t)(M / 8) * cols > want / 2)
-        return launch_matmul<false>(ctx, x, A, t, M, K, r, LoraTail{});
-    else
-        e = launch_pdl(lora_down_kernel<8>, dim3((M + 7) / 8, cols), dim3(LD_THREADS), 0, ctx->stream, x, A, t, M, K, r, r4);
+    const uint32_t mt = (uint64_t)M * cols <= want ? 1 : (uint64_t)(M / 4) * cols <= want ? 4 : 8;
+    if (mt == 8 && r == r4 && (uint64_t)(M / 8) * cols > want / 2) return launch_matmul<false>(ctx, x, A, t, M, K, r, LoraTail{});
+    auto kern = mt == 1 ? lora_down_kernel<1> : mt == 4 ? lora_down_kernel<4> : lora_down_kernel<8>;
+    cudaError_t e = cudaSuccess;
+    for (uint32_t c = 0; c < cols && e == cudaSuccess; c += 65535u)
+        e = launch_pdl(kern, dim3((M + mt - 1) / mt, cols - c < 65535u ? cols - c : 65535u), dim3(LD_THREADS), 0, ctx->stream, x, A, t, M, K, r, r4, c * 4u);
     if (e != cudaSuccess) return check_cuda(ctx, e, "lora_down");
     return after_launch(ctx, "lora_down");
 }
@@ -364,6 +361,10 @@ int need(rusty_cuda_ctx* ctx, const char* op, const char* name, const rusty_cuda
     return RUSTY_CUDA_OK;
 }
 
+// A launch holds 65535 row tiles, of 4 rows in the worst case; a call as many as of 64 rows.
+constexpr uint32_t PASS_ROWS = 65535u * 4u;
+bool too_many_rows(uint32_t M) { return M > 65535u * 64u; }
+
 template <bool NK>
 int matmul_entry(rusty_cuda_ctx* ctx, const char* op, const rusty_cuda_buf* a, const rusty_cuda_buf* b, rusty_cuda_buf* out, uint32_t M,
                  uint32_t K, uint32_t N) {
@@ -372,11 +373,10 @@ int matmul_entry(rusty_cuda_ctx* ctx, const char* op, const rusty_cuda_buf* a, c
     if ((rc = need(ctx, op, "b", b, (size_t)K * N * 4))) return rc;
     if ((rc = need(ctx, op, "out", out, (size_t)M * N * 4))) return rc;
     if (M == 0 || N == 0) return RUSTY_CUDA_OK;
-    if ((M + 63) / 64 > 65535) return fail(ctx, RUSTY_CUDA_ERR_INVALID_DIMENSIONS, "%s: M=%u too large", op, M);
+    if (too_many_rows(M)) return fail(ctx, RUSTY_CUDA_ERR_INVALID_DIMENSIONS, "%s: M=%u too large", op, M);
     DeviceGuard g(ctx->device);
-    constexpr uint32_t PASS = 65535u * 4u;   // a launch holds 65535 row tiles, of 4 rows in the worst case
-    for (uint32_t m0 = 0; m0 < M; m0 += PASS) {
-        const uint32_t rows = M - m0 < PASS ? M - m0 : PASS;
+    for (uint32_t m0 = 0; m0 < M; m0 += PASS_ROWS) {
+        const uint32_t rows = M - m0 < PASS_ROWS ? M - m0 : PASS_ROWS;
         if ((rc = launch_matmul<NK>(ctx, (const float*)a->ptr + (size_t)m0 * K, (const float*)b->ptr, (float*)out->ptr + (size_t)m0 * N, rows, K, N,
                                     LoraTail{})))
             return rc;
@@ -417,29 +417,30 @@ int rusty_cuda_linear_lora_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf* x, con
     if ((rc = need(ctx, op, "lora_b", lora_b, (size_t)rank * N * 4))) return rc;
     if ((rc = need(ctx, op, "y", y, (size_t)M * N * 4))) return rc;
     if (M == 0 || N == 0) return RUSTY_CUDA_OK;
-    if (M > 65535u * 4u || rank > 65535u * 4u) return fail(ctx, RUSTY_CUDA_ERR_INVALID_DIMENSIONS, "%s: M=%u or rank=%u too large", op, M, rank);
+    if (too_many_rows(M)) return fail(ctx, RUSTY_CUDA_ERR_INVALID_DIMENSIONS, "%s: M=%u too large", op, M);
     if (rank == 0)
         return weight ? rusty_cuda_matmul_f32(ctx, x, weight, y, M, K, N) : rusty_cuda_qlinear_forward(ctx, ql, x, RUSTY_CUDA_F32, M, y, RUSTY_CUDA_F32);
     // t = x . A lives in a pool buffer: later calls on this stream may take it over as soon as its reader is enqueued
-    const uint32_t r4 = (rank + 3u) & ~3u;
+    const uint32_t r4 = (rank + 3u) & ~3u, t_rows = M < PASS_ROWS ? M : PASS_ROWS;
     rusty_cuda_buf* t = nullptr;
-    if ((rc = rusty_cuda_buf_alloc(ctx, (size_t)M * r4 * 4, 1, &t))) return rc;
+    if ((rc = rusty_cuda_buf_alloc(ctx, (size_t)t_rows * r4 * 4, 1, &t))) return rc;
     DeviceGuard g(ctx->device);
-    const float* xp = (const float*)x->ptr;
-    if (weight) {
-        rc = launch_lora_down(ctx, xp, (const float*)lora_a->ptr, (float*)t->ptr, M, K, rank, r4);
-        if (!rc)
-            rc = launch_matmul<false>(ctx, xp, (const float*)weight->ptr, (float*)y->ptr, M, K, N,
+    if (ql) rc = qlinear_forward_cols(ctx, ql, x, RUSTY_CUDA_F32, M, y, RUSTY_CUDA_F32, N, 0);
+    for (uint32_t m0 = 0; m0 < M && !rc; m0 += PASS_ROWS) {
+        const uint32_t m = M - m0 < PASS_ROWS ? M - m0 : PASS_ROWS;
+        const float* xp = (const float*)x->ptr + (size_t)m0 * K;
+        float* yp = (float*)y->ptr + (size_t)m0 * N;
+        rc = launch_lora_down(ctx, xp, (const float*)lora_a->ptr, (float*)t->ptr, m, K, rank, r4);
+        if (rc) break;
+        if (weight) {
+            rc = launch_matmul<false>(ctx, xp, (const float*)weight->ptr, yp, m, K, N,
                                       LoraTail{(const float*)t->ptr, (const float*)lora_b->ptr, (int)rank, (int)r4});
-    } else {
-        rc = qlinear_forward_cols(ctx, ql, x, RUSTY_CUDA_F32, M, y, RUSTY_CUDA_F32, N, 0);
-        if (!rc) rc = launch_lora_down(ctx, xp, (const float*)lora_a->ptr, (float*)t->ptr, M, K, rank, r4);
-        if (!rc) {
+        } else {
             const unsigned gx = (N + LU_THREADS - 1) / LU_THREADS;
-            unsigned rows = (unsigned)(((uint64_t)M * gx + 4ull * ctx->sm_count - 1) / (4ull * ctx->sm_count));   // four blocks an SM
-            if (rows < (M + 65534u) / 65535u) rows = (M + 65534u) / 65535u;
-            cudaError_t e = launch_pdl(lora_up_add_kernel, dim3(gx, (M + rows - 1) / rows), dim3(LU_THREADS), 0, ctx->stream, (const float*)t->ptr,
-                                       (const float*)lora_b->ptr, (float*)y->ptr, M, N, (int)rank, r4, rows);
+            unsigned rows = (unsigned)(((uint64_t)m * gx + 4ull * ctx->sm_count - 1) / (4ull * ctx->sm_count));   // four blocks an SM
+            if (rows < (m + 65534u) / 65535u) rows = (m + 65534u) / 65535u;
+            cudaError_t e = launch_pdl(lora_up_add_kernel, dim3(gx, (m + rows - 1) / rows), dim3(LU_THREADS), 0, ctx->stream, (const float*)t->ptr,
+                                       (const float*)lora_b->ptr, yp, m, N, (int)rank, r4, rows);
             rc = e != cudaSuccess ? check_cuda(ctx, e, "lora_up_add") : after_launch(ctx, "lora_up_add");
         }
     }

@@ -245,3 +245,22 @@ def test_linear_lora_call(ctx, engine, oracle, M, K, N, rank):
         out = GuardedOutput(ctx, [M, N], DType.FP32)
         engine.linear_lora(ctx, tx, QLinear.from_host(ctx, q, s), ta, tb, out.tensor)
         assert rel_err(out.read(), x.astype(np.float64) @ (q * s[:, None].astype(np.float64)).T + branch) <= TOL_FP32
+
+
+@pytest.mark.parametrize("M,rank", [(262141, 4), (262150, 8), (3, 262141), (2, 262150)])
+def test_linear_lora_of_many_rows_or_columns(ctx, engine, M, rank):
+    """More rows than a launch holds row tiles of four, and a rank of more columns than a launch holds blocks of four: what the
+    products one by one took.  Small whole numbers, so that every sum is exact."""
+    K, N = 16, 64
+    rng = np.random.default_rng(M + rank)
+    x, w = rng.integers(-4, 5, size=(M, K)).astype(np.float32), rng.integers(-4, 5, size=(K, N)).astype(np.float32)
+    a, b = rng.integers(-2, 3, size=(K, rank)).astype(np.float32), rng.integers(-1, 2, size=(rank, N)).astype(np.float32)
+    tx, ta, tb = (UnifiedTensor.new(ctx, v, list(v.shape)) for v in (x, a, b))
+    low = (x @ a) @ b
+    out = GuardedOutput(ctx, [M, N])
+    engine.linear_lora(ctx, tx, UnifiedTensor.new(ctx, w, [K, N]), ta, tb, out.tensor)
+    assert_bits_equal(out.read(), x @ w + low)
+    q = rng.integers(-4, 5, size=(N, K), dtype=np.int8)
+    out = GuardedOutput(ctx, [M, N])
+    engine.linear_lora(ctx, tx, QLinear.from_host(ctx, q, np.ones(N, np.float32)), ta, tb, out.tensor)
+    assert_bits_equal(out.read(), x @ q.T.astype(np.float32) + low)
