@@ -577,7 +577,8 @@ def main():
         line["with_rms_norms"] = {"value": M / (rn["ms_step"] * 1e-3), "unit": "tokens/s", "ms_per_step": rn["ms_step"],
                                   "gpu_launches": rn["launches"],
                                   "note": "RMSNorm applied by the pre-pass of q|k|v, gate|up (with residual add) and lm_head; "
-                                          "no norm kernel is launched"}
+                                          "no norm kernel is launched" if M > 2 else
+                                          "RMSNorm a kernel of its own in front of q|k|v, gate|up (with residual add) and lm_head"}
 
     # The 70B stack's Linears are four times larger, so output-feature sharding pays there first: the same measurement
     # on llama2-70b-decode64 rides along as an extra key (never the headline).

@@ -142,6 +142,12 @@ class LinearStack:
                     self.norm_w[i] = UnifiedTensor.new(ctx, rng.uniform(0.5, 1.5, size=shape.d).astype(np.float32), [shape.d])
                     if name.endswith(".gate_up"):
                         self.norm_res[i] = res
+        # Where the norm does not ride in the Linear's pre-pass it is a kernel of its own and needs a buffer; a capture cannot
+        # allocate one.  (The pre-pass takes rows of up to 8192 at any batch.)
+        unfused = [w is not None and not (k <= 8192 and q.plan(M, x_dtype, y_dtype) == "tcgen05")
+                   for q, (_, k), w in zip(self.qls, self.dims, self.norm_w)]
+        normed = UnifiedTensor.empty(ctx, [M, shape.d]) if any(unfused) else None
+        self.normed: List[Optional[UnifiedTensor]] = [normed if u else None for u in unfused]
 
     # ---- accounting (algorithmic bytes / flops of ONE step on this rank) ----
     def weight_bytes(self) -> int:
@@ -169,11 +175,12 @@ class LinearStack:
             qlinear_forward_batch(self.ctx, self.qls, self._xs, self._ys, self.M, self.x_dtype, self.y_dtype)
             return
         eng = ComputeEngine(self.ctx)
-        for ql, x, y, w, r in zip(self.qls, self._xs, self._ys, self.norm_w, self.norm_res):
+        for ql, x, y, w, r, n in zip(self.qls, self._xs, self._ys, self.norm_w, self.norm_res, self.normed):
             if w is None:
                 eng.qlinear(self.ctx, x, ql, y)
             else:
-                eng.qlinear_normed(self.ctx, x, w, ql, y, residual=r, sum_out=self.norm_sum if r is not None else None)
+                eng.qlinear_normed(self.ctx, x, w, ql, y, residual=r, normed_out=n,
+                                   sum_out=self.norm_sum if r is not None else None)
 
     def capture(self) -> Graph:
         g = Graph(self.ctx)

@@ -31,3 +31,22 @@ def test_small_stack_outputs_match_the_reference_arithmetic(ctx, oracle, M, nati
         ref = oracle.matmul_bt(x, st.host_wf[i], mt=True)
         got = np.frombuffer(st._ys[i].to_bytes(ctx), np.float32).reshape(M, st.out_n[i])
         assert rel_err(got, ref) <= TOL_FP32, st.names[i]
+
+
+@pytest.mark.parametrize("native", [False, True])
+@pytest.mark.parametrize("M", [1, 2, 3])
+def test_stack_with_norms_under_capture(ctx, oracle, M, native):
+    """The step with the blocks' norms, recorded and replayed: at few rows, and in the native format, the norm is a kernel of its
+    own whose output needs a buffer, and nothing can be allocated while a capture is open."""
+    from rusty_b200 import DType
+    from rusty_b200.stack import LinearStack
+    from rusty_b200.workloads import StackShape
+    # (a width no other test uses: the pool must not happen to hold such a buffer)
+    st = LinearStack(ctx, StackShape("tiny", d=320, q=256, kv=64, ffn=640, vocab=1024, layers=2), M, DType.FP32, DType.FP32, seed=4, swiglu=True,
+                     norms=True, native=native, keep_host=True)
+    graph = st.capture()
+    graph.launch()
+    ctx.sync()
+    x, w = st.host_inputs[320], st.norm_w[-1].to_vec(ctx)
+    got = np.frombuffer(st.logits.to_bytes(ctx), np.float32).reshape(M, 1024)
+    assert rel_err(got, oracle.matmul_bt(oracle.rms_norm(x, w), st.host_wf[-1], mt=True)) <= TOL_FP32
