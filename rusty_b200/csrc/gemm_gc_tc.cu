@@ -15,7 +15,7 @@
 // int32 per plane (255 * 255 * K < 2^31 for K <= 32768) and int64 together, and 2^31 * sum_k u[n,k], a property of the weight
 // row, is taken off once at the end.  The largest |a| has to be the true one: max|x| max|s| over a stretch of k is far above it
 // where an outlier of x meets a small scale, and every factor of two of that is a bit of all other activations (an outlier of
-// 10^6 on a scale of 10^-6 cost 1e-3 of the result).  Up to eight rows every CTA multiplies x and s_g once more for it.  Larger
+// 10^6 on a scale of 10^-6 cost 1e-3 of the result).  Up to eight rows the CTAs multiply x and s_g once more for it.  Larger
 // batches know the largest |x| of a stage (128 k), its place and the second largest: the product at that place is one of the
 // row's, and second largest times the stage's largest |s| bounds the others; all products of a stage are taken only where
 // that bound has a larger exponent than the largest product so far (hardly ever for weights and activations of one scale).
@@ -94,6 +94,9 @@ struct GcParams {
     long long peer_delta[PEER_MAX_RANKS];
 };
 
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 // Magnitudes are compared as bits: a NaN or an infinity is above every number.
 __device__ __forceinline__ uint32_t abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
 __device__ __forceinline__ uint32_t abs_max(const float4& v) { return max(max(abs_bits(v.x), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w))); }
@@ -123,8 +126,10 @@ __device__ __forceinline__ int unit_exponent(uint32_t bits) {
     return min(157 - (int)(bits >> 23), 127);
 }
 
-// XT: type of the caller's x (RPW = 1 reads it as it is).  RB: row blocks of 32 (1 or 2); RPW: rows per converter warp (1, 2, 4 or 8; RB = 2 has 8)
-template <typename XT, int RB, int RPW>
+// XT: type of the caller's x (RPW = 1 reads it as it is).  RB: row blocks of 32 (1 or 2); RPW: rows per converter warp (1, 2, 4 or 8;
+// RB = 2 has 8).  MEET (RPW = 1): the cluster's CTAs share the look for the largest products (an instance of its own: the code of
+// both in one cost calls that do not meet 0.3 us in instruction fetches).
+template <typename XT, int RB, int RPW, bool MEET = false>
 __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ GcParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -153,19 +158,20 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
     const int st0 = nb * way / p.ways * BSUM, st1 = min(p.nst, nb * (way + 1) / p.ways * BSUM);
     const int active = min(CW, rows);          // converter warps that arrive on a stage
     pdl_launch_dependents();
-    // The scales are needed before the first weights are: asked for ahead of the ring's 70 KB, up to eight rows the first ones
-    // into registers.
+    // The scales are needed before the first weights are: asked for ahead of the ring's 70 KB.  Up to eight rows the first
+    // ones into registers, and where the cluster meets a CTA looks for the largest products of its own K range only.
     constexpr int AHEAD = 4;          // stages whose scales a converter warp holds while the rows go by (RPW = 1)
+    const int top0 = MEET ? st0 : 0, top1 = MEET ? st1 : p.nst;
     const float* gs = p.scales + (size_t)g * p.K + lane * 4;
     float4 sv[AHEAD];
     auto fetch_scales = [&](int st) {
 #pragma unroll
         for (int u = 0; u < AHEAD; ++u)
-            if (st + u * CW < p.nst) sv[u] = ldg_x4(gs + (st + u * CW) * SK);
+            if (st + u * CW < top1) sv[u] = ldg_x4(gs + (st + u * CW) * SK);
     };
     if (warp >= 2) {
-        if constexpr (RPW == 1) fetch_scales(warp - 2);
-        for (int k = (RPW == 1 ? AHEAD * CW * SK : 0) + ((int)threadIdx.x - 64) * 32; k < p.K; k += 32 * CW * 32)
+        if constexpr (RPW == 1) fetch_scales(top0 + warp - 2);
+        for (int k = (top0 + (RPW == 1 ? AHEAD * CW : 0)) * SK + ((int)threadIdx.x - 64) * 32; k < top1 * SK; k += 32 * CW * 32)
             asm volatile("prefetch.global.L2 [%0];" ::"l"(p.scales + (size_t)g * p.K + k));
     }
     if (threadIdx.x == 0) {
@@ -200,6 +206,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
     const int runit = warp >= 2 ? __ldg(p.rinfo + 8 * g + 4) : 0;
     const int rowsum_n = warp >= 2 ? __ldg(p.rowsum + g * GN + ((threadIdx.x - 64) & (GN - 1))) : 0;
 
+    if (MEET && warp < 2) cluster_arrive();   // for the converters' meeting; waited for at the end
     if (warp == 0) {
         // ------------------------------ producer ------------------------------
         // several row tiles read the weights again (from L2); one tile: a single pass
@@ -263,24 +270,29 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
         const int sub = shared_rows ? cw >> 2 : 0;
         const int nr = row_w < rows ? (rows - row_w + 7) / 8 : 0;       // rows of this warp
         if constexpr (RPW == 1) {
-            // every warp takes an eighth of K of every row
+            // every warp takes an eighth of the range of every row
             const XT* xr = reinterpret_cast<const XT*>(p.x) + (size_t)m0 * p.K + lane * 4;
-            for (int kb = cw; kb < p.nst; kb += AHEAD * CW) {
-                if (kb != cw) fetch_scales(kb);
+            for (int kb = top0 + cw; kb < top1; kb += AHEAD * CW) {
+                if (kb != top0 + cw) fetch_scales(kb);
                 for (int m = 0; m < rows; ++m) {
                     float4 v[AHEAD];
 #pragma unroll
                     for (int u = 0; u < AHEAD; ++u)
-                        if (kb + u * CW < p.nst) v[u] = ldg_x4<XT>(xr + (size_t)m * p.K + (kb + u * CW) * SK);
+                        if (kb + u * CW < top1) v[u] = ldg_x4<XT>(xr + (size_t)m * p.K + (kb + u * CW) * SK);
                     uint32_t top = 0u;
 #pragma unroll
                     for (int u = 0; u < AHEAD; ++u)
-                        if (kb + u * CW < p.nst) top = max(top, abs_max(v[u], sv[u]));
+                        if (kb + u * CW < top1) top = max(top, abs_max(v[u], sv[u]));
                     top = __reduce_max_sync(0xffffffffu, top);
                     if (lane == 0) atomicMax(s_top + m, top);
                 }
             }
-            asm volatile("bar.sync 1, %0;" ::"n"(32 * CW) : "memory");
+            if constexpr (MEET) {
+                cluster_arrive();
+                cluster_wait();
+            } else {
+                asm volatile("bar.sync 1, %0;" ::"n"(32 * CW) : "memory");
+            }
         } else {
             // (the unit depends on the exponent alone, and that is the true one here as well: a row has the same in any batch)
             const uint2* xt = p.xtop + (size_t)(m0 + row_w) * p.nst;
@@ -334,7 +346,9 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
         for (int i = 0; i < RPW; ++i) {
             scale[i] = 0.0f;
             if (i < nr) {
-                const uint32_t top = s_top[row_w + 8 * i];
+                uint32_t top = s_top[row_w + 8 * i];
+                if constexpr (MEET)
+                    for (int w = 1; w < p.ways; ++w) top = max(top, cg::this_cluster().map_shared_rank(s_top, (way + w) % p.ways)[row_w]);
                 const bool finite = top < 0x7f800000u;
                 const int e = unit_exponent(top);
                 // 2^e: between 2^-97 (products near the largest float) and 2^127, always a normal number
@@ -534,6 +548,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
         tc_fence_before();
     }
     cg::cluster_group cl = cg::this_cluster();
+    if (MEET && warp < 2) cluster_wait();
     if (p.ways > 1) cl.sync();
     else __syncthreads();
     if (warp == 1) {
@@ -689,9 +704,9 @@ __global__ void __launch_bounds__(256) gc_ratio_kernel(const float* __restrict__
     if (threadIdx.x < 8) info[8 * g + threadIdx.x] = threadIdx.x < RD ? s_sum[threadIdx.x] : threadIdx.x == 4 ? unit : 0;
 }
 
-template <typename XT, int RB, int RPW>
+template <typename XT, int RB, int RPW, bool MEET = false>
 cudaError_t launch_gc(rusty_cuda_ctx* ctx, const CUtensorMap& map_w, const GcParams& p, dim3 grid, size_t smem) {
-    auto kern = qlinear_gc_tc_kernel<XT, RB, RPW>;
+    auto kern = qlinear_gc_tc_kernel<XT, RB, RPW, MEET>;
     cudaError_t e = rusty::ensure_dynamic_smem((const void*)kern, ctx->device, smem);
     if (e != cudaSuccess) return e;
     return launch_pdl_cluster(kern, grid, dim3(GC_THREADS), (unsigned)p.ways, smem, ctx->stream, map_w, p);
@@ -781,6 +796,10 @@ int launch_gc_tc(rusty_cuda_ctx* ctx, const QLinearArgs& a) {
         // suffice, and the start and the end of a CTA cost as much as ten stages.
         p.ways = 1;
         while (tiles == 1 && p.ways < 4 && groups * p.ways * 2 <= 2 * ctx->sm_count && p.nst / (p.ways * 2) >= 4) p.ways *= 2;
+        // Meeting costs 2 us (one row x 4096 x 4096: 8.1 -> 10.0 us, four 10.5 -> 11.6), walking x and the scales beyond what the
+        // registers hold more than that with rows x stages (14336 x 3008 at one / two / eight rows: 16.4 / 18.4 / 30.6 us alone,
+        // 15.6 / 16.2 / 20.7 together; 11008 x 4096 at one / four: 15.1 / 20.3 and 15.5 / 17.6).
+        const bool meet = rpw == 1 && p.ways > 1 && p.nst > 32 && p.M * p.nst >= 100;
         const size_t fixed = 1024 + (size_t)rb * A_BYTES + (4 * MAX_STAGES + 2) * 8 + (size_t)rb * 32 * 24 + (size_t)p.nst * 4 + 64;
         const size_t budget = (ctx->smem_optin + 1024) / 2 - 1024;   // half an SM, less the 1 KiB every block pays
         int stages = budget > fixed ? (int)((budget - fixed) / (STAGE_BYTES + S_BYTES)) : 0;
@@ -792,7 +811,8 @@ int launch_gc_tc(rusty_cuda_ctx* ctx, const QLinearArgs& a) {
         cudaError_t e = rpw == 8   ? launch_gc<float, 2, 8>(ctx, map_w, p, grid, smem)
                         : rpw == 4 ? launch_gc<float, 1, 4>(ctx, map_w, p, grid, smem)
                         : rpw == 2 ? launch_gc<float, 1, 2>(ctx, map_w, p, grid, smem)
-                        : xb       ? launch_gc<__nv_bfloat16, 1, 1>(ctx, map_w, p, grid, smem)
+                        : xb       ? (meet ? launch_gc<__nv_bfloat16, 1, 1, true>(ctx, map_w, p, grid, smem) : launch_gc<__nv_bfloat16, 1, 1>(ctx, map_w, p, grid, smem))
+                        : meet     ? launch_gc<float, 1, 1, true>(ctx, map_w, p, grid, smem)
                                    : launch_gc<float, 1, 1>(ctx, map_w, p, grid, smem);
         if (e != cudaSuccess) return check_cuda(ctx, e, "qlinear_gc_tc");
         int rc = after_launch(ctx, "qlinear_gc_tc");
