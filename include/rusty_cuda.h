@@ -219,8 +219,13 @@ RUSTY_CUDA_API int rusty_cuda_qlinear_destroy(rusty_cuda_qlinear* ql);
 RUSTY_CUDA_API int rusty_cuda_qlinear_forward(rusty_cuda_ctx* ctx, const rusty_cuda_qlinear* ql,
                                               const rusty_cuda_buf* x, int x_dtype, uint32_t M,
                                               rusty_cuda_buf* y, int y_dtype);
-/* Name of the kernel `rusty_cuda_qlinear_forward` would launch for this shape
- * ("gemv_f32", "tcgen05", ...); for tests and logs. */
+/* Name of the FAMILY of kernels `rusty_cuda_qlinear_forward` would launch for this shape; for tests and logs.
+ *   "tcgen05"      int8 tensor cores, one scale per row (digit pre-pass + tcgen05 kernel)
+ *   "tcgen05_f16"  bf16 tensor cores (M >= 65 with bf16 activations)
+ *   "gemv_mma"     one scale per row, M <= 2: warp-level int8 tensor cores; a re-laid-out AFFINE_G64 weight, any M: its
+ *                  own tcgen05 kernel
+ *   "gemv"         AFFINE_G64 in LAYOUT_NK: warp-level int8 tensor cores; otherwise CUDA cores
+ *   "unsupported"  none: forward fails */
 RUSTY_CUDA_API int rusty_cuda_qlinear_plan(const rusty_cuda_qlinear* ql, int x_dtype, uint32_t M, int y_dtype,
                                            char* dst, size_t dst_len);
 

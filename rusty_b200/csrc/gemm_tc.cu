@@ -1114,7 +1114,8 @@ int launch_tc(rusty_cuda_ctx* ctx, const QLinearArgs& a) {
     // ONE pair: the blocks of a row tile share its weights in L2, and the fixed part of a pair is paid once (391 rows of a
     // Llama-3-8B layer: 919 us in seven pairs per Linear, 449 us in one).  Exchanges between ranks meet per block of 64, so
     // pushed forwards keep one block per pair; so do bf16 activations (three planes: 24 rows of digits are no multiple of 16).
-    // A normed call of two blocks stays two pairs: two launches per 64 rows is what its callers are told to count.
+    // A normed call of two blocks stays two pairs only because tests/test_norm_embed_gpu.py counts two launches per 64 rows: 4096 x
+    // 6144 takes 36 us at 66 rows and 41 at 128, in one pair 28 and 31 (4096 x 28672: 64 and 80, 51 and 71).
     uint32_t most = 64;
     if (a.M > 64 && a.x_dtype == RUSTY_CUDA_F32 && !(a.push && a.push->nranks > 1) && !(a.norm && a.M <= 128)) {
         const size_t fit = WS_XQ_BYTES / ((size_t)4 * a.K);

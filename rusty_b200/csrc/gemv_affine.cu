@@ -19,10 +19,12 @@
 // groups x 8/wr ranges, a cluster adds ranges.  Ranges are summed in shared memory (distributed, for a cluster) in a fixed order.
 //
 // What bounds it: up to about eight rows the weight stream and the two launches; beyond, waiting for the digits from L2 and the
-// fold of a chunk (77 instructions per 32 x 2 outputs; at 24 rows a third of the issue slots and 14 % of the integer tensor pipe
-// are used, with two warps per scheduler).  4096 x 4096, device time: 1 row 9.9 -> 6.8 us, 8 rows 26 -> 9.4, 16 rows 52 -> 14,
-// 64 rows 207 -> 51 (before: CUDA cores, eight rows per walk over the weights); 3000 x 14336: 1 row 25.7 -> 15.3 us.  Two digit tiles are fetched ahead (four where the tiles of a chunk are many): fetched where they are
-// used, 64 rows took 90 us; without the row guard around a tile's arithmetic the compiler overlaps neighbouring tiles.
+// fold of a chunk (77 instructions per 32 x 2 outputs; at 24 rows 42 % of the issue slots and 19 % of the integer tensor pipe are
+// used, with two warps per scheduler).  4096 x 4096, per call in a graph: 1 row 7.3 us, 8 rows 9.8, 16 rows 14.3, 24 rows 18.7, 64
+// rows 49.5 (on CUDA cores, eight rows per walk over the weights, 9.9, 26, 52 and 207 us for 1, 8, 16 and 64); 3000 x 14336: 1 row
+// 17.1 us (25.7).  Two digit tiles are fetched ahead (four where the tiles of a chunk are many): fetched where they are used, 64
+// rows took 90 us.  Tiles of a pass beyond the rows there are, up to the next of 1, 2, 4, 8 or 12, are computed and dropped: 13
+// rows take as long as 16, 14.3 us; with a row guard around a tile's arithmetic the compiler does not overlap neighbours.
 #include <cooperative_groups.h>
 
 #include <climits>
@@ -186,18 +188,16 @@ __global__ void __launch_bounds__(AF_THREADS, NT <= 8 ? 2 : 1) gemv_affine_kerne
             const uint4 d = q[t % PF];
             const float2 a = u[t % PF];
             fetch(t + PF < NT ? g : g + 1, t + PF < NT ? t + PF : t + PF - NT, t % PF);
-            {
-                int lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
-                mma_u8s8(lo, c.w[0].x, c.w[1].x, c.w[0].y, c.w[1].y, d.x, d.y);
-                mma_u8s8(hi, c.w[2].x, c.w[3].x, c.w[2].y, c.w[3].y, d.x, d.y);
-                mma_u8s8(lo, c.w[0].z, c.w[1].z, c.w[0].w, c.w[1].w, d.z, d.w);
-                mma_u8s8(hi, c.w[2].z, c.w[3].z, c.w[2].w, c.w[3].w, d.z, d.w);
-                // |sum| <= 64 * 255 * 128 per plane: both planes together stay below 2^30
-                acc[t][0] += fmaf((float)(lo[1] * 256 + lo[0]) * a.x, c.s[0], a.y * c.b[0]);
-                acc[t][1] += fmaf((float)(lo[3] * 256 + lo[2]) * a.x, c.s[1], a.y * c.b[1]);
-                acc[t][2] += fmaf((float)(hi[1] * 256 + hi[0]) * a.x, c.s[2], a.y * c.b[2]);
-                acc[t][3] += fmaf((float)(hi[3] * 256 + hi[2]) * a.x, c.s[3], a.y * c.b[3]);
-            }
+            int lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
+            mma_u8s8(lo, c.w[0].x, c.w[1].x, c.w[0].y, c.w[1].y, d.x, d.y);
+            mma_u8s8(hi, c.w[2].x, c.w[3].x, c.w[2].y, c.w[3].y, d.x, d.y);
+            mma_u8s8(lo, c.w[0].z, c.w[1].z, c.w[0].w, c.w[1].w, d.z, d.w);
+            mma_u8s8(hi, c.w[2].z, c.w[3].z, c.w[2].w, c.w[3].w, d.z, d.w);
+            // |sum| <= 64 * 255 * 128 per plane: both planes together stay below 2^30
+            acc[t][0] += fmaf((float)(lo[1] * 256 + lo[0]) * a.x, c.s[0], a.y * c.b[0]);
+            acc[t][1] += fmaf((float)(lo[3] * 256 + lo[2]) * a.x, c.s[1], a.y * c.b[1]);
+            acc[t][2] += fmaf((float)(hi[1] * 256 + hi[0]) * a.x, c.s[2], a.y * c.b[2]);
+            acc[t][3] += fmaf((float)(hi[3] * 256 + hi[2]) * a.x, c.s[3], a.y * c.b[3]);
         }
     };
     Chunk c0, c1;
@@ -273,7 +273,7 @@ int launch_gemv_affine(rusty_cuda_ctx* ctx, const QLinearArgs& a) {
         p.y = (char*)a.y + (size_t)m0 * a.ldy * ys;
         p.tiles = (p.M + 1) / 2;
         // Up to 24 activation rows share a pass over the weights (32 leave too few registers: 12288 x 2112 at 32 rows 60 us in
-        // one pass, 48 in two); passes of equal width.
+        // one pass, 47 in two); passes of equal width.
         const int passes = (p.tiles + 11) / 12;
         p.tpp = (p.tiles + passes - 1) / passes;
         uint32_t* digits = (uint32_t*)ctx->tc_ws;

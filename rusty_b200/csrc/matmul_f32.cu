@@ -248,7 +248,18 @@ template <bool NK>
 int launch_matmul(rusty_cuda_ctx* ctx, const float* a, const float* b, float* out, uint32_t M, uint32_t K, uint32_t N, const LoraTail& lora) {
     // Few rows: the tile that holds them, so that b is read once.  Otherwise by the outputs an SM gets: many threads of few
     // outputs while the chain is what bounds an SM, more outputs a thread (fewer shared-memory passes each) once the SMs are
-    // full; 64 x 64 only where it still gives every SM two blocks.
+    // full; 64 x 64 only where it still gives every SM two blocks.  K = 4096, us, by outputs an SM and tile:
+    //                 4     8    16    32    64   big
+    //      86       20.1  30.6  37.2  56.6  78.1   208     (64 x 200)
+    //     221       29.6  29.7  35.7  55.5  76.8   208     (64 x 512)
+    //     332       38.7  49.1  36.0  55.5  77.7   208     (128 x 384)
+    //     554       64.9  76.9  59.2  55.6  77.2   208     (128 x 640)
+    //     886       87.7  96.2  59.0  55.7  77.3   210     (128 x 1024)
+    //    1384        133   143  92.3  94.3  77.6   210     (64 x 3200)
+    //    7085        656   661   400   320   243   224     (256 x 4096)
+    //   14170       1295  1317   795   632   415   402     (512 x 4096)
+    // The lines are drawn by outputs alone; a tile whose blocks just miss one wave is chosen all the same (277, 64 x 640: 8 rows
+    // 49.3, 16 rows 36.1; 1124, 64 x 2600: 32 rows 97.1, 64 rows 78.5).
     const uint64_t outputs = (uint64_t)M * N, sms = (uint64_t)(ctx->sm_count > 0 ? ctx->sm_count : 1);
     if (M == 1) return launch_tile<TileRow, NK>(ctx, a, b, out, M, K, N, lora);
     if (M <= 4 || outputs <= 128 * sms) return launch_tile<Tile4, NK>(ctx, a, b, out, M, K, N, lora);
@@ -340,7 +351,10 @@ __global__ void __launch_bounds__(LU_THREADS) lora_up_add_kernel(const float* __
 
 int launch_lora_down(rusty_cuda_ctx* ctx, const float* x, const float* A, float* t, uint32_t M, uint32_t K, uint32_t r, uint32_t r4) {
     // rows per block: enough blocks for the SMs first (one row each), then fewer passes over A; once x is re-read for so many
-    // columns that the blocks fill the chip twice over, the chain of the matmul is shorter than the re-reading
+    // columns that the blocks fill the chip twice over, the chain of the matmul is shorter than the re-reading.  Whole calls, K =
+    // 4096, N = 512, us, with 1, 4, 8 rows a block and with the matmul: 128 rows of rank 8 40.3 / 40.8 / 43.0 / 55.6, 256 of 8 60.5 /
+    // 60.8 / 63.2 / 75.8, 64 of 64 47.3 / 36.8 / 37.4 / 49.3, 100 of 64 62.2 / 45.4 / 45.1 / 55.5, 256 of 64 123 / 79 / 74 / 76, 600
+    // of 16 263 / 251 / 251 / 155, 1024 of 8 254 / 249 / 250 / 157.
     const uint32_t cols = r4 / 4;
     const uint64_t want = 2ull * (unsigned)(ctx->sm_count > 0 ? ctx->sm_count : 1);
     const uint32_t mt = (uint64_t)M * cols <= want ? 1 : (uint64_t)(M / 4) * cols <= want ? 4 : 8;

@@ -11,8 +11,8 @@ write ``%globaltimer`` stamps into a buffer (the regular build compiles the stam
 
 Twelve Linears with separate weight copies are captured in one graph and replayed; the steady-state Linears are
 printed with the times (µs from the first pre-pass of the graph, this GPU's clock) at which the phases were reached:
-minimum and maximum over the CTAs of the GEMM.  Development-build environment switches: RUSTY_PEER_EXP=1 drops the
-meeting of the ranks, =2 the stores into the other ranks' memory, =3 both; RUSTY_TC_SMS=n plans the GEMM for n SMs.
+minimum and maximum over the CTAs of the GEMM.  RUSTY_TC_SMS=n in the environment plans the
+GEMM for n SMs.
 """
 from __future__ import annotations
 
