@@ -166,8 +166,10 @@ __global__ void __launch_bounds__(GM_THREADS, 2) gemv_mma_kernel(const __grid_co
             const uint64_t pol = policy_evict_first();
             // What the ring will not hold at first: into L2 now, so that it is a short trip later.  Long streams
             // are left alone (the ring runs far ahead of the consumers there anyway).
+            // (not the stage that ends in a tail: map_w has no part of it, and may be a 2-D map where there is no other stage)
             if (total <= 3 * p.stages)
-                for (int i = p.stages + 2; i < total; ++i) tma_prefetch_3d(&map_w, 0, row0 + group_start(i / p.nch), (i % p.nch) * (KC / 128));
+                for (int i = p.stages + 2; i < total; ++i)
+                    if (!p.tail || i % p.nch < p.nch - 1) tma_prefetch_3d(&map_w, 0, row0 + group_start(i / p.nch), (i % p.nch) * (KC / 128));
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;

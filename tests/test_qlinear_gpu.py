@@ -69,6 +69,16 @@ def test_gemv_shapes_sym(ctx, engine, oracle, M, K, N):
     assert rel_err(got, ref) <= TOL_FP32
 
 
+@pytest.mark.parametrize("M", [1, 2])
+@pytest.mark.parametrize("K,N", [(576, 32000), (960, 24000), (400, 40000), (1040, 20000), (2064, 9472)])
+def test_gemv_tail_over_many_rows(ctx, engine, oracle, M, K, N):
+    """K with a tail and so many rows that a CTA asks for stages ahead of its ring: the tail's stage is not part of the 3-D map,
+    and with a single stage along K there is no such map."""
+    x, q, s = sym_row_linear(K + N + M, M, K, N)
+    got = _forward(ctx, engine, QLinear.from_host(ctx, q, s), x)
+    assert rel_err(got, oracle.matmul_bt(x, oracle.dequantize_rowscale(q, s), mt=True)) <= TOL_FP32
+
+
 @pytest.mark.parametrize("M,K,N", [(1, 4096, 1024), (3, 11008, 256), (4, 192, 19)])
 def test_gemv_shapes_affine(ctx, engine, oracle, M, K, N):
     x, q, _ = sym_row_linear(K + N + M, M, K, N)
