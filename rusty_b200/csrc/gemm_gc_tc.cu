@@ -105,12 +105,15 @@ __device__ __forceinline__ uint32_t abs_max(const float4& x, const float4& s) { 
     return abs_max(make_float4(__fmul_rn(x.x, s.x), __fmul_rn(x.y, s.y), __fmul_rn(x.z, s.z), __fmul_rn(x.w, s.w)));
 }
 
+__device__ __forceinline__ float4 ldg_x4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }   // of the weight's own tables
+// Activations: not through the read-only path, which wants data nobody writes while the kernel runs; this kernel is there while the
+// ones in front of it still write x, its copy and xtop (at the same addresses on every call).
 template <typename XT>
-__device__ __forceinline__ float4 ldg_x4(const XT* p) {
+__device__ __forceinline__ float4 ld_x4(const XT* p) {
     if constexpr (sizeof(XT) == 4) {
-        return __ldg(reinterpret_cast<const float4*>(p));
+        return *reinterpret_cast<const float4*>(p);
     } else {
-        const uint2 raw = __ldg(reinterpret_cast<const uint2*>(p));
+        const uint2 raw = *reinterpret_cast<const uint2*>(p);
         return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
                            __uint_as_float(raw.y & 0xffff0000u));
     }
@@ -279,7 +282,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
                     float4 v[AHEAD];
 #pragma unroll
                     for (int u = 0; u < AHEAD; ++u)
-                        if (kb + u * CW < top1) v[u] = ldg_x4<XT>(xr + (size_t)m * p.K + (kb + u * CW) * SK);
+                        if (kb + u * CW < top1) v[u] = ld_x4<XT>(xr + (size_t)m * p.K + (kb + u * CW) * SK);
                     uint32_t top = 0u;
 #pragma unroll
                     for (int u = 0; u < AHEAD; ++u)
@@ -307,7 +310,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
                 float s1[RPW];
 #pragma unroll
                 for (int i = 0; i < RPW; ++i)
-                    if (i < nr) v[i] = __ldg(xt + (size_t)(8 * i) * p.nst + st);
+                    if (i < nr) v[i] = xt[(size_t)(8 * i) * p.nst + st];
 #pragma unroll
                 for (int i = 0; i < RPW; ++i)
                     if (i < nr) s1[i] = __ldg(p.scales + (size_t)g * p.K + st * SK + (v[i].y & 0xffffu));
@@ -325,9 +328,9 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
                     if (__any_sync(0xffffffffu, rest[i] >> 23 > top[i] >> 23)) {
                         for (int base = 0; base < p.nst; base += 32) {
                             const int st = base + lane;
-                            const uint32_t b = st < p.nst ? rest_bound(__ldg(xt + (size_t)(8 * i) * p.nst + st), st) >> 23 : 0u;
+                            const uint32_t b = st < p.nst ? rest_bound(xt[(size_t)(8 * i) * p.nst + st], st) >> 23 : 0u;
                             uint32_t todo = __ballot_sync(0xffffffffu, b > top[i] >> 23);
-                            auto stage_max = [&](int s) { return abs_max(ldg_x4(xr + (size_t)s * p.xstep + i * (8 * SK)), ldg_x4(gs + s * SK)); };
+                            auto stage_max = [&](int s) { return abs_max(ld_x4(xr + (size_t)s * p.xstep + i * (8 * SK)), ldg_x4(gs + s * SK)); };
                             while (todo) {     // two stages at a time
                                 const int sa = base + __ffs(todo) - 1;
                                 todo &= todo - 1;
@@ -379,7 +382,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
                 for (int h = 0; h < GS; ++h)
                     if (st + h < st1)
 #pragma unroll
-                        for (int i = 0; i < GR; ++i) v[i * GS + h] = ldg_x4<XT>(q + h * p.xstep + (half * GR + i) * (8 * SK));
+                        for (int i = 0; i < GR; ++i) v[i * GS + h] = ld_x4<XT>(q + h * p.xstep + (half * GR + i) * (8 * SK));
             };
             uint4 sq;
             int slot = 0, ab = 0;
@@ -469,7 +472,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
                 for (int i = 0; i < nr; ++i) {
                     double hi = 0.0, lo = 0.0;
                     for (int st = st0; st < st1; ++st) {
-                        const float4 x4 = ldg_x4<XT>(xb + (size_t)st * p.xstep + i * (RPW == 1 ? 8 * p.K : 8 * SK)), b4 = ldg_x4(gb + st * SK);
+                        const float4 x4 = ld_x4<XT>(xb + (size_t)st * p.xstep + i * (RPW == 1 ? 8 * p.K : 8 * SK)), b4 = ldg_x4(gb + st * SK);
                         const double d = fma((double)x4.x, (double)b4.x, fma((double)x4.y, (double)b4.y, fma((double)x4.z, (double)b4.z, (double)x4.w * (double)b4.w)));
                         const double u = __hiloint2double(__double2hiint(d), __double2loint(d) & (int)0xe0000000);
                         hi += u;
@@ -610,7 +613,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
 // converters read it, [K/128][Mp][128]: a warp's rows of a stage then lie at constant offsets, and rows M .. Mp and k beyond K
 // (zeros) need no checks.  A block takes 1024 k of a row.  K % 4 == 0.
 template <typename XT>
-__global__ void __launch_bounds__(256) gc_prepare_kernel(const XT* __restrict__ x, float* __restrict__ xs, uint2* __restrict__ xtop, int M, int Mp,
+__global__ void __launch_bounds__(256) gc_prepare_kernel(const XT* x, float* xs, uint2* xtop, int M, int Mp,
                                                          int K) {
     pdl_launch_dependents();
     pdl_wait();
@@ -619,7 +622,7 @@ __global__ void __launch_bounds__(256) gc_prepare_kernel(const XT* __restrict__ 
     const int Kp = (K + SK - 1) / SK * SK;
     const int k = (blockIdx.y * 256 + threadIdx.x) * 4;
     if (k < Kp) {                                        // (a warp is inside or outside)
-        const float4 v = m < M && k < K ? ldg_x4<XT>(row + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 v = m < M && k < K ? ld_x4<XT>(row + k) : make_float4(0.f, 0.f, 0.f, 0.f);
         *reinterpret_cast<float4*>(xs + ((size_t)(k / SK) * Mp + m) * SK + (k & (SK - 1))) = v;
         const uint32_t c[4] = {abs_bits(v.x), abs_bits(v.y), abs_bits(v.z), abs_bits(v.w)};
         uint32_t best = c[0], next = 0u, at = 0u;

@@ -104,7 +104,7 @@ constexpr int DIG_MAXV = 8;   // passes of a row held in registers between the m
 // reference); the row is normalised in registers between the load and the maximum, so it must fit there
 // (K <= DIG_MAXV * 4 * threads of the row), and the normalised row and the sum are written out where asked for.
 template <typename XT, int D, bool NORM>
-__global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* __restrict__ x, int8_t* __restrict__ xq,
+__global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* x, int8_t* __restrict__ xq,
                                                                     float* __restrict__ inv_s, int M, int Mpad, int K, int R,
                                                                     const PeerPush push, const NormArgs nrm, long long* dbg) {
     __shared__ float red[DIG_THREADS / 32];

@@ -83,7 +83,7 @@ __device__ __forceinline__ int xs_index(int m, int nchunks, int k) {
 template <int MB, int R, int U, typename XT, typename YT>
 __global__ void __launch_bounds__(GEMV_THREADS, (MB <= 2 ? 2 : 1))
 gemv_nk_kernel(const uint8_t* __restrict__ W, const float* __restrict__ scales,
-               const XT* __restrict__ x, YT* __restrict__ y, int M, int N, int K, int ldy, int y_col0, int act) {
+               const XT* x, YT* __restrict__ y, int M, int N, int K, int ldy, int y_col0, int act) {
     extern __shared__ __align__(16) float smem[];
     const int nchunks = (K + CHUNK - 1) / CHUNK;
     float* xs = smem;
@@ -222,7 +222,7 @@ constexpr int KN_SLICES = 64;            // k-slices per block
 template <int MB, int U, bool AFFINE, typename XT, typename YT>
 __global__ void __launch_bounds__(KN_THREADS)
 gemv_kn_kernel(const uint8_t* __restrict__ W, const float* __restrict__ scales, const float* __restrict__ biases,
-               const XT* __restrict__ x, YT* __restrict__ y, int M, int N, int K, int ldy, int y_col0) {
+               const XT* x, YT* __restrict__ y, int M, int N, int K, int ldy, int y_col0) {
     extern __shared__ __align__(16) float smem[];
     float* xs = smem;                             // [MB][K]
     float* red = smem + (size_t)MB * K;           // [KN_SLICES][MB][KN_COLS]

@@ -82,7 +82,7 @@ __device__ __forceinline__ float2 ld_ahead(const float2* p) {
 
 // Digits of x: a half warp takes 64 k of a row.  Rows M .. 2 tiles are zeros.
 template <typename XT>
-__global__ void __launch_bounds__(256) affine_prepare_kernel(const XT* __restrict__ x, uint32_t* digits, float2* aux, int M, int K, int tiles) {
+__global__ void __launch_bounds__(256) affine_prepare_kernel(const XT* x, uint32_t* digits, float2* aux, int M, int K, int tiles) {
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31, m = blockIdx.y;

@@ -272,10 +272,11 @@ int launch_matmul(rusty_cuda_ctx* ctx, const float* a, const float* b, float* ou
 
 // t[M, r4] = x[M, K] . A[K, r] (zeros in columns r .. r4), the adapter's first product.  Here the order of the sum is free (f32
 // throughout): a block takes MT rows of x and four columns of A, its threads cut K between them, so that the product costs
-// two trips to L2 instead of a chain of K links.
+// two trips to L2 instead of a chain of K links.  (No read-only loads here and in the kernel below: what they read may be the work
+// of kernels that still run when these start.)
 constexpr int LD_THREADS = 256;
 template <int MT>
-__global__ void __launch_bounds__(LD_THREADS) lora_down_kernel(const float* __restrict__ x, const float* __restrict__ A, float* __restrict__ t,
+__global__ void __launch_bounds__(LD_THREADS) lora_down_kernel(const float* x, const float* A, float* t,
                                                                uint32_t M, uint32_t K, uint32_t r, uint32_t r4, uint32_t col0) {
     __shared__ float red[LD_THREADS / 32][MT * 4];
     pdl_wait();
@@ -293,15 +294,15 @@ __global__ void __launch_bounds__(LD_THREADS) lora_down_kernel(const float* __re
         float av[4];
         const float* pa = A + (size_t)k * r + c0;
         if (vec) {
-            const float4 q = __ldg(reinterpret_cast<const float4*>(pa));
+            const float4 q = *reinterpret_cast<const float4*>(pa);
             av[0] = q.x; av[1] = q.y; av[2] = q.z; av[3] = q.w;
         } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) av[j] = c0 + j < r ? __ldg(pa + j) : 0.0f;
+            for (int j = 0; j < 4; ++j) av[j] = c0 + j < r ? pa[j] : 0.0f;
         }
 #pragma unroll
         for (int i = 0; i < MT; ++i) {
-            const float xv = m0 + i < M ? __ldg(x + (size_t)(m0 + i) * K + k) : 0.0f;
+            const float xv = m0 + i < M ? x[(size_t)(m0 + i) * K + k] : 0.0f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xv, av[j], acc[i][j]);
         }
@@ -327,7 +328,7 @@ __global__ void __launch_bounds__(LD_THREADS) lora_down_kernel(const float* __re
 // y[M, N] += t[M, r4] . b[r, N], behind a quantised Linear that has written y.  One thread per column, the block's rows one
 // after the other: b stays in registers up to rank 16.
 constexpr int LU_THREADS = 256, LU_KEEP = 16;
-__global__ void __launch_bounds__(LU_THREADS) lora_up_add_kernel(const float* __restrict__ t, const float* __restrict__ b, float* y, uint32_t M,
+__global__ void __launch_bounds__(LU_THREADS) lora_up_add_kernel(const float* t, const float* b, float* y, uint32_t M,
                                                                  uint32_t N, int r, uint32_t r4, uint32_t rows) {
     pdl_launch_dependents();
     pdl_wait();
@@ -335,7 +336,7 @@ __global__ void __launch_bounds__(LU_THREADS) lora_up_add_kernel(const float* __
     if (n >= N) return;
     float bv[LU_KEEP];
 #pragma unroll
-    for (int q = 0; q < LU_KEEP; ++q) bv[q] = q < r ? __ldg(b + (size_t)q * N + n) : 0.0f;
+    for (int q = 0; q < LU_KEEP; ++q) bv[q] = q < r ? b[(size_t)q * N + n] : 0.0f;
     const uint32_t m1 = min(M, (blockIdx.y + 1) * rows);
     for (uint32_t m = blockIdx.y * rows; m < m1; ++m) {
         const float* tr = t + (size_t)m * r4;
@@ -343,8 +344,8 @@ __global__ void __launch_bounds__(LU_THREADS) lora_up_add_kernel(const float* __
         float s = 0.0f;
 #pragma unroll
         for (int q = 0; q < LU_KEEP; ++q)
-            if (q < r) s = fmaf(__ldg(tr + q), bv[q], s);
-        for (int q = LU_KEEP; q < r; ++q) s = fmaf(__ldg(tr + q), __ldg(b + (size_t)q * N + n), s);
+            if (q < r) s = fmaf(tr[q], bv[q], s);
+        for (int q = LU_KEEP; q < r; ++q) s = fmaf(tr[q], b[(size_t)q * N + n], s);
         y[(size_t)m * N + n] = __fadd_rn(v, s);
     }
 }

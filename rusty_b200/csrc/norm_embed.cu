@@ -27,7 +27,7 @@ namespace {
 // threads walking the row twice it took 4.8 us a call, with every load in flight at once 2.6.  K % 4 == 0.
 constexpr int RN_V = 4;
 template <int T>
-__global__ void __launch_bounds__(T) rms_norm_rows_kernel(const float* __restrict__ x, const float* residual, const float* __restrict__ weight,
+__global__ void __launch_bounds__(T) rms_norm_rows_kernel(const float* x, const float* residual, const float* __restrict__ weight,
                                                           float* out, float* sum_out, int K, float eps) {
     __shared__ float red[T / 32];
     pdl_launch_dependents();
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(T) rms_norm_rows_kernel(const float* __restric
 }
 
 // out[t, :] = table[ids[t], :], 16 bytes per thread access; dim % 4 == 0.
-__global__ void __launch_bounds__(256) embedding_rows_kernel(const float* __restrict__ table, const uint32_t* __restrict__ ids,
+__global__ void __launch_bounds__(256) embedding_rows_kernel(const float* __restrict__ table, const uint32_t* ids,
                                                              float* __restrict__ out, size_t n_ids, uint32_t vocab, uint32_t dim,
                                                              rusty_cuda_dev_status* status) {
     pdl_launch_dependents();
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(256) embedding_rows_kernel(const float* __rest
     const size_t per_row = dim / 4, total = n_ids * per_row;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t t = i / per_row, c = i - t * per_row;
-        const uint32_t id = __ldg(ids + t);
+        const uint32_t id = ids[t];
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (id < vocab) {
             v = __ldg(reinterpret_cast<const float4*>(table + (size_t)id * dim) + c);

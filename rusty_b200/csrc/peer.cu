@@ -39,7 +39,7 @@ __global__ void peer_wait_kernel(const PeerPush pp) {
 // Copies rows [0,M) x bytes [0,row_bytes) of a local slice (rows ld_bytes apart) to the same addresses of every
 // other arena.  VEC = bytes per thread access.
 template <int VEC>
-__global__ void __launch_bounds__(256) peer_push_kernel(const uint8_t* __restrict__ src, int M, size_t row_bytes, size_t ld_bytes,
+__global__ void __launch_bounds__(256) peer_push_kernel(const uint8_t* src, int M, size_t row_bytes, size_t ld_bytes,
                                                         const PeerPush pp) {
     pdl_launch_dependents();
     pdl_wait();

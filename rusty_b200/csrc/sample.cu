@@ -31,7 +31,7 @@ __device__ __forceinline__ bool beats(const Cand& a, const Cand& b, bool b_valid
 
 // best of row m of x[M, ld] over columns [0, n), indices reported as col0 + column; NaN never wins.
 // valid == false: no candidate (empty row or all NaN).
-__device__ __forceinline__ void row_argmax(const float* __restrict__ x, int n, unsigned int col0, Cand& best, bool& valid) {
+__device__ __forceinline__ void row_argmax(const float* x, int n, unsigned int col0, Cand& best, bool& valid) {
     __shared__ float s_v[AM_THREADS / 32];
     __shared__ unsigned int s_i[AM_THREADS / 32];
     __shared__ int s_ok[AM_THREADS / 32];
@@ -88,7 +88,7 @@ __device__ __forceinline__ void row_argmax(const float* __restrict__ x, int n, u
 // L2).  One block of 1024 threads per row took 19 us for 1 x 32000 and 65 us for 32 x 128256 logits; 8 blocks of 512: 4 and
 // 6 us.  Candidates are compared as (order-preserving key, index) with two warp reductions.
 constexpr int AR_THREADS = 512;
-__global__ void __launch_bounds__(AR_THREADS) argmax_rows_kernel(const float* __restrict__ x, int n, size_t ld,
+__global__ void __launch_bounds__(AR_THREADS) argmax_rows_kernel(const float* x, int n, size_t ld,
                                                                  unsigned int* __restrict__ out_idx, float* __restrict__ out_val) {
     __shared__ unsigned int s_key[AR_THREADS / 32], s_idx[AR_THREADS / 32];
     __shared__ uint2 s_cand[8];   // in block 0 of the cluster: every block's best
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(AR_THREADS) argmax_rows_kernel(const float* __
 
 // Sharded form, first half: this rank's candidate of every row goes into slot `rank` of the candidate table of EVERY
 // rank's arena ([G][M] x {value bits, index + 1}; index + 1 == 0 means "no candidate"), then the CTA signals.
-__global__ void __launch_bounds__(AM_THREADS) argmax_rows_push_kernel(const float* __restrict__ x, int n, size_t ld, unsigned int col0,
+__global__ void __launch_bounds__(AM_THREADS) argmax_rows_push_kernel(const float* x, int n, size_t ld, unsigned int col0,
                                                                       uint2* __restrict__ table, int M, const PeerPush pp) {
     pdl_launch_dependents();
     pdl_wait();

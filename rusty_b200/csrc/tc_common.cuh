@@ -162,6 +162,8 @@ __device__ __forceinline__ bool peer_sync_block(const PeerPush& pp, int b, unsig
 // Programmatic dependent launch: let the next kernel in the stream start its
 // prologue now / wait until everything earlier in the stream has finished and
 // its writes are visible.  Both are no-ops for a kernel launched the plain way.
+// What an earlier kernel may write is read with ordinary loads behind the wait: read-only ones (ld.global.nc: __ldg, or what the
+// compiler makes of a const __restrict__ parameter) want data that nobody writes while the kernel runs, and this one runs already.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -339,7 +341,7 @@ inline unsigned row_cluster(uint32_t M, uint32_t N, int sm_count) {
 // Calls f(value, column) for this block's slice of row[0, n): thread t of block r of S walks ascending columns, 16 bytes a
 // load where the row is aligned, four loads in flight.
 template <int THREADS, typename F>
-__device__ __forceinline__ void walk_row_slice(const float* __restrict__ row, int n, unsigned r, unsigned S, F&& f) {
+__device__ __forceinline__ void walk_row_slice(const float* row, int n, unsigned r, unsigned S, F&& f) {
     const int tid = threadIdx.x;
     if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
         const float4* r4 = reinterpret_cast<const float4*>(row);
@@ -349,7 +351,7 @@ __device__ __forceinline__ void walk_row_slice(const float* __restrict__ row, in
             float4 v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-                if (i0 + u * THREADS < hi) v[u] = __ldg(r4 + i0 + u * THREADS);
+                if (i0 + u * THREADS < hi) v[u] = r4[i0 + u * THREADS];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int i = i0 + u * THREADS;
@@ -368,7 +370,7 @@ __device__ __forceinline__ void walk_row_slice(const float* __restrict__ row, in
             float v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-                if (i0 + u * THREADS < hi) v[u] = __ldg(row + i0 + u * THREADS);
+                if (i0 + u * THREADS < hi) v[u] = row[i0 + u * THREADS];
 #pragma unroll
             for (int u = 0; u < 4; ++u)
                 if (i0 + u * THREADS < hi) f(v[u], i0 + u * THREADS);

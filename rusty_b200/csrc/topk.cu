@@ -72,7 +72,7 @@ struct RadixScratch {
     unsigned int warp[T / 32];
 };
 template <int T>
-__device__ void radix_topk(const float* __restrict__ row, int n, unsigned int col0, int k, unsigned long long* cand, RadixScratch<T>& s) {
+__device__ void radix_topk(const float* row, int n, unsigned int col0, int k, unsigned long long* cand, RadixScratch<T>& s) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         s.prefix = 0u;
@@ -173,7 +173,7 @@ __device__ void radix_topk(const float* __restrict__ row, int n, unsigned int co
 
 // Sharded, first half.  One block per row (rows b, b + grid, ...): the row's k winners, sorted, as items into slot `rank` of
 // every rank's candidate table ([G][M][k], zero-padded).
-__global__ void __launch_bounds__(TK_THREADS) topk_rows_push_kernel(const float* __restrict__ x, int n, size_t ld, unsigned int col0, int k, int M,
+__global__ void __launch_bounds__(TK_THREADS) topk_rows_push_kernel(const float* x, int n, size_t ld, unsigned int col0, int k, int M,
                                                                     unsigned long long* __restrict__ table, const PeerPush pp) {
     __shared__ RadixScratch<TK_THREADS> scratch;
     __shared__ unsigned long long cand[TK_MAX_K];
@@ -230,7 +230,7 @@ __device__ __forceinline__ uint32_t stat_key_of(float v) {
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
-__global__ void __launch_bounds__(RC_THREADS) logits_rows_kernel(const float* __restrict__ x, int n, size_t ld, int k, int glog,
+__global__ void __launch_bounds__(RC_THREADS) logits_rows_kernel(const float* x, int n, size_t ld, int k, int glog,
                                                                  unsigned int* __restrict__ out_idx, float* __restrict__ out_val,
                                                                  float inv_t, float* __restrict__ out_max, float* __restrict__ out_sum) {
     extern __shared__ __align__(16) unsigned char row_smem[];

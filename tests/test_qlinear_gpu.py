@@ -702,3 +702,26 @@ def test_affine_out_in_sums(ctx, engine, M, K, N, act):
     x[M - 1] *= np.float32(2.0 ** -100)          # the scaled rows of a chunk keep their bits however small they are
     tiny = _forward(ctx, engine, QLinear.from_host(ctx, u, sg.reshape(-1), bg.reshape(-1)), x, x_dtype=dt, y_dtype=DType.FP32)[M - 1]
     assert np.linalg.norm(tiny[cols] - exact[M - 1] * 2.0 ** -100) / np.linalg.norm(exact[M - 1] * 2.0 ** -100) <= 2.0 ** -24 * (17.0 / 3.0) ** 0.5 * 1.25   # (one row's sample)
+
+
+@pytest.mark.parametrize("weights,M", [("sym", 1), ("sym", 5), ("native", 1), ("native", 4), ("native", 8), ("native", 13), ("native", 40), ("affine", 2), ("affine", 13)])
+def test_activations_rewritten_between_calls(ctx, engine, weights, M):
+    """Forwards back to back over one activation buffer that a kernel rewrites in between, small enough that kernels of several
+    steps are on the device together: each sees its own step's values, bit for bit as when nothing else runs."""
+    K, N, steps = 1024, 256, 24
+    rng = np.random.default_rng(M)
+    if weights == "sym":
+        ql = QLinear.from_host(ctx, rng.integers(-127, 128, size=(N, K), dtype=np.int8), rng.uniform(0.001, 0.02, size=N).astype(np.float32))
+    else:
+        u = rng.integers(0, 256, size=(K, N) if weights == "native" else (N, K), dtype=np.uint8)
+        sg = rng.uniform(0.001, 0.02, size=K * N // 64).astype(np.float32)
+        ql = QLinear.from_host(ctx, u, sg, -128.0 * sg, layout=capi.LAYOUT_KN if weights == "native" else capi.LAYOUT_NK)
+    xs = [rng.standard_normal((M, K)).astype(np.float32) for _ in range(3)]
+    want = [_forward(ctx, engine, ql, x) for x in xs]
+    src, zero = [UnifiedTensor.new(ctx, x, [M, K]) for x in xs], UnifiedTensor.zeros(ctx, [M, K])
+    x, ys = UnifiedTensor.empty(ctx, [M, K]), [UnifiedTensor.empty(ctx, [M, N]) for _ in range(steps)]
+    for i in range(steps):
+        engine.add(ctx, src[i % 3], zero, x)
+        engine.qlinear(ctx, x, ql, ys[i])
+    for i in range(steps):
+        assert_bits_equal(ys[i].to_vec(ctx).reshape(M, N), want[i % 3])

@@ -264,3 +264,25 @@ def test_linear_lora_of_many_rows_or_columns(ctx, engine, M, rank):
     out = GuardedOutput(ctx, [M, N])
     engine.linear_lora(ctx, tx, QLinear.from_host(ctx, q, np.ones(N, np.float32)), ta, tb, out.tensor)
     assert_bits_equal(out.read(), x @ q.T.astype(np.float32) + low)
+
+
+@pytest.mark.parametrize("M,rank", [(100, 16), (200, 32), (200, 30), (300, 64)])
+def test_linear_lora_first_products_back_to_back(ctx, engine, M, rank):
+    """The adapter's first product with four rows a block, with eight (16-byte and single loads of A) and as a matmul of its own,
+    over an f32 and a quantised weight: calls back to back over an x that a kernel rewrites in between, against float64."""
+    K, N, steps = 256, 192, 6
+    rng = np.random.default_rng(M + rank)
+    w, a, b = (rng.standard_normal(s).astype(np.float32) for s in ((K, N), (K, rank), (rank, N)))
+    q, s = rng.integers(-127, 128, size=(N, K), dtype=np.int8), rng.uniform(0.001, 0.02, size=N).astype(np.float32)
+    ta, tb = UnifiedTensor.new(ctx, a, [K, rank]), UnifiedTensor.new(ctx, b, [rank, N])
+    weights = ((UnifiedTensor.new(ctx, w, [K, N]), w.astype(np.float64)), (QLinear.from_host(ctx, q, s), (q * s[:, None].astype(np.float64)).T))
+    xs = [rng.standard_normal((M, K)).astype(np.float32) for _ in range(3)]
+    src, zero = [UnifiedTensor.new(ctx, x, [M, K]) for x in xs], UnifiedTensor.zeros(ctx, [M, K])
+    for tw, wf in weights:
+        x, ys = UnifiedTensor.empty(ctx, [M, K]), [UnifiedTensor.empty(ctx, [M, N]) for _ in range(steps)]
+        for i in range(steps):
+            engine.add(ctx, src[i % 3], zero, x)
+            engine.linear_lora(ctx, x, tw, ta, tb, ys[i])
+        for i in range(steps):
+            x64 = xs[i % 3].astype(np.float64)
+            assert rel_err(ys[i].to_vec(ctx).reshape(M, N), x64 @ wf + (x64 @ a) @ b) <= TOL_FP32
