@@ -33,11 +33,11 @@
 // epilogue in the end.  Two CTAs fit an SM.
 // A K range per CTA of a cluster (1, 2 or 4) where there are too few groups; their int64 sums meet in distributed shared memory.
 //
-// What bounds it: few rows, the weight stream and the fixed part of a launch; 4096 x 4096, per call in a graph: 1 row 8.0 us, 4 rows
-// 10.5, 8 rows 13.1, 13 rows 12.5, 32 rows 17.6, 64 rows 28.4 (a GEMV kernel with a pair of rows per CTA: 4 rows 13.2, 32 rows 58.6);
-// 12288 x 2112, whose last stage is half empty (rows padded at create), 1 row 10.8 us, 64 rows 38 (on CUDA cores 15.5 and 600).
-// Many rows: 512 x 4096 x 4096 takes 121 us and is at the limit of no unit (ncu: issue slots 51 %, the data pipe of shared memory
-// and L1 50 %, ALU 36 %, tensor cores 18 %); a converter waits for x from L2 (5 % of its loads hit L1) and for its A buffer, and
+// What bounds it: few rows, the weight stream and the fixed part of a launch; 4096 x 4096, per call in a graph: 1 row 8.2 us, 4 rows
+// 10.8, 8 rows 13.4, 13 rows 12.2, 32 rows 17.0, 64 rows 26.5 (a GEMV kernel with a pair of rows per CTA: 4 rows 13.2, 32 rows 58.6);
+// 12288 x 2112, whose last stage is half empty (rows padded at create), 1 row 11.1 us, 64 rows 36.5 (on CUDA cores 15.5 and 600).
+// Many rows: 512 x 4096 x 4096 takes 113 us and is at the limit of no unit (ncu: issue slots 46 %, the data pipe of shared memory
+// and L1 52 %, ALU 31 %, tensor cores 18 %); a converter waits for x from L2 (6 % of its loads hit L1) and for its A buffer, and
 // the 512 CTAs are 1.7 waves of the 296 that fit.
 #include <cooperative_groups.h>
 

@@ -353,9 +353,10 @@ __global__ void __launch_bounds__(LU_THREADS) lora_up_add_kernel(const float* t,
 int launch_lora_down(rusty_cuda_ctx* ctx, const float* x, const float* A, float* t, uint32_t M, uint32_t K, uint32_t r, uint32_t r4) {
     // rows per block: enough blocks for the SMs first (one row each), then fewer passes over A; once x is re-read for so many
     // columns that the blocks fill the chip twice over, the chain of the matmul is shorter than the re-reading.  Whole calls, K =
-    // 4096, N = 512, us, with 1, 4, 8 rows a block and with the matmul: 128 rows of rank 8 40.3 / 40.8 / 43.0 / 55.6, 256 of 8 60.5 /
-    // 60.8 / 63.2 / 75.8, 64 of 64 47.3 / 36.8 / 37.4 / 49.3, 100 of 64 62.2 / 45.4 / 45.1 / 55.5, 256 of 64 123 / 79 / 74 / 76, 600
-    // of 16 263 / 251 / 251 / 155, 1024 of 8 254 / 249 / 250 / 157.
+    // 4096, N = 512, us, with 1, 4, 8 rows a block and with the matmul: 128 rows of rank 8 38.8 / 39.9 / 41.8 / 55.6, 256 of 8 60.0 /
+    // 60.2 / 61.9 / 75.9, 64 of 64 46.9 / 36.5 / 36.4 / 49.3, 100 of 64 62.1 / 45.3 / 44.6 / 55.5, 256 of 64 121 / 77 / 73 / 76, 600
+    // of 16 263 / 250 / 250 / 154, 1024 of 8 254 / 248 / 250 / 157.  (The line is drawn by blocks alone: 100 and 256 of 64 lie
+    // behind it all the same.)
     const uint32_t cols = r4 / 4;
     const uint64_t want = 2ull * (unsigned)(ctx->sm_count > 0 ? ctx->sm_count : 1);
     const uint32_t mt = (uint64_t)M * cols <= want ? 1 : (uint64_t)(M / 4) * cols <= want ? 4 : 8;
