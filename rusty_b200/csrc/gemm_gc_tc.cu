@@ -34,7 +34,7 @@
 // A K range per CTA of a cluster (1, 2 or 4) where there are too few groups; their int64 sums meet in distributed shared memory.
 //
 // What bounds it: few rows, the weight stream and the fixed part of a launch; 4096 x 4096, per call in a graph: 1 row 8.2 us, 4 rows
-// 10.8, 8 rows 13.4, 13 rows 12.2, 32 rows 17.0, 64 rows 26.5 (a GEMV kernel with a pair of rows per CTA: 4 rows 13.2, 32 rows 58.6);
+// 10.5, 8 rows 12.8, 13 rows 12.2, 32 rows 17.0, 64 rows 26.5 (a GEMV kernel with a pair of rows per CTA: 4 rows 13.2, 32 rows 58.6);
 // 12288 x 2112, whose last stage is half empty (rows padded at create), 1 row 11.1 us, 64 rows 36.5 (on CUDA cores 15.5 and 600).
 // Many rows: 512 x 4096 x 4096 takes 113 us and is at the limit of no unit (ncu: issue slots 46 %, the data pipe of shared memory
 // and L1 52 %, ALU 31 %, tensor cores 18 %); a converter waits for x from L2 (6 % of its loads hit L1) and for its A buffer, and
@@ -101,8 +101,12 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // Magnitudes are compared as bits: a NaN or an infinity is above every number.
 __device__ __forceinline__ uint32_t abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
 __device__ __forceinline__ uint32_t abs_max(const float4& v) { return max(max(abs_bits(v.x), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w))); }
-__device__ __forceinline__ uint32_t abs_max(const float4& x, const float4& s) {   // of the products, rounded as the converters round them
-    return abs_max(make_float4(__fmul_rn(x.x, s.x), __fmul_rn(x.y, s.y), __fmul_rn(x.z, s.z), __fmul_rn(x.w, s.w)));
+// Largest of top and the magnitudes of four products, rounded as the converters round them.  Two three-operand maxima that take the
+// magnitudes by themselves: every CTA walks all rows x K of them (as integers, four more instructions).  A NaN stays one.
+__device__ __forceinline__ float top_of(float top, const float4& x, const float4& s) {
+    asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(top) : "f"(__fmul_rn(x.x, s.x)), "f"(__fmul_rn(x.y, s.y)));
+    asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(top) : "f"(__fmul_rn(x.z, s.z)), "f"(__fmul_rn(x.w, s.w)));
+    return top;
 }
 
 __device__ __forceinline__ float4 ldg_x4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }   // of the weight's own tables
@@ -283,11 +287,11 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
 #pragma unroll
                     for (int u = 0; u < AHEAD; ++u)
                         if (kb + u * CW < top1) v[u] = ld_x4<XT>(xr + (size_t)m * p.K + (kb + u * CW) * SK);
-                    uint32_t top = 0u;
+                    float most = 0.0f;
 #pragma unroll
                     for (int u = 0; u < AHEAD; ++u)
-                        if (kb + u * CW < top1) top = max(top, abs_max(v[u], sv[u]));
-                    top = __reduce_max_sync(0xffffffffu, top);
+                        if (kb + u * CW < top1) most = top_of(most, v[u], sv[u]);
+                    const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(most));
                     if (lane == 0) atomicMax(s_top + m, top);
                 }
             }
@@ -330,7 +334,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
                             const int st = base + lane;
                             const uint32_t b = st < p.nst ? rest_bound(xt[(size_t)(8 * i) * p.nst + st], st) >> 23 : 0u;
                             uint32_t todo = __ballot_sync(0xffffffffu, b > top[i] >> 23);
-                            auto stage_max = [&](int s) { return abs_max(ld_x4(xr + (size_t)s * p.xstep + i * (8 * SK)), ldg_x4(gs + s * SK)); };
+                            auto stage_max = [&](int s) { return __float_as_uint(top_of(0.0f, ld_x4(xr + (size_t)s * p.xstep + i * (8 * SK)), ldg_x4(gs + s * SK))); };
                             while (todo) {     // two stages at a time
                                 const int sa = base + __ffs(todo) - 1;
                                 todo &= todo - 1;
@@ -800,10 +804,11 @@ int launch_gc_tc(rusty_cuda_ctx* ctx, const QLinearArgs& a) {
         // suffice, and the start and the end of a CTA cost as much as ten stages.
         p.ways = 1;
         while (tiles == 1 && p.ways < 4 && groups * p.ways * 2 <= 2 * ctx->sm_count && p.nst / (p.ways * 2) >= 4) p.ways *= 2;
-        // Meeting costs 2 us (one row x 4096 x 4096: 8.1 -> 10.0 us, four 10.5 -> 11.6), walking x and the scales beyond what the
-        // registers hold more than that with rows x stages (14336 x 3008 at one / two / eight rows: 16.4 / 18.4 / 30.6 us alone,
-        // 15.6 / 16.2 / 20.7 together; 11008 x 4096 at one / four: 15.1 / 20.3 and 15.5 / 17.6).
-        const bool meet = rpw == 1 && p.ways > 1 && p.nst > 32 && p.M * p.nst >= 100;
+        // Meeting costs 1 to 2 us, walking x and the scales beyond what the registers hold more than that with rows x stages.  One
+        // CTA alone / together, us: 4096 x 4096 at one / eight rows 8.2 / 10.0 and 12.8 / 13.4; 5120 x 4096 at three / four / six
+        // 12.0 / 12.6, 13.1 / 13.2, 15.0 / 14.0; 8192 x 4096 at two / four 13.2 / 13.9, 15.5 / 15.0; 11008 x 4096 at one / two /
+        // eight 15.4 / 15.8, 16.6 / 16.5, 24.9 / 19.6; 14336 x 3008 at one / eight 16.5 / 16.0, 28.3 / 20.3.
+        const bool meet = rpw == 1 && p.ways > 1 && p.nst > 32 && (p.M * p.nst >= 160 || p.nst > 96);
         const size_t fixed = 1024 + (size_t)rb * A_BYTES + (4 * MAX_STAGES + 2) * 8 + (size_t)rb * 32 * 24 + (size_t)p.nst * 4 + 64;
         const size_t budget = (ctx->smem_optin + 1024) / 2 - 1024;   // half an SM, less the 1 KiB every block pays
         int stages = budget > fixed ? (int)((budget - fixed) / (STAGE_BYTES + S_BYTES)) : 0;
