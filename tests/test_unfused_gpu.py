@@ -286,3 +286,34 @@ def test_linear_lora_first_products_back_to_back(ctx, engine, M, rank):
         for i in range(steps):
             x64 = xs[i % 3].astype(np.float64)
             assert rel_err(ys[i].to_vec(ctx).reshape(M, N), x64 @ wf + (x64 @ a) @ b) <= TOL_FP32
+
+
+@pytest.mark.parametrize("M,K,N,rank", [(1, 4096, 260, 2), (5, 1028, 1024, 8), (8, 1024, 1100, 3), (9, 2052, 516, 17), (16, 4096, 260, 64), (17, 1040, 1012, 1),
+                                        (33, 1024, 4100, 30), (100, 8192, 132, 4)])
+def test_linear_lora_with_k_cut(ctx, engine, M, K, N, rank):
+    """The f32 weight's kernel that cuts K and multiplies on the tensor cores, at ragged rows, columns, units of k and ranks.  Bound: the
+    split costs a product at most 2^-22 of itself, and at most 48 additions of 2^-24 of the sum of magnitudes lie on an output's way."""
+    rng = np.random.default_rng(M + K + N)
+    x, w = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((K, N)).astype(np.float32)
+    x[:, rng.integers(0, K, size=4)] *= 1000.0
+    a, b = rng.standard_normal((K, rank)).astype(np.float32), rng.standard_normal((rank, N)).astype(np.float32)
+    tx, tw = UnifiedTensor.new(ctx, x, [M, K]), UnifiedTensor.new(ctx, w, [K, N])
+    ta, tb = UnifiedTensor.new(ctx, a, [K, rank]), UnifiedTensor.new(ctx, b, [rank, N])
+    x64, t64 = x.astype(np.float64), x.astype(np.float64) @ a
+    want = x64 @ w + t64 @ b
+    sizes = np.abs(x64) @ np.abs(w) + (np.abs(x64) @ np.abs(a)) @ np.abs(b)
+    out = GuardedOutput(ctx, [M, N], DType.FP32)
+    engine.linear_lora(ctx, tx, tw, ta, tb, out.tensor)
+    got = out.read()
+    assert (np.abs(got - want) <= 52 * 2.0**-24 * sizes).all()
+    # an infinity stays one, in its row (of x) or its column (of W)
+    xi, wi = x.copy(), w.copy()
+    xi[M // 2, 3], wi[K - 1, N // 2] = np.inf, -np.inf
+    out = GuardedOutput(ctx, [M, N], DType.FP32)
+    engine.linear_lora(ctx, UnifiedTensor.new(ctx, xi, [M, K]), UnifiedTensor.new(ctx, wi, [K, N]), ta, UnifiedTensor.zeros(ctx, [rank, N]), out.tensor)
+    got = out.read()
+    rows, cols = np.arange(M) != M // 2, np.arange(N) != N // 2
+    assert np.isfinite(got[rows][:, cols]).all()
+    assert np.array_equal(got[rows, N // 2], np.sign(xi[rows, K - 1]) * -np.inf)
+    # the infinite x times A makes an infinite or undefined t, and that times a zero B is undefined, as in the products one by one
+    assert np.isnan(got[M // 2]).all()
