@@ -103,16 +103,19 @@ constexpr int DIG_MAXV = 8;   // passes of a row held in registers between the m
 // NORM: the activations are RMSNorm(x [+ residual]) * weight (norm_embed.cu gives the formula and its lines in the
 // reference); the row is normalised in registers between the load and the maximum, so it must fit there
 // (K <= DIG_MAXV * 4 * threads of the row), and the normalised row and the sum are written out where asked for.
-template <typename XT, int D, bool NORM>
+template <typename XT, int D, bool NORM, bool SPLIT>
 __global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* x, int8_t* __restrict__ xq,
                                                                     float* __restrict__ inv_s, int M, int Mpad, int K, int R,
                                                                     const PeerPush push, const NormArgs nrm, long long* dbg) {
     __shared__ float red[DIG_THREADS / 32];
     __shared__ float red_ss[DIG_THREADS / 32];
+    __shared__ uint32_t part_max[2];
     const int tid = threadIdx.x;
+    const int part = SPLIT ? (int)blockIdx.x & 1 : 0;         // SPLIT: which half of the row (R = 1)
+    const int k0 = part ? K / 8 * 4 : 0, k1 = SPLIT && !part ? K / 8 * 4 : K;
     const int tpr = DIG_THREADS / R;               // threads per row (512 or 256)
     const int grp = tid / tpr, tg = tid - grp * tpr;
-    const int mq = blockIdx.x * R + grp;           // row inside row block blockIdx.y
+    const int mq = (SPLIT ? (int)blockIdx.x >> 1 : (int)blockIdx.x * R) + grp;   // row inside row block blockIdx.y
     const int m = (int)blockIdx.y * Mpad + mq;
     xq += (size_t)blockIdx.y * D * Mpad * K;
     PDBG(tid == 0 && blockIdx.x == 0, 0);
@@ -128,24 +131,24 @@ __global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* x,
     }
     const int step = tpr * 4;                       // activations one pass of the row's threads covers
     if (m >= M) {
-        for (int k = tg * 4; k < K; k += step)
+        for (int k = k0 + tg * 4; k < k1; k += step)
 #pragma unroll
             for (int d = 0; d < D; ++d) *reinterpret_cast<uint32_t*>(xq + (size_t)(d * Mpad + mq) * K + k) = 0u;
-        return;   // whole row groups leave together: the named barrier below is per group
+        return;   // whole row groups (and clusters) leave together: the named barrier below is per group
     }
     const XT* xr = x + (size_t)m * K;
     float4 v[DIG_MAXV];
 #pragma unroll
     for (int j = 0; j < DIG_MAXV; ++j) {
-        const int k = tg * 4 + j * step;
-        v[j] = k < K ? load_row4<XT>(xr + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const int k = k0 + tg * 4 + j * step;
+        v[j] = k < k1 ? load_row4<XT>(xr + k) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if constexpr (NORM) {
         float ss = 0.0f;
 #pragma unroll
         for (int j = 0; j < DIG_MAXV; ++j) {
-            const int k = tg * 4 + j * step;
-            if (k < K) {
+            const int k = k0 + tg * 4 + j * step;
+            if (k < k1) {
                 if (nrm.residual) {
                     const float4 r = *reinterpret_cast<const float4*>(nrm.residual + (size_t)m * K + k);
                     v[j].x += r.x; v[j].y += r.y; v[j].z += r.z; v[j].w += r.w;
@@ -166,8 +169,8 @@ __global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* x,
         const float inv_rms = 1.0f / sqrtf(tot / (float)K + nrm.eps);
 #pragma unroll
         for (int j = 0; j < DIG_MAXV; ++j) {
-            const int k = tg * 4 + j * step;
-            if (k < K) {
+            const int k = k0 + tg * 4 + j * step;
+            if (k < k1) {
                 const float4 w = __ldg(reinterpret_cast<const float4*>(nrm.weight + k));
                 v[j].x = v[j].x * inv_rms * w.x; v[j].y = v[j].y * inv_rms * w.y;
                 v[j].z = v[j].z * inv_rms * w.z; v[j].w = v[j].w * inv_rms * w.w;
@@ -182,12 +185,18 @@ __global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* x,
     };
 #pragma unroll
     for (int j = 0; j < DIG_MAXV; ++j) fold(v[j]);
-    for (int k = tg * 4 + DIG_MAXV * step; k < K; k += step) fold(load_row4<XT>(xr + k));
+    for (int k = k0 + tg * 4 + DIG_MAXV * step; k < k1; k += step) fold(load_row4<XT>(xr + k));
     mx = __reduce_max_sync(0xffffffffu, mx);
     if ((tid & 31) == 0) red[tid >> 5] = __uint_as_float(mx);
     asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(tpr) : "memory");   // the row's threads only
     const int wpr = tpr / 32;                       // warps per row: 16 or 8
-    const float vmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(red[grp * wpr + (tid & (wpr - 1))])));
+    uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(red[grp * wpr + (tid & (wpr - 1))]));
+    if constexpr (SPLIT) {
+        if (tid < 2) st_cluster_u32(part_max + part, (uint32_t)tid, top);
+        cluster_sync_all();
+        top = max(part_max[0], part_max[1]);
+    }
+    const float vmax = __uint_as_float(top);
     // s = the power of two that puts vmax*s into [64, 128) but not above 127
     int e2 = 0;
     if (vmax >= 1.0e-30f && vmax <= 3.0e38f) {
@@ -202,7 +211,7 @@ __global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* x,
     const bool finite = vmax <= 3.0e38f;
     const float sc = finite ? __uint_as_float((uint32_t)(127 + e2) << 23) : 0.0f;
     // 1/s_m * 256^-(D-1): both powers of two, so the product is exact; inf/nan poisons the row
-    if (tg == 0) inv_s[m] = finite ? ldexpf(1.0f, -e2 - 8 * (D - 1)) : __int_as_float(0x7fc00000);
+    if (tg == 0 && part == 0) inv_s[m] = finite ? ldexpf(1.0f, -e2 - 8 * (D - 1)) : __int_as_float(0x7fc00000);
     // Straight-line code over the registers (a rolled loop had to pick its registers with a chain of selects: 78.4 -> 71.7 us
     // for the pair at 64 x 28672 x 8192).  4 elements x 4 digit bytes -> digit planes x 4 element bytes; byte b = digit b from the
     // least significant, byte D-1 = the top digit = plane 0.
@@ -216,10 +225,10 @@ __global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* x,
     };
 #pragma unroll
     for (int j = 0; j < DIG_MAXV; ++j) {
-        const int k = tg * 4 + j * step;
-        if (k < K) turn(v[j], k);
+        const int k = k0 + tg * 4 + j * step;
+        if (k < k1) turn(v[j], k);
     }
-    for (int k = tg * 4 + DIG_MAXV * step; k < K; k += step) turn(load_row4<XT>(xr + k), k);
+    for (int k = k0 + tg * 4 + DIG_MAXV * step; k < k1; k += step) turn(load_row4<XT>(xr + k), k);
     PDBG(tid == 0 && blockIdx.x == 0, 2);
 }
 
@@ -248,7 +257,7 @@ struct TcParams {
     int act;                 // RUSTY_CUDA_ACT_SWIGLU_PAIRS: rows 2j, 2j+1 -> y[:, (y_col0 + 2j) / 2] = silu(gate) * up
     int epi_warps;           // 4 or 8 epilogue warps: two per tensor-memory lane quarter split the activation rows between them
     int stages;
-    int red_bytes;           // epilogue staging area: a partial tile (Mpad x 128 x 8 bytes), at least 12 KiB
+    int red_bytes;           // epilogue staging area: 8 rows x 128 x 8 bytes for every four epilogue warps
     uint32_t idesc;
     uint32_t tmem_cols;
     rusty_cuda_dev_status* status;
@@ -273,14 +282,15 @@ __device__ __forceinline__ void split_tile(const TcParams& p, int t, int& wt, in
     }
 }
 
-// Every role of the CTA walks the same segment list.
+// Every role of the CTA walks the same segment list.  PAIR: the two CTAs of a pair walk the same one, and "CTA" in what follows is the pair.
+template <bool PAIR>
 struct Sched {
     const TcParams& p;
+    int c;          // this CTA
     int g, g_end;   // position inside the stream-K space
     int dp_next;    // next whole tile
     int seg_index;
-    __device__ Sched(const TcParams& pp) : p(pp) {
-        const int c = blockIdx.x;
+    __device__ Sched(const TcParams& pp) : p(pp), c(PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x) {
         if (p.sk_ways > 0) {
             // one piece per CTA, cut at the same places in every tile: g walks the piece's k-blocks
             const int lt = c / p.sk_ways, j = c % p.sk_ways;
@@ -308,7 +318,7 @@ struct Sched {
                 s.nseg = last_cta - s.first_cta + 1;
             }
             // head piece (the CTA's run starts inside this tile) -> even slot, tail piece -> odd slot
-            s.slot = 2 * (int)blockIdx.x + ((int)blockIdx.x * p.sk_per_cta >= lt * p.kb_total ? 0 : 1);
+            s.slot = 2 * c + (c * p.sk_per_cta >= lt * p.kb_total ? 0 : 1);
             g += s.kb1 - s.kb0;
             ++seg_index;
             return true;
@@ -320,7 +330,7 @@ struct Sched {
             s.nseg = 1;
             s.slot = 0;
             s.first_cta = 0;
-            dp_next += gridDim.x;
+            dp_next += PAIR ? gridDim.x >> 1 : gridDim.x;
             ++seg_index;
             return true;
         }
@@ -368,19 +378,30 @@ __device__ __forceinline__ void finalize_store4(const TcParams& p, YT* y, const 
     }
 }
 
-// BLOCKS: several row blocks (nblk > 1)
-template <typename YT, bool BLOCKS>
+// A piece's words as they are now.  Volatile: __ldcg is not, and a loop that waits for its result can be taken apart into one load
+// and an endless wait.
+__device__ __forceinline__ ulonglong2 poll_cg(const ulonglong2* p) {
+    ulonglong2 v;
+    asm volatile("ld.global.cg.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
+    return v;
+}
+
+// BLOCKS: several row blocks (nblk > 1).  PAIR: a unit of work is 256 weight rows on a pair of CTAs, 128 each; a CTA brings half of the
+// digit tile, and the tensor cores of both read both halves.
+template <typename YT, bool BLOCKS, bool PAIR>
 __global__ void __launch_bounds__(TC_MAX_THREADS, 1)
 qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                      const __grid_constant__ TcParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // carve: [A stages][B stages][barriers]
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int b_stage_bytes = p.NB * BK;
+    const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
+    const int nb_cta = PAIR ? p.NB / 2 : p.NB;      // digit rows of a stage that this CTA holds
+    const int b_stage_bytes = nb_cta * BK;
     const int a_stage_bytes = p.tpu * A_TILE_BYTES;
     uint8_t* sA = smem;
     uint8_t* sB = smem + (size_t)p.stages * a_stage_bytes;
-    // epilogue staging of a whole tile's folded sums: [Mpad/2][128] x 16 bytes
+    // epilogue staging of eight rows' folded sums for each half of the epilogue warps: [2][4][128] x 16 bytes
     int4* stage_red = reinterpret_cast<int4*>(sB + (size_t)p.stages * b_stage_bytes);
     uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(stage_red) + (size_t)p.red_bytes);
     uint64_t* full = bars;                      // [stages]
@@ -418,17 +439,24 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(&acc_full[a], 1);
-            mbar_init(&acc_empty[a], (uint32_t)p.epi_warps);
+            mbar_init(&acc_empty[a], (uint32_t)(PAIR ? 2 * p.epi_warps : p.epi_warps));
         }
         *abort_flag = 0;
         fence_barrier_init();
     }
-    if (warp == 1) tmem_alloc(tmem_slot, p.tmem_cols);
+    if (warp == 1) {
+        if constexpr (PAIR) tmem_alloc_pair(tmem_slot, p.tmem_cols);
+        else tmem_alloc(tmem_slot, p.tmem_cols);
+    }
     tc_fence_before();
-    __syncthreads();
+    if constexpr (PAIR) cluster_sync_all();   // the other CTA's barriers are counted by this one's copies and arrivals
+    else __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     if (threadIdx.x == 0) DBG(1);
+    // first weight row of unit t that is this CTA's
+    auto unit_row = [&](int t) { return PAIR ? (2 * t + (int)rank) * BM : t * p.bmu; };
+    auto slot_of = [&](int i) { return PAIR ? (size_t)(2 * i + (int)rank) : (size_t)i; };
 
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
@@ -438,22 +466,28 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         uint32_t phase = 0;
         int issued = 0;
         bool ok = true;
-        Sched sched(p);
+        Sched<PAIR> sched(p);
         Segment sg;
+        // PAIR: the even CTA's barrier counts both CTAs' copies (the odd one's may land before it has said how many to expect: the
+        // phase cannot end without that)
+        auto load = [&](void* dst, const CUtensorMap* map, int c0, int c1, int st, uint64_t pol) {
+            if constexpr (PAIR) tma_load_2d_pair(dst, map, c0, c1, mapa_u32(&full[st], 0), pol);
+            else tma_load_2d(dst, map, c0, c1, &full[st], pol);
+        };
         // The weights do not depend on earlier kernels: start streaming them at once.  The digit planes do, so
         // the first ring-full of stages gets its weight tile now and its digit tile after pdl_wait().
         int early = 0;           // stages whose weight tile is already in flight
         auto late_digits = [&]() {   // walks the early stages once more
             pdl_wait();
             DBG1(1);
-            Sched again(p);
+            Sched<PAIR> again(p);
             Segment e;
             int n = 0;
             while (n < early && again.next(e)) {
                 int w_row, x_row;
                 split_tile<BLOCKS>(p, e.t, w_row, x_row);
                 for (int kb = e.kb0; kb < e.kb1 && n < early; ++kb, ++n) {
-                    if (elect_one()) tma_load_2d(sB + (size_t)n * b_stage_bytes, &map_x, kb * BK, x_row * p.NB, &full[n], pol_x);
+                    if (elect_one()) load(sB + (size_t)n * b_stage_bytes, &map_x, kb * BK, x_row * p.NB + (int)rank * nb_cta, n, pol_x);
                     __syncwarp();
                 }
             }
@@ -462,8 +496,8 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         while (ok && sched.next(sg)) {
             int w_row, x_row;
             split_tile<BLOCKS>(p, sg.t, w_row, x_row);
-            w_row *= p.bmu;
-            x_row *= p.NB;
+            w_row = unit_row(w_row);
+            x_row = x_row * p.NB + (int)rank * nb_cta;
             for (int kb = sg.kb0; kb < sg.kb1; ++kb) {
                 const bool ahead = !waited && early < p.stages;
                 if (!ahead) {
@@ -474,9 +508,9 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                     if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, p.status, 1)) { ok = false; break; }
                 }
                 if (elect_one()) {
-                    mbar_expect_tx(&full[stage], (uint32_t)(a_stage_bytes + b_stage_bytes));
-                    tma_load_2d(sA + (size_t)stage * a_stage_bytes, &map_w, kb * BK, w_row, &full[stage], pol_w);
-                    if (!ahead) tma_load_2d(sB + (size_t)stage * b_stage_bytes, &map_x, kb * BK, x_row, &full[stage], pol_x);
+                    if (!PAIR || rank == 0) mbar_expect_tx(&full[stage], (uint32_t)((a_stage_bytes + b_stage_bytes) * (PAIR ? 2 : 1)));
+                    load(sA + (size_t)stage * a_stage_bytes, &map_w, kb * BK, w_row, stage, pol_w);
+                    if (!ahead) load(sB + (size_t)stage * b_stage_bytes, &map_x, kb * BK, x_row, stage, pol_x);
                 }
                 __syncwarp();
                 if (ahead) ++early;
@@ -487,7 +521,12 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         if (!waited) late_digits();   // fewer k-blocks than ring slots
         DBG1(3);
         if (!ok) {
-            // give the copies still in flight a bounded chance to land before the CTA tears down
+            // give the copies still in flight a bounded chance to land before the CTA tears down (PAIR: the odd CTA's are counted
+            // elsewhere, and whether the other's will be issued nobody knows: time it is)
+            if constexpr (PAIR) {
+                const long long t0 = clock64();
+                while (clock64() - t0 < 4000000ll) {}
+            } else
             for (int j = 0; j < p.stages && j < issued; ++j) {
                 const int idx = issued - 1 - j;
                 uint64_t* bar = &full[idx % p.stages];
@@ -501,8 +540,8 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         // the whole warp walks the segments and waits; one elected lane issues
         int stage = 0;
         uint32_t phase = 0;
-        bool ok = true;
-        Sched sched(p);
+        bool ok = !PAIR || rank == 0;        // the even CTA issues for both
+        Sched<PAIR> sched(p);
         Segment sg;
         for (int i = 0; ok && sched.next(sg); ++i) {
             const int ab = i & 1;
@@ -520,12 +559,20 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
 #pragma unroll
                         for (int k4 = 0; k4 < BK / UMMA_K; ++k4) {
                             // advance 32 bytes along K inside the 128-byte swizzle atom: +2 in 16-byte units
-                            umma_i8(d_tmem + (uint32_t)(h * p.NB), da + (uint64_t)(h * (A_TILE_BYTES >> 4) + 2 * k4), db + (uint64_t)(2 * k4), p.idesc,
-                                    (kb > sg.kb0 || k4 > 0) ? 1u : 0u);
+                            if constexpr (PAIR)
+                                umma_i8_pair(d_tmem, da + (uint64_t)(2 * k4), db + (uint64_t)(2 * k4), p.idesc, (kb > sg.kb0 || k4 > 0) ? 1u : 0u);
+                            else
+                                umma_i8(d_tmem + (uint32_t)(h * p.NB), da + (uint64_t)(h * (A_TILE_BYTES >> 4) + 2 * k4), db + (uint64_t)(2 * k4), p.idesc,
+                                        (kb > sg.kb0 || k4 > 0) ? 1u : 0u);
                         }
                     }
-                    umma_commit(&empty[stage]);
-                    if (kb == sg.kb1 - 1) umma_commit(&acc_full[ab]);
+                    if constexpr (PAIR) {
+                        umma_commit_pair(&empty[stage]);
+                        if (kb == sg.kb1 - 1) umma_commit_pair(&acc_full[ab]);
+                    } else {
+                        umma_commit(&empty[stage]);
+                        if (kb == sg.kb1 - 1) umma_commit(&acc_full[ab]);
+                    }
                 }
                 __syncwarp();
                 if (++stage == p.stages) { stage = 0; phase ^= 1u; }
@@ -545,12 +592,13 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         // rows, in units of 8.  With 4 epilogue warps every warp takes them all.
         const int m_split = p.epi_warps == 8 ? ((p.Mpad / 8 + 1) / 2) * 8 : p.Mpad;
         const int m_lo = (warp - 2) < 4 ? 0 : m_split, m_hi = (warp - 2) < 4 ? m_split : p.Mpad;
+        int4* const my_red = stage_red + ((warp - 2) < 4 ? 0 : 4) * BM + r;
         // per-row factors of the pre-pass: once into shared memory (a load from global memory per output costs
         // an L2 round trip each time)
         for (int m = et; m < (BLOCKS ? p.nblk * p.Mpad : p.Mpad); m += EPI_THREADS) s_rowf[m] = __ldcg(p.row_factor + m);
         asm volatile("bar.sync 1, %0;" ::"r"(EPI_THREADS) : "memory");
-        int cut_t[2], cut_j[2], cut_n[2], cut_f[2], n_cut = 0;  // shared tiles this CTA holds a piece of
-        Sched sched(p);
+        int n_cut = 0;                          // shared tiles this CTA holds a piece of, two at most
+        Sched<PAIR> sched(p);
         Segment sg;
         for (int i = 0;; ++i) {
             const bool have = ok && sched.next(sg);
@@ -560,12 +608,15 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             // behind.  No counters, no fences: a word carries its own arrival.  The CTAs of the grid are resident
             // together (one wave) and every piece is written before its holder waits here, so a wait cannot depend
             // on a CTA that has not started.
+            Sched<PAIR> again(p);                // finds them again (an array of them would be in local memory)
             for (int e = 0; ok && e < n_cut && !have; ++e) {
-                const int nseg = cut_n[e], j = cut_j[e], fcta = cut_f[e];
-                const int lt = cut_t[e] - p.dp_tiles;
+                do again.next(sg);
+                while (sg.nseg == 1);            // (a run longer than a tile may hold a whole one first)
+                const int nseg = sg.nseg, fcta = sg.first_cta;
+                const int j = sched.c - fcta, lt = sg.t - p.dp_tiles;
                 int n_base, m_base;
-                split_tile<BLOCKS>(p, cut_t[e], n_base, m_base);
-                n_base *= p.bmu;
+                split_tile<BLOCKS>(p, sg.t, n_base, m_base);
+                n_base = unit_row(n_base);
                 m_base *= p.Mpad;
                 const size_t slot_items = (size_t)p.tpu * (p.Mpad / 2) * BM;   // a slot: [tile of the unit][m / 2][row] x 16 bytes
                 // this CTA's share of the tile's rows, cut in units of two rows so that a (gate, up) pair stays together
@@ -576,16 +627,19 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                 int row = et % rows, mp = et / rows;
                 const int step_row = EPI_THREADS % rows, step_mp = EPI_THREADS / rows;
                 const long long t_begin = clock64();
+                // Two items at a time.  (Four spilled, and code that runs once per launch is paid by the instruction: without the spills
+                // 4096 x 4096 takes 9.4 instead of 11.6 us at 4 rows, 11.2 instead of 12.7 at 32.)
+                constexpr int U = 2;
                 // the loop bounds are the same for every thread: the pair epilogue needs whole warps
-                for (int base = 0; base < items; base += 4 * EPI_THREADS) {
+                for (int base = 0; base < items; base += U * EPI_THREADS) {
                     const int it0 = base + et;
-                    long long s0[4] = {0, 0, 0, 0}, s1[4] = {0, 0, 0, 0};
-                    uint32_t off[4];
-                    int rw[4], mq[4];
-                    bool in[4];
-                    float wsc[4];   // the rows' weight scales: fetched with the pieces, not behind them (the residuals too: spills, slower)
+                    long long s0[U] = {}, s1[U] = {};
+                    uint32_t off[U];
+                    int rw[U], mq[U];
+                    bool in[U];
+                    float wsc[U];   // the rows' weight scales: fetched with the pieces, not behind them (the residuals too: spills, slower)
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
+                    for (int u = 0; u < U; ++u) {
                         rw[u] = lo + row;
                         mq[u] = mp;
                         in[u] = it0 + u * EPI_THREADS < items;
@@ -599,26 +653,27 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                         }
                     }
 #pragma unroll 1
-                    for (int q0 = 0; q0 < nseg; q0 += 4) {   // four pieces x four items: sixteen loads in flight per trip
+                    for (int q0 = 0; q0 < nseg; q0 += 4) {   // four pieces x two items: eight loads in flight per trip
                         ulonglong2* slot[4];
-                        ulonglong2 v[4][4];
+                        ulonglong2 v[4][U];
 #pragma unroll
                         for (int w = 0; w < 4; ++w) {
                             // piece q of the tile sits with CTA fcta + q: its head piece (even slot) if that CTA's run
                             // of k-blocks starts inside this tile, else its tail piece (odd slot)
                             const int c = fcta + min(q0 + w, nseg - 1);
-                            slot[w] = p.part + (size_t)(2 * c + (c * p.sk_per_cta >= lt * p.kb_total ? 0 : 1)) * slot_items;
-#pragma unroll
-                            for (int u = 0; u < 4; ++u)
-                                v[w][u] = (in[u] && q0 + w < nseg) ? __ldcg(slot[w] + off[u]) : make_ulonglong2(1ull, 1ull);
+                            slot[w] = p.part + slot_of(2 * c + (c * p.sk_per_cta >= lt * p.kb_total ? 0 : 1)) * slot_items;
                         }
-                        // every word carries its own "valid" tag in bit 0: one combined test for the common case ...
                         unsigned long long allv = 1ull;
 #pragma unroll
                         for (int w = 0; w < 4; ++w)
 #pragma unroll
-                            for (int u = 0; u < 4; ++u) allv &= v[w][u].x & v[w][u].y;
-                        // ... and a rolled re-poll of the whole batch while some piece has not landed yet
+                            for (int u = 0; u < U; ++u) v[w][u] = (in[u] && q0 + w < nseg) ? poll_cg(slot[w] + off[u]) : make_ulonglong2(1ull, 1ull);
+                        // every word carries its own "valid" tag in bit 0: one combined test for the common case ...
+#pragma unroll
+                        for (int w = 0; w < 4; ++w)
+#pragma unroll
+                            for (int u = 0; u < U; ++u) allv &= v[w][u].x & v[w][u].y;
+                        // ... and the batch again while some piece has not landed yet
                         while (!(allv & 1ull)) {
                             if (*abort_flag || clock64() - t_begin > WAIT_LIMIT_CYCLES) {
                                 *abort_flag = 1;
@@ -630,15 +685,15 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
 #pragma unroll
                             for (int w = 0; w < 4; ++w)
 #pragma unroll
-                                for (int u = 0; u < 4; ++u) {
-                                    if (in[u] && q0 + w < nseg) v[w][u] = __ldcg(slot[w] + off[u]);
+                                for (int u = 0; u < U; ++u) {
+                                    if (in[u] && q0 + w < nseg) v[w][u] = poll_cg(slot[w] + off[u]);
                                     allv &= v[w][u].x & v[w][u].y;
                                 }
                         }
 #pragma unroll
                         for (int w = 0; w < 4; ++w) {
 #pragma unroll
-                            for (int u = 0; u < 4; ++u) {
+                            for (int u = 0; u < U; ++u) {
                                 if (in[u] && q0 + w < nseg) __stcg(slot[w] + off[u], make_ulonglong2(0ull, 0ull));
                                 s0[u] += (long long)v[w][u].x >> 1;   // arithmetic shift: drops the tag, keeps the sign
                                 s1[u] += (long long)v[w][u].y >> 1;
@@ -649,17 +704,14 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                         ok = false;
                         break;
                     }
-#pragma unroll
-                    for (int u = 0; u < 4; u += 2) {  // two items = four outputs per trip
-                        const bool v0 = in[u] && n_base + rw[u] < p.N, v1 = in[u + 1] && n_base + rw[u + 1] < p.N;
-                        const int n0 = n_base + rw[u], n1 = n_base + rw[u + 1];
-                        const int m0 = m_base + (v0 ? 2 * mq[u] : 0), m1 = m_base + (v1 ? 2 * mq[u + 1] : 0);
-                        const long long a4[4] = {s0[u], s1[u], s0[u + 1], s1[u + 1]};
-                        const int n4[4] = {n0, n0, n1, n1}, m4[4] = {m0, m0 + 1, m1, m1 + 1};
-                        const float s4[4] = {wsc[u], wsc[u], wsc[u + 1], wsc[u + 1]};
-                        const bool l4[4] = {v0 && m0 < p.M, v0 && m0 + 1 < p.M, v1 && m1 < p.M, v1 && m1 + 1 < p.M};
-                        finalize_store4<YT>(p, y, n4, m4, a4, s4, s_rowf, po, l4);
-                    }
+                    const bool v0 = in[0] && n_base + rw[0] < p.N, v1 = in[1] && n_base + rw[1] < p.N;
+                    const int n0 = n_base + rw[0], n1 = n_base + rw[1];
+                    const int m0 = m_base + (v0 ? 2 * mq[0] : 0), m1 = m_base + (v1 ? 2 * mq[1] : 0);
+                    const long long a4[4] = {s0[0], s1[0], s0[1], s1[1]};
+                    const int n4[4] = {n0, n0, n1, n1}, m4[4] = {m0, m0 + 1, m1, m1 + 1};
+                    const float s4[4] = {wsc[0], wsc[0], wsc[1], wsc[1]};
+                    const bool l4[4] = {v0 && m0 < p.M, v0 && m0 + 1 < p.M, v1 && m1 < p.M, v1 && m1 + 1 < p.M};
+                    finalize_store4<YT>(p, y, n4, m4, a4, s4, s_rowf, po, l4);
                 }
                 if (threadIdx.x == 64) DBG(11);
             }
@@ -670,21 +722,24 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             tc_fence_after();
             if (threadIdx.x == 64) DBG(6 + 4 * (i & 1));
             {
-                // Fold the digit planes into one exact 64-bit integer per output.  A whole tile is staged in shared
-                // memory ([m/2][row] x 16 bytes) and converted from there in a rolled loop (unrolled register code
-                // that runs once per tile costs an instruction fetch per line and was twice as slow); a piece of a
-                // shared tile goes straight into this CTA's slot in global memory, every word tagged valid.
+                // Fold the digit planes into one exact 64-bit integer per output.  A whole tile's are staged in shared
+                // memory, eight activation rows at a time (all at once they took the room of ring stages), and converted
+                // from there in a rolled loop (unrolled register code that runs once per tile costs an instruction fetch
+                // per line and was twice as slow); a piece of a shared tile goes straight into this CTA's slot in
+                // global memory, every word tagged valid.
                 const bool whole = sg.nseg == 1;
                 int n_base, m_base;
                 split_tile<BLOCKS>(p, sg.t, n_base, m_base);
-                n_base *= p.bmu;
+                n_base = unit_row(n_base);
                 m_base *= p.Mpad;
                 for (int ht = 0; ht < p.tpu; ++ht) {   // the unit's tiles, one accumulator each
                     const int n = n_base + ht * BM + r;
                     const bool row_ok = n < p.N;
+                    const float sc = whole && row_ok ? __ldg(p.scales + n) : 0.0f;
                     const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)((ab * p.tpu + ht) * p.NB);
-                    ulonglong2* slot = p.part + ((size_t)sg.slot * p.tpu + ht) * (p.Mpad / 2) * BM;
-                    for (int m0 = m_lo; m0 < m_hi; m0 += 8) {
+                    ulonglong2* slot = p.part + (slot_of(sg.slot) * p.tpu + ht) * (p.Mpad / 2) * BM;
+                    // sums of eight activation rows, two at a time
+                    auto fold = [&](int m0, auto&& put) {
                         int32_t c[4][8];
 #pragma unroll
                         for (int d = 0; d < 4; ++d)
@@ -700,39 +755,45 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                                     a1 = a1 * 256 + c[d][2 * h + 1];
                                 }
                             if (!row_ok) a0 = a1 = 0;
-                            if (whole) {
-                                int4 v;
-                                v.x = (int)(a0 & 0xffffffffll);
-                                v.y = (int)(a0 >> 32);
-                                v.z = (int)(a1 & 0xffffffffll);
-                                v.w = (int)(a1 >> 32);
-                                stage_red[(size_t)(m0 / 2 + h) * BM + r] = v;
-                            } else {   // |sum| < 2^56: room for the tag; two 64-bit words, each stored whole
+                            put(h, a0, a1);
+                        }
+                    };
+                    if (!whole) {   // |sum| < 2^56: room for the tag; two 64-bit words, each stored whole
+#pragma unroll 1
+                        for (int m0 = m_lo; m0 < m_hi; m0 += 8)
+                            fold(m0, [&](int h, long long a0, long long a1) {
                                 __stcg(slot + (size_t)(m0 / 2 + h) * BM + r,
                                        make_ulonglong2((unsigned long long)((a0 << 1) | 1), (unsigned long long)((a1 << 1) | 1)));
+                            });
+                    } else {
+#pragma unroll 1
+                        for (int m0 = m_lo; m0 < m_hi; m0 += 8) {
+                            fold(m0, [&](int h, long long a0, long long a1) {
+                                my_red[h * BM] = make_int4((int)(a0 & 0xffffffffll), (int)(a0 >> 32), (int)(a1 & 0xffffffffll), (int)(a1 >> 32));
+                            });
+                            // every thread reads back only what it staged itself: no barrier needed
+#pragma unroll 1
+                            for (int m = m0; m < min(m0 + 8, p.M - m_base); m += 4) {
+                                const int4* from = my_red + (m - m0) / 2 * BM;
+                                const longlong2 t0 = *reinterpret_cast<const longlong2*>(from);
+                                const longlong2 t1 = *reinterpret_cast<const longlong2*>(from + BM);
+                                const long long a4[4] = {t0.x, t0.y, t1.x, t1.y};
+                                const int mg = m_base + m;
+                                const int n4[4] = {n, n, n, n}, m4[4] = {mg, mg + 1, mg + 2, mg + 3};
+                                const float s4[4] = {sc, sc, sc, sc};
+                                const bool l4[4] = {row_ok, row_ok && mg + 1 < p.M, row_ok && mg + 2 < p.M, row_ok && mg + 3 < p.M};
+                                finalize_store4<YT>(p, y, n4, m4, a4, s4, s_rowf, po, l4);
                             }
                         }
                     }
                     if (ht == p.tpu - 1) {   // the accumulators of this unit have been read
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(&acc_empty[ab]);
-                        if (threadIdx.x == 64) DBG(7 + 4 * (i & 1));
-                    }
-                    if (whole) {
-                        // every thread reads back only what it staged itself: no barrier needed
-                        const float sc = row_ok ? __ldg(p.scales + n) : 0.0f;
-#pragma unroll 1
-                        for (int m = m_lo; m < min(m_hi, p.M - m_base); m += 4) {  // in units of 8: the staged rows m .. m+3 exist
-                            const longlong2 t0 = *reinterpret_cast<const longlong2*>(&stage_red[(size_t)(m >> 1) * BM + r]);
-                            const longlong2 t1 = *reinterpret_cast<const longlong2*>(&stage_red[(size_t)((m >> 1) + 1) * BM + r]);
-                            const long long a4[4] = {t0.x, t0.y, t1.x, t1.y};
-                            const int mg = m_base + m;
-                            const int n4[4] = {n, n, n, n}, m4[4] = {mg, mg + 1, mg + 2, mg + 3};
-                            const float s4[4] = {sc, sc, sc, sc};
-                            const bool l4[4] = {row_ok, row_ok && mg + 1 < p.M, row_ok && mg + 2 < p.M, row_ok && mg + 3 < p.M};
-                            finalize_store4<YT>(p, y, n4, m4, a4, s4, s_rowf, po, l4);
+                        if (lane == 0) {
+                            if constexpr (PAIR) mbar_arrive_cluster(mapa_u32(&acc_empty[ab], 0));
+                            else mbar_arrive(&acc_empty[ab]);
                         }
+                        if (threadIdx.x == 64) DBG(7 + 4 * (i & 1));
                     }
                 }
                 if (whole) {
@@ -740,28 +801,21 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                     continue;
                 }
                 // The conversion is shared between the CTAs that hold the tile's pieces and is done after the CTA's
-                // last segment (above): remember the tile and which piece this was.
-                if (n_cut < 2) {
-                    cut_t[n_cut] = sg.t;
-                    cut_j[n_cut] = (int)blockIdx.x - sg.first_cta;
-                    cut_n[n_cut] = sg.nseg;
-                    cut_f[n_cut] = sg.first_cta;
-                    ++n_cut;
-                } else {
-                    ok = false;  // cannot happen: a run of k-blocks starts and ends inside at most two shared tiles
-                    if (threadIdx.x == 64 && atomicExch(&p.status->timeout_flag, 1u) == 0u) p.status->timeout_where = 7;
-                }
+                // last segment (above).
+                ++n_cut;
                 if (threadIdx.x == 64) DBG(8 + 4 * (i & 1));
             }
         }
     }
 
     tc_fence_before();
-    __syncthreads();
+    if constexpr (PAIR) cluster_sync_all();   // neither CTA leaves while the other's MMAs, copies or arrivals may reach it
+    else __syncthreads();
     if (threadIdx.x == 0) DBG(14);
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, p.tmem_cols);
+        if constexpr (PAIR) tmem_dealloc_pair(tmem_base, p.tmem_cols);
+        else tmem_dealloc(tmem_base, p.tmem_cols);
     }
     if (threadIdx.x == 0) DBG(15);
 }
@@ -859,19 +913,21 @@ cudaError_t launch_digitize(cudaStream_t stream, const void* x, int8_t* xq, floa
                             const PeerPush& push, long long* dbg, const NormArgs* norm = nullptr) {
     // Mpad is a multiple of 8 and at most 64: one row per block up to 32 rows, two beyond; several row blocks (a prompt, where
     // the GEMM is long): one row per block
+    // Long rows: one a block from 8192 activations on (two a block left 256 threads to reload what their registers do not hold: a
+    // call of 64 x 14336 x 4096 29.7 -> 26.1 us), and beyond 16384 a cluster of two blocks a row (64 x 28672 x 8192 67.0 -> 58.9, of
+    // which one row a block gives 60.9; at 32 rows 53.6 -> 51.8; four blocks: no gain).  Between ranks a block of this kernel is a
+    // meeting point, of which there are 64: one block a row.
     int R = 1;
-    while (nblk == 1 && (Mpad / R > DIG_MAX_BLOCKS || Mpad % R != 0)) R <<= 1;   // R in {1, 2}: the rows' thread groups share a block evenly
-    const int blocks = Mpad / R;
-    if constexpr (std::is_same<XT, float>::value) {
-        if (norm) {
-            if (D == 4)
-                return launch_pdl(digitize_x_kernel<XT, 4, true>, dim3(blocks, nblk), dim3(DIG_THREADS), 0, stream, (const XT*)x, xq, inv_s, M, Mpad, K, R, push, *norm, dbg);
-            return launch_pdl(digitize_x_kernel<XT, 3, true>, dim3(blocks, nblk), dim3(DIG_THREADS), 0, stream, (const XT*)x, xq, inv_s, M, Mpad, K, R, push, *norm, dbg);
-        }
-    }
-    if (D == 4)
-        return launch_pdl(digitize_x_kernel<XT, 4, false>, dim3(blocks, nblk), dim3(DIG_THREADS), 0, stream, (const XT*)x, xq, inv_s, M, Mpad, K, R, push, NormArgs{}, dbg);
-    return launch_pdl(digitize_x_kernel<XT, 3, false>, dim3(blocks, nblk), dim3(DIG_THREADS), 0, stream, (const XT*)x, xq, inv_s, M, Mpad, K, R, push, NormArgs{}, dbg);
+    const int cs = K > DIG_MAXV * 4 * DIG_THREADS && push.nranks <= 1 ? 2 : 1;
+    while (nblk == 1 && K < 8192 && (Mpad / R > DIG_MAX_BLOCKS || Mpad % R != 0)) R <<= 1;   // R in {1, 2}: the rows' thread groups share a block evenly
+    const dim3 grid(Mpad / R * cs, nblk);
+    auto go = [&](auto kern, const NormArgs& n) {
+        return launch_pdl_cluster(kern, grid, dim3(DIG_THREADS), (unsigned)cs, 0, stream, (const XT*)x, xq, inv_s, M, Mpad, K, R, push, n, dbg);
+    };
+    if constexpr (std::is_same<XT, float>::value)
+        if (norm) return D == 4 ? go(digitize_x_kernel<XT, 4, true, false>, *norm) : go(digitize_x_kernel<XT, 3, true, false>, *norm);   // (K <= 16384)
+    if (cs == 2) return D == 4 ? go(digitize_x_kernel<XT, 4, false, true>, NormArgs{}) : go(digitize_x_kernel<XT, 3, false, true>, NormArgs{});
+    return D == 4 ? go(digitize_x_kernel<XT, 4, false, false>, NormArgs{}) : go(digitize_x_kernel<XT, 3, false, false>, NormArgs{});
 }
 
 }  // namespace
@@ -1025,31 +1081,44 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
     p.kb_total = (p.K + BK - 1) / BK;
     TcSchedule sc{};
     p.tpu = 1;
-    if (two_tiles > 0 && 4 * NB <= 512 && a.N > (uint32_t)BM) {
+    // A pair of CTAs per unit of 256 rows halves the digit bytes a CTA pulls from L2, where they are more than the weights' (an SM
+    // takes in some 46 bytes a clock: 64 rows, a weight tile of 16 KB and a digit tile of 32, streamed at 4.4 TB/s).  It costs about 1
+    // us a launch (clusters are placed later and leave together), so only where units are taken whole or their pieces are long.
+    // One CTA / pairs, us: 32 x 4096 x 28672 31.3 / 28.9, 64 x 8192 x 57344 124 / 110, 64 x 28672 x 8192 (pieces of 112 k-blocks)
+    // 71.7 / 67.0, 391 x 4096 x 28672 159 / 127; short pieces: 64 x 4096 x 4096 15.4 / 16.8, 32 x 4096 x 4096 12.7 / 13.7.
+    bool pair = NB >= 128 && NB % 32 == 0 && a.N > (uint32_t)BM && ctx->sm_count >= 4;
+    if (pair) {
+        const int units = (p.N + 2 * BM - 1) / (2 * BM) * nblk;
+        plan_tc_schedule(units, p.kb_total, ctx->sm_count / 2, dp_percent, WS_ACC_BYTES / ((size_t)2 * Mpad * BM * 8), &sc);
+        pair = sc.sk_tiles == 0 || sc.dp_tiles > 0 || (NB > 192 && sc.sk_per_cta >= 32);
+    }
+    const int group = pair ? 2 : 1;      // CTAs that work on one unit
+    if (!pair && two_tiles > 0 && 4 * NB <= 512 && a.N > (uint32_t)BM) {
         const int units = (p.N + 2 * BM - 1) / (2 * BM) * nblk;
         plan_tc_schedule(units, p.kb_total, ctx->sm_count, dp_percent, WS_ACC_BYTES / ((size_t)2 * Mpad * BM * 8), &sc);
         if (two_tiles >= 2 || sc.sk_tiles == 0) p.tpu = 2;
     }
     p.bmu = p.tpu * BM;
-    p.tiles = (p.N + p.bmu - 1) / p.bmu * nblk;
-    int sched_sms = ctx->sm_count;
+    p.tiles = (p.N + group * p.bmu - 1) / (group * p.bmu) * nblk;
+    int sched_sms = ctx->sm_count / group;
+    const size_t slots_cap = WS_ACC_BYTES / ((size_t)group * p.tpu * Mpad * BM * 8);
     {   // tuning aid: schedule as if the GPU had fewer SMs
         static const int sms_env = getenv("RUSTY_TC_SMS") ? atoi(getenv("RUSTY_TC_SMS")) : 0;
         if (sms_env > 0 && sms_env < sched_sms) sched_sms = sms_env;
     }
-    plan_tc_schedule(p.tiles, p.kb_total, sched_sms, dp_percent, WS_ACC_BYTES / ((size_t)p.tpu * Mpad * BM * 8), &sc);
+    plan_tc_schedule(p.tiles, p.kb_total, sched_sms, dp_percent, slots_cap, &sc);
     // A GEMM CTA and a pre-pass block do not fit one SM together (registers), and the NEXT pair's pre-pass blocks are
     // resident (two per SM, up to 16 SMs) while this GEMM's CTAs are placed.  A short launch whose every tile is cut
     // (fewer tiles than SMs) and whose grid leaves those SMs no room gets its last CTAs placed only after the pre-pass
     // has finished, 2-5 us late: plan it for 16 SMs fewer (q|k|v 6144 x 4096: 144 -> 96 CTAs, 18.2 -> 16.8 us).
     // RUSTY_TC_ROOM=0 turns the rule off (tuning aid).
     static const bool leave_room = !(getenv("RUSTY_TC_ROOM") && atoi(getenv("RUSTY_TC_ROOM")) == 0);
-    if (leave_room && sc.dp_tiles == 0 && sc.grid > sched_sms - 16 && sched_sms > 32) {
+    if (leave_room && sc.dp_tiles == 0 && sc.grid > sched_sms - 16 / group && sched_sms > 32 / group) {
         TcSchedule alt{};
-        plan_tc_schedule(p.tiles, p.kb_total, sched_sms - 16, dp_percent, WS_ACC_BYTES / ((size_t)p.tpu * Mpad * BM * 8), &alt);
+        plan_tc_schedule(p.tiles, p.kb_total, sched_sms - 16 / group, dp_percent, slots_cap, &alt);
         if (alt.dp_tiles == 0) sc = alt;
     }
-    int grid = sc.grid;
+    const int grid = sc.grid * group;
     p.dp_tiles = sc.dp_tiles;
     p.sk_tiles = sc.sk_tiles;
     p.sk_per_cta = sc.sk_per_cta;
@@ -1069,19 +1138,19 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
     p.dbg = dbg;
     p.push = push;
     // int8 x int8 -> int32, both K-major: c_format=S32(2)@4, a_format=INT8(1)@7, b_format=INT8(1)@10, N>>3 @17, M>>4 @24
-    p.idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NB >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    p.idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NB >> 3) << 17) | ((uint32_t)(group * BM >> 4) << 24);
     uint32_t cols = 32;
     while (cols < (uint32_t)(2 * p.tpu * NB)) cols <<= 1;   // two sets of accumulators: the epilogue of one unit overlaps the next
     p.tmem_cols = cols;
-    const int a_stage = p.tpu * A_TILE_BYTES, b_stage = NB * BK;
+    const int a_stage = p.tpu * A_TILE_BYTES, b_stage = NB / group * BK;
     // Half of the SM's shared memory at most for narrow batches, so that the next kernel's CTA can move in beside this
     // one and prefetch its weights while this one drains (RUSTY_TC_FULL_SMEM=1: take it all, 8 stages).
     static const bool full_smem = getenv("RUSTY_TC_FULL_SMEM") != nullptr;
     size_t budget = ctx->smem_optin > 4096 ? ctx->smem_optin - 4096 : 0;
     if (!full_smem && NB <= 32 && 4 * (size_t)a_stage + 4096 <= budget / 2)
         budget = budget / 2 - 1024;  // narrow batches: leave room for the next kernel's CTA on the SM
-    // epilogue staging of one whole 128-row tile (its folded sums); launches without whole tiles need none
-    const size_t red_bytes = p.dp_tiles > 0 ? (size_t)Mpad * 8 * BM : 0;
+    // epilogue staging of whole tiles' sums, eight rows at a time; launches without whole tiles need none
+    const size_t red_bytes = p.dp_tiles > 0 ? (size_t)(p.epi_warps / 4) * 8 * 8 * BM : 0;
     const size_t rowf_bytes = (size_t)nblk * Mpad * 4;
     int stages = budget > red_bytes + rowf_bytes + 2048 ? (int)((budget - 1024 - 512 - red_bytes - rowf_bytes) / (size_t)(a_stage + b_stage)) : 0;
     if (stages > 8) stages = 8;
@@ -1092,18 +1161,24 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
 
     CUtensorMap map_w, map_x;
     if (!make_map_u8(&map_w, a.w, a.N, a.K, (uint32_t)p.bmu) ||
-        !make_map_u8(&map_x, xq, (uint64_t)D * Mpad * nblk, a.K, (uint32_t)NB))
+        !make_map_u8(&map_x, xq, (uint64_t)D * Mpad * nblk, a.K, (uint32_t)(NB / group)))
         return fail(ctx, RUSTY_CUDA_ERR_KERNEL_EXECUTION, "tensor-core path: cuTensorMapEncodeTiled failed");
 
     const bool yb = a.y_dtype == RUSTY_CUDA_BF16;
 
-    auto kern = nblk > 1 ? (yb ? qlinear_i8_tc_kernel<__nv_bfloat16, true> : qlinear_i8_tc_kernel<float, true>)
-                         : (yb ? qlinear_i8_tc_kernel<__nv_bfloat16, false> : qlinear_i8_tc_kernel<float, false>);
+    auto pick = [&](auto blocks, auto paired) {
+        constexpr bool B = decltype(blocks)::value, P = decltype(paired)::value;
+        return yb ? qlinear_i8_tc_kernel<__nv_bfloat16, B, P> : qlinear_i8_tc_kernel<float, B, P>;
+    };
+    using std::true_type;
+    using std::false_type;
+    auto kern = nblk > 1 ? (pair ? pick(true_type{}, true_type{}) : pick(true_type{}, false_type{}))
+                         : (pair ? pick(false_type{}, true_type{}) : pick(false_type{}, false_type{}));
     {
         cudaError_t e = ensure_dynamic_smem((const void*)kern, ctx->device, smem);
         if (e != cudaSuccess) return check_cuda(ctx, e, "qlinear_i8_tc: cudaFuncSetAttribute");
     }
-    le = launch_pdl(kern, dim3(grid), dim3(64 + 32 * p.epi_warps), smem, ctx->stream, map_w, map_x, p);
+    le = launch_pdl_cluster(kern, dim3(grid), dim3(64 + 32 * p.epi_warps), (unsigned)group, smem, ctx->stream, map_w, map_x, p);
     if (le != cudaSuccess) return check_cuda(ctx, le, "qlinear_i8_tc");
     return after_launch(ctx, "qlinear_i8_tc");
 }
@@ -1292,7 +1367,7 @@ extern "C" RUSTY_CUDA_API int rusty_cuda_qlinear_i8_forward_static(const void* w
     CUtensorMap map_w, map_x;
     if (!make_map_u8(&map_w, w_i8, N, K, BM) || !make_map_u8(&map_x, xq, (uint64_t)D * Mpad, K, (uint32_t)NB))
         return fail(nullptr, RUSTY_CUDA_ERR_KERNEL_EXECUTION, "qlinear_i8_forward_static: cuTensorMapEncodeTiled failed");
-    auto kern = qlinear_i8_tc_kernel<float, false>;
+    auto kern = qlinear_i8_tc_kernel<float, false, false>;
     // Raise the kernel's dynamic shared-memory limit to the device maximum: enough for this launch and never
     // below what another entry point has asked for.
     cudaFuncAttributes fa;

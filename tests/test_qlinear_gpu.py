@@ -633,6 +633,21 @@ def test_f32_prompts_in_row_blocks(ctx, engine, M, K, N):
         assert rel_err_rows(y.read(), g * u / (1.0 + np.exp(-np.maximum(g, -80.0)))) <= TOL_FP32
 
 
+@pytest.mark.parametrize("M,K,N,xdt", [(25, 144, 19237, "f32"), (32, 1040, 37889, "f32"), (64, 4112, 515, "f32"), (64, 16400, 385, "f32"), (7, 20000, 129, "f32"),
+                                       (40, 9232, 260, "f32"), (64, 8208, 2100, "f32"), (64, 272, 18950, "bf16"), (130, 400, 9500, "f32")])
+def test_pairs_of_ctas_and_long_rows(ctx, engine, M, K, N, xdt):
+    """Units of 256 weight rows on two CTAs (whole ones, whole ones and cut ones, long pieces; a last unit of one half or less) and
+    rows of activations cut over one block or two, against float64: four digit planes and two roundings leave 2e-6 of a row's
+    largest output at most, three planes 2e-5; twice the same bits."""
+    x, q, s = sym_row_linear(M + K + N, M, K, N)
+    bf = xdt == "bf16"
+    xe = bf16_bits_to_f32(f32_to_bf16_bits(x)).reshape(M, K) if bf else x
+    ql = QLinear.from_host(ctx, q, s)
+    got = _forward(ctx, engine, ql, x, x_dtype=DType.BF16 if bf else DType.FP32)
+    assert rel_err_rows(got, xe.astype(np.float64) @ (q * s[:, None].astype(np.float64)).T) <= (2e-5 if bf else 2e-6)
+    assert_bits_equal(_forward(ctx, engine, ql, x, x_dtype=DType.BF16 if bf else DType.FP32), got)
+
+
 @pytest.mark.parametrize("M,K,N", [(512, 4096, 11008), (78, 4096, 4096), (300, 2048, 6144), (244, 14336, 1024), (600, 1024, 9472)])
 def test_prefill_same_bits_on_every_run(ctx, engine, M, K, N):
     """Whole tiles, equal pieces, runs of stages and pieces in front of whole tiles: exact enough for f32 sums, and the same
