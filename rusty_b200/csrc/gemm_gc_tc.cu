@@ -34,11 +34,9 @@
 // A K range per CTA of a cluster (1, 2 or 4) where there are too few groups; their int64 sums meet in distributed shared memory.
 //
 // What bounds it: few rows, the weight stream and the fixed part of a launch; 4096 x 4096, per call in a graph: 1 row 8.2 us, 4 rows
-// 10.5, 8 rows 12.8, 13 rows 12.2, 32 rows 17.0, 64 rows 26.5 (a GEMV kernel with a pair of rows per CTA: 4 rows 13.2, 32 rows 58.6);
-// 12288 x 2112, whose last stage is half empty (rows padded at create), 1 row 11.1 us, 64 rows 36.5 (on CUDA cores 15.5 and 600).
-// Many rows: 512 x 4096 x 4096 takes 113 us and is at the limit of no unit (ncu: issue slots 46 %, the data pipe of shared memory
-// and L1 52 %, ALU 31 %, tensor cores 18 %); a converter waits for x from L2 (6 % of its loads hit L1) and for its A buffer, and
-// the 512 CTAs are 1.7 waves of the 296 that fit.
+// 10.5, 8 rows 12.8, 13 rows 12.4, 32 rows 16.3 (a GEMV kernel with a pair of rows per CTA: 4 rows 13.2, 32 rows 58.6);
+// 12288 x 2112, whose last stage is half empty (rows padded at create), 1 row 11.1 us (on CUDA cores 15.5).
+// Beyond 32 rows see the kernel for them, below.
 #include <cooperative_groups.h>
 
 #include <climits>
@@ -68,10 +66,10 @@ constexpr int MAX_STAGES = 8;
 // The A operand of a stage, 128 rows of 128 bytes per row block.  A CTA of few rows fills the first 32 RPW rows only, and its
 // buffers lie that close together: the MMA then multiplies what follows (other buffers, the ring) into rows nobody reads.
 constexpr int A_BYTES = 32 * 1024;
-template <int RB, int RPW>
-constexpr int A_PITCH = RB == 2 ? 32 * 1024 : RPW * 4096;
-template <int RB, int RPW>
-constexpr int A_BUFS = RB == 2 ? 2 : 8 / RPW;
+template <int RPW>
+constexpr int A_PITCH = RPW * 4096;
+template <int RPW>
+constexpr int A_BUFS = 8 / RPW;
 
 struct GcParams {
     const float* scales;         // [N/64][K]
@@ -134,33 +132,61 @@ __device__ __forceinline__ int unit_exponent(uint32_t bits) {
     return min(157 - (int)(bits >> 23), 127);
 }
 
-// XT: type of the caller's x (RPW = 1 reads it as it is).  RB: row blocks of 32 (1 or 2); RPW: rows per converter warp (1, 2, 4 or 8;
-// RB = 2 has 8).  MEET (RPW = 1): the cluster's CTAs share the look for the largest products (an instance of its own: the code of
+// What the outputs of a row and group share: its unit 2^-e (NaN: poisoned) and what r adds to the sums, from the sums with r's bytes and
+// ones.
+__device__ __forceinline__ double2 row_terms(const long long (&ext)[RD + 1], const int4& rsum, int runit, int e, int K) {
+    // sum_k q r: the offsets off the planes, then r's own 2^31 off its top byte
+    const long long sq = ext[RD] - ((long long)K << 31);
+    const double top = (double)(ext[0] - ((long long)rsum.x << 31) - 128 * sq);
+    const double rest = (double)(ext[1] - ((long long)rsum.y << 31)) * 65536.0 + (double)(ext[2] - ((long long)rsum.z << 31)) * 256.0 +
+                        (double)(ext[3] - ((long long)rsum.w << 31));
+    const double r_unit = runit == INT_MIN ? 0.0 : __longlong_as_double((long long)(1023 - runit) << 52);
+    // 2^-e as a double from its exponent field; the sum is exact up to here
+    return make_double2((top * 16777216.0 + rest) * r_unit, e == INT_MIN ? (double)__int_as_float(0x7fc00000) : __longlong_as_double((long long)(1023 - e) << 52));
+}
+__device__ __forceinline__ void store_output(const GcParams& p, float f, size_t at) {
+    auto put = [&](auto* y0, auto value) {
+        auto* dst = y0 + at;
+        *dst = value;
+#pragma unroll
+        for (int r = 0; r < PEER_MAX_RANKS - 1; ++r)   // the same element of every other rank's y, over NVLink
+            if (r < p.n_peers) *reinterpret_cast<decltype(dst)>(reinterpret_cast<char*>(dst) + p.peer_delta[r]) = value;
+    };
+    if (p.y_bf16) {
+        if (p.residual) f += __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.residual)[at]);
+        put(reinterpret_cast<__nv_bfloat16*>(p.y), __float2bfloat16_rn(f));
+    } else {
+        if (p.residual) f = __fadd_rn(reinterpret_cast<const float*>(p.residual)[at], f);
+        put(reinterpret_cast<float*>(p.y), f);
+    }
+}
+
+// Up to 32 rows.  XT: type of the caller's x (RPW = 1 reads it as it is).  RPW: rows per converter warp (1, 2 or 4).  MEET (RPW = 1): the cluster's CTAs share the look for the largest products (an instance of its own: the code of
 // both in one cost calls that do not meet 0.3 us in instruction fetches).
-template <typename XT, int RB, int RPW, bool MEET = false>
+template <typename XT, int RPW, bool MEET = false>
 __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ GcParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    constexpr int PITCH = A_PITCH<RB, RPW>, BUFS = A_BUFS<RB, RPW>, TCOLS = RB == 2 ? 256 : 128;
+    constexpr int PITCH = A_PITCH<RPW>, BUFS = A_BUFS<RPW>, TCOLS = 128;
     uint8_t* sA = smem;                                              // [BUFS] x PITCH
-    uint8_t* sIn = smem + RB * A_BYTES;                              // [stages][STAGE_BYTES]
+    uint8_t* sIn = smem + A_BYTES;                                   // [stages][STAGE_BYTES]
     uint8_t* sSc = sIn + (size_t)p.stages * STAGE_BYTES;             // [stages][S_BYTES]
     uint64_t* in_full = reinterpret_cast<uint64_t*>(sSc + (size_t)p.stages * S_BYTES);
     uint64_t* in_empty = in_full + MAX_STAGES;
     uint64_t* a_full = in_empty + MAX_STAGES;
     uint64_t* a_empty = a_full + MAX_STAGES;
     uint64_t* d_full = a_empty + MAX_STAGES;
-    double2* s_bias = reinterpret_cast<double2*>(d_full + 2);        // [RB * 32]: a group without r: this K range's bias term, in two parts
-    int* s_exp = reinterpret_cast<int*>(s_bias + RB * 32);           // [RB * 32]: e of a row, or INT_MIN: poisoned
-    uint32_t* s_top = reinterpret_cast<uint32_t*>(s_exp + RB * 32);  // [RB * 32]: largest |a| of a row (bits, its exponent at least)
-    float* s_smax = reinterpret_cast<float*>(s_top + RB * 32);       // [K / 128]
+    double2* s_bias = reinterpret_cast<double2*>(d_full + 2);        // [32]: a group without r: this K range's bias term, in two parts
+    int* s_exp = reinterpret_cast<int*>(s_bias + 32);           // [32]: e of a row, or INT_MIN: poisoned
+    uint32_t* s_top = reinterpret_cast<uint32_t*>(s_exp + 32);  // [32]: largest |a| of a row (bits, its exponent at least)
+    float* s_smax = reinterpret_cast<float*>(s_top + 32);       // [K / 128]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_smax + p.nst);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = warp_id(), lane = threadIdx.x & 31;
     const int g = blockIdx.y;
-    const int way = (int)blockIdx.x % p.ways, m0 = ((int)blockIdx.x / p.ways) * (RB * 32);
-    const int rows = min(RB * 32, p.M - m0);
+    const int way = (int)blockIdx.x % p.ways, m0 = ((int)blockIdx.x / p.ways) * (32);
+    const int rows = min(32, p.M - m0);
     // K ranges start at multiples of BSUM stages: the f32 pieces of the bias sum do not depend on how K is cut
     const int nb = (p.nst + BSUM - 1) / BSUM;
     const int st0 = nb * way / p.ways * BSUM, st1 = min(p.nst, nb * (way + 1) / p.ways * BSUM);
@@ -195,7 +221,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
         *abort_flag = 0;
         fence_barrier_init();
     }
-    if (threadIdx.x >= 64 && threadIdx.x < 64 + RB * 32) {
+    if (threadIdx.x >= 64 && threadIdx.x < 64 + 32) {
         s_top[threadIdx.x - 64] = 0u;
         s_bias[threadIdx.x - 64] = make_double2(0.0, 0.0);
     }
@@ -218,7 +244,7 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
     if (warp == 0) {
         // ------------------------------ producer ------------------------------
         // several row tiles read the weights again (from L2); one tile: a single pass
-        const uint64_t pol = p.M > RB * 32 ? policy_evict_last() : policy_evict_first();
+        const uint64_t pol = p.M > 32 ? policy_evict_last() : policy_evict_first();
         int s = 0, issued = 0;
         uint32_t ph = 0;
         for (int st = st0; st < st1; ++st, ++issued) {
@@ -247,15 +273,11 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
         for (int st = st0; st < st1; ++st) {
             if (!mbar_wait(&in_full[s], ph, abort_flag, p.status, 42) || !mbar_wait(&a_full[ab], aph, abort_flag, p.status, 43)) break;
             tc_fence_after();
-            const uint64_t db = make_smem_desc(smem_u32(sIn + (size_t)s * STAGE_BYTES));
+            const uint64_t da = make_smem_desc(smem_u32(sA + (size_t)ab * PITCH)), db = make_smem_desc(smem_u32(sIn + (size_t)s * STAGE_BYTES));
             if (elect_one()) {
 #pragma unroll
-                for (int rb = 0; rb < RB; ++rb) {
-                    const uint64_t da = make_smem_desc(smem_u32(sA + (size_t)ab * PITCH + (size_t)rb * 16384));
-#pragma unroll
-                    for (int k4 = 0; k4 < SK / 32; ++k4)
-                        umma_i8(tmem_base + (uint32_t)(rb * NC), da + (uint64_t)(2 * k4), db + (uint64_t)(2 * k4), idesc, (st > st0 || k4 > 0) ? 1u : 0u);
-                }
+                for (int k4 = 0; k4 < SK / 32; ++k4)
+                    umma_i8(tmem_base, da + (uint64_t)(2 * k4), db + (uint64_t)(2 * k4), idesc, (st > st0 || k4 > 0) ? 1u : 0u);
                 umma_commit(&in_empty[s]);
                 umma_commit(&a_empty[ab]);
                 if (st == st1 - 1) umma_commit(d_full);
@@ -365,11 +387,9 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
             }
         }
         if (nr > 0) {
-            // Work items (row, stage) in groups of four: 4 stages of one row, 2 of two, one of four, half a stage of eight.  The x
+            // Work items (row, stage) in groups of four: 4 stages of one row, 2 of two, one of four.  The x
             // values of a group are loaded while the group before it is converted.
-            constexpr int GS = RPW >= 4 ? 1 : 4 / RPW;          // stages of a group
-            constexpr int GR = RPW >= 4 ? 4 : RPW;              // rows of a group
-            constexpr int HALVES = RPW / GR;                    // groups per stage (RPW = 8: two)
+            constexpr int GS = 4 / RPW;                         // stages of a group
             const int step = shared_rows ? 2 * BSUM : GS;       // from one group's first stage to the next one's
             // where this lane's four bytes of plane pl go: row 4m + pl of the tile, 16-byte chunk lane / 4 under the 128-byte
             // swizzle; m's parity is the first row's
@@ -381,24 +401,22 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
             bool ok = true;
             // (RPW > 1: the copy's rows are 512 bytes, and there are rows enough for the whole tile: no checks, constant offsets)
             const XT* xw = reinterpret_cast<const XT*>(p.x) + (RPW == 1 ? (size_t)(m0 + row_w) * p.K : (size_t)(m0 + row_w) * SK) + lane * 4 + st0 * p.xstep;
-            auto fetch = [&](float4 (&v)[4], const XT* q, int st, int half) {
+            auto fetch = [&](float4 (&v)[4], const XT* q, int st) {
 #pragma unroll
                 for (int h = 0; h < GS; ++h)
                     if (st + h < st1)
 #pragma unroll
-                        for (int i = 0; i < GR; ++i) v[i * GS + h] = ld_x4<XT>(q + h * p.xstep + (half * GR + i) * (8 * SK));
+                        for (int i = 0; i < RPW; ++i) v[i * GS + h] = ld_x4<XT>(q + h * p.xstep + i * (8 * SK));
             };
             uint4 sq;
-            int slot = 0, ab = 0;
-            uint32_t ph = 0, aph = 0, at[4];
+            int ab = 0;
+            uint32_t at[4];
             // waits for stage idx's scales and biases and for its A buffer
             auto enter = [&](int idx) {
-                if constexpr (RB == 1) {   // eight stages and a power of two of buffers
-                    slot = idx & (MAX_STAGES - 1);
-                    ph = ((uint32_t)idx / MAX_STAGES) & 1u;
-                    ab = idx & (BUFS - 1);
-                    aph = ((uint32_t)idx / BUFS) & 1u;
-                }
+                // eight stages and a power of two of buffers
+                const int slot = idx & (MAX_STAGES - 1);
+                const uint32_t ph = ((uint32_t)idx / MAX_STAGES) & 1u, aph = ((uint32_t)idx / BUFS) & 1u;
+                ab = idx & (BUFS - 1);
                 if (!mbar_wait(&in_full[slot], ph, abort_flag, p.status, 44)) return false;
                 sq = lds128(sv0 + (uint32_t)slot * S_BYTES);
                 if (!mbar_wait(&a_empty[ab], aph ^ 1u, abort_flag, p.status, 45)) return false;
@@ -424,49 +442,28 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMA reads through the async proxy
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&a_full[ab]);
-                if constexpr (RB == 2) {
-                    if (++slot == p.stages) { slot = 0; ph ^= 1u; }
-                    if (++ab == BUFS) { ab = 0; aph ^= 1u; }
-                }
             };
             float4 xa[4], xb[4];
-            if constexpr (HALVES == 2) {
-                const bool both = nr > GR;      // rows of a half are converted together, real or not
-                fetch(xa, xw, st0, 0);
-                for (int st = st0; st < st1; ++st) {
-                    if (both) fetch(xb, xw, st, 1);
-                    if (!enter(st - st0)) { ok = false; break; }
+            auto convert = [&](const float4 (&v)[4], int st) {
 #pragma unroll
-                    for (int i = 0; i < GR; ++i) item(xa[i], i);
-                    xw += p.xstep;
-                    fetch(xa, xw, st + 1, 0);
-                    if (both)
+                for (int h = 0; h < GS; ++h) {
+                    if (!ok || st + h >= st1) return;
+                    if (!enter(st + h - st0)) { ok = false; return; }
 #pragma unroll
-                        for (int i = 0; i < GR; ++i) item(xb[i], GR + i);
+                    for (int i = 0; i < RPW; ++i) item(v[i * GS + h], i);
                     leave();
                 }
-            } else {
-                auto convert = [&](const float4 (&v)[4], int st) {
-#pragma unroll
-                    for (int h = 0; h < GS; ++h) {
-                        if (!ok || st + h >= st1) return;
-                        if (!enter(st + h - st0)) { ok = false; return; }
-#pragma unroll
-                        for (int i = 0; i < GR; ++i) item(v[i * GS + h], i);
-                        leave();
-                    }
-                };
-                int st = st0 + sub * BSUM;
-                xw += (size_t)(sub * BSUM) * p.xstep;
-                const size_t stride = (size_t)step * p.xstep;
-                fetch(xa, xw, st, 0);
-                for (; ok && st < st1; st += 2 * step) {
-                    fetch(xb, xw + stride, st + step, 0);
-                    convert(xa, st);
-                    xw += 2 * stride;
-                    fetch(xa, xw, st + 2 * step, 0);
-                    convert(xb, st + step);
-                }
+            };
+            int st = st0 + sub * BSUM;
+            xw += (size_t)(sub * BSUM) * p.xstep;
+            const size_t stride = (size_t)step * p.xstep;
+            fetch(xa, xw, st);
+            for (; ok && st < st1; st += 2 * step) {
+                fetch(xb, xw + stride, st + step);
+                convert(xa, st);
+                xw += 2 * stride;
+                fetch(xa, xw, st + 2 * step);
+                convert(xb, st + step);
             }
             if (runit == INT_MIN && sub == 0) {
                 // A group without r: x . b in double.  Upper 24 bits and the rest of every four terms are added up apart: exact
@@ -492,8 +489,8 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
             }
         }
         // ------------------------------ epilogue, first half ------------------
-        // accumulators -> shared memory as [warp][row 4m + p][column], in the memory of the A tiles (RB = 1) or of A tiles
-        // and ring alike: every MMA has read them once d_full is reached
+        // accumulators -> shared memory as [warp][row 4m + p][column], in the memory of the A tiles: every MMA has read them once
+        // d_full is reached
         if (st1 > st0) mbar_wait(d_full, 0, abort_flag, p.status, 46);
     }
     // All K ranges of a tile: bytes -> int64 sums per output, exact, parked in shared memory; then each CTA of the cluster adds
@@ -502,55 +499,39 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    constexpr int LDW = RB == 1 ? 37 : 33;                             // words between rows of a warp's corner: no bank conflicts
+    constexpr int LDW = 37;                                            // words between rows of a warp's corner: no bank conflicts
     uint32_t* s_raw = reinterpret_cast<uint32_t*>(smem);               // [CW][32][LDW]
-    long long* s_sum = reinterpret_cast<long long*>(smem + 40 * 1024); // [RB * 32][GN]
-    long long* s_ext = s_sum + RB * 32 * GN;                           // [RB * 32][RD + 1]: the bias columns
+    long long* s_sum = reinterpret_cast<long long*>(smem + 40 * 1024); // [32][GN]
+    long long* s_ext = s_sum + 32 * GN;                           // [32][RD + 1]: the bias columns
     const bool failed = *abort_flag != 0;
     if (warp >= 2 && !failed) {
         const int cw = warp - 2, q = warp & 3, half = cw >> 2;         // lane quarter of tensor memory, half of the columns
         uint32_t* mine = s_raw + (size_t)cw * 32 * LDW;
+        const int row0 = q * 8;
+        if (row0 < rows) {
+            const uint32_t from = tmem_base + ((uint32_t)(q * 32) << 16);
+            uint32_t v[2][16], ext[16];
 #pragma unroll
-        for (int rb = 0; rb < RB; ++rb) {
-            if (rb * 32 + q * 8 < rows) {
-                const uint32_t from = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(rb * NC);
-                uint32_t v[2][16], ext[16];
+            for (int c = 0; c < 2; ++c) tmem_ld16(from + half * 32 + c * 16, v[c]);
+            if (half == 1) tmem_ld16(from + GN, ext);
+            tmem_ld_wait();
 #pragma unroll
-                for (int c = 0; c < 2; ++c) tmem_ld16(from + half * 32 + c * 16, v[c]);
-                if (half == 1) tmem_ld16(from + GN, ext);
-                tmem_ld_wait();
+            for (int c = 0; c < 2; ++c)
 #pragma unroll
-                for (int c = 0; c < 2; ++c)
+                for (int e = 0; e < 16; ++e) mine[lane * LDW + c * 16 + e] = v[c][e];
+            if (half == 1)
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) mine[lane * LDW + c * 16 + e] = v[c][e];
-                if (RB == 1 && half == 1)
-#pragma unroll
-                    for (int e = 0; e <= RD; ++e) mine[lane * LDW + 32 + e] = ext[e];
-                __syncwarp();
-                auto sum_at = [&](int m, int c) {
-                    const uint32_t* r = mine + (4 * m) * LDW + c;
-                    return ((((long long)r[0] * 256 + r[LDW]) * 256 + r[2 * LDW]) * 256) + r[3 * LDW];
-                };
-                const int row0 = rb * 32 + q * 8;
-                if constexpr (RB == 1) {
-                    // a loop over the rows there are and not its copies: code that runs once waits for its instructions
+                for (int e = 0; e <= RD; ++e) mine[lane * LDW + 32 + e] = ext[e];
+            __syncwarp();
+            auto sum_at = [&](int m, int c) {
+                const uint32_t* r = mine + (4 * m) * LDW + c;
+                return ((((long long)r[0] * 256 + r[LDW]) * 256 + r[2 * LDW]) * 256) + r[3 * LDW];
+            };
+            // a loop over the rows there are and not its copies: code that runs once waits for its instructions
 #pragma unroll 1
-                    for (int m = 0; m < min(8, rows - row0); ++m) {
-                        s_sum[(size_t)(row0 + m) * GN + half * 32 + lane] = sum_at(m, lane);
-                        if (half == 1 && lane <= RD) s_ext[(size_t)(row0 + m) * (RD + 1) + lane] = sum_at(m, 32 + lane);
-                    }
-                } else {
-#pragma unroll
-                    for (int m = 0; m < 8; ++m) s_sum[(size_t)(row0 + m) * GN + half * 32 + lane] = sum_at(m, lane);
-                    if (half == 1) {
-                        __syncwarp();
-#pragma unroll
-                        for (int e = 0; e <= RD; ++e) mine[lane * LDW + e] = ext[e];
-                        __syncwarp();
-                        for (int i = lane; i < 8 * (RD + 1); i += 32) s_ext[(size_t)row0 * (RD + 1) + i] = sum_at(i / (RD + 1), i % (RD + 1));
-                    }
-                }
-                __syncwarp();
+            for (int m = 0; m < min(8, rows - row0); ++m) {
+                s_sum[(size_t)(row0 + m) * GN + half * 32 + lane] = sum_at(m, lane);
+                if (half == 1 && lane <= RD) s_ext[(size_t)(row0 + m) * (RD + 1) + lane] = sum_at(m, 32 + lane);
             }
         }
         tc_fence_before();
@@ -582,30 +563,384 @@ __global__ void __launch_bounds__(GC_THREADS, 2) qlinear_gc_tc_kernel(const __gr
                     bhi += b.x;
                     blo += b.y;
                 }
-            // sum_k q r: the offsets off the planes, then r's own 2^31 off its top byte
-            const long long sq = ext[RD] - ((long long)p.K << 31);
-            const double top = (double)(ext[0] - ((long long)rsum.x << 31) - 128 * sq);
-            const double rest = (double)(ext[1] - ((long long)rsum.y << 31)) * 65536.0 + (double)(ext[2] - ((long long)rsum.z << 31)) * 256.0 +
-                                (double)(ext[3] - ((long long)rsum.w << 31));
-            const double r_unit = runit == INT_MIN ? 0.0 : __longlong_as_double((long long)(1023 - runit) << 52);
-            const int e = s_exp[j];
-            // 2^-e as a double from its exponent field; the sum is exact up to here
-            const double unit = e == INT_MIN ? (double)__int_as_float(0x7fc00000) : __longlong_as_double((long long)(1023 - e) << 52);
-            float f = __double2float_rn(((double)(sum - rs) + (top * 16777216.0 + rest) * r_unit) * unit + (bhi + blo));
-            const size_t at = (size_t)(m0 + j) * p.ldy + p.y_col0 + col;
-            auto put = [&](auto* y0, auto value) {
-                auto* dst = y0 + at;
-                *dst = value;
+            const double2 terms = row_terms(ext, rsum, runit, s_exp[j], p.K);
+            store_output(p, __double2float_rn(((double)(sum - rs) + terms.x) * terms.y + (bhi + blo)), (size_t)(m0 + j) * p.ldy + p.y_col0 + col);
+        }
+    }
+    if (p.ways > 1) cl.sync();   // the others have read this CTA's sums
+}
+
+// ---- more than 32 rows ------------------------------------------------------------------------------------------------------
+// The same arithmetic, tables and meeting of K ranges on tiles of 64 rows x TWO groups, one CTA an SM with sixteen converter warps:
+// four rows of x in a warp's registers are multiplied by the scales of both groups before the next four are needed, and x crosses
+// L2 -> SM half as often.  512 x 4096 x 4096 takes 92 us; one group a CTA of eight converter warps, two CTAs an SM: 112.  What bounds it: a
+// stage takes 2000 cycles, of which the conversions to integers need 1130 (16 an SM a clock), the MMAs 640 and the shared-memory pipe
+// 1300; the converters meet at two buffers of A, and 256 CTAs are 1.7 waves of 148.
+constexpr int WG = 2, WCW = 16, WROWS = 64, WR = WROWS / WCW;      // groups, converter warps, rows of a tile, rows a warp
+constexpr int W_THREADS = 32 * (2 + WCW);
+constexpr int W_ABUF = 32 * 1024;              // A operand of a stage and group: 64 rows x 4 planes x 128 bytes
+constexpr int W_IN = WG * STAGE_BYTES, W_SC = WG * S_BYTES;
+constexpr int W_LDW = 33;                      // words between rows of a warp's corner in the epilogue: no bank conflicts
+constexpr size_t W_SUM_AT = (size_t)WCW * 32 * W_LDW * 4 + 512;    // the sums' place behind the corners (16-byte aligned)
+
+// a * s, two at a time, each half rounded like __fmul_rn
+__device__ __forceinline__ void mul2(float& r0, float& r1, float a0, float a1, float s0, float s1) {
+    asm("{\n\t.reg .b64 a, s;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 s, {%4, %5};\n\tmul.rn.f32x2 a, a, s;\n\tmov.b64 {%0, %1}, a;\n\t}"
+        : "=f"(r0), "=f"(r1)
+        : "f"(a0), "f"(a1), "f"(s0), "f"(s1));
+}
+
+__global__ void __launch_bounds__(W_THREADS, 1) qlinear_gc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ GcParams p) {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* sA = smem;                                              // [2][WG] x W_ABUF
+    uint8_t* sIn = smem + 2 * WG * W_ABUF;                           // [stages][WG] x STAGE_BYTES
+    uint8_t* sSc = sIn + (size_t)p.stages * W_IN;                    // [stages][WG] x S_BYTES
+    uint64_t* in_full = reinterpret_cast<uint64_t*>(sSc + (size_t)p.stages * W_SC);
+    uint64_t* in_empty = in_full + MAX_STAGES;
+    uint64_t* a_full = in_empty + MAX_STAGES;                        // [2]
+    uint64_t* a_empty = a_full + 2;
+    uint64_t* d_full = a_empty + 2;
+    double2* s_bias = reinterpret_cast<double2*>(d_full + 2);        // [WG][64]: a group without r: this K range's bias term, in two parts
+    int* s_exp = reinterpret_cast<int*>(s_bias + WG * WROWS);        // [WG][64]: e of a row, or INT_MIN: poisoned
+    float* s_smax = reinterpret_cast<float*>(s_exp + WG * WROWS);    // [WG][K / 128]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_smax + WG * p.nst);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = warp_id(), lane = threadIdx.x & 31;
+    const int groups = p.N / GN;
+    // an odd last group is computed twice and stored once
+    auto group_of = [&](int q) { return min((int)blockIdx.y * WG + q, groups - 1); };
+    const int way = (int)blockIdx.x % p.ways, m0 = ((int)blockIdx.x / p.ways) * WROWS;
+    const int rows = min(WROWS, p.M - m0);
+    const int nb = (p.nst + BSUM - 1) / BSUM;
+    const int st0 = nb * way / p.ways * BSUM, st1 = min(p.nst, nb * (way + 1) / p.ways * BSUM);
+    const int active = min(WCW, rows);         // converter warps that arrive on a stage
+    pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < p.stages; ++s) {
+            mbar_init(&in_full[s], 1);
+            mbar_init(&in_empty[s], 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&a_full[s], (uint32_t)active);
+            mbar_init(&a_empty[s], 1);
+        }
+        mbar_init(d_full, 1);
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (threadIdx.x >= 64 && threadIdx.x < 64 + WG * WROWS) s_bias[threadIdx.x - 64] = make_double2(0.0, 0.0);
+    if (warp == 1) {
+        for (int s = 0; s < p.stages * WG; ++s) sts32(smem_u32(sIn + (size_t)s * STAGE_BYTES + W_BYTES + RD * SK) + lane * 4, 0x01010101u);   // ones
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        tmem_alloc(tmem_slot, 512);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        // ------------------------------ producer ------------------------------
+        const uint64_t pol = p.M > WROWS ? policy_evict_last() : policy_evict_first();
+        int s = 0, issued = 0;
+        uint32_t ph = 0;
+        for (int st = st0; st < st1; ++st, ++issued) {
+            if (!mbar_wait(&in_empty[s], ph ^ 1u, abort_flag, p.status, 41)) break;
+            if (elect_one()) {
+                mbar_expect_tx(&in_full[s], (uint32_t)(WG * TX_BYTES));
 #pragma unroll
-                for (int r = 0; r < PEER_MAX_RANKS - 1; ++r)   // the same element of every other rank's y, over NVLink
-                    if (r < p.n_peers) *reinterpret_cast<decltype(dst)>(reinterpret_cast<char*>(dst) + p.peer_delta[r]) = value;
+                for (int q = 0; q < WG; ++q) {
+                    const int g = group_of(q);
+                    uint8_t* dst = sIn + (size_t)s * W_IN + q * STAGE_BYTES;
+                    tma_load_2d(dst, &map_w, st * SK, g * GN, &in_full[s], pol);
+                    bulk_load(dst + W_BYTES, p.rbytes + ((size_t)g * p.nst + st) * (RD * SK), RD * SK, &in_full[s]);
+                    bulk_load(sSc + (size_t)s * W_SC + q * S_BYTES, p.scales + (size_t)g * p.K + st * SK, S_BYTES, &in_full[s]);
+                }
+            }
+            __syncwarp();
+            if (++s == p.stages) { s = 0; ph ^= 1u; }
+        }
+        // whatever happened to the other roles: no copy is in flight when this CTA's shared memory is used for other things
+        for (int j = max(0, issued - p.stages); j < issued; ++j) {
+            const long long t0 = clock64();
+            while (!mbar_try_wait(&in_full[j % p.stages], (uint32_t)(j / p.stages) & 1u) && clock64() - t0 < 4000000ll) {}
+        }
+    } else if (warp == 1) {
+        // ------------------------------ MMA issuer ----------------------------
+        constexpr uint32_t idesc = (2u << 4) | ((uint32_t)(NC >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        int s = 0, ab = 0;
+        uint32_t ph = 0, aph = 0;
+        for (int st = st0; st < st1; ++st) {
+            if (!mbar_wait(&in_full[s], ph, abort_flag, p.status, 42) || !mbar_wait(&a_full[ab], aph, abort_flag, p.status, 43)) break;
+            tc_fence_after();
+            if (elect_one()) {
+#pragma unroll
+                for (int q = 0; q < WG; ++q) {
+                    const uint64_t db = make_smem_desc(smem_u32(sIn + (size_t)s * W_IN + q * STAGE_BYTES));
+#pragma unroll
+                    for (int rb = 0; rb < 2; ++rb) {
+                        const uint64_t da = make_smem_desc(smem_u32(sA + (size_t)(ab * WG + q) * W_ABUF + (size_t)rb * 16384));
+#pragma unroll
+                        for (int k4 = 0; k4 < SK / 32; ++k4)
+                            umma_i8(tmem_base + (uint32_t)((q * 2 + rb) * NC), da + (uint64_t)(2 * k4), db + (uint64_t)(2 * k4), idesc, (st > st0 || k4 > 0) ? 1u : 0u);
+                    }
+                }
+                umma_commit(&a_empty[ab]);
+                umma_commit(&in_empty[s]);
+                if (st == st1 - 1) umma_commit(d_full);
+            }
+            __syncwarp();
+            if (++s == p.stages) { s = 0; ph ^= 1u; }
+            ab ^= 1;
+            if (ab == 0) aph ^= 1u;
+        }
+    } else {
+        // ------------------------------ converters ----------------------------
+        const int cw = warp - 2, ct = threadIdx.x - 64;
+        for (int i = ct; i < WG * p.nst; i += 32 * WCW) s_smax[i] = __ldg(p.smax + (size_t)group_of(i / p.nst) * p.nst + i % p.nst);   // the weight's own: before the wait
+        pdl_wait();   // x and xtop come from the previous kernel
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * WCW) : "memory");
+        const int nr = cw < rows ? (rows - cw + WCW - 1) / WCW : 0;     // rows of this warp: cw, cw + 16, ...
+        // The largest product of every row and group, as in the kernel above: the places of the stages' largest |x| first, all
+        // products of a stage where the bound of the others has a larger exponent.
+        const uint2* xt = p.xtop + (size_t)(m0 + cw) * p.nst;
+        const float* xr = reinterpret_cast<const float*>(p.x) + (size_t)(m0 + cw) * SK + lane * 4;
+        const float* gs[WG] = {p.scales + (size_t)group_of(0) * p.K, p.scales + (size_t)group_of(1) * p.K};
+        auto rest_bound = [&](uint2 v, int q, int st) { return abs_bits(__fmul_rn(__uint_as_float(v.y & 0xffff0000u), s_smax[q * p.nst + st])); };
+        float scale[WG][WR];
+        {
+            uint32_t top[WG][WR], rest[WG][WR];
+#pragma unroll
+            for (int i = 0; i < WR; ++i) top[0][i] = top[1][i] = rest[0][i] = rest[1][i] = 0u;
+            for (int st = lane; st < p.nst; st += 32) {
+                uint2 v[WR];
+                float s1[WG][WR];
+#pragma unroll
+                for (int i = 0; i < WR; ++i)
+                    if (i < nr) v[i] = xt[(size_t)(WCW * i) * p.nst + st];
+#pragma unroll
+                for (int i = 0; i < WR; ++i)
+                    if (i < nr)
+#pragma unroll
+                        for (int q = 0; q < WG; ++q) s1[q][i] = __ldg(gs[q] + st * SK + (v[i].y & 0xffffu));
+#pragma unroll
+                for (int i = 0; i < WR; ++i)
+                    if (i < nr)
+#pragma unroll
+                        for (int q = 0; q < WG; ++q) {
+                            top[q][i] = max(top[q][i], abs_bits(__fmul_rn(__uint_as_float(v[i].x), s1[q][i])));
+                            rest[q][i] = max(rest[q][i], rest_bound(v[i], q, st));
+                        }
+            }
+#pragma unroll
+            for (int q = 0; q < WG; ++q)
+#pragma unroll
+                for (int i = 0; i < WR; ++i) {
+                    scale[q][i] = 0.0f;
+                    if (i >= nr) continue;
+                    uint32_t t = __reduce_max_sync(0xffffffffu, top[q][i]);
+                    if (__any_sync(0xffffffffu, rest[q][i] >> 23 > t >> 23)) {
+#pragma unroll 1
+                        for (int base = 0; base < p.nst; base += 32) {
+                            const int st = base + lane;
+                            const uint32_t b = st < p.nst ? rest_bound(xt[(size_t)(WCW * i) * p.nst + st], q, st) >> 23 : 0u;
+                            uint32_t todo = __ballot_sync(0xffffffffu, b > t >> 23);
+                            while (todo) {
+                                const int sa = base + __ffs(todo) - 1;
+                                todo &= todo - 1;
+                                t = max(t, __reduce_max_sync(0xffffffffu, __float_as_uint(top_of(0.0f, ld_x4(xr + (size_t)sa * p.xstep + i * (WCW * SK)), ldg_x4(gs[q] + sa * SK + lane * 4)))));
+                                todo &= __ballot_sync(0xffffffffu, b > t >> 23);
+                            }
+                        }
+                    }
+                    const bool finite = t < 0x7f800000u;
+                    const int e = unit_exponent(t);
+                    scale[q][i] = finite ? __uint_as_float((uint32_t)(127 + e) << 23) : 0.0f;   // 2^e, a normal number
+                    if (lane == 0) s_exp[q * WROWS + cw + WCW * i] = finite ? e : INT_MIN;
+                }
+        }
+        if (nr > 0) {
+            // where this lane's four bytes of plane pl go: row 4m + pl of the tile, 16-byte chunk lane / 4 under the 128-byte swizzle;
+            // m's parity is the first row's
+            uint32_t off[4];
+#pragma unroll
+            for (int pl = 0; pl < 4; ++pl)
+                off[pl] = smem_u32(sA) + (uint32_t)(cw * 512 + pl * 128 + ((((lane >> 2) ^ pl) << 4) ^ ((cw & 1) << 6)) + (lane & 3) * 4);
+            const uint32_t sv0 = smem_u32(sSc) + lane * 16;
+            const float* xw = xr + (size_t)st0 * p.xstep;
+            int slot = 0, ab = 0;
+            uint32_t ph = 0, aph = 0;
+            auto fetch = [&](float4 (&v)[WR], int st) {
+                if (st < st1)
+#pragma unroll
+                    for (int i = 0; i < WR; ++i) v[i] = ld_x4(xw + i * (WCW * SK));     // (the copy has rows enough for the whole tile)
+                xw += p.xstep;
             };
-            if (p.y_bf16) {
-                if (p.residual) f += __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.residual)[at]);
-                put(reinterpret_cast<__nv_bfloat16*>(p.y), __float2bfloat16_rn(f));
-            } else {
-                if (p.residual) f = __fadd_rn(reinterpret_cast<const float*>(p.residual)[at], f);
-                put(reinterpret_cast<float*>(p.y), f);
+            auto convert = [&](const float4 (&v)[WR]) {
+                if (!mbar_wait(&in_full[slot], ph, abort_flag, p.status, 44)) return false;
+                uint4 sq[WG];
+#pragma unroll
+                for (int q = 0; q < WG; ++q) sq[q] = lds128(sv0 + (uint32_t)(slot * W_SC + q * S_BYTES));
+                const uint32_t buf = (uint32_t)(ab * WG * W_ABUF);
+                auto item = [&](const float4& x4, int q, int i) {
+                    float a0, a1, a2, a3;
+                    mul2(a0, a1, x4.x, x4.y, __uint_as_float(sq[q].x), __uint_as_float(sq[q].y));
+                    mul2(a2, a3, x4.z, x4.w, __uint_as_float(sq[q].z), __uint_as_float(sq[q].w));
+                    mul2(a0, a1, a0, a1, scale[q][i], scale[q][i]);
+                    mul2(a2, a3, a2, a3, scale[q][i], scale[q][i]);
+                    const int q0 = __float2int_rn(a0), q1 = __float2int_rn(a1), q2 = __float2int_rn(a2), q3 = __float2int_rn(a3);
+                    // 4 integers x 4 bytes -> 4 planes x 4 k; plane 0 is the top byte, its sign bit flipped: q + 2^31
+                    const uint32_t t0 = __byte_perm(q0, q1, 0x5140), t1 = __byte_perm(q2, q3, 0x5140);
+                    const uint32_t t2 = __byte_perm(q0, q1, 0x7362), t3 = __byte_perm(q2, q3, 0x7362);
+                    const uint32_t at = buf + (uint32_t)(q * W_ABUF + i * (WCW * 512));
+                    sts32(off[0] + at, __byte_perm(t2, t3, 0x7632) ^ 0x80808080u);
+                    sts32(off[1] + at, __byte_perm(t2, t3, 0x5410));
+                    sts32(off[2] + at, __byte_perm(t0, t1, 0x7632));
+                    sts32(off[3] + at, __byte_perm(t0, t1, 0x5410));
+                };
+                if (!mbar_wait(&a_empty[ab], aph ^ 1u, abort_flag, p.status, 45)) return false;
+#pragma unroll
+                for (int q = 0; q < WG; ++q)
+#pragma unroll
+                    for (int i = 0; i < WR; ++i) item(v[i], q, i);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMA reads through the async proxy
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&a_full[ab]);    // (group by group, four buffers: 512 rows 92 -> 97 us)
+                if (++slot == p.stages) { slot = 0; ph ^= 1u; }
+                ab ^= 1;
+                if (ab == 0) aph ^= 1u;
+                return true;
+            };
+            float4 xa[WR], xb[WR];
+            fetch(xa, st0);
+            for (int st = st0; st < st1; st += 2) {
+                fetch(xb, st + 1);
+                if (!convert(xa) || st + 1 >= st1) break;
+                fetch(xa, st + 2);
+                if (!convert(xb)) break;
+            }
+#pragma unroll 1
+            for (int q = 0; q < WG; ++q) {
+                if (__ldg(p.rinfo + 8 * group_of(q) + 4) != INT_MIN) continue;
+                // a group without r: x . b in double, upper 24 bits and the rest of every four terms apart: exact sums
+                const float* xb0 = reinterpret_cast<const float*>(p.x) + (size_t)(m0 + cw) * SK + lane * 4;
+                const float* gb = p.biases + (size_t)group_of(q) * p.K + lane * 4;
+                for (int i = 0; i < nr; ++i) {
+                    double hi = 0.0, lo = 0.0;
+                    for (int st = st0; st < st1; ++st) {
+                        const float4 x4 = ld_x4(xb0 + (size_t)st * p.xstep + i * (WCW * SK)), b4 = ldg_x4(gb + st * SK);
+                        const double d = fma((double)x4.x, (double)b4.x, fma((double)x4.y, (double)b4.y, fma((double)x4.z, (double)b4.z, (double)x4.w * (double)b4.w)));
+                        const double u = __hiloint2double(__double2hiint(d), __double2loint(d) & (int)0xe0000000);
+                        hi += u;
+                        lo += d - u;
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        hi += __shfl_xor_sync(0xffffffffu, hi, o);
+                        lo += __shfl_xor_sync(0xffffffffu, lo, o);
+                    }
+                    if (lane == 0) s_bias[q * WROWS + cw + WCW * i] = make_double2(hi, lo);
+                }
+            }
+        }
+        if (st1 > st0) mbar_wait(d_full, 0, abort_flag, p.status, 46);
+    }
+    // bytes -> int64 sums per output, exact, parked where A and the ring were; then each CTA of the cluster adds up and writes its
+    // share of the rows (a wait that gave up leaves the loops above in every role; the barriers below are reached all the same)
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    long long* s_sum = reinterpret_cast<long long*>(smem + W_SUM_AT);  // [WG][64][GN]
+    long long* s_ext = s_sum + WG * WROWS * GN;                        // [WG][64][RD + 1]: the bias columns
+    const bool failed = *abort_flag != 0;
+    if (warp >= 2 && !failed) {
+        const int cw = warp - 2, quarter = warp & 3, half = (cw >> 2) & 1, q = cw >> 3;   // lanes of tensor memory, columns, group
+        uint32_t* mine = reinterpret_cast<uint32_t*>(smem) + (size_t)cw * 32 * W_LDW;
+#pragma unroll 1
+        for (int rb = 0; rb < 2; ++rb) {
+            const int row0 = rb * 32 + quarter * 8;
+            if (row0 >= rows) continue;
+            const uint32_t from = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((q * 2 + rb) * NC);
+            uint32_t v[2][16], ext[16];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) tmem_ld16(from + half * 32 + c * 16, v[c]);
+            tmem_ld16(from + GN, ext);
+            tmem_ld_wait();
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int e = 0; e < 16; ++e) mine[lane * W_LDW + c * 16 + e] = v[c][e];
+            __syncwarp();
+            auto sum_at = [&](int m, int c) {
+                const uint32_t* w = mine + (4 * m) * W_LDW + c;
+                return ((((long long)w[0] * 256 + w[W_LDW]) * 256 + w[2 * W_LDW]) * 256) + w[3 * W_LDW];
+            };
+#pragma unroll
+            for (int m = 0; m < 8; ++m) s_sum[(size_t)(q * WROWS + row0 + m) * GN + half * 32 + lane] = sum_at(m, lane);
+            __syncwarp();
+            if (half == 1) {
+#pragma unroll
+                for (int e = 0; e <= RD; ++e) mine[lane * W_LDW + e] = ext[e];
+                __syncwarp();
+                for (int i = lane; i < 8 * (RD + 1); i += 32) s_ext[(size_t)(q * WROWS + row0) * (RD + 1) + i] = sum_at(i / (RD + 1), i % (RD + 1));
+            }
+            __syncwarp();
+        }
+        tc_fence_before();
+    }
+    cg::cluster_group cl = cg::this_cluster();
+    if (p.ways > 1) cl.sync();
+    else __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, 512);
+    }
+    if (warp >= 2 && !failed) {
+        const int t = threadIdx.x - 64, n = t & (GN - 1), q = (t >> 6) & 1;      // 512 threads: both groups' 64 columns, every fourth row
+        const int g = (int)blockIdx.y * WG + q;
+        double2* s_terms = reinterpret_cast<double2*>(smem);           // [WG][64], where the corners were
+        double* s_plus = reinterpret_cast<double*>(s_terms + WG * WROWS);
+        if (t < WG * WROWS && (t & (WROWS - 1)) < rows) {
+            const int tg = group_of(t / WROWS), runit = __ldg(p.rinfo + 8 * tg + 4);
+            const int4 rsum = __ldg(reinterpret_cast<const int4*>(p.rinfo) + 2 * tg);
+            long long ext[RD + 1] = {0, 0, 0, 0, 0};
+            double bhi = 0.0, blo = 0.0;
+            for (int w = 0; w < p.ways; ++w) {
+                const long long* se = (p.ways > 1 ? cl.map_shared_rank(s_ext, w) : s_ext) + (size_t)t * (RD + 1);
+#pragma unroll
+                for (int i = 0; i <= RD; ++i) ext[i] += se[i];
+                if (runit == INT_MIN) {
+                    const double2 b = (p.ways > 1 ? cl.map_shared_rank(s_bias, w) : s_bias)[t];
+                    bhi += b.x;
+                    blo += b.y;
+                }
+            }
+            s_terms[t] = row_terms(ext, rsum, runit, s_exp[t], p.K);
+            s_plus[t] = bhi + blo;
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * WCW) : "memory");
+        if (g < groups) {
+            const long long rs = (long long)__ldg(p.rowsum + g * GN + n) << 31;
+            // four rows at a time: one by one the way from a sum to its f32 is a chain of 300 cycles
+            for (int j0 = (t >> 7) + 4 * way; j0 < rows; j0 += 16 * p.ways) {
+                long long sum[4] = {0, 0, 0, 0};
+                for (int w = 0; w < p.ways; ++w) {
+                    const long long* from = (p.ways > 1 ? cl.map_shared_rank(s_sum, w) : s_sum) + (size_t)(q * WROWS) * GN + n;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (j0 + u * 4 * p.ways < rows) sum[u] += from[(size_t)(j0 + u * 4 * p.ways) * GN];
+                }
+                float f[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int at_row = q * WROWS + min(j0 + u * 4 * p.ways, rows - 1);
+                    f[u] = __double2float_rn(((double)(sum[u] - rs) + s_terms[at_row].x) * s_terms[at_row].y + s_plus[at_row]);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (j0 + u * 4 * p.ways < rows) store_output(p, f[u], (size_t)(m0 + j0 + u * 4 * p.ways) * p.ldy + p.y_col0 + g * GN + n);
             }
         }
     }
@@ -712,9 +1047,9 @@ __global__ void __launch_bounds__(256) gc_ratio_kernel(const float* __restrict__
     if (threadIdx.x < 8) info[8 * g + threadIdx.x] = threadIdx.x < RD ? s_sum[threadIdx.x] : threadIdx.x == 4 ? unit : 0;
 }
 
-template <typename XT, int RB, int RPW, bool MEET = false>
+template <typename XT, int RPW, bool MEET = false>
 cudaError_t launch_gc(rusty_cuda_ctx* ctx, const CUtensorMap& map_w, const GcParams& p, dim3 grid, size_t smem) {
-    auto kern = qlinear_gc_tc_kernel<XT, RB, RPW, MEET>;
+    auto kern = qlinear_gc_tc_kernel<XT, RPW, MEET>;
     cudaError_t e = rusty::ensure_dynamic_smem((const void*)kern, ctx->device, smem);
     if (e != cudaSuccess) return e;
     return launch_pdl_cluster(kern, grid, dim3(GC_THREADS), (unsigned)p.ways, smem, ctx->stream, map_w, p);
@@ -779,13 +1114,36 @@ int launch_gc_tc(rusty_cuda_ctx* ctx, const QLinearArgs& a) {
         p.x = (const char*)a.x + (size_t)m0 * a.K * xs;
         p.y = (char*)a.y + (size_t)m0 * a.ldy * ys;
         p.residual = a.residual ? (const char*)a.residual + (size_t)m0 * a.ldy * ys : nullptr;
+        // K ranges: as many CTAs as the SMs hold (two an SM; the wide kernel one), four stages each at least.  More than two tiles of
+        // rows (wide: one): none, the CTAs suffice, and the start and the end of a CTA cost as much as ten stages.
+        const int groups = p.N / GN;
+        auto ways_of = [&](int ctas, int slots, bool cut) {
+            int w = 1;
+            while (cut && w < 4 && ctas * w * 2 <= slots && p.nst / (w * 2) >= 4) w *= 2;
+            return w;
+        };
+        // Beyond 32 rows: tiles of 32 on the narrow kernel or of 64 x two groups on the wide one, which does four times the work of a
+        // CTA in 41 us where 2 an SM of the others take 27 (32 stages), but starts and ends in 14 instead of 8 us and fills whole
+        // waves less well.  us, narrow / wide: 64 x 4096 x 4096 23.3 / 25.3, 64 x 4096 x 1024 13.1 / 23.7, 64 x 4096 x 11008 55.3 / 47.2, 96 x
+        // 4096 x 4096 33.2 / 44.9, 200 x 4096 x 4096 62.9 / 47.7, 512 x 4096 x 4096 118 / 91.4, 512 x 4096 x 11008 295 / 224.
+        bool wide = false;
+        if (p.M > 32) {
+            const int tn = (p.M + 31) / 32, tw = (p.M + WROWS - 1) / WROWS, un = groups * tn, uw = (groups + WG - 1) / WG * tw;
+            const int wn = ways_of(un, 2 * ctx->sm_count, tn <= 2), ww = ways_of(uw, ctx->sm_count, tw == 1);
+            auto us = [&](int ctas, int slots, int ways, double us32, double fixed) {
+                return (double)((ctas * ways + slots - 1) / slots) * us32 * p.nst / 32.0 / ways + fixed;
+            };
+            wide = us(uw, ctx->sm_count, ww, 41.0, 6.0 + (p.M < WROWS ? p.M : WROWS) / 8) < us(un, 2 * ctx->sm_count, wn, 27.0, 8.0);
+        }
         // rows per converter warp; up to 8 rows the converters read x as it is and find its maxima themselves (16 KB a row from
         // L2 at K = 4096, while the first weights arrive) if x has no partial stage: the copy pads it
-        const int rpw = p.M <= 8 && p.K == (int)a.K ? 1 : p.M <= 16 ? 2 : p.M <= 32 ? 4 : 8;
-        const int rb = rpw == 8 ? 2 : 1, tile = rpw == 8 ? 64 : 8 * rpw, tiles = (p.M + tile - 1) / tile;
+        const int rpw = p.M <= 8 && p.K == (int)a.K ? 1 : p.M <= 16 ? 2 : 4;
+        const int tile = wide ? WROWS : 8 * rpw, tiles = (p.M + tile - 1) / tile;
+        const int units = wide ? (groups + WG - 1) / WG : groups;
+        p.ways = ways_of(units * tiles, (wide ? 1 : 2) * ctx->sm_count, tiles <= (wide ? 1 : 2));
         p.xstep = SK;
         p.xtop = nullptr;
-        if (rpw > 1) {
+        if (wide || rpw > 1) {
             const int Mp = tiles * tile;
             float* xbuf = (float*)ctx->tc_ws;
             uint2* xtop = (uint2*)(xbuf + (size_t)Mp * p.K);
@@ -799,30 +1157,32 @@ int launch_gc_tc(rusty_cuda_ctx* ctx, const QLinearArgs& a) {
             p.xtop = xtop;
             p.xstep = (size_t)Mp * SK;
         }
-        const int groups = p.N / GN;
-        // K ranges: as many CTAs as two an SM hold, four stages each at least.  More than one tile of rows: none, the CTAs
-        // suffice, and the start and the end of a CTA cost as much as ten stages.
-        p.ways = 1;
-        while (tiles == 1 && p.ways < 4 && groups * p.ways * 2 <= 2 * ctx->sm_count && p.nst / (p.ways * 2) >= 4) p.ways *= 2;
         // Meeting costs 1 to 2 us, walking x and the scales beyond what the registers hold more than that with rows x stages.  One
         // CTA alone / together, us: 4096 x 4096 at one / eight rows 8.2 / 10.0 and 12.8 / 13.4; 5120 x 4096 at three / four / six
         // 12.0 / 12.6, 13.1 / 13.2, 15.0 / 14.0; 8192 x 4096 at two / four 13.2 / 13.9, 15.5 / 15.0; 11008 x 4096 at one / two /
         // eight 15.4 / 15.8, 16.6 / 16.5, 24.9 / 19.6; 14336 x 3008 at one / eight 16.5 / 16.0, 28.3 / 20.3.
         const bool meet = rpw == 1 && p.ways > 1 && p.nst > 32 && (p.M * p.nst >= 160 || p.nst > 96);
-        const size_t fixed = 1024 + (size_t)rb * A_BYTES + (4 * MAX_STAGES + 2) * 8 + (size_t)rb * 32 * 24 + (size_t)p.nst * 4 + 64;
-        const size_t budget = (ctx->smem_optin + 1024) / 2 - 1024;   // half an SM, less the 1 KiB every block pays
-        int stages = budget > fixed ? (int)((budget - fixed) / (STAGE_BYTES + S_BYTES)) : 0;
+        const size_t stage_bytes = wide ? W_IN + W_SC : STAGE_BYTES + S_BYTES;
+        const size_t fixed = wide ? 1024 + (size_t)2 * WG * W_ABUF + (2 * MAX_STAGES + 6) * 8 + (size_t)WG * WROWS * 20 + (size_t)WG * p.nst * 4 + 64
+                                  : 1024 + (size_t)A_BYTES + (4 * MAX_STAGES + 2) * 8 + (size_t)32 * 24 + (size_t)p.nst * 4 + 64;
+        const size_t budget = wide ? ctx->smem_optin : (ctx->smem_optin + 1024) / 2 - 1024;   // an SM, or half of it less the 1 KiB every block pays
+        int stages = budget > fixed ? (int)((budget - fixed) / stage_bytes) : 0;
         if (stages > MAX_STAGES) stages = MAX_STAGES;
-        if (stages < (rb == 1 ? MAX_STAGES : 4)) return fail(ctx, RUSTY_CUDA_ERR_UNSUPPORTED, "gc_tc: the ring does not fit shared memory");
+        if (stages < (wide ? 3 : MAX_STAGES)) return fail(ctx, RUSTY_CUDA_ERR_UNSUPPORTED, "gc_tc: the ring does not fit shared memory");
         p.stages = stages;
-        const size_t smem = fixed + (size_t)stages * (STAGE_BYTES + S_BYTES);
-        const dim3 grid((unsigned)(tiles * p.ways), (unsigned)groups);
-        cudaError_t e = rpw == 8   ? launch_gc<float, 2, 8>(ctx, map_w, p, grid, smem)
-                        : rpw == 4 ? launch_gc<float, 1, 4>(ctx, map_w, p, grid, smem)
-                        : rpw == 2 ? launch_gc<float, 1, 2>(ctx, map_w, p, grid, smem)
-                        : xb       ? (meet ? launch_gc<__nv_bfloat16, 1, 1, true>(ctx, map_w, p, grid, smem) : launch_gc<__nv_bfloat16, 1, 1>(ctx, map_w, p, grid, smem))
-                        : meet     ? launch_gc<float, 1, 1, true>(ctx, map_w, p, grid, smem)
-                                   : launch_gc<float, 1, 1>(ctx, map_w, p, grid, smem);
+        const size_t smem = fixed + (size_t)stages * stage_bytes;
+        const dim3 grid((unsigned)(tiles * p.ways), (unsigned)units);
+        cudaError_t e;
+        if (wide) {
+            e = rusty::ensure_dynamic_smem((const void*)qlinear_gc_wide_kernel, ctx->device, smem);
+            if (e == cudaSuccess) e = launch_pdl_cluster(qlinear_gc_wide_kernel, grid, dim3(W_THREADS), (unsigned)p.ways, smem, ctx->stream, map_w, p);
+        } else {
+            e = rpw == 4   ? launch_gc<float, 4>(ctx, map_w, p, grid, smem)
+                : rpw == 2 ? launch_gc<float, 2>(ctx, map_w, p, grid, smem)
+                : xb       ? (meet ? launch_gc<__nv_bfloat16, 1, true>(ctx, map_w, p, grid, smem) : launch_gc<__nv_bfloat16, 1>(ctx, map_w, p, grid, smem))
+                : meet     ? launch_gc<float, 1, true>(ctx, map_w, p, grid, smem)
+                           : launch_gc<float, 1>(ctx, map_w, p, grid, smem);
+        }
         if (e != cudaSuccess) return check_cuda(ctx, e, "qlinear_gc_tc");
         int rc = after_launch(ctx, "qlinear_gc_tc");
         if (rc) return rc;

@@ -536,6 +536,37 @@ def test_native_affine_batches(ctx, engine, oracle, M, K, N):
     assert np.isnan(got[0]).all() and np.isfinite(got[1:]).all()
 
 
+@pytest.mark.parametrize("M,K,N", [(33, 4096, 4160), (63, 4100, 10944), (200, 1412, 4160), (321, 772, 9664)])
+def test_native_affine_wide_tiles(ctx, engine, M, K, N):
+    """Tiles of 64 rows x two groups (an odd last group, cut along K and not, ragged rows and stages): outliers on small scales in every
+    stage, one group whose biases are no multiple of its scales, a row of zeros and an infinity; every row as alone."""
+    rng = np.random.default_rng(M + K + N)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    sg = rng.uniform(0.001, 0.02, size=(K, N // 64)).astype(np.float32)
+    at = np.arange(0, K, 128) + rng.integers(0, 4, size=(K + 127) // 128)
+    x[:, at] *= np.float32(1e6)
+    sg[at] *= np.float32(1e-6)
+    x[5] = 0.0
+    bg = (-128.0 * sg * rng.uniform(0.9, 1.1, size=sg.shape)).astype(np.float32)
+    bg[:, N // 64 - 2] *= 1e3
+    ukn = rng.integers(0, 256, size=(K, N), dtype=np.uint8)
+    ql = QLinear.from_host(ctx, ukn, sg, bg, layout=capi.LAYOUT_KN)
+    got = _forward(ctx, engine, ql, x)
+    wf = ukn.astype(np.float64) * np.repeat(sg.astype(np.float64), 64, axis=1) + np.repeat(bg.astype(np.float64), 64, axis=1)
+    exact = x.astype(np.float64) @ wf
+    live = np.arange(M) != 5
+    assert not got[5].any()
+    for g in (0, N // 128, N // 64 - 2, N // 64 - 1):
+        assert rel_err_rows(got[live, 64 * g:64 * g + 64], exact[live, 64 * g:64 * g + 64]) <= 1e-6
+    assert rel_err_rows(got[live], exact[live]) <= 1e-6
+    for m in (0, 32, M - 1):
+        assert_bits_equal(got[m:m + 1], _forward(ctx, engine, ql, x[m:m + 1]))
+    x[M - 1, 1] = np.inf
+    got2 = _forward(ctx, engine, ql, x)
+    assert np.isnan(got2[M - 1]).all()
+    assert_bits_equal(got2[:M - 1], got[:M - 1])
+
+
 @pytest.mark.parametrize("M,K,N", [(1, 4096, 64), (4, 11008, 64), (8, 4352, 128), (9, 4096, 64), (13, 8192, 128), (32, 4100, 64), (64, 4096, 192), (65, 4096, 64), (150, 2112, 128)])
 @pytest.mark.parametrize("outliers", ["one", "per_stage"])
 def test_native_affine_outliers_on_small_scales(ctx, engine, M, K, N, outliers):
