@@ -90,7 +90,12 @@ __device__ __forceinline__ float4 load_row4<__nv_bfloat16>(const __nv_bfloat16* 
 
 constexpr int DIG_THREADS = 512;
 constexpr int DIG_MAX_BLOCKS = 32;
-constexpr int DIG_MAXV = 8;   // passes of a row held in registers between the maximum and the digits
+constexpr int DIG_MAXV = 8;   // most passes of a row held in registers
+// planes: f32 activations 4, 31 bits below the row maximum.  Three (23 bits) hold the fp32 tolerance only while the row's largest element
+// stays within ~25x of its rms: with one outlier of 1000x every other element keeps 13 bits and the result is too far off.  bf16
+// activations carry 8 significant bits each: 3.
+template <typename XT>
+constexpr int DIG_PLANES = sizeof(XT) == 4 ? 4 : 3;
 
 // A few fat blocks on purpose: grid = min(32, Mpad) blocks of 512 threads, R = Mpad / grid activation rows per block
 // (1 or 2), 512 / R threads per row (its own named barrier).  The kernel is launched early (programmatic dependent
@@ -103,13 +108,16 @@ constexpr int DIG_MAXV = 8;   // passes of a row held in registers between the m
 // NORM: the activations are RMSNorm(x [+ residual]) * weight (norm_embed.cu gives the formula and its lines in the
 // reference); the row is normalised in registers between the load and the maximum, so it must fit there
 // (K <= DIG_MAXV * 4 * threads of the row), and the normalised row and the sum are written out where asked for.
-template <typename XT, int D, bool NORM, bool SPLIT>
+// V: passes of a row held in registers between the maximum and the digits, 2, 4 or 8 (a kernel that runs for 1.5 us is paid by the
+// instruction: with eight for all 4096 x 4096 took 11.2 us instead of 10.7 at 32 rows, 10.4 instead of 9.6 at 16).
+template <typename XT, int V, bool NORM, bool SPLIT>
 __global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* x, int8_t* __restrict__ xq,
                                                                     float* __restrict__ inv_s, int M, int Mpad, int K, int R,
                                                                     const PeerPush push, const NormArgs nrm, long long* dbg) {
     __shared__ float red[DIG_THREADS / 32];
     __shared__ float red_ss[DIG_THREADS / 32];
     __shared__ uint32_t part_max[2];
+    constexpr int D = DIG_PLANES<XT>;
     const int tid = threadIdx.x;
     const int part = SPLIT ? (int)blockIdx.x & 1 : 0;         // SPLIT: which half of the row (R = 1)
     const int k0 = part ? K / 8 * 4 : 0, k1 = SPLIT && !part ? K / 8 * 4 : K;
@@ -137,16 +145,16 @@ __global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* x,
         return;   // whole row groups (and clusters) leave together: the named barrier below is per group
     }
     const XT* xr = x + (size_t)m * K;
-    float4 v[DIG_MAXV];
+    float4 v[V];
 #pragma unroll
-    for (int j = 0; j < DIG_MAXV; ++j) {
+    for (int j = 0; j < V; ++j) {
         const int k = k0 + tg * 4 + j * step;
         v[j] = k < k1 ? load_row4<XT>(xr + k) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if constexpr (NORM) {
         float ss = 0.0f;
 #pragma unroll
-        for (int j = 0; j < DIG_MAXV; ++j) {
+        for (int j = 0; j < V; ++j) {
             const int k = k0 + tg * 4 + j * step;
             if (k < k1) {
                 if (nrm.residual) {
@@ -168,7 +176,7 @@ __global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* x,
         for (int off = 4; off > 0; off >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, off);
         const float inv_rms = 1.0f / sqrtf(tot / (float)K + nrm.eps);
 #pragma unroll
-        for (int j = 0; j < DIG_MAXV; ++j) {
+        for (int j = 0; j < V; ++j) {
             const int k = k0 + tg * 4 + j * step;
             if (k < k1) {
                 const float4 w = __ldg(reinterpret_cast<const float4*>(nrm.weight + k));
@@ -184,8 +192,8 @@ __global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* x,
                          max(__float_as_uint(f.z) & 0x7fffffffu, __float_as_uint(f.w) & 0x7fffffffu)));
     };
 #pragma unroll
-    for (int j = 0; j < DIG_MAXV; ++j) fold(v[j]);
-    for (int k = k0 + tg * 4 + DIG_MAXV * step; k < k1; k += step) fold(load_row4<XT>(xr + k));
+    for (int j = 0; j < V; ++j) fold(v[j]);
+    for (int k = k0 + tg * 4 + V * step; k < k1; k += step) fold(load_row4<XT>(xr + k));
     mx = __reduce_max_sync(0xffffffffu, mx);
     if ((tid & 31) == 0) red[tid >> 5] = __uint_as_float(mx);
     asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(tpr) : "memory");   // the row's threads only
@@ -224,11 +232,11 @@ __global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* x,
         for (int d = 0; d < D; ++d) *reinterpret_cast<uint32_t*>(xq + (size_t)(d * Mpad + mq) * K + k) = by[D - 1 - d];
     };
 #pragma unroll
-    for (int j = 0; j < DIG_MAXV; ++j) {
+    for (int j = 0; j < V; ++j) {
         const int k = k0 + tg * 4 + j * step;
         if (k < k1) turn(v[j], k);
     }
-    for (int k = k0 + tg * 4 + DIG_MAXV * step; k < k1; k += step) turn(load_row4<XT>(xr + k), k);
+    for (int k = k0 + tg * 4 + V * step; k < k1; k += step) turn(load_row4<XT>(xr + k), k);
     PDBG(tid == 0 && blockIdx.x == 0, 2);
 }
 
@@ -900,16 +908,10 @@ void plan_tc_schedule(int tiles, int kb_total, int sm_count, int dp_percent, siz
     *out = s;
 }
 
-int pick_digits(int x_dtype, uint32_t rows) {
-    // f32 activations: 4 planes = 31 bits below the row maximum.  Three planes (23 bits) hold the fp32 tolerance only
-    // while the row's largest element stays within ~25x of its rms: with one outlier of 1000x every other element
-    // keeps 13 bits and the result is too far off.  bf16 activations carry 8 significant bits each: 3 planes.
-    (void)rows;
-    return x_dtype == RUSTY_CUDA_F32 ? 4 : 3;
-}
+int pick_digits(int x_dtype) { return x_dtype == RUSTY_CUDA_F32 ? DIG_PLANES<float> : DIG_PLANES<__nv_bfloat16>; }
 
 template <typename XT>
-cudaError_t launch_digitize(cudaStream_t stream, const void* x, int8_t* xq, float* inv_s, int M, int Mpad, int nblk, int K, int D,
+cudaError_t launch_digitize(cudaStream_t stream, const void* x, int8_t* xq, float* inv_s, int M, int Mpad, int nblk, int K,
                             const PeerPush& push, long long* dbg, const NormArgs* norm = nullptr) {
     // Mpad is a multiple of 8 and at most 64: one row per block up to 32 rows, two beyond; several row blocks (a prompt, where
     // the GEMM is long): one row per block
@@ -924,10 +926,16 @@ cudaError_t launch_digitize(cudaStream_t stream, const void* x, int8_t* xq, floa
     auto go = [&](auto kern, const NormArgs& n) {
         return launch_pdl_cluster(kern, grid, dim3(DIG_THREADS), (unsigned)cs, 0, stream, (const XT*)x, xq, inv_s, M, Mpad, K, R, push, n, dbg);
     };
+    const int passes = (K / cs + 4 * (DIG_THREADS / R) - 1) / (4 * (DIG_THREADS / R));
     if constexpr (std::is_same<XT, float>::value)
-        if (norm) return D == 4 ? go(digitize_x_kernel<XT, 4, true, false>, *norm) : go(digitize_x_kernel<XT, 3, true, false>, *norm);   // (K <= 16384)
-    if (cs == 2) return D == 4 ? go(digitize_x_kernel<XT, 4, false, true>, NormArgs{}) : go(digitize_x_kernel<XT, 3, false, true>, NormArgs{});
-    return D == 4 ? go(digitize_x_kernel<XT, 4, false, false>, NormArgs{}) : go(digitize_x_kernel<XT, 3, false, false>, NormArgs{});
+        if (norm)   // (K <= 16384: not split)
+            return passes <= 2   ? go(digitize_x_kernel<XT, 2, true, false>, *norm)
+                   : passes <= 4 ? go(digitize_x_kernel<XT, 4, true, false>, *norm)
+                                 : go(digitize_x_kernel<XT, 8, true, false>, *norm);
+    if (cs == 2) return go(digitize_x_kernel<XT, 8, false, true>, NormArgs{});
+    return passes <= 2   ? go(digitize_x_kernel<XT, 2, false, false>, NormArgs{})
+           : passes <= 4 ? go(digitize_x_kernel<XT, 4, false, false>, NormArgs{})
+                         : go(digitize_x_kernel<XT, 8, false, false>, NormArgs{});
 }
 
 }  // namespace
@@ -1026,7 +1034,7 @@ bool tc_norm_fused(uint32_t M, uint32_t K) {
 // One launch pair (digitise + GEMM) for `rows` activation rows in `nblk` equal blocks of at most 64.
 static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void* x, void* y, uint32_t rows, int nblk, const NormArgs* norm) {
     const int M = (int)rows, Mpad = ((M + nblk - 1) / nblk + 7) / 8 * 8;
-    const int D = pick_digits(a.x_dtype, rows);
+    const int D = pick_digits(a.x_dtype);
     const int NB = (D * Mpad + 15) / 16 * 16;
     uint8_t* ws = (uint8_t*)ctx->tc_ws;
     int8_t* xq = (int8_t*)ws;
@@ -1050,8 +1058,8 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
     {
         if (norm && (a.x_dtype != RUSTY_CUDA_F32 || !tc_norm_fused(a.M, a.K)))
             return fail(ctx, RUSTY_CUDA_ERR_INVALID_OPERATION, "qlinear_forward: the norm cannot be applied by this call's pre-pass");
-        le = a.x_dtype == RUSTY_CUDA_BF16 ? launch_digitize<__nv_bfloat16>(ctx->stream, x, xq, inv_s, M, Mpad, nblk, (int)a.K, D, push, dbg ? dbg + 150 * 16 : nullptr)
-                                          : launch_digitize<float>(ctx->stream, x, xq, inv_s, M, Mpad, nblk, (int)a.K, D, push, dbg ? dbg + 150 * 16 : nullptr, norm);
+        le = a.x_dtype == RUSTY_CUDA_BF16 ? launch_digitize<__nv_bfloat16>(ctx->stream, x, xq, inv_s, M, Mpad, nblk, (int)a.K, push, dbg ? dbg + 150 * 16 : nullptr)
+                                          : launch_digitize<float>(ctx->stream, x, xq, inv_s, M, Mpad, nblk, (int)a.K, push, dbg ? dbg + 150 * 16 : nullptr, norm);
         if (le != cudaSuccess) return check_cuda(ctx, le, "digitize_x");
         rc = after_launch(ctx, "digitize_x");
         if (rc) return rc;
@@ -1320,7 +1328,7 @@ extern "C" RUSTY_CUDA_API int rusty_cuda_qlinear_i8_forward_static(const void* w
     if (e != cudaSuccess) return check_cuda(nullptr, e, "qlinear_i8_forward_static: clearing the scratch");
 
     const int Mi = (int)M, Mpad = 8, D = 4, NB = 32;
-    e = launch_digitize<float>(st, x_f32, xq, factor, Mi, Mpad, 1, (int)K, D, PeerPush{}, nullptr);
+    e = launch_digitize<float>(st, x_f32, xq, factor, Mi, Mpad, 1, (int)K, PeerPush{}, nullptr);
     if (e != cudaSuccess) return check_cuda(nullptr, e, "qlinear_i8_forward_static: digitize_x");
 
     TcParams p{};
