@@ -414,6 +414,12 @@ RUSTY_CUDA_API int rusty_cuda_softmax_stats_rows_f32(rusty_cuda_ctx* ctx, const 
 RUSTY_CUDA_API int rusty_cuda_sampler_candidates_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf* logits, uint32_t M, uint32_t N, uint32_t k,
                                                      float temperature, uint32_t* host_idx, float* host_val, float* host_max,
                                                      float* host_sum);
+/* Temperature / top-p sampling of one token per row on the device (Sampler::sample, rusty-loader/src/tokenizer.rs:161-204, in f32 and in
+ * its order of operations), over the row's k largest logits: host_draws[m] in [0, 1) is the row's random number, host_tokens[m] the
+ * token, or 0xffffffff where the k largest do not hold top_p of the probability (the host then draws from the whole row).
+ * Blocking, like the call above. */
+RUSTY_CUDA_API int rusty_cuda_sample_top_p_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf* logits, uint32_t M, uint32_t N, uint32_t k,
+                                               float temperature, float top_p, const float* host_draws, uint32_t* host_tokens);
 /* top_k over output-feature shards: every rank passes its own columns [M, Nl] (global index = rank * Nl + column);
  * only k (value, index) pairs per row and rank cross NVLink, every rank ends with the k global winners.
  * table: a buffer of the arena, nranks * M * k * 8 bytes, at the same offset on every rank.  k * nranks <= 2048. */

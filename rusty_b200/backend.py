@@ -401,6 +401,19 @@ class ComputeEngine:
                                                       val.ctypes.data, mx.ctypes.data, sm.ctypes.data), ctx.handle)
         return idx, val, mx, sm
 
+    def sample_top_p(self, ctx: CudaContext, input: UnifiedTensor, k: int, temperature: float, top_p: float, draws: np.ndarray):
+        """One token of every row of input[..., N] as u32 [M], drawn from its k largest logits by draws[M] (f32 in [0, 1)); 0xffffffff
+        where those hold less than top_p of the probability; blocking."""
+        N = int(input.shape[-1])
+        M = math.prod(input.shape[:-1])
+        draws = np.ascontiguousarray(draws, np.float32)
+        if draws.shape != (M,):
+            raise ValueError(f"sample_top_p: {M} draws needed, {draws.shape} given")
+        tokens = np.empty(M, np.uint32)
+        check(lib().rusty_cuda_sample_top_p_f32(ctx.handle, input.buffer(), M, N, k, float(temperature), float(top_p), draws.ctypes.data,
+                                                tokens.ctypes.data), ctx.handle)
+        return tokens
+
     def qlinear(self, ctx: CudaContext, x: UnifiedTensor, w: QLinear, out: UnifiedTensor) -> None:
         """out[M,N] = x[M,K] (.) w, fused dequantise + multiply."""
         m = int(math.prod(x.shape[:-1]))

@@ -230,15 +230,26 @@ __device__ __forceinline__ uint32_t stat_key_of(float v) {
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
+// The draw of temperature / top-p sampling from the row's k winners (Sampler::sample, rusty-loader/src/tokenizer.rs:161-204): in f32 and in
+// the reference's order of operations.  One token per row instead of k pairs: the walk over them on the host, in numpy, took 60 us
+// for 32 rows.
+constexpr uint32_t NO_TOKEN = 0xffffffffu;     // the winners' probabilities do not reach top_p: the row has to be drawn from as a whole
+struct DrawArgs {
+    const float* draws;    // [M] uniform numbers in [0, 1); null: no draw
+    uint32_t* tokens;      // [M]
+    float temperature, top_p;
+};
+
 __global__ void __launch_bounds__(RC_THREADS) logits_rows_kernel(const float* x, int n, size_t ld, int k, int glog,
                                                                  unsigned int* __restrict__ out_idx, float* __restrict__ out_val,
-                                                                 float inv_t, float* __restrict__ out_max, float* __restrict__ out_sum) {
+                                                                 float inv_t, float* __restrict__ out_max, float* __restrict__ out_sum, const DrawArgs draw) {
     extern __shared__ __align__(16) unsigned char row_smem[];
     RowShared& sh = *reinterpret_cast<RowShared*>(row_smem);
     cg::cluster_group cl = cg::this_cluster();
     const unsigned S = cl.num_blocks(), r = cl.block_rank(), m = blockIdx.x / S;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool stats = out_sum != nullptr;
+    const bool stats = out_sum != nullptr || draw.draws != nullptr;
+    const float rnd = draw.draws && r == 0 && tid == 0 ? draw.draws[m] : 0.0f;     // (from host memory: asked for early)
     if (tid == 0) sh.count = 0u;
     pdl_launch_dependents();
     cl.barrier_arrive();          // the blocks of the cluster have started and cleared their counters (waited for below)
@@ -313,16 +324,23 @@ __global__ void __launch_bounds__(RC_THREADS) logits_rows_kernel(const float* x,
     }
     cl.sync();
     if (r != 0) return;
-    if (stats && tid == 0) {
-        float t = 0.0f;
-        for (unsigned b = 0; b < S; ++b) t += sh.sum_of[b];
-        out_max[m] = mx;
-        out_sum[m] = t;
+    float total = 0.0f;
+    if (stats) {
+        for (unsigned b = 0; b < S; ++b) total += sh.sum_of[b];
+        if (tid == 0 && out_sum) {
+            out_max[m] = mx;
+            out_sum[m] = total;
+        }
     }
     if (k == 0) return;
     unsigned int* oi = out_idx + (size_t)m * k;
     float* ov = out_val ? out_val + (size_t)m * k : nullptr;
+    unsigned long long* sorted = sh.u.s.sorted;           // (draw: where the group maxima were)
     auto put = [&](int at, unsigned long long it) {
+        if (draw.draws) {
+            sorted[at] = it;
+            return;
+        }
         oi[at] = it ? 0xffffffffu - (uint32_t)(it & 0xffffffffull) : 0u;
         if (ov) ov[at] = it ? value_of((uint32_t)(it >> 32)) : __int_as_float(0xff800000);
     };
@@ -335,32 +353,75 @@ __global__ void __launch_bounds__(RC_THREADS) logits_rows_kernel(const float* x,
             if (rank < k) put(rank, mine);
         }
         for (int i = (int)C + tid; i < k; i += RC_THREADS) put(i, 0ull);
-        return;
-    }
-    const unsigned long long* winners;
-    if (C <= (uint32_t)RC_CAP) {
+    } else if (C <= (uint32_t)RC_CAP) {
         int P = 1;
         while (P < (int)C) P <<= 1;
         for (int i = (int)C + tid; i < P; i += RC_THREADS) sh.cand[i] = 0ull;
         bitonic_desc(sh.cand, P);
-        winners = sh.cand;
+        for (int i = tid; i < k; i += RC_THREADS) put(i, sh.cand[i]);
     } else {
-        radix_topk<RC_THREADS>(row, n, 0u, k, sh.u.s.sorted, sh.u.s.radix);
-        winners = sh.u.s.sorted;
+        radix_topk<RC_THREADS>(row, n, 0u, k, sorted, sh.u.s.radix);
+        if (!draw.draws)
+            for (int i = tid; i < k; i += RC_THREADS) put(i, sorted[i]);
     }
-    for (int i = tid; i < k; i += RC_THREADS) put(i, winners[i]);
+    if (!draw.draws) return;
+    __syncthreads();
+    float* probs = reinterpret_cast<float*>(sh.cand);     // [k]
+    uint32_t idx[TK_MAX_K / RC_THREADS];
+    float prob[TK_MAX_K / RC_THREADS];
+    const float top = __fdiv_rn(mx, draw.temperature);
+#pragma unroll
+    for (int u = 0; u < TK_MAX_K / RC_THREADS; ++u) {
+        const int i = tid + u * RC_THREADS;
+        const unsigned long long it = i < k ? sorted[i] : 0ull;
+        idx[u] = it ? 0xffffffffu - (uint32_t)(it & 0xffffffffull) : 0u;
+        const float v = it ? value_of((uint32_t)(it >> 32)) : __int_as_float(0xff800000);
+        prob[u] = __fdiv_rn(expf(__fdiv_rn(v, draw.temperature) - top), total);
+    }
+    __syncthreads();                                       // (the candidates and the sorted items have been read)
+    uint32_t* index = reinterpret_cast<uint32_t*>(sorted);
+#pragma unroll
+    for (int u = 0; u < TK_MAX_K / RC_THREADS; ++u) {
+        const int i = tid + u * RC_THREADS;
+        if (i < k) {
+            probs[i] = prob[u];
+            index[i] = idx[u];
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        float cum = 0.0f;
+        int last = -1;
+        for (int i = 0; i < k && last < 0; ++i) {
+            cum = __fadd_rn(cum, probs[i]);
+            if (cum >= draw.top_p) last = i;
+        }
+        uint32_t token = NO_TOKEN;
+        if (last >= 0) {
+            token = index[0];
+            float c = 0.0f;
+            for (int i = 0; i <= last; ++i) {
+                c = __fadd_rn(c, __fdiv_rn(probs[i], cum));
+                if (rnd < c) {
+                    token = index[i];
+                    break;
+                }
+            }
+        }
+        draw.tokens[m] = token;
+    }
 }
 
 // k == 0: no top-k; out_sum == null: no statistics.
 cudaError_t launch_logits_rows(rusty_cuda_ctx* ctx, const float* x, uint32_t M, uint32_t N, uint32_t k, unsigned int* out_idx, float* out_val,
-                               float temperature, float* out_max, float* out_sum) {
+                               float temperature, float* out_max, float* out_sum, const DrawArgs& draw = DrawArgs{}) {
     const unsigned S = row_cluster(M, N, ctx->sm_count);
     int glog = 5;
     while (glog > 0 && (uint64_t)S * (RC_THREADS >> glog) < 2ull * k) --glog;
     cudaError_t e = ensure_dynamic_smem((const void*)logits_rows_kernel, ctx->device, sizeof(RowShared));
     if (e != cudaSuccess) return e;
     return launch_pdl_cluster(logits_rows_kernel, dim3(M * S), dim3(RC_THREADS), S, sizeof(RowShared), ctx->stream, x, (int)N, (size_t)N, (int)k,
-                              glog, out_idx, out_val, out_sum ? 1.0f / temperature : 0.0f, out_max, out_sum);
+                              glog, out_idx, out_val, out_sum || draw.draws ? 1.0f / temperature : 0.0f, out_max, out_sum, draw);
 }
 
 // Sharded, second half: once every rank's candidates have landed, the best k of the G x k items of each row.
@@ -439,20 +500,18 @@ int rusty_cuda_softmax_stats_rows_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf*
     return after_launch(ctx, "softmax_stats_rows");
 }
 
-int rusty_cuda_sampler_candidates_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf* logits, uint32_t M, uint32_t N, uint32_t k, float temperature,
-                                      uint32_t* host_idx, float* host_val, float* host_max, float* host_sum) {
-    RUSTY_REQUIRE_CTX(ctx);
-    if (!logits || !host_idx || !host_val || !host_max || !host_sum)
-        return fail(ctx, RUSTY_CUDA_ERR_INVALID_OPERATION, "sampler_candidates: null argument");
-    if (ctx->capturing) return fail(ctx, RUSTY_CUDA_ERR_INVALID_OPERATION, "sampler_candidates: not allowed while a graph capture is open");
-    if (!(temperature > 0.0f)) return fail(ctx, RUSTY_CUDA_ERR_INVALID_OPERATION, "sampler_candidates: temperature must be > 0 (greedy choice is argmax_rows)");
-    if (k == 0 || k > (uint32_t)TK_MAX_K) return fail(ctx, RUSTY_CUDA_ERR_INVALID_DIMENSIONS, "sampler_candidates: k=%u must lie in 1..%d", k, TK_MAX_K);
-    if (N > 0x7fffffffu) return fail(ctx, RUSTY_CUDA_ERR_INVALID_DIMENSIONS, "sampler_candidates: N=%u too large", N);
+// What both calls for a sampling host check.
+static int sampler_check(rusty_cuda_ctx* ctx, const char* op, const rusty_cuda_buf* logits, uint32_t M, uint32_t N, uint32_t k, float temperature) {
+    if (ctx->capturing) return fail(ctx, RUSTY_CUDA_ERR_INVALID_OPERATION, "%s: not allowed while a graph capture is open", op);
+    if (!(temperature > 0.0f)) return fail(ctx, RUSTY_CUDA_ERR_INVALID_OPERATION, "%s: temperature must be > 0 (greedy choice is argmax_rows)", op);
+    if (k == 0 || k > (uint32_t)TK_MAX_K) return fail(ctx, RUSTY_CUDA_ERR_INVALID_DIMENSIONS, "%s: k=%u must lie in 1..%d", op, k, TK_MAX_K);
+    if (N > 0x7fffffffu) return fail(ctx, RUSTY_CUDA_ERR_INVALID_DIMENSIONS, "%s: N=%u too large", op, N);
     if (logits->bytes < (size_t)M * N * 4)
-        return fail(ctx, RUSTY_CUDA_ERR_INVALID_DIMENSIONS, "sampler_candidates: [%u,%u] logits need %zu bytes", M, N, (size_t)M * N * 4);
-    if (M == 0) return RUSTY_CUDA_OK;
-    DeviceGuard g(ctx->device);
-    const size_t pairs = (size_t)M * k, need = pairs * 8 + (size_t)M * 8;
+        return fail(ctx, RUSTY_CUDA_ERR_INVALID_DIMENSIONS, "%s: [%u,%u] logits need %zu bytes", op, M, N, (size_t)M * N * 4);
+    return RUSTY_CUDA_OK;
+}
+// The context's pinned staging memory, of `need` bytes at least, and its address on the device.
+static int sampler_stage(rusty_cuda_ctx* ctx, const char* op, size_t need, void** dev) {
     if (ctx->host_stage_bytes < need) {
         if (ctx->host_stage) cudaFreeHost(ctx->host_stage);   // (nothing in flight uses it: every use ends with a wait)
         ctx->host_stage = nullptr;
@@ -461,13 +520,24 @@ int rusty_cuda_sampler_candidates_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf*
         if (e != cudaSuccess) {
             cudaGetLastError();
             ctx->host_stage = nullptr;
-            return fail(ctx, RUSTY_CUDA_ERR_MEMORY_ALLOCATION, "sampler_candidates: pinned staging of %zu bytes", need);
+            return fail(ctx, RUSTY_CUDA_ERR_MEMORY_ALLOCATION, "%s: pinned staging of %zu bytes", op, need);
         }
         ctx->host_stage_bytes = need;
     }
+    return check_cuda(ctx, cudaHostGetDevicePointer(dev, ctx->host_stage, 0), "sampler: staging");
+}
+
+int rusty_cuda_sampler_candidates_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf* logits, uint32_t M, uint32_t N, uint32_t k, float temperature,
+                                      uint32_t* host_idx, float* host_val, float* host_max, float* host_sum) {
+    RUSTY_REQUIRE_CTX(ctx);
+    const char* op = "sampler_candidates";
+    if (!logits || !host_idx || !host_val || !host_max || !host_sum) return fail(ctx, RUSTY_CUDA_ERR_INVALID_OPERATION, "%s: null argument", op);
+    int rc = sampler_check(ctx, op, logits, M, N, k, temperature);
+    if (rc || M == 0) return rc;
+    DeviceGuard g(ctx->device);
+    const size_t pairs = (size_t)M * k;
     void* dev = nullptr;
-    int rc = check_cuda(ctx, cudaHostGetDevicePointer(&dev, ctx->host_stage, 0), "sampler_candidates: staging");
-    if (rc) return rc;
+    if ((rc = sampler_stage(ctx, op, pairs * 8 + (size_t)M * 8, &dev))) return rc;
     // one kernel, whose last block per row stores the results into host memory: no copies behind it
     unsigned int* d_idx = (unsigned int*)dev;
     float *d_val = (float*)(d_idx + pairs), *d_max = d_val + pairs, *d_sum = d_max + M;
@@ -480,6 +550,27 @@ int rusty_cuda_sampler_candidates_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf*
     memcpy(host_val, h + pairs * 4, pairs * 4);
     memcpy(host_max, h + pairs * 8, (size_t)M * 4);
     memcpy(host_sum, h + pairs * 8 + (size_t)M * 4, (size_t)M * 4);
+    return RUSTY_CUDA_OK;
+}
+
+int rusty_cuda_sample_top_p_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf* logits, uint32_t M, uint32_t N, uint32_t k, float temperature, float top_p,
+                                const float* host_draws, uint32_t* host_tokens) {
+    RUSTY_REQUIRE_CTX(ctx);
+    const char* op = "sample_top_p";
+    if (!logits || !host_draws || !host_tokens) return fail(ctx, RUSTY_CUDA_ERR_INVALID_OPERATION, "%s: null argument", op);
+    int rc = sampler_check(ctx, op, logits, M, N, k, temperature);
+    if (rc || M == 0) return rc;
+    DeviceGuard g(ctx->device);
+    void* dev = nullptr;
+    if ((rc = sampler_stage(ctx, op, (size_t)M * 8, &dev))) return rc;
+    memcpy(ctx->host_stage, host_draws, (size_t)M * 4);
+    uint32_t* tokens = (uint32_t*)dev + M;
+    cudaError_t e = launch_logits_rows(ctx, (const float*)logits->ptr, M, N, k, nullptr, nullptr, temperature, nullptr, nullptr,
+                                       DrawArgs{(const float*)dev, tokens, temperature, top_p});
+    if (e != cudaSuccess) return check_cuda(ctx, e, op);
+    if ((rc = after_launch(ctx, op))) return rc;
+    if ((rc = rusty_cuda_sync(ctx))) return rc;
+    memcpy(host_tokens, (const char*)ctx->host_stage + (size_t)M * 4, (size_t)M * 4);
     return RUSTY_CUDA_OK;
 }
 

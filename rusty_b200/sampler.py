@@ -1,11 +1,11 @@
 """Host-side mirror of rusty-loader's Sampler (rusty-loader/src/tokenizer.rs:134-204).
 
 Greedy choice (temperature <= 0) also exists on the device (`ComputeEngine.argmax_rows`, sharded form in
-`rusty_b200.shard`); temperature / top-p sampling stays on the host, as in the reference, in f32 arithmetic and in the
+`rusty_b200.shard`); `Sampler.sample` is the reference's temperature / top-p sampling, in f32 arithmetic and in the
 reference's order of operations: scale by 1/temperature, soft-max with the maximum subtracted, sort by probability
 (descending, stable), take the shortest prefix whose sum reaches top_p, renormalise, draw.  `sample_rows_from_device`
-does the same walk over the k largest logits of each row and the row's soft-max statistics, both computed on the
-device, so that k pairs and two floats per row cross PCIe instead of the whole vocabulary; a row whose nucleus does not
+has the same walk done on the device, over the k largest logits of each row and the row's soft-max statistics, so that
+one number goes there and one token comes back per row instead of the whole vocabulary; a row whose nucleus does not
 fit into k falls back to reading its logits.
 """
 from __future__ import annotations
@@ -87,7 +87,8 @@ class Sampler:
 
     def sample_rows_from_device(self, ctx, engine, logits, k: int = 64):
         """One token per row of a device tensor logits[M, N] (f32).  temperature <= 0: the device arg-max.  Otherwise
-        the device's top-k and soft-max statistics, then the reference's nucleus walk on the host."""
+        the reference's nucleus walk on the device, over the k largest logits and the row's soft-max statistics; a row whose
+        nucleus is longer than k is sampled from its whole logits, here.  One number is drawn per row, in row order."""
         from .backend import DType, UnifiedTensor
         M, N = math.prod(logits.shape[:-1]), int(logits.shape[-1])
         if self.temperature <= 0.0:
@@ -95,38 +96,13 @@ class Sampler:
             engine.argmax_rows(ctx, logits, tok)
             return [int(t) for t in tok.to_bytes(ctx).view(np.uint32)]
         k = max(1, min(int(k), N, 1024))
-        idx, val, mx, sm = engine.sampler_candidates(ctx, logits, k, float(self.temperature))
-        return self._walk_rows(idx, val, mx, sm, lambda: logits.to_vec(ctx).reshape(M, N))
-
-    def _walk_rows(self, idx, val, row_max, exp_sum, host_logits):
-        """`sample_from_candidates` for all rows at once, with the same f32 arithmetic in the same order (np.cumsum adds
-        an f32 row from left to right) and the same order of draws; `host_logits` fetches the rows of nuclei longer
-        than k."""
-        t = self.temperature
-        scaled = val / t                                                         # f32 throughout
-        probs = np.exp(scaled - (row_max / t)[:, None]) / exp_sum[:, None]
-        cum = np.cumsum(probs, axis=1, dtype=np.float32)
-        reached = cum >= self.top_p
-        last = reached.argmax(axis=1)                                            # the first candidate that reaches top_p
-        rows = np.arange(len(idx))
-        found = reached[rows, last]
-        steps = np.cumsum(probs / cum[rows, last][:, None], axis=1, dtype=np.float32)
-        out = []
+        rand = self._rand
+        draws = np.array([rand() for _ in range(M)], np.float32)
+        out = engine.sample_top_p(ctx, logits, k, float(self.temperature), float(self.top_p), draws).tolist()
         fetched = None
-        rand, pick = self._rand, last + 1
-        if found.all():                                                          # no row draws from its whole logits
-            draws = np.array([rand() for _ in rows], np.float32)
-            below = draws[:, None] < steps
-            at = below.argmax(axis=1)
-            at[~(below[rows, at] & (at < pick))] = 0
-            return idx[rows, at].tolist()
-        for m in rows:
-            if not found[m]:   # the nucleus is longer than k: the reference's own path over the whole row
+        for m, token in enumerate(out):
+            if token == 0xFFFFFFFF:
                 if fetched is None:
-                    fetched = host_logits()
-                out.append(self.sample(fetched[m]))
-                continue
-            r = np.float32(rand())
-            at = int(np.argmax(r < steps[m]))
-            out.append(int(idx[m, at if r < steps[m, at] and at < pick[m] else 0]))
+                    fetched = logits.to_vec(ctx).reshape(M, N)
+                out[m] = Sampler(self.temperature, self.top_p, rand=lambda: draws[m]).sample(fetched[m])
         return out
