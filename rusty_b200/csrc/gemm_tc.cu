@@ -265,6 +265,7 @@ struct TcParams {
     int act;                 // RUSTY_CUDA_ACT_SWIGLU_PAIRS: rows 2j, 2j+1 -> y[:, (y_col0 + 2j) / 2] = silu(gate) * up
     int epi_warps;           // 4 or 8 epilogue warps: two per tensor-memory lane quarter split the activation rows between them
     int stages;
+    int prefetch;            // stages behind the ring's that are asked into L2 before the digits are there
     int red_bytes;           // epilogue staging area: 8 rows x 128 x 8 bytes for every four epilogue warps
     uint32_t idesc;
     uint32_t tmem_cols;
@@ -500,6 +501,18 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                 }
             }
         };
+        // What the ring does not hold yet goes into L2 while the digits are made.
+        auto prefetch = [&](Sched<PAIR> walk, Segment e, int kb) {
+            for (int n = 0; n < p.prefetch;) {
+                int w_row, x_row;
+                split_tile<BLOCKS>(p, e.t, w_row, x_row);
+                for (; kb < e.kb1 && n < p.prefetch; ++kb, ++n)
+                    if (elect_one()) tma_prefetch_2d(&map_w, kb * BK, unit_row(w_row));
+                if (n >= p.prefetch || !walk.next(e)) break;
+                kb = e.kb0;
+            }
+            __syncwarp();
+        };
         bool waited = false;
         while (ok && sched.next(sg)) {
             int w_row, x_row;
@@ -510,6 +523,7 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                 const bool ahead = !waited && early < p.stages;
                 if (!ahead) {
                     if (!waited) {
+                        prefetch(sched, sg, kb);
                         late_digits();
                         waited = true;
                     }
@@ -1164,6 +1178,10 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
     if (stages > 8) stages = 8;
     if (stages < 2) return fail(ctx, RUSTY_CUDA_ERR_UNSUPPORTED, "tensor-core path: tile does not fit shared memory");
     p.stages = stages;
+    // Eight stages where tiles are taken whole (32 x 4096 x 28672 26.8 -> 25.8 us, 16 rows 25.1 -> 23.8, 32 x 4096 x 128256 87.4 -> 84.5; sixteen:
+    // 25.8, 24.7, 84.3), four where they are cut (32 x 14336 x 4096 20.0 -> 19.7; eight 19.7, sixteen 20.2).  Not for row blocks, whose
+    // CTAs share the weights.
+    p.prefetch = nblk > 1 ? 0 : p.dp_tiles > 0 ? 8 : 4;
     p.red_bytes = (int)red_bytes;
     const size_t smem = 1024 + (size_t)stages * (a_stage + b_stage) + red_bytes + (size_t)(2 * stages + 4) * 8 + 256 + rowf_bytes;
 
