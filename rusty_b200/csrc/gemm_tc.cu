@@ -253,7 +253,7 @@ struct TcParams {
     int M, Mpad, D, NB;      // NB = UMMA N = roundup16(D*Mpad)
     int nblk;                // blocks of Mpad activation rows; tile t is row tile t / nblk of the weight, row block t % nblk
     int N, K;
-    int tpu, bmu;            // row tiles of 128 per work unit (1 or 2: two tiles share every digit tile they multiply), rows per unit
+    int tpu, bmu;            // row tiles of 128 per work unit (1 or 2: two tiles share every digit tile they multiply), rows per unit and CTA (tpu = 1: 128 or less)
     int tiles, kb_total;     // work units (called tiles below), k-blocks per unit
     // Schedule.  The last `sk_tiles` row tiles are cut stream-K fashion: their
     // sk_tiles*kb_total k-blocks form one linear space dealt out in contiguous
@@ -407,7 +407,7 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
     const int nb_cta = PAIR ? p.NB / 2 : p.NB;      // digit rows of a stage that this CTA holds
     const int b_stage_bytes = nb_cta * BK;
-    const int a_stage_bytes = p.tpu * A_TILE_BYTES;
+    const int a_stage_bytes = p.bmu * BK;           // (a unit of fewer than 128 rows: the MMA multiplies what lies behind it into rows nobody reads)
     uint8_t* sA = smem;
     uint8_t* sB = smem + (size_t)p.stages * a_stage_bytes;
     // epilogue staging of eight rows' folded sums for each half of the epilogue warps: [2][4][128] x 16 bytes
@@ -464,7 +464,7 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     const uint32_t tmem_base = *tmem_slot;
     if (threadIdx.x == 0) DBG(1);
     // first weight row of unit t that is this CTA's
-    auto unit_row = [&](int t) { return PAIR ? (2 * t + (int)rank) * BM : t * p.bmu; };
+    auto unit_row = [&](int t) { return (PAIR ? 2 * t + (int)rank : t) * p.bmu; };
     auto slot_of = [&](int i) { return PAIR ? (size_t)(2 * i + (int)rank) : (size_t)i; };
 
     if (warp == 0) {
@@ -756,7 +756,7 @@ qlinear_i8_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                 m_base *= p.Mpad;
                 for (int ht = 0; ht < p.tpu; ++ht) {   // the unit's tiles, one accumulator each
                     const int n = n_base + ht * BM + r;
-                    const bool row_ok = n < p.N;
+                    const bool row_ok = n < p.N && ht * BM + r < p.bmu;
                     const float sc = whole && row_ok ? __ldg(p.scales + n) : 0.0f;
                     const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)((ab * p.tpu + ht) * p.NB);
                     ulonglong2* slot = p.part + (slot_of(sg.slot) * p.tpu + ht) * (p.Mpad / 2) * BM;
@@ -1114,13 +1114,25 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
         plan_tc_schedule(units, p.kb_total, ctx->sm_count / 2, dp_percent, WS_ACC_BYTES / ((size_t)2 * Mpad * BM * 8), &sc);
         pair = sc.sk_tiles == 0 || sc.dp_tiles > 0 || (NB > 192 && sc.sk_per_cta >= 32);
     }
+    // Too many tiles for two CTAs each and too few for the SMs (74 < tiles < 107): runs of k-blocks would leave most CTAs with pieces of
+    // two tiles to exchange.  Units of as many rows (a multiple of eight) as give every CTA one whole unit instead, on pairs where
+    // there are digits to share.  Runs / units of N / 148 rows, us: 4 x 4096 x 12288 16.3 / 13.7, 16 rows 16.9 / 14.3, 32 rows 20.1 / 17.0,
+    // 64 rows 27.1 / 21.9; 4 x 1024 x 9000 9.7 / 6.5; 32 x 8192 x 10240 26.1 / 25.5, but 4 rows 22.5 / 23.5: a CTA walks all of K.
+    const int even_rows = (p.N + ctx->sm_count * 8 - 1) / (ctx->sm_count * 8) * 8;
+    bool even = false;
+    if (nblk == 1 && even_rows <= BM && a.N > (uint32_t)BM && (p.kb_total <= 32 || NB >= 128)) {
+        plan_tc_schedule((p.N + BM - 1) / BM, p.kb_total, ctx->sm_count, dp_percent, WS_ACC_BYTES / ((size_t)Mpad * BM * 8), &sc);
+        even = sc.dp_tiles == 0 && sc.sk_tiles > 0 && sc.sk_ways == 0;
+        if (even) pair = NB >= 64 && NB % 32 == 0 && p.kb_total >= 16 && ctx->sm_count % 2 == 0;
+    }
     const int group = pair ? 2 : 1;      // CTAs that work on one unit
-    if (!pair && two_tiles > 0 && 4 * NB <= 512 && a.N > (uint32_t)BM) {
+    if (!pair && !even && two_tiles > 0 && 4 * NB <= 512 && a.N > (uint32_t)BM) {
         const int units = (p.N + 2 * BM - 1) / (2 * BM) * nblk;
         plan_tc_schedule(units, p.kb_total, ctx->sm_count, dp_percent, WS_ACC_BYTES / ((size_t)2 * Mpad * BM * 8), &sc);
         if (two_tiles >= 2 || sc.sk_tiles == 0) p.tpu = 2;
     }
     p.bmu = p.tpu * BM;
+    if (even) p.bmu = even_rows;
     p.tiles = (p.N + group * p.bmu - 1) / (group * p.bmu) * nblk;
     int sched_sms = ctx->sm_count / group;
     const size_t slots_cap = WS_ACC_BYTES / ((size_t)group * p.tpu * Mpad * BM * 8);
@@ -1164,7 +1176,7 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
     uint32_t cols = 32;
     while (cols < (uint32_t)(2 * p.tpu * NB)) cols <<= 1;   // two sets of accumulators: the epilogue of one unit overlaps the next
     p.tmem_cols = cols;
-    const int a_stage = p.tpu * A_TILE_BYTES, b_stage = NB / group * BK;
+    const int a_stage = p.bmu * BK, b_stage = NB / group * BK;
     // Half of the SM's shared memory at most for narrow batches, so that the next kernel's CTA can move in beside this
     // one and prefetch its weights while this one drains (RUSTY_TC_FULL_SMEM=1: take it all, 8 stages).
     static const bool full_smem = getenv("RUSTY_TC_FULL_SMEM") != nullptr;

@@ -665,9 +665,11 @@ def test_f32_prompts_in_row_blocks(ctx, engine, M, K, N):
 
 
 @pytest.mark.parametrize("M,K,N,xdt", [(25, 144, 19237, "f32"), (32, 1040, 37889, "f32"), (64, 4112, 515, "f32"), (64, 16400, 385, "f32"), (7, 20000, 129, "f32"),
-                                       (40, 9232, 260, "f32"), (64, 8208, 2100, "f32"), (64, 272, 18950, "bf16"), (130, 400, 9500, "f32")])
+                                       (40, 9232, 260, "f32"), (64, 8208, 2100, "f32"), (64, 272, 18950, "bf16"), (130, 400, 9500, "f32"), (5, 1040, 9601, "f32"),
+                                       (20, 2064, 12289, "f32"), (64, 4112, 10002, "f32"), (16, 528, 13500, "bf16")])
 def test_pairs_of_ctas_and_long_rows(ctx, engine, M, K, N, xdt):
-    """Units of 256 weight rows on two CTAs (whole ones, whole ones and cut ones, long pieces; a last unit of one half or less) and
+    """Units of 256 weight rows on two CTAs (whole ones, whole ones and cut ones, long pieces; a last unit of one half or less), units of
+    N / 148 rows on one CTA or two, and
     rows of activations cut over one block or two, against float64: four digit planes and two roundings leave 2e-6 of a row's
     largest output at most, three planes 2e-5; twice the same bits."""
     x, q, s = sym_row_linear(M + K + N, M, K, N)
