@@ -1101,6 +1101,26 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
     // RUSTY_TC_DP_PERCENT: least share of the SMs that whole tiles must keep streaming (default 72; 101 turns the rule off).
     static const int dp_percent = getenv("RUSTY_TC_DP_PERCENT") ? atoi(getenv("RUSTY_TC_DP_PERCENT")) : 72;
     p.kb_total = (p.K + BK - 1) / BK;
+    // The schedule of `tiles` units on groups of CTAs.
+    // A GEMM CTA and a pre-pass block do not fit one SM together (registers), and the NEXT pair's pre-pass blocks are
+    // resident (two per SM, up to 16 SMs) while this GEMM's CTAs are placed.  A short launch whose every tile is cut
+    // (fewer tiles than SMs) and whose grid leaves those SMs no room gets its last CTAs placed only after the pre-pass
+    // has finished, 2-5 us late: plan it for 16 SMs fewer (q|k|v 6144 x 4096: 144 -> 96 CTAs, 18.2 -> 16.8 us).
+    // RUSTY_TC_ROOM=0 turns the rule off (tuning aid).
+    auto plan = [&](int tiles, int group, int tpu, TcSchedule* out) {
+        int sms = ctx->sm_count / group;
+        const size_t slots_cap = WS_ACC_BYTES / ((size_t)group * tpu * Mpad * BM * 8);
+        // tuning aid: schedule as if the GPU had fewer SMs
+        static const int sms_env = getenv("RUSTY_TC_SMS") ? atoi(getenv("RUSTY_TC_SMS")) : 0;
+        if (sms_env > 0 && sms_env < sms) sms = sms_env;
+        plan_tc_schedule(tiles, p.kb_total, sms, dp_percent, slots_cap, out);
+        static const bool leave_room = !(getenv("RUSTY_TC_ROOM") && atoi(getenv("RUSTY_TC_ROOM")) == 0);
+        if (leave_room && out->dp_tiles == 0 && out->grid > sms - 16 / group && sms > 32 / group) {
+            TcSchedule alt{};
+            plan_tc_schedule(tiles, p.kb_total, sms - 16 / group, dp_percent, slots_cap, &alt);
+            if (alt.dp_tiles == 0) *out = alt;
+        }
+    };
     TcSchedule sc{};
     p.tpu = 1;
     // A pair of CTAs per unit of 256 rows halves the digit bytes a CTA pulls from L2, where they are more than the weights' (an SM
@@ -1114,15 +1134,17 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
         plan_tc_schedule(units, p.kb_total, ctx->sm_count / 2, dp_percent, WS_ACC_BYTES / ((size_t)2 * Mpad * BM * 8), &sc);
         pair = sc.sk_tiles == 0 || sc.dp_tiles > 0 || (NB > 192 && sc.sk_per_cta >= 32);
     }
-    // Too many tiles for two CTAs each and too few for the SMs (74 < tiles < 107): runs of k-blocks would leave most CTAs with pieces of
+    // Too many tiles for two CTAs each and too few for the SMs (66 < tiles < 107): runs of k-blocks would leave most CTAs with pieces of
     // two tiles to exchange.  Units of as many rows (a multiple of eight) as give every CTA one whole unit instead, on pairs where
-    // there are digits to share.  Runs / units of N / 148 rows, us: 4 x 4096 x 12288 16.3 / 13.7, 16 rows 16.9 / 14.3, 32 rows 20.1 / 17.0,
-    // 64 rows 27.1 / 21.9; 4 x 1024 x 9000 9.7 / 6.5; 32 x 8192 x 10240 26.1 / 25.5, but 4 rows 22.5 / 23.5: a CTA walks all of K.
+    // there are digits to share.  Runs / units of N / 148 rows, us: 4 x 4096 x 12288 16.3 / 13.9, 16 rows 16.9 / 14.4, 32 rows 20.1 / 17.1,
+    // 64 rows 27.1 / 21.9; 32 x 2048 x 9000 14.5 / 11.3; 32 x 8192 x 10240 26.1 / 25.5, but 4 rows 22.5 / 23.5: a CTA walks all of K.  And up to
+    // 1024 activations, where the exchange of any cut is longer than the walk: 4 x 1024 x 4096 7.2 / 6.8, 64 rows 12.6 / 11.0.
+    // (Two pieces a tile and 2048 activations, 4 x 2048 x 8192: 8.9 / 9.4.)
     const int even_rows = (p.N + ctx->sm_count * 8 - 1) / (ctx->sm_count * 8) * 8;
     bool even = false;
     if (nblk == 1 && even_rows <= BM && a.N > (uint32_t)BM && (p.kb_total <= 32 || NB >= 128)) {
-        plan_tc_schedule((p.N + BM - 1) / BM, p.kb_total, ctx->sm_count, dp_percent, WS_ACC_BYTES / ((size_t)Mpad * BM * 8), &sc);
-        even = sc.dp_tiles == 0 && sc.sk_tiles > 0 && sc.sk_ways == 0;
+        plan((p.N + BM - 1) / BM, 1, 1, &sc);
+        even = sc.dp_tiles == 0 && sc.sk_tiles > 0 && (sc.sk_ways == 0 || p.kb_total <= 8);
         if (even) pair = NB >= 64 && NB % 32 == 0 && p.kb_total >= 16 && ctx->sm_count % 2 == 0;
     }
     const int group = pair ? 2 : 1;      // CTAs that work on one unit
@@ -1134,24 +1156,7 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
     p.bmu = p.tpu * BM;
     if (even) p.bmu = even_rows;
     p.tiles = (p.N + group * p.bmu - 1) / (group * p.bmu) * nblk;
-    int sched_sms = ctx->sm_count / group;
-    const size_t slots_cap = WS_ACC_BYTES / ((size_t)group * p.tpu * Mpad * BM * 8);
-    {   // tuning aid: schedule as if the GPU had fewer SMs
-        static const int sms_env = getenv("RUSTY_TC_SMS") ? atoi(getenv("RUSTY_TC_SMS")) : 0;
-        if (sms_env > 0 && sms_env < sched_sms) sched_sms = sms_env;
-    }
-    plan_tc_schedule(p.tiles, p.kb_total, sched_sms, dp_percent, slots_cap, &sc);
-    // A GEMM CTA and a pre-pass block do not fit one SM together (registers), and the NEXT pair's pre-pass blocks are
-    // resident (two per SM, up to 16 SMs) while this GEMM's CTAs are placed.  A short launch whose every tile is cut
-    // (fewer tiles than SMs) and whose grid leaves those SMs no room gets its last CTAs placed only after the pre-pass
-    // has finished, 2-5 us late: plan it for 16 SMs fewer (q|k|v 6144 x 4096: 144 -> 96 CTAs, 18.2 -> 16.8 us).
-    // RUSTY_TC_ROOM=0 turns the rule off (tuning aid).
-    static const bool leave_room = !(getenv("RUSTY_TC_ROOM") && atoi(getenv("RUSTY_TC_ROOM")) == 0);
-    if (leave_room && sc.dp_tiles == 0 && sc.grid > sched_sms - 16 / group && sched_sms > 32 / group) {
-        TcSchedule alt{};
-        plan_tc_schedule(p.tiles, p.kb_total, sched_sms - 16 / group, dp_percent, slots_cap, &alt);
-        if (alt.dp_tiles == 0) sc = alt;
-    }
+    plan(p.tiles, group, p.tpu, &sc);
     const int grid = sc.grid * group;
     p.dp_tiles = sc.dp_tiles;
     p.sk_tiles = sc.sk_tiles;
