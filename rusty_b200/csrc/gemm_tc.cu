@@ -1188,8 +1188,10 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
     size_t budget = ctx->smem_optin > 4096 ? ctx->smem_optin - 4096 : 0;
     if (!full_smem && NB <= 32 && 4 * (size_t)a_stage + 4096 <= budget / 2)
         budget = budget / 2 - 1024;  // narrow batches: leave room for the next kernel's CTA on the SM
-    // epilogue staging of whole tiles' sums, eight rows at a time; launches without whole tiles need none
-    const size_t red_bytes = p.dp_tiles > 0 ? (size_t)(p.epi_warps / 4) * 8 * 8 * BM : 0;
+    // epilogue staging of whole tiles' sums, eight rows at a time; launches without whole tiles need none.  A run of k-blocks as long as a
+    // tile holds whole ones as well (few k-blocks, few tiles: 59 x 624 x 600).
+    const bool whole_tiles = p.dp_tiles > 0 || (p.sk_ways == 0 && p.sk_per_cta >= p.kb_total);
+    const size_t red_bytes = whole_tiles ? (size_t)(p.epi_warps / 4) * 8 * 8 * BM : 0;
     const size_t rowf_bytes = (size_t)nblk * Mpad * 4;
     int stages = budget > red_bytes + rowf_bytes + 2048 ? (int)((budget - 1024 - 512 - red_bytes - rowf_bytes) / (size_t)(a_stage + b_stage)) : 0;
     if (stages > 8) stages = 8;

@@ -664,6 +664,16 @@ def test_f32_prompts_in_row_blocks(ctx, engine, M, K, N):
         assert rel_err_rows(y.read(), g * u / (1.0 + np.exp(-np.maximum(g, -80.0)))) <= TOL_FP32
 
 
+@pytest.mark.parametrize("M,K,N", [(59, 624, 2097), (59, 624, 600), (5, 624, 600), (20, 560, 900), (64, 720, 1500), (130, 624, 700), (300, 624, 5000), (100, 560, 130)])
+def test_runs_of_k_blocks_as_long_as_a_tile(ctx, engine, M, K, N):
+    """Few k-blocks and few tiles: the schedule cuts nothing and has no whole waves either, so that whole tiles come as runs; they are
+    staged in shared memory like any others.  Against float64 (2e-6 of a row's largest output: four digit planes, two roundings)."""
+    x, q, s = sym_row_linear(M + K + N, M, K, N)
+    got = _forward(ctx, engine, QLinear.from_host(ctx, q, s), x)
+    assert rel_err_rows(got, x.astype(np.float64) @ (q * s[:, None].astype(np.float64)).T) <= 2e-6
+    ctx.sync()
+
+
 @pytest.mark.parametrize("M,K,N,xdt", [(25, 144, 19237, "f32"), (32, 1040, 37889, "f32"), (64, 4112, 515, "f32"), (64, 16400, 385, "f32"), (7, 20000, 129, "f32"),
                                        (40, 9232, 260, "f32"), (64, 8208, 2100, "f32"), (64, 272, 18950, "bf16"), (130, 400, 9500, "f32"), (5, 1040, 9601, "f32"),
                                        (20, 2064, 12289, "f32"), (64, 4112, 10002, "f32"), (16, 528, 13500, "bf16")])
