@@ -98,12 +98,12 @@ template <typename XT>
 constexpr int DIG_PLANES = sizeof(XT) == 4 ? 4 : 3;
 
 // A few fat blocks on purpose: grid = min(32, Mpad) blocks of 512 threads, R = Mpad / grid activation rows per block
-// (1 or 2), 512 / R threads per row (its own named barrier).  The kernel is launched early (programmatic dependent
+// (1 or 2), 512 / R threads per row (its own named barrier); rows from 8192 activations on have a block each whatever Mpad is, and
+// beyond 16384 a cluster of two (SPLIT; they meet for the maximum).  The kernel is launched early (programmatic dependent
 // launch) and parks in griddepcontrol.wait while the GEMM before it still runs; many small parked blocks pile up on the
 // few SMs that GEMM left free and keep the next GEMM's CTAs from being placed there.  Thirty-two blocks of at most 64
 // registers a thread fit beside a GEMM CTA on any SM and cannot fill more than eight.  Rows M..Mpad-1 are written as
-// zeros.  A row of up to 16384 activations (one row per block) stays in registers between its maximum and its digits:
-// one round trip to memory, all loads in flight together.
+// zeros.  What a row's threads hold in registers between its maximum and its digits is read once, all loads in flight together.
 //
 // NORM: the activations are RMSNorm(x [+ residual]) * weight (norm_embed.cu gives the formula and its lines in the
 // reference); the row is normalised in registers between the load and the maximum, so it must fit there
@@ -1145,7 +1145,15 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
     if (nblk == 1 && even_rows <= BM && a.N > (uint32_t)BM && (p.kb_total <= 32 || NB >= 128)) {
         plan((p.N + BM - 1) / BM, 1, 1, &sc);
         even = sc.dp_tiles == 0 && sc.sk_tiles > 0 && (sc.sk_ways == 0 || p.kb_total <= 8);
-        if (even) pair = NB >= 64 && NB % 32 == 0 && p.kb_total >= 16 && ctx->sm_count % 2 == 0;
+        if (even) {
+            const bool on_pairs = NB >= 64 && NB % 32 == 0 && p.kb_total >= 16 && ctx->sm_count % 2 == 0;
+            const int rows = even_rows * (on_pairs ? 2 : 1);
+            plan((p.N + rows - 1) / rows, on_pairs ? 2 : 1, 1, &sc);
+            // Whole units or none: a piece is stored with all 128 rows and taken away again with the unit's, and what stays behind in a
+            // slot counts as arrived in the next launch.  (Very few k-blocks: the plan may cut these units as well.)
+            even = sc.sk_tiles == 0;
+            if (even) pair = on_pairs;
+        }
     }
     const int group = pair ? 2 : 1;      // CTAs that work on one unit
     if (!pair && !even && two_tiles > 0 && 4 * NB <= 512 && a.N > (uint32_t)BM) {
