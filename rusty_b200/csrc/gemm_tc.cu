@@ -1137,12 +1137,13 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
     // Too many tiles for two CTAs each and too few for the SMs (66 < tiles < 107): runs of k-blocks would leave most CTAs with pieces of
     // two tiles to exchange.  Units of as many rows (a multiple of eight) as give every CTA one whole unit instead, on pairs where
     // there are digits to share.  Runs / units of N / 148 rows, us: 4 x 4096 x 12288 16.3 / 13.9, 16 rows 16.9 / 14.4, 32 rows 20.1 / 17.1,
-    // 64 rows 27.1 / 21.9; 32 x 2048 x 9000 14.5 / 11.3; 32 x 8192 x 10240 26.1 / 25.5, but 4 rows 22.5 / 23.5: a CTA walks all of K.  And up to
+    // 64 rows 27.1 / 21.9; 32 x 2048 x 9000 14.5 / 11.3; not for longer rows, where a CTA's walk of all of K is the longer part: 4 x 8192 x 10240
+    // 22.5 / 23.5, 32 rows 25.6 / 25.6, 64 rows 33.3 / 32.5, but a 70B-shaped stack 600 / 606.  And up to
     // 1024 activations, where the exchange of any cut is longer than the walk: 4 x 1024 x 4096 7.2 / 6.8, 64 rows 12.6 / 11.0.
     // (Two pieces a tile and 2048 activations, 4 x 2048 x 8192: 8.9 / 9.4.)
     const int even_rows = (p.N + ctx->sm_count * 8 - 1) / (ctx->sm_count * 8) * 8;
     bool even = false;
-    if (nblk == 1 && even_rows <= BM && a.N > (uint32_t)BM && (p.kb_total <= 32 || NB >= 128)) {
+    if (nblk == 1 && even_rows <= BM && a.N > (uint32_t)BM && p.kb_total <= 32) {
         plan((p.N + BM - 1) / BM, 1, 1, &sc);
         even = sc.dp_tiles == 0 && sc.sk_tiles > 0 && (sc.sk_ways == 0 || p.kb_total <= 8);
         if (even) {
