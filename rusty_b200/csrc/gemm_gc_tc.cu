@@ -93,9 +93,6 @@ struct GcParams {
     long long peer_delta[PEER_MAX_RANKS];
 };
 
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
 // Magnitudes are compared as bits: a NaN or an infinity is above every number.
 __device__ __forceinline__ uint32_t abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
 __device__ __forceinline__ uint32_t abs_max(const float4& v) { return max(max(abs_bits(v.x), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w))); }

@@ -128,6 +128,8 @@ __global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* x,
     xq += (size_t)blockIdx.y * D * Mpad * K;
     PDBG(tid == 0 && blockIdx.x == 0, 0);
     pdl_launch_dependents();
+    if constexpr (SPLIT)
+        if (m < M) cluster_arrive();   // this block runs: the other may store into it (waited for before the store)
     pdl_wait();  // x may come from the previous kernel, and that kernel may still be reading the digit planes
     PDBG(tid == 0 && blockIdx.x == 0, 1);
     if (push.nranks > 1) {
@@ -200,6 +202,7 @@ __global__ void __launch_bounds__(DIG_THREADS, 2) digitize_x_kernel(const XT* x,
     const int wpr = tpr / 32;                       // warps per row: 16 or 8
     uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(red[grp * wpr + (tid & (wpr - 1))]));
     if constexpr (SPLIT) {
+        cluster_wait();
         if (tid < 2) st_cluster_u32(part_max + part, (uint32_t)tid, top);
         cluster_sync_all();
         top = max(part_max[0], part_max[1]);
