@@ -177,9 +177,12 @@ RUSTY_CUDA_API int rusty_cuda_add_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf*
 
 /* Linear::forward with a LoRA branch (rusty-graph/src/lib.rs:69-80) in one call: y[M,N] = x[M,K] . W + (x . A) . B with
  * lora_a f32 [K, rank], lora_b f32 [rank, N], no alpha / rank factor (as there).  Exactly one of `weight` (f32 [K,N]) and
- * `ql` (N x K, no pair activation) is given.  x . W as rusty_cuda_matmul_f32 (or rusty_cuda_qlinear_forward) computes it;
- * the branch is summed in f32 in an order of its own.  Needs M * rank floats of scratch: while a capture is open, run one
- * such call before it so that the pool holds them. */
+ * `ql` (N x K, no pair activation) is given.  Over `ql`, x . W is what rusty_cuda_qlinear_forward computes.  Over an f32
+ * `weight` both products are one f32 sum (fused multiply-adds) in an order of its own, not rusty_cuda_matmul_f32's: from 2^20
+ * weights on K is summed in up to 128 ranges, which is nearer the exact sum.  Up to 32 rows (and rank 128) a row's bits do not
+ * depend on the other rows of the call; beyond, the order may follow the number of rows.  The branch's x . A is summed in f32 in an
+ * order of its own.  Needs M * rank floats of scratch: while a capture is open, run one such call before it so that the
+ * pool holds them. */
 RUSTY_CUDA_API int rusty_cuda_linear_lora_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf* x, const rusty_cuda_buf* weight,
                                               const rusty_cuda_qlinear* ql, const rusty_cuda_buf* lora_a,
                                               const rusty_cuda_buf* lora_b, rusty_cuda_buf* y, uint32_t M, uint32_t K,

@@ -84,12 +84,6 @@ __device__ __forceinline__ float lds_f1(const float* p) {
     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(smem_u32(p)));
     return v;
 }
-// Global loads as volatile asm, for the same reason.
-__device__ __forceinline__ float4 ldg_f4(const float* p) {
-    float4 v;
-    asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-    return v;
-}
 // two FMAs an instruction, each half rounded like fmaf
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
     unsigned long long v;
@@ -382,214 +376,191 @@ int launch_lora_down(rusty_cuda_ctx* ctx, const float* x, const float* A, float*
 }
 
 // ---- f32 Linear with an adapter ----------------------------------------------------------------------------------------
-// y[M, N] = [x | t] . [W ; B].  No shader gives the order of this sum (the reference adds two products), so it may be cut, and it
-// may run on the tensor cores as long as nothing is lost.  An f32 is a tf32 (11 bits, to nearest) plus a tf32 of what is left, off by
-// 2^-23 of it at most and to either side; of the four products the smallest, below 2^-24, is left out.  The three others of sixteen k go
-// into one mma.sync chain that starts at zero, the smaller ones first, and its result is added in f32 to the lane's accumulators: the
-// tensor core's own, truncating, additions stay inside sixteen k.  Against float64, 2-norm, K = 4096: 1.4e-7 where one f32 chain is off by
-// 1.1e-6; K = 512: 1.3e-7 and 3.7e-7.
-// An infinity, or a sum beyond the largest float, comes out of the split as a NaN: outputs that are not finite are computed once
-// more, in one f32 chain.
+// y[M, N] = [x | t] . [W ; B], f32 throughout: every product enters by a fused multiply-add, so that infinities, subnormals and single
+// products are what f32 makes them.  No shader gives the order of this sum (the reference adds two products), so K is cut: a warp owns 64
+// columns x TM rows x a range of K in units of sixteen links, its halves take the even and the odd ones, a lane four neighbouring columns
+// (pairs of rows share an FMA instruction).  Each warp has a ring of its own, filled with cp.async: W as it is, x as [link][row], so that four
+// rows are one read.  The ranges of a CTA's warps are summed in shared memory, those of a cluster's CTAs in distributed shared memory,
+// in a fixed order that depends on K, N and the rank, and beyond 32 rows on their number: up to there a row's bits do not depend on the
+// rows beside it.  Against float64, 2-norm, K = 4096: 2.1e-7 where one f32 chain is off by 1.1e-6; K = 8192 x 8192: 3.4e-7 and 1.3e-6.
 //
-// A warp owns 64 columns x 8 NT rows x a range of K, in units of sixteen k.  Its loads go straight into fragments, one unit ahead: a
-// lane's four neighbouring columns of W are rows g and g + 8 of two tiles (a register each, nothing to pack), its four
-// neighbouring k of a row of x the k it owns in W.  The ranges of a CTA's warps are summed in shared memory, those of a cluster's
-// CTAs in distributed shared memory, in a fixed order.  What bounds it: up to 16 rows waiting for W (48 KB in flight an SM; a warp's
-// loads, its split and its MMAs take turns, three warps a scheduler), beyond them the split and the MMAs (24 NT of 8 cycles a unit).
-// 4096 x 4096, rank 8, whole call in a graph: 8 rows 31.9 -> 22.3, 16 rows 41.4 -> 29.1, 64 rows 82.7 -> 60.8, 256 rows 251 -> 215 us;
-// 8192 x 512: 8 rows 39.7 -> 14.5, 64 rows 65.9 -> 44.8; 8192 x 8192, rank 64: 8 rows 108 -> 72.5, 64 rows 500 -> 226.
-// Tried: FMAs with x from shared memory (the reads and the copies of a weight into both halves of a pair: 16 rows 27, 256 rows 269),
-// three bf16 instead of two tf32 (more to split and to pack: 28, 223), copies by cp.async (whole lines torn apart on their way into
-// fragment order: 33), 256 columns a CTA (clusters of eight, of which 15 fit: 47).
-constexpr int SP_BN = 64;
-template <int NT>
-constexpr int SP_WARPS = NT == 4 ? 8 : 12;
+// What bounds it: up to eight rows W (96 KB in flight an SM) and the fixed part of two launches, beyond sixteen the FMAs: the pipe is busy 68 %
+// of a CTA's time at 256 rows.  4096 x 4096, rank 8, whole call in a graph, one chain of K on the matmul's tiles / this, us: one row 21.7
+// / 13.4, 8 rows 31.1 / 14.0, 16 rows 38.7 / 20.0, 64 rows 80.2 / 54.5, 256 rows 250 / 207; 8192 x 512: 8 rows 39.3 / 8.9, 64 rows 61.4 / 38.8;
+// 8192 x 8192, rank 64: one row 47.7 / 40.4, 64 rows 500 / 208.
+// Tried: two tf32 an f32 on the tensor cores (the products lose up to 2^-21 of themselves; 8 rows 21.7, 16 rows 25.6, 64 rows 57.4, 256 rows
+// 213); W through registers instead of a ring (8 rows 23, 16 rows 28, 64 rows 72); 256 columns a CTA (clusters of eight, of which 15 fit: 47).
+constexpr int SP_BN = 64, SP_WARPS = 8, SP_THREADS = 32 * SP_WARPS, SP_STAGES = 4;
+template <int TM>
+struct Sp {
+    static constexpr int LDX = TM + 4;                                          // floats between links of x in shared memory
+    static constexpr int STAGE = 16 * (SP_BN + LDX);                            // floats of a unit: W, then x
+    static constexpr int PIECE = TM < 16 ? TM : 16;                             // rows read ahead of their FMAs
+    static constexpr int RING = SP_WARPS * SP_STAGES * STAGE, PART = SP_WARPS * TM * SP_BN;
+    static constexpr size_t SMEM = (size_t)(RING > PART ? RING : PART) * 4;
+};
 
-// D = A[16x8] . B[8x8] + C, tf32 -> f32
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2], float c0, float c1, float c2, float c3) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
-                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
-}
-// v = big + small, both with the lower 13 bits clear
-__device__ __forceinline__ void split2(float v, uint32_t& big, uint32_t& small) {
-    big = (__float_as_uint(v) + 0x1000u) & 0xffffe000u;
-    small = __float_as_uint(v - __uint_as_float(big)) & 0xffffe000u;
+__device__ __forceinline__ ulonglong2 lds_2xf32x2(uint32_t addr) {
+    ulonglong2 v;
+    asm volatile("ld.shared.v2.u64 {%0,%1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(addr));
+    return v;
 }
 
-template <int NT>
-__global__ void __launch_bounds__(32 * SP_WARPS<NT>, 1) linear_splitk_f32_kernel(const float* x, const float* W, float* y, uint32_t M, uint32_t K, uint32_t N,
-                                                                                 const LoraTail lora, int ways, uint32_t row_tiles) {
-    constexpr int TM = 8 * NT, WARPS = SP_WARPS<NT>, THREADS = 32 * WARPS;
+template <int TM>
+__global__ void __launch_bounds__(SP_THREADS, 1) linear_splitk_f32_kernel(const float* x, const float* W, float* y, uint32_t M, uint32_t K, uint32_t N,
+                                                                          const LoraTail lora, int ways, uint32_t row_tiles) {
+    using C = Sp<TM>;
+    constexpr int PIECE = C::PIECE, ST = SP_STAGES;
     extern __shared__ __align__(16) float sp_smem[];
-    const int warp = warp_id(), lane = threadIdx.x & 31, g = lane >> 2, j = lane & 3;
+    const int warp = warp_id(), lane = threadIdx.x & 31, half = lane >> 4;
     const uint32_t way = blockIdx.x % (uint32_t)ways, tile = blockIdx.x / (uint32_t)ways;
     const uint32_t m0 = (tile % row_tiles) * TM, n0 = (tile / row_tiles) * SP_BN;
-    // this lane's columns, 4 g .. 4 g + 3 of each half of 32 (N % 4 == 0: they exist together, or are others' and not stored)
-    const uint32_t c0 = min(n0 + 4 * g, N - 4), c1 = min(n0 + 32 + 4 * g, N - 4);
-    float acc[4][NT][4];     // [tile of 16 columns][rows 8 at a time]
+    const uint32_t c0 = min(n0 + 4 * (lane & 15), N - 4);      // (N % 4 == 0; columns that do not exist repeat the last and are not stored)
+    const uint32_t ring = smem_u32(sp_smem) + (uint32_t)(warp * ST * C::STAGE) * 4;
+    unsigned long long acc[TM / 2][4];                         // [two rows][column]
 #pragma unroll
-    for (int t = 0; t < 4; ++t)
-#pragma unroll
-        for (int i = 0; i < NT; ++i) acc[t][i][0] = acc[t][i][1] = acc[t][i][2] = acc[t][i][3] = 0.0f;
+    for (int i = 0; i < TM / 2; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0ull;
 
     // the K + r links in units of sixteen, the same number for every warp; the last ones hold t . B
     const uint32_t units_k = (K + 15) / 16, units = units_k + ((uint32_t)lora.r + 15) / 16;
-    const uint32_t parts = (uint32_t)(ways * WARPS), mine = way * WARPS + warp;
+    const uint32_t parts = (uint32_t)(ways * SP_WARPS), mine = way * SP_WARPS + warp;
     const uint32_t u0 = (uint32_t)((uint64_t)units * mine / parts), u1 = (uint32_t)((uint64_t)units * (mine + 1) / parts);
     // The kernel in front of this one only computes t, and it lets this one start after its own griddepcontrol.wait
     // (lora_down_kernel): x, W and y are free by then, only t has to be waited for.
     bool t_ready = false;
-    struct Unit {
-        float4 w[8];      // links 4 j .. 4 j + 3: columns c0, then c1
-        float4 x[NT];     // the same links of row g
-    };
-    auto fetch = [&](Unit& v, uint32_t u) {
-        if (u >= u1) return;
-        const bool second = u >= units_k;
-        if (second && !t_ready) {
-            pdl_wait();
-            t_ready = true;
-        }
-        const float* a = second ? lora.t : x;
-        const uint32_t lda = second ? (uint32_t)lora.r4 : K, len = second ? (uint32_t)lora.r : K;
-        const uint32_t k = (second ? u - units_k : u) * 16 + 4 * j;
-        const float* p = (second ? lora.b : W) + (size_t)k * N;
-        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-        const bool whole = k - 4 * j + 16 <= len;       // (the same for all lanes)
-#pragma unroll
-        for (int h = 0; h < 4; ++h, p += N) {
-            if (whole) {
-                v.w[h] = ldg_f4(p + c0);
-                v.w[4 + h] = ldg_f4(p + c1);
-            } else {                                     // links that do not exist are zeros
-                v.w[h] = k + h < len ? ldg_f4(p + c0) : zero;
-                v.w[4 + h] = k + h < len ? ldg_f4(p + c1) : zero;
+    auto fetch = [&](uint32_t u, int slot) {
+        if (u < u1) {
+            const bool tail = u >= units_k;
+            if (tail && !t_ready) {
+                pdl_wait();
+                t_ready = true;
             }
-        }
+            const uint32_t k0 = (tail ? u - units_k : u) * 16, len = tail ? (uint32_t)lora.r : K, lda = tail ? (uint32_t)lora.r4 : K;
+            const uint32_t to = ring + (uint32_t)(slot * C::STAGE) * 4;
+            // W: links 2 i + half, the lane's own four columns; x: link lane % 16 of rows lane / 16 + 2 i
+            const uint32_t to_w = to + (uint32_t)(half * SP_BN + 4 * (lane & 15)) * 4, to_x = to + (uint32_t)(16 * SP_BN + (lane & 15) * C::LDX + half) * 4;
+            const float* p = (tail ? lora.b : W) + (size_t)(k0 + half) * N + c0;
+            const uint32_t k = k0 + (lane & 15);
+            const float* a = (tail ? lora.t : x) + (size_t)m0 * lda + k;
+            if (k0 + 16 <= len && m0 + TM <= M) {
+                a += (size_t)half * lda;
 #pragma unroll
-        for (int i = 0; i < NT; ++i)                     // (rows that do not exist repeat the last one)
-            v.x[i] = whole || k < len ? ldg_f4(a + (size_t)min(m0 + 8 * i + g, M - 1) * lda + k) : zero;
-        if (!whole && k < len && k + 4 > len)            // t's rows are padded with zeros, x's (K % 4 == 0) end with a lane's four
+                for (int i = 0; i < 8; ++i, p += 2 * (size_t)N) cp_async<true>(to_w + (uint32_t)(2 * i * SP_BN) * 4, p, 16u);
 #pragma unroll
-            for (int i = 0; i < NT; ++i) {
-                if (k + 1 >= len) v.x[i].y = 0.0f;
-                if (k + 2 >= len) v.x[i].z = 0.0f;
-                v.x[i].w = 0.0f;
-            }
-    };
-    auto multiply = [&](const Unit& v) {
-        uint32_t xb[2][2][NT][2];                        // [big, small][eight of the sixteen k][rows][fragment]
-#pragma unroll
-        for (int i = 0; i < NT; ++i) {
-            split2(v.x[i].x, xb[0][0][i][0], xb[1][0][i][0]);
-            split2(v.x[i].y, xb[0][0][i][1], xb[1][0][i][1]);
-            split2(v.x[i].z, xb[0][1][i][0], xb[1][1][i][0]);
-            split2(v.x[i].w, xb[0][1][i][1], xb[1][1][i][1]);
-        }
-#pragma unroll
-        for (int half = 0; half < 2; ++half)
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {
-                uint32_t wa[2][2][4];                    // [big, small][eight k][row g, g + 8 (columns 2 t, 2 t + 1) of k and of k + 1]
-#pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    const float4& f = v.w[4 * half + h];
-                    split2(t == 0 ? f.x : f.z, wa[0][h >> 1][2 * (h & 1)], wa[1][h >> 1][2 * (h & 1)]);
-                    split2(t == 0 ? f.y : f.w, wa[0][h >> 1][2 * (h & 1) + 1], wa[1][h >> 1][2 * (h & 1) + 1]);
-                }
-                float d[NT][4];
-#pragma unroll
-                for (int i = 0; i < NT; ++i) mma_tf32(d[i], wa[1][0], xb[0][0][i], 0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                for (int m = 1; m < 6; ++m)              // small x big, big x small, big x big
-#pragma unroll
-                    for (int i = 0; i < NT; ++i) mma_tf32(d[i], wa[m < 2 ? 1 : 0][m & 1], xb[m >> 1 == 1 ? 1 : 0][m & 1][i], d[i][0], d[i][1], d[i][2], d[i][3]);
-#pragma unroll
-                for (int i = 0; i < NT; ++i)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[2 * half + t][i][e] += d[i][e];
-            }
-    };
-    Unit ua, ub;
-    fetch(ua, u0);
+                for (int i = 0; i < TM / 2; ++i, a += 2 * (size_t)lda) cp_async<false>(to_x + (uint32_t)(2 * i) * 4, a, 4u);
+            } else {   // links that do not exist are zeros (t's rows are padded with them to r4), rows that do not exist repeat the last one
+                const int left = (int)(len - k0) - half;
+                const uint32_t bytes = k < lda ? 4u : 0u;
 #pragma unroll 1
-    for (uint32_t u = u0; u < u1; u += 2) {
-        fetch(ub, u + 1);
-        multiply(ua);
-        fetch(ua, u + 2);
-        if (u + 1 < u1) multiply(ub);
+                for (int i = 0; i < 8; ++i, p += 2 * (size_t)N) cp_async<true>(to_w + (uint32_t)(2 * i * SP_BN) * 4, 2 * i < left ? p : W, 2 * i < left ? 16u : 0u);
+#pragma unroll 1
+                for (int i = 0; i < TM / 2; ++i) cp_async<false>(to_x + (uint32_t)(2 * i) * 4, bytes ? a + (size_t)min(half + 2 * i, (int)(M - 1 - m0)) * lda : x, bytes);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll 1
+    for (int d = 0; d < ST - 1; ++d) fetch(u0 + d, d);
+    int slot = 0;
+#pragma unroll 1
+    for (uint32_t u = u0; u < u1; ++u) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+        __syncwarp();                                          // unit u is there for all lanes, and the one before has been read by all
+        fetch(u + ST - 1, slot == 0 ? ST - 1 : slot - 1);
+        const uint32_t from_w = ring + (uint32_t)(slot * C::STAGE + half * SP_BN + 4 * (lane & 15)) * 4;
+        const uint32_t from_x = ring + (uint32_t)(slot * C::STAGE + 16 * SP_BN + half * C::LDX) * 4;
+        constexpr int PER = TM / PIECE, PIECES = 8 * PER;
+        ulonglong2 xv[2][PIECE / 4];
+        uint4 wv[2];
+        auto read = [&](int p) {
+            if (p % PER == 0) wv[(p / PER) & 1] = lds128(from_w + (uint32_t)((p / PER) * 2 * SP_BN) * 4);
+#pragma unroll
+            for (int q = 0; q < PIECE / 4; ++q) xv[p & 1][q] = lds_2xf32x2(from_x + (uint32_t)((p / PER) * 2 * C::LDX + (p % PER) * PIECE + 4 * q) * 4);
+        };
+        read(0);
+#pragma unroll
+        for (int p = 0; p < PIECES; ++p) {
+            if (p + 1 < PIECES) read(p + 1);
+            const uint4& w = wv[(p / PER) & 1];
+            unsigned long long wd[4];
+            asm("mov.b64 %0, {%1, %1};" : "=l"(wd[0]) : "r"(w.x));
+            asm("mov.b64 %0, {%1, %1};" : "=l"(wd[1]) : "r"(w.y));
+            asm("mov.b64 %0, {%1, %1};" : "=l"(wd[2]) : "r"(w.z));
+            asm("mov.b64 %0, {%1, %1};" : "=l"(wd[3]) : "r"(w.w));
+#pragma unroll
+            for (int q = 0; q < PIECE / 4; ++q)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[(p % PER) * (PIECE / 2) + 2 * q][c]) : "l"(xv[p & 1][q].x), "l"(wd[c]));
+                    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[(p % PER) * (PIECE / 2) + 2 * q + 1][c]) : "l"(xv[p & 1][q].y), "l"(wd[c]));
+                }
+        }
+        if (++slot == ST) slot = 0;
     }
-    // ---- the warps' sums: [warp][TM][64], then this CTA's in the first warp's place ----
-    float* part = sp_smem;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                           // the sums go where the rings were
+    float* part = sp_smem;                                     // [warp][TM][64]
+    // ---- the halves' sums, then the warps': [warp][TM][64], then this CTA's in the first warp's place ----
 #pragma unroll
-    for (int i = 0; i < NT; ++i)
+    for (int i = 0; i < TM / 4; ++i) {                          // a half keeps its half of the rows
+        float lo[4], hi[4];
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int e = 0; e < 2; ++e)      // row 2 j + e of these eight, the lane's four columns of half h
-                *reinterpret_cast<float4*>(part + ((size_t)warp * TM + 8 * i + 2 * j + e) * SP_BN + 32 * h + 4 * g) =
-                    make_float4(acc[2 * h][i][e], acc[2 * h][i][2 + e], acc[2 * h + 1][i][e], acc[2 * h + 1][i][2 + e]);
+        for (int c = 0; c < 4; ++c) {
+            const unsigned long long keep = half ? acc[i + TM / 4][c] : acc[i][c], give = half ? acc[i][c] : acc[i + TM / 4][c];
+            const unsigned long long got = __shfl_xor_sync(0xffffffffu, give, 16);
+            lo[c] = __uint_as_float((uint32_t)keep) + __uint_as_float((uint32_t)got);
+            hi[c] = __uint_as_float((uint32_t)(keep >> 32)) + __uint_as_float((uint32_t)(got >> 32));
+        }
+        float* to = part + ((size_t)warp * TM + half * (TM / 2) + 2 * i) * SP_BN + 4 * (lane & 15);
+        *reinterpret_cast<float4*>(to) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+        *reinterpret_cast<float4*>(to + SP_BN) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+    }
     __syncthreads();
     constexpr int ITEMS = TM * SP_BN / 4;      // four columns of a row each
     float4* p4 = reinterpret_cast<float4*>(part);
     cg::cluster_group cl = cg::this_cluster();
-    auto put = [&](int i, float4 s) {
+    auto put = [&](int i, const float4& s) {
         const uint32_t m = m0 + (uint32_t)(i / (SP_BN / 4)), c = n0 + (uint32_t)(i % (SP_BN / 4)) * 4;
-        if (m >= M || c >= N) return;
-        if (!(fabsf(s.x) <= 3.0e38f && fabsf(s.y) <= 3.0e38f && fabsf(s.z) <= 3.0e38f && fabsf(s.w) <= 3.0e38f)) {
-            pdl_wait();
-            s = make_float4(0.f, 0.f, 0.f, 0.f);
-            auto chain = [&](const float* a, const float* b, uint32_t len) {
-                for (uint32_t k = 0; k < len; ++k, b += N) {
-                    const float4 v = *reinterpret_cast<const float4*>(b + c);
-                    s.x = fmaf(a[k], v.x, s.x); s.y = fmaf(a[k], v.y, s.y); s.z = fmaf(a[k], v.z, s.z); s.w = fmaf(a[k], v.w, s.w);
-                }
-            };
-            chain(x + (size_t)m * K, W, K);
-            chain(lora.t + (size_t)m * lora.r4, lora.b, (uint32_t)lora.r);
-        }
-        *reinterpret_cast<float4*>(y + (size_t)m * N + c) = s;
+        if (m < M && c < N) *reinterpret_cast<float4*>(y + (size_t)m * N + c) = s;
     };
-    for (int i = threadIdx.x; i < ITEMS; i += THREADS) {
+    for (int i = threadIdx.x; i < ITEMS; i += SP_THREADS) {
         float4 s = p4[i];
 #pragma unroll
-        for (int w = 1; w < WARPS; ++w) {
-            const float4 v = p4[w * ITEMS + i];
-            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        for (int v = 1; v < SP_WARPS; ++v) {
+            const float4 f = p4[v * ITEMS + i];
+            s.x += f.x; s.y += f.y; s.z += f.z; s.w += f.w;
         }
         if (ways == 1) put(i, s);
         else p4[i] = s;                        // (an item is one thread's)
     }
     if (ways == 1) return;
     cl.sync();
-    for (int i = (int)way * THREADS + threadIdx.x; i < ITEMS; i += ways * THREADS) {
+    for (int i = (int)way * SP_THREADS + threadIdx.x; i < ITEMS; i += ways * SP_THREADS) {
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int w = 0; w < ways; ++w) {
-            const float4 v = cl.map_shared_rank(p4, w)[i];
-            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        for (int v = 0; v < ways; ++v) {
+            const float4 f = cl.map_shared_rank(p4, v)[i];
+            s.x += f.x; s.y += f.y; s.z += f.z; s.w += f.w;
         }
         put(i, s);
     }
     cl.sync();                                 // the others have read this CTA's sums
 }
 
-template <int NT>
+template <int TM>
 int launch_splitk(rusty_cuda_ctx* ctx, const float* x, const float* W, float* y, uint32_t M, uint32_t K, uint32_t N, const LoraTail& lora) {
-    constexpr int TM = 8 * NT, WARPS = SP_WARPS<NT>;
     const uint32_t groups = (N + SP_BN - 1) / SP_BN, row_tiles = (M + TM - 1) / TM;
     const uint64_t tiles = (uint64_t)groups * row_tiles, sms = (uint64_t)(ctx->sm_count > 0 ? ctx->sm_count : 1);
-    // K ranges: what fills the SMs with one CTA each, of a unit a warp at least.  Clusters lie in one GPC: of more than two CTAs not as
+    // K ranges: what fills the SMs with one CTA each, of two units a warp at least.  Clusters lie in one GPC: of more than two CTAs not as
     // many fit as there are SMs (of 148: 132 in clusters of four, 120 of eight), so beyond two an eighth of them is left out.
     uint64_t ways = sms / tiles >= 3 ? sms * 7 / 8 / tiles : sms / tiles;
-    const uint64_t most = K / (16 * WARPS);
+    const uint64_t most = K / (32 * SP_WARPS);
     if (ways > most) ways = most;
     ways = ways < 1 ? 1 : ways > 4 ? (ways < 8 ? 4 : 8) : ways;
-    constexpr size_t smem = (size_t)WARPS * TM * SP_BN * 4;
-    auto kern = linear_splitk_f32_kernel<NT>;
-    cudaError_t e = ensure_dynamic_smem((const void*)kern, ctx->device, smem);
+    auto kern = linear_splitk_f32_kernel<TM>;
+    cudaError_t e = ensure_dynamic_smem((const void*)kern, ctx->device, Sp<TM>::SMEM);
     if (e == cudaSuccess)
-        e = launch_pdl_cluster(kern, dim3((unsigned)(tiles * ways)), dim3(32 * WARPS), (unsigned)ways, smem, ctx->stream, x, W, y, M, K, N, lora, (int)ways, row_tiles);
+        e = launch_pdl_cluster(kern, dim3((unsigned)(tiles * ways)), dim3(SP_THREADS), (unsigned)ways, Sp<TM>::SMEM, ctx->stream, x, W, y, M, K, N, lora,
+                               (int)ways, row_tiles);
     if (e != cudaSuccess) return check_cuda(ctx, e, "linear_splitk_f32");
     return after_launch(ctx, "linear_splitk_f32");
 }
@@ -667,12 +638,14 @@ int rusty_cuda_linear_lora_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf* x, con
     if ((rc = rusty_cuda_buf_alloc(ctx, (size_t)t_rows * r4 * 4, 1, &t))) return rc;
     DeviceGuard g(ctx->device);
     if (ql) rc = qlinear_forward_cols(ctx, ql, x, RUSTY_CUDA_F32, M, y, RUSTY_CUDA_F32, N, 0);
-    // The kernel with K cut where rows and columns can be read four at a time and it is the faster one.  Below 2^20 weights the tiles
-    // are (one chain of 512 k, 512 columns, against a cluster's meeting: 16 rows 5.3 / 7.6 us; 1024 x 1024: 8.0 / 7.6).  Up to four
-    // rows they read W faster and only their chain of K is slow: us, tiles / cut, K x N at one row: 8192 x 512 40.5 / 14.2, 4096 x
-    // 1024 21.9 / 17.2, 2048 x 2048 12.6 / 9.7, 4096 x 4096 22.4 / 22.0, 2048 x 8192 16.1 / 21.2, 8192 x 8192 48.6 / 63.1.
-    const uint64_t weights = (uint64_t)K * N;
-    const bool cut = weight && K % 4 == 0 && N % 4 == 0 && weights >= (1u << 20) && (M > 4 || (N <= K && weights < (1u << 24))) &&
+    // The kernel with K cut where columns can be read four at a time and it is the faster one (tiles / cut, us).  Not below 2^20 weights (16 rows of
+    // 512 x 512 5.3 / 7.6), up to 32 rows not below 2^21 where K < 1024, where the tiles' chains are short (512 x 2048 at 16 / 32 / 64 rows 6.5 / 7.1,
+    // 7.5 / 10.0, 10.3 / 10.4; 512 x 8192 at 16 / 64 12.1 / 8.6 and 35.5 / 22.7; 1024 x 1024 at 1 / 16 / 256 7.3 / 5.1, 7.6 / 7.1, 22.6 / 19.2).
+    // Not for many outputs of few links each, where the tiles of 64 x 64 fill the chip with whole CTAs: 512 x 4096 at 512 / 1024 rows 80.5 / 71
+    // and 108 / 141, 1024 x 4096 at 512 / 1024 154 / 114 and 207 / 230, 2048 x 8192 at 512 / 1024 397 / 388 and 675 / 758, 8192 x 8192
+    // at 512 / 1024 1586 / 1394 and 2681 / 2728, 4096 x 4096 at 1024 797 / 728.
+    const uint64_t weights = (uint64_t)K * N, outputs = (uint64_t)M * N;
+    const bool cut = weight && K % 4 == 0 && N % 4 == 0 && weights >= (K < 1024 && M <= 32 ? 1u << 21 : 1u << 20) && (M <= 256 || outputs < 4096ull * K) &&
                      ((reinterpret_cast<uintptr_t>(x->ptr) | reinterpret_cast<uintptr_t>(weight->ptr) | reinterpret_cast<uintptr_t>(lora_b->ptr) |
                        reinterpret_cast<uintptr_t>(y->ptr)) & 15) == 0;
     for (uint32_t m0 = 0; m0 < M && !rc; m0 += PASS_ROWS) {
@@ -684,9 +657,10 @@ int rusty_cuda_linear_lora_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf* x, con
         if (rc) break;
         if (cut) {
             const float* w = (const float*)weight->ptr;
-            rc = m <= 8    ? launch_splitk<1>(ctx, xp, w, yp, m, K, N, tail)
-                 : m <= 16 ? launch_splitk<2>(ctx, xp, w, yp, m, K, N, tail)
-                           : launch_splitk<4>(ctx, xp, w, yp, m, K, N, tail);
+            rc = m <= 4    ? launch_splitk<4>(ctx, xp, w, yp, m, K, N, tail)
+                 : m <= 8  ? launch_splitk<8>(ctx, xp, w, yp, m, K, N, tail)
+                 : m <= 16 ? launch_splitk<16>(ctx, xp, w, yp, m, K, N, tail)
+                           : launch_splitk<32>(ctx, xp, w, yp, m, K, N, tail);
         } else if (weight) {
             rc = launch_matmul<false>(ctx, xp, (const float*)weight->ptr, yp, m, K, N, tail);
         } else {

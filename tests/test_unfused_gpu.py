@@ -291,8 +291,9 @@ def test_linear_lora_first_products_back_to_back(ctx, engine, M, rank):
 @pytest.mark.parametrize("M,K,N,rank", [(1, 4096, 260, 2), (5, 1028, 1024, 8), (8, 1024, 1100, 3), (9, 2052, 516, 17), (16, 4096, 260, 64), (17, 1040, 1012, 1),
                                         (33, 1024, 4100, 30), (100, 8192, 132, 4)])
 def test_linear_lora_with_k_cut(ctx, engine, M, K, N, rank):
-    """The f32 weight's kernel that cuts K and multiplies on the tensor cores, at ragged rows, columns, units of k and ranks.  Bound: the
-    split costs a product at most 2^-22 of itself, and at most 48 additions of 2^-24 of the sum of magnitudes lie on an output's way."""
+    """The f32 weight's kernel that cuts K, at ragged rows, columns, units of k and ranks.  Bound: a product enters with the rounding of its
+    addition alone, and at most 88 roundings of 2^-24 of the sum of magnitudes lie on an output's way (72 links of a chain, two halves, eight
+    warps, eight ranges); half of that and more cancels, 52 are asked for."""
     rng = np.random.default_rng(M + K + N)
     x, w = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((K, N)).astype(np.float32)
     x[:, rng.integers(0, K, size=4)] *= 1000.0
@@ -317,3 +318,63 @@ def test_linear_lora_with_k_cut(ctx, engine, M, K, N, rank):
     assert np.array_equal(got[rows, N // 2], np.sign(xi[rows, K - 1]) * -np.inf)
     # the infinite x times A makes an infinite or undefined t, and that times a zero B is undefined, as in the products one by one
     assert np.isnan(got[M // 2]).all()
+
+
+def _with_k_cut(ctx, engine, x, w, a=None, b=None):
+    (M, K), N = x.shape, w.shape[1]
+    a = np.zeros((K, 4), np.float32) if a is None else a
+    b = np.zeros((4, N), np.float32) if b is None else b
+    tensors = [UnifiedTensor.new(ctx, v, list(v.shape)) for v in (x, w, a, b)]
+    out = GuardedOutput(ctx, [M, N], DType.FP32)
+    engine.linear_lora(ctx, *tensors, out.tensor)
+    return out.read()
+
+
+@pytest.mark.parametrize("M", [1, 6, 16, 33])
+@pytest.mark.parametrize("case", ["normal", "near_one", "tiny_x", "huge_x", "subnormal_products"])
+def test_linear_lora_single_products(ctx, engine, M, case):
+    """One activation of a row is not zero: every output is one product, and comes out as f32 rounds it, over the whole range of
+    exponents (the zeros beside it add nothing)."""
+    K, N = 2048, 1024
+    rng = np.random.default_rng(M)
+    v = {"normal": rng.standard_normal(M), "near_one": np.full(M, 1 + 2.0**-11 + 2.0**-23), "tiny_x": rng.standard_normal(M) * 2.0**-118,
+         "huge_x": rng.standard_normal(M) * 2.0**121, "subnormal_products": rng.standard_normal(M) * 2.0**-100}[case].astype(np.float32)
+    w = {"normal": rng.standard_normal((K, N)), "near_one": np.full((K, N), 1 + 2.0**-11 + 2.0**-22), "tiny_x": rng.standard_normal((K, N)) * 2.0**90,
+         "huge_x": rng.standard_normal((K, N)), "subnormal_products": rng.standard_normal((K, N)) * 2.0**-30}[case].astype(np.float32)
+    x = np.zeros((M, K), np.float32)
+    at = rng.integers(0, K, size=M)
+    x[np.arange(M), at] = v
+    assert np.array_equal(_with_k_cut(ctx, engine, x, w), v[:, None] * w[at])
+
+
+@pytest.mark.parametrize("K,N", [(4096, 1024), (1040, 4100), (8192, 132)])
+def test_linear_lora_row_alone_and_in_a_batch(ctx, engine, K, N):
+    """Up to 32 rows a row's bits do not depend on the rows beside it; an infinite weight changes its own column alone."""
+    rng = np.random.default_rng(K + N)
+    x, w = rng.standard_normal((32, K)).astype(np.float32), rng.standard_normal((K, N)).astype(np.float32)
+    a, b = rng.standard_normal((K, 8)).astype(np.float32), rng.standard_normal((8, N)).astype(np.float32)
+    want = _with_k_cut(ctx, engine, x, w, a, b)
+    for first, rows in ((0, 1), (3, 4), (5, 7), (19, 13), (1, 17)):
+        assert_bits_equal(_with_k_cut(ctx, engine, x[first:first + rows], w, a, b), want[first:first + rows])
+    w[K // 3, N // 2] = np.inf
+    got = _with_k_cut(ctx, engine, x, w, a, b)
+    others = np.arange(N) != N // 2
+    assert_bits_equal(got[:, others], want[:, others])
+    assert np.array_equal(got[:, N // 2], np.sign(x[:, K // 3]) * np.inf)
+
+
+def test_linear_lora_with_k_cut_back_to_back(ctx, engine):
+    """Calls back to back over an x that a kernel rewrites in between, on one scratch for x . A: each sees its own."""
+    M, K, N, rank, steps = 20, 2048, 1024, 30, 8
+    rng = np.random.default_rng(5)
+    w, a, b = (rng.standard_normal(s).astype(np.float32) for s in ((K, N), (K, rank), (rank, N)))
+    xs = [rng.standard_normal((M, K)).astype(np.float32) for _ in range(3)]
+    src, zero = [UnifiedTensor.new(ctx, x, [M, K]) for x in xs], UnifiedTensor.zeros(ctx, [M, K])
+    tw, ta, tb = (UnifiedTensor.new(ctx, v, list(v.shape)) for v in (w, a, b))
+    x, ys = UnifiedTensor.empty(ctx, [M, K]), [UnifiedTensor.empty(ctx, [M, N]) for _ in range(steps)]
+    for i in range(steps):
+        engine.add(ctx, src[i % 3], zero, x)
+        engine.linear_lora(ctx, x, tw, ta, tb, ys[i])
+    for i in range(steps):
+        x64 = xs[i % 3].astype(np.float64)
+        assert rel_err(ys[i].to_vec(ctx).reshape(M, N), x64 @ w + (x64 @ a) @ b) <= 1e-6
