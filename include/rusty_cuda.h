@@ -420,7 +420,8 @@ RUSTY_CUDA_API int rusty_cuda_sampler_candidates_f32(rusty_cuda_ctx* ctx, const 
 /* Temperature / top-p sampling of one token per row on the device (Sampler::sample, rusty-loader/src/tokenizer.rs:161-204, in f32 and in
  * its order of operations), over the row's k largest logits: host_draws[m] in [0, 1) is the row's random number, host_tokens[m] the
  * token, or 0xffffffff where the k largest do not hold top_p of the probability (the host then draws from the whole row).
- * Blocking, like the call above. */
+ * exp is the device's, within two units in the last place, and the row's sum is taken in another order than a host's: a number
+ * that close to the border of two tokens may fall to either.  Blocking, like the call above. */
 RUSTY_CUDA_API int rusty_cuda_sample_top_p_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf* logits, uint32_t M, uint32_t N, uint32_t k,
                                                float temperature, float top_p, const float* host_draws, uint32_t* host_tokens);
 /* top_k over output-feature shards: every rank passes its own columns [M, Nl] (global index = rank * Nl + column);

@@ -58,8 +58,9 @@ class Sampler:
         return nucleus[0] if nucleus else 0
 
     def sample_from_candidates(self, idx, val, row_max: float, exp_sum: float):
-        """The nucleus walk over candidates sorted by value (descending; equal values by ascending index), given the
-        row's largest logit and sum exp((x - max) / T) over ALL logits.  Returns the token, or None when the
+        """The nucleus walk of `ComputeEngine.sample_top_p` on the host, for callers of `ComputeEngine.sampler_candidates`:
+        over candidates sorted by value (descending; equal values by ascending index), given the row's largest logit and
+        sum exp((x - max) / T) over ALL logits.  Returns the token, or None when the
         candidates' probability mass does not reach top_p (the nucleus is longer than the list)."""
         t = self.temperature
         scaled = (np.asarray(val, np.float32) / t).astype(np.float32)            # the reference's order: scale, then subtract
