@@ -97,13 +97,13 @@ constexpr int DIG_MAXV = 8;   // most passes of a row held in registers
 template <typename XT>
 constexpr int DIG_PLANES = sizeof(XT) == 4 ? 4 : 3;
 
-// A few fat blocks on purpose: grid = min(32, Mpad) blocks of 512 threads, R = Mpad / grid activation rows per block
-// (1 or 2), 512 / R threads per row (its own named barrier); rows from 8192 activations on have a block each whatever Mpad is, and
-// beyond 16384 a cluster of two (SPLIT; they meet for the maximum).  The kernel is launched early (programmatic dependent
-// launch) and parks in griddepcontrol.wait while the GEMM before it still runs; many small parked blocks pile up on the
-// few SMs that GEMM left free and keep the next GEMM's CTAs from being placed there.  Thirty-two blocks of at most 64
-// registers a thread fit beside a GEMM CTA on any SM and cannot fill more than eight.  Rows M..Mpad-1 are written as
-// zeros.  What a row's threads hold in registers between its maximum and its digits is read once, all loads in flight together.
+// A few fat blocks on purpose, 512 threads each: a block takes one row, two of a single row block of more than 32 rows (512 / R
+// threads per row, its own named barrier), so that there are 32 blocks at most; rows from 8192 activations on have a block
+// each (64 at most in a row block), beyond 16384 a cluster of two (SPLIT; they meet for the maximum).  The kernel is launched early
+// (programmatic dependent launch) and parks in griddepcontrol.wait, two blocks an SM, while the GEMM before it still runs; many small
+// parked blocks pile up on the few SMs that GEMM left free and keep the next GEMM's CTAs from being placed there (from 16 rows on
+// the registers of a GEMM CTA, 320 x 168, and of a block do not fit one SM together).  Rows M..Mpad-1 are written as zeros.
+// What a row's threads hold in registers between its maximum and its digits is read once, all loads in flight together.
 //
 // NORM: the activations are RMSNorm(x [+ residual]) * weight (norm_embed.cu gives the formula and its lines in the
 // reference); the row is normalised in registers between the load and the maximum, so it must fit there
@@ -1039,8 +1039,9 @@ bool tc_supported(const rusty_cuda_ctx* ctx, const QLinearArgs& a) {
 // The kernel pair below stores into the peers' arenas itself, except in the small-batch mode that has no pre-pass.
 bool tc_pushes_fused(uint32_t M) { return M >= tc_min_rows(); }
 
-// The pre-pass normalises a row held in registers: 8 x 4 activations per thread, 512 threads a row up to 32 rows and
-// 256 beyond (two rows share a block).
+// The pre-pass normalises a row held in registers: 8 x 4 activations per thread, 512 threads a row up to 32 rows and 256
+// beyond, where two rows share a block.  (From 8192 activations on they do not, and rows of up to 16384 would fit there as
+// well: those take a norm kernel in front.)
 bool tc_norm_fused(uint32_t M, uint32_t K) {
     if (M < (uint32_t)tc_min_rows()) return false;
     const uint32_t Mpad = (M + 7u) & ~7u;
@@ -1098,17 +1099,22 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
     // digit tile a CTA loads then multiplies 256 weight rows instead of 128, which takes a quarter off the bytes a
     // CTA pulls from L2 (the digits are re-read by every row tile; the weights are not).  Only where the units are
     // then taken whole: a unit's epilogue is twice a tile's, which cut units (whose pieces cross CTAs after the
-    // stream) cannot afford.  Measured on batch 32: gate|up 31.9 -> 29.9 us, LM head 98.1 -> 95.9 us; with cut units
-    // the whole stack loses 6 %.  RUSTY_TC_TWO_TILES = 0 / 1 / 2: never / by that rule / always (tuning aid).
+    // stream) cannot afford (a batch-32 stack lost 6 % with them).  One tile a unit / two, us: 4096 x 28672 at 4 / 8 / 16 / 24 rows
+    // 24.1 / 20.8, 24.6 / 21.5, 22.7 / 22.0, 24.7 / 24.8; 4096 x 128256 83.0 / 77.3, 84.4 / 78.0, 80.2 / 79.8, 85.2 / 84.1; 8192 x 57344 at 8 /
+    // 24 88.7 / 73.8, 83.6 / 79.9.  (From 128 digit columns on pairs of CTAs share the digits instead: below.)
+    // RUSTY_TC_TWO_TILES = 0 / 1 / 2: never / by that rule / always (tuning aid).
     static const int two_tiles = getenv("RUSTY_TC_TWO_TILES") ? atoi(getenv("RUSTY_TC_TWO_TILES")) : 1;
     // RUSTY_TC_DP_PERCENT: least share of the SMs that whole tiles must keep streaming (default 72; 101 turns the rule off).
     static const int dp_percent = getenv("RUSTY_TC_DP_PERCENT") ? atoi(getenv("RUSTY_TC_DP_PERCENT")) : 72;
     p.kb_total = (p.K + BK - 1) / BK;
     // The schedule of `tiles` units on groups of CTAs.
     // A GEMM CTA and a pre-pass block do not fit one SM together (registers), and the NEXT pair's pre-pass blocks are
-    // resident (two per SM, up to 16 SMs) while this GEMM's CTAs are placed.  A short launch whose every tile is cut
-    // (fewer tiles than SMs) and whose grid leaves those SMs no room gets its last CTAs placed only after the pre-pass
-    // has finished, 2-5 us late: plan it for 16 SMs fewer (q|k|v 6144 x 4096: 144 -> 96 CTAs, 18.2 -> 16.8 us).
+    // resident (two per SM: 16 SMs up to 8191 activations, 64 at most for longer rows) while this GEMM's CTAs are placed.  A
+    // short launch whose every tile is cut (fewer tiles than SMs) and whose grid leaves those SMs no room gets its last CTAs
+    // placed only after the pre-pass has finished, 2-5 us late: plan it for 16 SMs fewer (q|k|v 6144 x 4096: 144 -> 96 CTAs, 18.2 ->
+    // 16.8 us).  Not for more where the next rows are long (this launch does not know them): none / 16 / 32 / 64 SMs left, us: four
+    // 8B-shaped layers and the head at 32 rows 424 / 415 / 430 / 466, two 70B-shaped ones at 64 rows 598 / 600 / 627 / 598, 28672 x
+    // 8192 and 8192 x 10240 in turn at 32 rows 75.0 / 74.7 / 78.7 / 77.2, at 64 rows 88.0 / 88.3 / 102.7 / 93.2.
     // RUSTY_TC_ROOM=0 turns the rule off (tuning aid).
     auto plan = [&](int tiles, int group, int tpu, TcSchedule* out) {
         int sms = ctx->sm_count / group;
@@ -1139,11 +1145,14 @@ static int launch_tc_rows(rusty_cuda_ctx* ctx, const QLinearArgs& a, const void*
     }
     // Too many tiles for two CTAs each and too few for the SMs (66 < tiles < 107): runs of k-blocks would leave most CTAs with pieces of
     // two tiles to exchange.  Units of as many rows (a multiple of eight) as give every CTA one whole unit instead, on pairs where
-    // there are digits to share.  Runs / units of N / 148 rows, us: 4 x 4096 x 12288 16.3 / 13.9, 16 rows 16.9 / 14.4, 32 rows 20.1 / 17.1,
-    // 64 rows 27.1 / 21.9; 32 x 2048 x 9000 14.5 / 11.3; not for longer rows, where a CTA's walk of all of K is the longer part: 4 x 8192 x 10240
-    // 22.5 / 23.5, 32 rows 25.6 / 25.6, 64 rows 33.3 / 32.5, but a 70B-shaped stack 600 / 606.  And up to
-    // 1024 activations, where the exchange of any cut is longer than the walk: 4 x 1024 x 4096 7.2 / 6.8, 64 rows 12.6 / 11.0.
-    // (Two pieces a tile and 2048 activations, 4 x 2048 x 8192: 8.9 / 9.4.)
+    // there are digits to share.  Runs / units of N / 148 rows, us, the same call again and again: 4 x 4096 x 12288 16.3 / 13.9, 16 rows
+    // 16.9 / 14.4, 32 rows 20.1 / 17.1, 64 rows 27.1 / 21.9; 32 x 2048 x 9000 14.5 / 11.3.  In turn with a Linear of 4096 outputs, whose
+    // pre-pass finds fewer SMs free, at 4 / 16 / 32 / 64 rows: 4096 x 12288 24.1 / 23.8, 25.7 / 26.4, 30.2 / 28.6, 40.3 / 36.5; 4096 x
+    // 10240 23.6 / 23.5, 23.6 / 26.8, 28.7 / 28.5, 39.0 / 36.6; a layer of 7B shapes 63.2 / 63.6, 65.6 / 66.2, 76.7 / 74.5, 100.4 / 94.4.
+    // The line at 4096 activations: beyond it a CTA's walk of all of K is the longer part, and what few rows lose grows: 6144 x 10240 29.0 /
+    // 29.8, 28.6 / 32.4, 33.7 / 34.6, 46.9 / 46.0; 8192 x 10240 33.7 / 38.3, 33.8 / 38.6, 39.8 / 41.0, 50.5 / 48.7; 8192 x 12288 at 16 / 32 / 64 rows 37.1
+    // / 38.0, 41.5 / 40.6, 53.2 / 48.3; a 70B-shaped stack 600 / 606.  And up to 1024 activations, where the exchange of any cut is longer
+    // than the walk: 4 x 1024 x 4096 7.2 / 6.8, 64 rows 12.6 / 11.0.  (Two pieces a tile and 2048 activations, 4 x 2048 x 8192: 8.9 / 9.4.)
     const int even_rows = (p.N + ctx->sm_count * 8 - 1) / (ctx->sm_count * 8) * 8;
     bool even = false;
     if (nblk == 1 && even_rows <= BM && a.N > (uint32_t)BM && p.kb_total <= 32) {
