@@ -188,6 +188,42 @@ def test_rows_cut_over_a_cluster(ctx, engine, oracle, M, N, k):
     assert np.max(np.abs(c_sm - want_sm) / want_sm) < 2e-6
 
 
+@pytest.mark.parametrize("M,N,k", [(1, 1, 1), (3, 300, 7), (40, 4096, 64), (2, 70001, 1024), (5, 128256, 513)])
+def test_top_p_draw_on_the_device(ctx, engine, M, N, k):
+    """The nucleus walk on the device against the host's over the whole row: flat and peaked rows, one value only, NaN and
+    infinities, the smallest draw; rows whose nucleus is longer than k are handed back."""
+    from rusty_b200.sampler import Sampler
+    rng = np.random.default_rng(M + N + k)
+    logits = (rng.standard_normal((M, N)) * rng.uniform(0.5, 6.0, size=(M, 1))).astype(np.float32)
+    if M > 2:
+        logits[1, : N // 2] = np.nan
+        logits[2] = np.float32(-3.0)
+        logits[0, N // 3] = np.float32(-np.inf)
+    t = UnifiedTensor.new(ctx, logits, [M, N])
+    for temp, top_p in ((0.7, 0.9), (1.3, 0.4), (0.2, 0.98)):
+        draws = rng.random(M).astype(np.float32)
+        draws[0] = 0.0
+        got = engine.sample_top_p(ctx, t, k, temp, top_p, draws)
+        idx, val, mx, sm = engine.sampler_candidates(ctx, t, k, temp)
+        for m in range(M):
+            # exp differs by three units in the last place between here and there, and a sum of k terms rounds k times: a draw, or a
+            # top_p, that close to a sum may fall to either side
+            near = (4 + k) * 2.0**-24
+            want = set()
+            for dr in (0.0, -near, near):
+                for dp in (0.0, -near, near):
+                    w = Sampler(temp, top_p + dp, rand=lambda: np.float32(draws[m] + dr)).sample_from_candidates(idx[m], val[m], mx[m], sm[m])
+                    want.add(0xFFFFFFFF if w is None else w)
+            assert int(got[m]) in want, (temp, top_p, m)
+            assert len(want) <= 3
+    from rusty_b200 import BackendError
+    with pytest.raises(BackendError) as e:
+        engine.sample_top_p(ctx, t, k, 0.0, 0.9, draws)
+    assert e.value.kind == "InvalidOperation"
+    with pytest.raises(ValueError):
+        engine.sample_top_p(ctx, t, k, 1.0, 0.9, draws[:-1] if M > 1 else np.zeros(2, np.float32))
+
+
 def _winners(row, k, temp):
     """Of one row: indexes and values of its k largest logits in descending order (equal ones by ascending index; no NaN, nothing that is
     not above -1e9; index 0 and -inf where there are fewer), its largest number, and the sum of exp((x - max) / T) in 64 bits."""
@@ -201,8 +237,8 @@ def _winners(row, k, temp):
 
 
 @pytest.mark.parametrize("M,N,k", [(1, 1, 1), (3, 300, 7), (40, 4096, 64), (2, 70001, 1024), (5, 128256, 513)])
-def test_top_p_draw_on_the_device(ctx, engine, M, N, k):
-    """The nucleus walk on the device against the host's over candidates and sums that numpy takes from the logits: flat and peaked
+def test_top_p_draw_from_the_logits(ctx, engine, M, N, k):
+    """The same draw against the host's walk over candidates and sums that numpy takes from the logits: flat and peaked
     rows, one value only, NaN and infinities, the smallest draw; rows whose nucleus is longer than k are handed back."""
     from rusty_b200.sampler import Sampler
     rng = np.random.default_rng(M + N + k)
@@ -228,9 +264,3 @@ def test_top_p_draw_on_the_device(ctx, engine, M, N, k):
                     want.add(0xFFFFFFFF if w is None else w)
             assert int(got[m]) in want, (temp, top_p, m)
             assert len(want) <= 3
-    from rusty_b200 import BackendError
-    with pytest.raises(BackendError) as e:
-        engine.sample_top_p(ctx, t, k, 0.0, 0.9, draws)
-    assert e.value.kind == "InvalidOperation"
-    with pytest.raises(ValueError):
-        engine.sample_top_p(ctx, t, k, 1.0, 0.9, draws[:-1] if M > 1 else np.zeros(2, np.float32))
