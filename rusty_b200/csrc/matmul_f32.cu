@@ -442,19 +442,24 @@ __global__ void __launch_bounds__(SP_THREADS, 1) linear_splitk_f32_kernel(const 
             const float* p = (tail ? lora.b : W) + (size_t)(k0 + half) * N + c0;
             const uint32_t k = k0 + (lane & 15);
             const float* a = (tail ? lora.t : x) + (size_t)m0 * lda + k;
-            if (k0 + 16 <= len && m0 + TM <= M) {
-                a += (size_t)half * lda;
+            // Rows that do not exist are not copied: whatever lies there goes into sums that are not stored.  (A rolled loop that repeated the
+            // last row in their place made every ragged number of rows wait for its copies: 4096 x 4096 at 24 / 40 / 213 rows 44.4 / 79.6 / 227 us
+            // instead of 31.9 / 53.4 / 200.)
+            const int rows = (int)min((uint32_t)TM, M - m0) - half;
+            a += (size_t)half * lda;
+            if (k0 + 16 <= len) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i, p += 2 * (size_t)N) cp_async<true>(to_w + (uint32_t)(2 * i * SP_BN) * 4, p, 16u);
 #pragma unroll
-                for (int i = 0; i < TM / 2; ++i, a += 2 * (size_t)lda) cp_async<false>(to_x + (uint32_t)(2 * i) * 4, a, 4u);
-            } else {   // links that do not exist are zeros (t's rows are padded with them to r4), rows that do not exist repeat the last one
+                for (int i = 0; i < TM / 2; ++i, a += 2 * (size_t)lda)
+                    if (2 * i < rows) cp_async<false>(to_x + (uint32_t)(2 * i) * 4, a, 4u);
+            } else {   // links that do not exist are zeros (t's rows are padded with them to r4)
                 const int left = (int)(len - k0) - half;
                 const uint32_t bytes = k < lda ? 4u : 0u;
 #pragma unroll 1
                 for (int i = 0; i < 8; ++i, p += 2 * (size_t)N) cp_async<true>(to_w + (uint32_t)(2 * i * SP_BN) * 4, 2 * i < left ? p : W, 2 * i < left ? 16u : 0u);
 #pragma unroll 1
-                for (int i = 0; i < TM / 2; ++i) cp_async<false>(to_x + (uint32_t)(2 * i) * 4, bytes ? a + (size_t)min(half + 2 * i, (int)(M - 1 - m0)) * lda : x, bytes);
+                for (int i = 0; 2 * i < rows; ++i, a += 2 * (size_t)lda) cp_async<false>(to_x + (uint32_t)(2 * i) * 4, bytes ? a : x, bytes);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
