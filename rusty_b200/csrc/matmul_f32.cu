@@ -415,7 +415,8 @@ __global__ void __launch_bounds__(SP_THREADS, 1) linear_splitk_f32_kernel(const 
     const int warp = warp_id(), lane = threadIdx.x & 31, half = lane >> 4;
     const uint32_t way = blockIdx.x % (uint32_t)ways, tile = blockIdx.x / (uint32_t)ways;
     const uint32_t m0 = (tile % row_tiles) * TM, n0 = (tile / row_tiles) * SP_BN;
-    const uint32_t c0 = min(n0 + 4 * (lane & 15), N - 4);      // (N % 4 == 0; columns that do not exist repeat the last and are not stored)
+    const uint32_t c0 = n0 + 4 * (lane & 15);                  // this lane's four columns (N % 4 == 0: there or not)
+    const bool there = c0 < N;
     const uint32_t ring = smem_u32(sp_smem) + (uint32_t)(warp * ST * C::STAGE) * 4;
     unsigned long long acc[TM / 2][4];                         // [two rows][column]
 #pragma unroll
@@ -442,22 +443,24 @@ __global__ void __launch_bounds__(SP_THREADS, 1) linear_splitk_f32_kernel(const 
             const float* p = (tail ? lora.b : W) + (size_t)(k0 + half) * N + c0;
             const uint32_t k = k0 + (lane & 15);
             const float* a = (tail ? lora.t : x) + (size_t)m0 * lda + k;
-            // Rows that do not exist are not copied: whatever lies there goes into sums that are not stored.  (A rolled loop that repeated the
+            // Rows and columns that do not exist are not copied: whatever lies there goes into sums that are not stored.  (A rolled loop that repeated the
             // last row in their place made every ragged number of rows wait for its copies: 4096 x 4096 at 24 / 40 / 213 rows 44.4 / 79.6 / 227 us
             // instead of 31.9 / 53.4 / 200.)
             const int rows = (int)min((uint32_t)TM, M - m0) - half;
             a += (size_t)half * lda;
             if (k0 + 16 <= len) {
+                if (there)
 #pragma unroll
-                for (int i = 0; i < 8; ++i, p += 2 * (size_t)N) cp_async<true>(to_w + (uint32_t)(2 * i * SP_BN) * 4, p, 16u);
+                    for (int i = 0; i < 8; ++i, p += 2 * (size_t)N) cp_async<true>(to_w + (uint32_t)(2 * i * SP_BN) * 4, p, 16u);
 #pragma unroll
                 for (int i = 0; i < TM / 2; ++i, a += 2 * (size_t)lda)
                     if (2 * i < rows) cp_async<false>(to_x + (uint32_t)(2 * i) * 4, a, 4u);
             } else {   // links that do not exist are zeros (t's rows are padded with them to r4)
                 const int left = (int)(len - k0) - half;
                 const uint32_t bytes = k < lda ? 4u : 0u;
+                if (there)
 #pragma unroll 1
-                for (int i = 0; i < 8; ++i, p += 2 * (size_t)N) cp_async<true>(to_w + (uint32_t)(2 * i * SP_BN) * 4, 2 * i < left ? p : W, 2 * i < left ? 16u : 0u);
+                    for (int i = 0; i < 8; ++i, p += 2 * (size_t)N) cp_async<true>(to_w + (uint32_t)(2 * i * SP_BN) * 4, 2 * i < left ? p : W, 2 * i < left ? 16u : 0u);
 #pragma unroll 1
                 for (int i = 0; 2 * i < rows; ++i, a += 2 * (size_t)lda) cp_async<false>(to_x + (uint32_t)(2 * i) * 4, bytes ? a : x, bytes);
             }
