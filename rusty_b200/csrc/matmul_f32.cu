@@ -84,6 +84,12 @@ __device__ __forceinline__ float lds_f1(const float* p) {
     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(smem_u32(p)));
     return v;
 }
+// A global load as volatile asm, for the same reason.
+__device__ __forceinline__ float4 ldg_f4(const float* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
 // two FMAs an instruction, each half rounded like fmaf
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
     unsigned long long v;
@@ -379,15 +385,17 @@ int launch_lora_down(rusty_cuda_ctx* ctx, const float* x, const float* A, float*
 // y[M, N] = [x | t] . [W ; B], f32 throughout: every product enters by a fused multiply-add, so that infinities, subnormals and single
 // products are what f32 makes them.  No shader gives the order of this sum (the reference adds two products), so K is cut: a warp owns 64
 // columns x TM rows x a range of K in units of sixteen links, its halves take the even and the odd ones, a lane four neighbouring columns
-// (pairs of rows share an FMA instruction).  Each warp has a ring of its own, filled with cp.async: W as it is, x as [link][row], so that four
-// rows are one read.  The ranges of a CTA's warps are summed in shared memory, those of a cluster's CTAs in distributed shared memory,
-// in a fixed order that depends on K, N and the rank, and beyond 32 rows on their number: up to there a row's bits do not depend on the
-// rows beside it.  Against float64, 2-norm, K = 4096: 2.1e-7 where one f32 chain is off by 1.1e-6; K = 8192 x 8192: 3.4e-7 and 1.3e-6.
+// (pairs of rows share an FMA instruction).  Each warp has a ring of its own: W as it is, by cp.async, and x as [link][row], so that four
+// rows are one read: from 16 rows on by way of registers, a unit ahead (a copy of four bytes a lane takes the copy pipe some 15 cycles; 32 x 912
+// x 7172 19.6 -> 17.8 us), below that by such copies.  The ranges of a CTA's warps are summed in shared memory, those of a cluster's
+// CTAs in distributed shared memory, in a fixed order that depends on K, N and the rank, and beyond 32 rows on their number: up to there a
+// row's bits do not depend on the rows beside it.  Against float64, 2-norm, K = 4096: 2.1e-7 where one f32 chain is off by 1.1e-6; K =
+// 8192 x 8192: 3.4e-7 and 1.3e-6.
 //
-// What bounds it: up to eight rows W (96 KB in flight an SM) and the fixed part of two launches, beyond sixteen the FMAs: the pipe is busy 68 %
-// of a CTA's time at 256 rows.  4096 x 4096, rank 8, whole call in a graph, one chain of K on the matmul's tiles / this, us: one row 21.7
-// / 13.4, 8 rows 31.1 / 14.0, 16 rows 38.7 / 20.0, 64 rows 80.2 / 54.5, 256 rows 250 / 207; 8192 x 512: 8 rows 39.3 / 8.9, 64 rows 61.4 / 38.8;
-// 8192 x 8192, rank 64: one row 47.7 / 40.4, 64 rows 500 / 208.
+// What bounds it: up to eight rows W (96 KB in flight an SM) and the fixed part of two launches, beyond sixteen the FMAs: the pipe is busy 65 %
+// of a CTA's time at 256 rows.  4096 x 4096, rank 8, whole call in a graph, one chain of K on the matmul's tiles / this, us: one row 21.6
+// / 13.2, 8 rows 31.2 / 13.9, 16 rows 37.8 / 19.8, 64 rows 79.5 / 52.7, 256 rows 248 / 197; 8192 x 512: 8 rows 39.3 / 9.0, 64 rows 60.0 / 20.3;
+// 8192 x 8192, rank 64: one row 47.2 / 40.2, 64 rows 495 / 203.
 // Tried: two tf32 an f32 on the tensor cores (the products lose up to 2^-21 of themselves; 8 rows 21.7, 16 rows 25.6, 64 rows 57.4, 256 rows
 // 213); W through registers instead of a ring (8 rows 23, 16 rows 28, 64 rows 72); 256 columns a CTA (clusters of eight, of which 15 fit: 47).
 constexpr int SP_BN = 64, SP_WARPS = 8, SP_THREADS = 32 * SP_WARPS, SP_STAGES = 4;
@@ -396,6 +404,8 @@ struct Sp {
     static constexpr int LDX = TM + 4;                                          // floats between links of x in shared memory
     static constexpr int STAGE = 16 * (SP_BN + LDX);                            // floats of a unit: W, then x
     static constexpr int PIECE = TM < 16 ? TM : 16;                             // rows read ahead of their FMAs
+    static constexpr bool X_REGS = TM >= 16;                                    // x goes to shared memory by way of registers
+    static constexpr int XV = X_REGS ? TM / 8 : 1;
     static constexpr int RING = SP_WARPS * SP_STAGES * STAGE, PART = SP_WARPS * TM * SP_BN;
     static constexpr size_t SMEM = (size_t)(RING > PART ? RING : PART) * 4;
 };
@@ -405,6 +415,8 @@ __device__ __forceinline__ ulonglong2 lds_2xf32x2(uint32_t addr) {
     asm volatile("ld.shared.v2.u64 {%0,%1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(addr));
     return v;
 }
+
+__device__ __forceinline__ void sts_f1(uint32_t addr, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
 
 template <int TM>
 __global__ void __launch_bounds__(SP_THREADS, 1) linear_splitk_f32_kernel(const float* x, const float* W, float* y, uint32_t M, uint32_t K, uint32_t N,
@@ -443,38 +455,77 @@ __global__ void __launch_bounds__(SP_THREADS, 1) linear_splitk_f32_kernel(const 
             const float* p = (tail ? lora.b : W) + (size_t)(k0 + half) * N + c0;
             const uint32_t k = k0 + (lane & 15);
             const float* a = (tail ? lora.t : x) + (size_t)m0 * lda + k;
-            // Rows and columns that do not exist are not copied: whatever lies there goes into sums that are not stored.  (A rolled loop that repeated the
-            // last row in their place made every ragged number of rows wait for its copies: 4096 x 4096 at 24 / 40 / 213 rows 44.4 / 79.6 / 227 us
-            // instead of 31.9 / 53.4 / 200.)
+            // Rows and columns that do not exist are not copied: whatever lies there goes into sums that are not stored.  (Copies of the last
+            // ones in their place: a rolled loop over rows took 79.6 us for 40 x 4096 x 4096, now 52.1, and lanes that copied one address
+            // 139.8 us for 194 x 3152 x 3980, now 123.)
             const int rows = (int)min((uint32_t)TM, M - m0) - half;
             a += (size_t)half * lda;
             if (k0 + 16 <= len) {
                 if (there)
 #pragma unroll
                     for (int i = 0; i < 8; ++i, p += 2 * (size_t)N) cp_async<true>(to_w + (uint32_t)(2 * i * SP_BN) * 4, p, 16u);
+                if constexpr (!C::X_REGS)
 #pragma unroll
-                for (int i = 0; i < TM / 2; ++i, a += 2 * (size_t)lda)
-                    if (2 * i < rows) cp_async<false>(to_x + (uint32_t)(2 * i) * 4, a, 4u);
+                    for (int i = 0; i < TM / 2; ++i, a += 2 * (size_t)lda)
+                        if (2 * i < rows) cp_async<false>(to_x + (uint32_t)(2 * i) * 4, a, 4u);
             } else {   // links that do not exist are zeros (t's rows are padded with them to r4)
                 const int left = (int)(len - k0) - half;
                 const uint32_t bytes = k < lda ? 4u : 0u;
                 if (there)
 #pragma unroll 1
                     for (int i = 0; i < 8; ++i, p += 2 * (size_t)N) cp_async<true>(to_w + (uint32_t)(2 * i * SP_BN) * 4, 2 * i < left ? p : W, 2 * i < left ? 16u : 0u);
+                if constexpr (!C::X_REGS)
 #pragma unroll 1
-                for (int i = 0; 2 * i < rows; ++i, a += 2 * (size_t)lda) cp_async<false>(to_x + (uint32_t)(2 * i) * 4, bytes ? a : x, bytes);
+                    for (int i = 0; 2 * i < rows; ++i, a += 2 * (size_t)lda) cp_async<false>(to_x + (uint32_t)(2 * i) * 4, bytes ? a : x, bytes);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    // X_REGS: a lane takes four links of rows lane / 4 + 8 i, a unit ahead of their stores
+    float4 xn[C::XV];
+    auto load_x = [&](float4 (&v)[C::XV], uint32_t u) {
+        if (u >= u1) return;
+        const bool tail = u >= units_k;
+        if (tail && !t_ready) {
+            pdl_wait();
+            t_ready = true;
+        }
+        const uint32_t lda = tail ? (uint32_t)lora.r4 : K, k = (tail ? u - units_k : u) * 16 + 4 * (lane & 3), row = m0 + (lane >> 2);
+        const float* a = (tail ? lora.t : x) + (size_t)row * lda + k;
+#pragma unroll
+        for (int i = 0; i < C::XV; ++i, a += 8 * (size_t)lda)
+            v[i] = k < lda && row + 8 * i < M ? ldg_f4(a) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto store_x = [&](const float4 (&v)[C::XV], int slot) {
+        const int at = (lane >> 2) + 8 * ((lane >> 1) & 1);
+        const uint32_t to = ring + (uint32_t)(slot * C::STAGE + 16 * SP_BN + 4 * (lane & 3) * C::LDX) * 4;
+#pragma unroll
+        for (int i = 0; i < C::XV; ++i) {
+            const uint32_t d = to + (uint32_t)((at + 8 * i) & (TM - 1)) * 4;
+            sts_f1(d, v[i].x);
+            sts_f1(d + C::LDX * 4, v[i].y);
+            sts_f1(d + 2 * C::LDX * 4, v[i].z);
+            sts_f1(d + 3 * C::LDX * 4, v[i].w);
+        }
+    };
 #pragma unroll 1
     for (int d = 0; d < ST - 1; ++d) fetch(u0 + d, d);
+    if constexpr (C::X_REGS) {
+        float4 first[C::XV];
+        load_x(first, u0);
+        load_x(xn, u0 + 1);
+        store_x(first, 0);
+    }
     int slot = 0;
 #pragma unroll 1
     for (uint32_t u = u0; u < u1; ++u) {
         asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
         __syncwarp();                                          // unit u is there for all lanes, and the one before has been read by all
         fetch(u + ST - 1, slot == 0 ? ST - 1 : slot - 1);
+        if constexpr (C::X_REGS) {
+            store_x(xn, slot == ST - 1 ? 0 : slot + 1);
+            load_x(xn, u + 2);
+        }
         const uint32_t from_w = ring + (uint32_t)(slot * C::STAGE + half * SP_BN + 4 * (lane & 15)) * 4;
         const uint32_t from_x = ring + (uint32_t)(slot * C::STAGE + 16 * SP_BN + half * C::LDX) * 4;
         constexpr int PER = TM / PIECE, PIECES = 8 * PER;
@@ -483,7 +534,10 @@ __global__ void __launch_bounds__(SP_THREADS, 1) linear_splitk_f32_kernel(const 
         auto read = [&](int p) {
             if (p % PER == 0) wv[(p / PER) & 1] = lds128(from_w + (uint32_t)((p / PER) * 2 * SP_BN) * 4);
 #pragma unroll
-            for (int q = 0; q < PIECE / 4; ++q) xv[p & 1][q] = lds_2xf32x2(from_x + (uint32_t)((p / PER) * 2 * C::LDX + (p % PER) * PIECE + 4 * q) * 4);
+            for (int q = 0; q < PIECE / 4; ++q) {
+                const int row = ((p % PER) * PIECE + 4 * q + (C::X_REGS ? 8 * ((p / PER) >> 2) : 0)) & (TM - 1);
+                xv[p & 1][q] = lds_2xf32x2(from_x + (uint32_t)((p / PER) * 2 * C::LDX + row) * 4);
+            }
         };
         read(0);
 #pragma unroll
