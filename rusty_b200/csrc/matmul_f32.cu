@@ -608,16 +608,21 @@ __global__ void __launch_bounds__(SP_THREADS, 1) linear_splitk_f32_kernel(const 
     cl.sync();                                 // the others have read this CTA's sums
 }
 
+// K ranges (CTAs of a cluster) for so many tiles: what fills the SMs with one CTA each, of a unit a warp at least.  Clusters lie in one
+// GPC: of more than two CTAs not as many fit as there are SMs (of 148: 132 in clusters of four, 120 of eight), so beyond two an
+// eighth of them is left out, and of eight only as many CTAs are taken as fit (4096 x 1024 at 16 rows: 16 clusters of eight 16.5 us, of four 12.1).
+uint64_t splitk_ways(uint64_t tiles, uint32_t K, uint64_t sms) {
+    uint64_t ways = sms / tiles >= 3 ? sms * 7 / 8 / tiles : sms / tiles;
+    const uint64_t most = K / (16 * SP_WARPS);
+    if (ways > most) ways = most;
+    return ways < 1 ? 1 : ways <= 4 ? ways : ways < 8 || tiles * 8 > sms * 13 / 16 ? 4 : 8;
+}
+
 template <int TM>
 int launch_splitk(rusty_cuda_ctx* ctx, const float* x, const float* W, float* y, uint32_t M, uint32_t K, uint32_t N, const LoraTail& lora) {
     const uint32_t groups = (N + SP_BN - 1) / SP_BN, row_tiles = (M + TM - 1) / TM;
     const uint64_t tiles = (uint64_t)groups * row_tiles, sms = (uint64_t)(ctx->sm_count > 0 ? ctx->sm_count : 1);
-    // K ranges: what fills the SMs with one CTA each, of two units a warp at least.  Clusters lie in one GPC: of more than two CTAs not as
-    // many fit as there are SMs (of 148: 132 in clusters of four, 120 of eight), so beyond two an eighth of them is left out.
-    uint64_t ways = sms / tiles >= 3 ? sms * 7 / 8 / tiles : sms / tiles;
-    const uint64_t most = K / (32 * SP_WARPS);
-    if (ways > most) ways = most;
-    ways = ways < 1 ? 1 : ways > 4 ? (ways < 8 ? 4 : 8) : ways;
+    const uint64_t ways = splitk_ways(tiles, K, sms);
     auto kern = linear_splitk_f32_kernel<TM>;
     cudaError_t e = ensure_dynamic_smem((const void*)kern, ctx->device, Sp<TM>::SMEM);
     if (e == cudaSuccess)
@@ -701,13 +706,12 @@ int rusty_cuda_linear_lora_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf* x, con
     DeviceGuard g(ctx->device);
     if (ql) rc = qlinear_forward_cols(ctx, ql, x, RUSTY_CUDA_F32, M, y, RUSTY_CUDA_F32, N, 0);
     // The kernel with K cut where columns can be read four at a time and it is the faster one (tiles / cut, us).  Not below 2^20 weights (16 rows of
-    // 512 x 512 5.3 / 7.6), up to 32 rows not below 2^21 where K < 1024, where the tiles' chains are short (512 x 2048 at 16 / 32 / 64 rows 6.5 / 7.1,
-    // 7.5 / 10.0, 10.3 / 10.4; 512 x 8192 at 16 / 64 12.1 / 8.6 and 35.5 / 22.7; 1024 x 1024 at 1 / 16 / 256 7.3 / 5.1, 7.6 / 7.1, 22.6 / 19.2).
-    // Not for many outputs of few links each, where the tiles of 64 x 64 fill the chip with whole CTAs: 512 x 4096 at 512 / 1024 rows 80.5 / 71
-    // and 108 / 141, 1024 x 4096 at 512 / 1024 154 / 114 and 207 / 230, 2048 x 8192 at 512 / 1024 397 / 388 and 675 / 758, 8192 x 8192
-    // at 512 / 1024 1586 / 1394 and 2681 / 2728, 4096 x 4096 at 1024 797 / 728.
+    // 512 x 512 4.7 / 5.8; 512 x 2048 at 16 / 32 / 64 rows 6.2 / 6.0, 7.3 / 7.7, 10.3 / 7.3; 512 x 8192 at 16 / 64 11.6 / 8.7 and 35.5 / 20.8;
+    // 1024 x 1024 at 1 / 16 / 256 7.1 / 4.3, 7.8 / 6.5, 22.6 / 17.4).  Not beyond 512 rows for many outputs of few links each, where the tiles of
+    // 64 x 64 fill the chip with whole CTAs: 512 x 4096 at 512 / 1024 rows 80.2 / 67.0 and 108 / 134, 1024 x 4096 153 / 106 and 206 / 214, 2048 x
+    // 8192 390 / 365 and 675 / 734, 8192 x 8192 1530 / 1308 and 2656 / 2651, 4096 x 4096 588 / 345 and 795 / 705.
     const uint64_t weights = (uint64_t)K * N, outputs = (uint64_t)M * N;
-    const bool cut = weight && K % 4 == 0 && N % 4 == 0 && weights >= (K < 1024 && M <= 32 ? 1u << 21 : 1u << 20) && (M <= 256 || outputs < 4096ull * K) &&
+    const bool cut = weight && K % 4 == 0 && N % 4 == 0 && weights >= (1u << 20) && (M <= 512 || outputs < 4096ull * K) &&
                      ((reinterpret_cast<uintptr_t>(x->ptr) | reinterpret_cast<uintptr_t>(weight->ptr) | reinterpret_cast<uintptr_t>(lora_b->ptr) |
                        reinterpret_cast<uintptr_t>(y->ptr)) & 15) == 0;
     for (uint32_t m0 = 0; m0 < M && !rc; m0 += PASS_ROWS) {
