@@ -632,6 +632,24 @@ int launch_splitk(rusty_cuda_ctx* ctx, const float* x, const float* W, float* y,
     return after_launch(ctx, "linear_splitk_f32");
 }
 
+// Rows a tile.  Up to 32 rows one tile holds them, and a row's sum is cut the same way whatever the tile.  Beyond, tiles of 32 or of 16: a unit takes
+// a CTA 1.1 or 0.6 us, its start and end 4 or 3 and one more in a cluster; the tiles of 16 win where they fill the waves better.
+// All of 32 / of 16, us: 38 x 912 x 2992 16.1 / 10.6, 99 x 4592 x 1244 58.1 / 36.2, 200 x 1552 x 684 25.6 / 17.6, 256 x 4096 x 4096 199.7 / 197.3; 64 x
+// 4096 x 4096 52.8 / 58.5, 83 x 880 x 5996 29.6 / 36.2.  Of 125 shapes beyond 32 rows the rule takes the slower one for six, 4 % slower at most.
+int launch_splitk_rows(rusty_cuda_ctx* ctx, const float* x, const float* W, float* y, uint32_t M, uint32_t K, uint32_t N, const LoraTail& lora) {
+    if (M <= 4) return launch_splitk<4>(ctx, x, W, y, M, K, N, lora);
+    if (M <= 8) return launch_splitk<8>(ctx, x, W, y, M, K, N, lora);
+    if (M <= 16) return launch_splitk<16>(ctx, x, W, y, M, K, N, lora);
+    if (M <= 32) return launch_splitk<32>(ctx, x, W, y, M, K, N, lora);
+    const uint64_t sms = (uint64_t)(ctx->sm_count > 0 ? ctx->sm_count : 1);
+    auto us = [&](uint32_t tm, double unit, double ends) {
+        const uint64_t tiles = (uint64_t)((N + SP_BN - 1) / SP_BN) * ((M + tm - 1) / tm), ways = splitk_ways(tiles, K, sms);
+        const double units = (double)((K + 15) / 16 + (lora.r + 15) / 16) / (double)(SP_WARPS * ways);
+        return (double)((tiles * ways + sms - 1) / sms) * (units * unit + ends + (ways > 1 ? 1.0 : 0.0));
+    };
+    return us(16, 0.6, 3.0) < us(32, 1.1, 4.0) ? launch_splitk<16>(ctx, x, W, y, M, K, N, lora) : launch_splitk<32>(ctx, x, W, y, M, K, N, lora);
+}
+
 int need(rusty_cuda_ctx* ctx, const char* op, const char* name, const rusty_cuda_buf* b, size_t bytes) {
     if (!b) return fail(ctx, RUSTY_CUDA_ERR_INVALID_OPERATION, "%s: buffer '%s' is null", op, name);
     if (b->bytes < bytes)
@@ -722,11 +740,7 @@ int rusty_cuda_linear_lora_f32(rusty_cuda_ctx* ctx, const rusty_cuda_buf* x, con
         rc = launch_lora_down(ctx, xp, (const float*)lora_a->ptr, (float*)t->ptr, m, K, rank, r4);
         if (rc) break;
         if (cut) {
-            const float* w = (const float*)weight->ptr;
-            rc = m <= 4    ? launch_splitk<4>(ctx, xp, w, yp, m, K, N, tail)
-                 : m <= 8  ? launch_splitk<8>(ctx, xp, w, yp, m, K, N, tail)
-                 : m <= 16 ? launch_splitk<16>(ctx, xp, w, yp, m, K, N, tail)
-                           : launch_splitk<32>(ctx, xp, w, yp, m, K, N, tail);
+            rc = launch_splitk_rows(ctx, xp, (const float*)weight->ptr, yp, m, K, N, tail);
         } else if (weight) {
             rc = launch_matmul<false>(ctx, xp, (const float*)weight->ptr, yp, m, K, N, tail);
         } else {

@@ -378,3 +378,28 @@ def test_linear_lora_with_k_cut_back_to_back(ctx, engine):
     for i in range(steps):
         x64 = xs[i % 3].astype(np.float64)
         assert rel_err(ys[i].to_vec(ctx).reshape(M, N), x64 @ w + (x64 @ a) @ b) <= 1e-6
+
+
+@pytest.mark.parametrize("M,K,N,rank", [(33, 640, 1640, 8), (47, 1040, 1000, 4), (48, 912, 2992, 1), (49, 2052, 1028, 17), (64, 1024, 1024, 8),
+                                        (65, 4096, 260, 64), (200, 1552, 684, 12), (257, 512, 2052, 30)])
+def test_linear_lora_with_k_cut_beyond_32_rows(ctx, engine, M, K, N, rank):
+    """Tiles of 16 and of 32 rows, the last of each with a row, half of them or all; a last group of columns with 4 to 64.  Bound: what f32
+    sums may be off, each addition by 2^-24 of the magnitudes before it: the links of half a warp's range, seventeen sums of ranges, and for
+    the branch the K links of x . A before them."""
+    rng = np.random.default_rng(M + K + N + rank)
+    x, w, a, b = (rng.standard_normal(s).astype(np.float32) for s in ((M, K), (K, N), (K, rank), (rank, N)))
+    got = _with_k_cut(ctx, engine, x, w, a, b).astype(np.float64)
+    x64, w64, a64, b64 = (v.astype(np.float64) for v in (x, w, a, b))
+    links = 8 * -(-(-(-K // 16) + -(-rank // 16)) // 8) + 18
+    may = 2.0**-24 * (links * (abs(x64) @ abs(w64)) + (links + K) * (abs(x64) @ abs(a64) @ abs(b64)))
+    assert (abs(got - (x64 @ w64 + (x64 @ a64) @ b64)) <= may).all()
+
+
+def test_linear_lora_short_rows_alone_and_in_a_batch(ctx, engine):
+    """The same bits for a row alone and in a batch of up to 32 where K is short and cut over a cluster."""
+    K, N = 640, 1640
+    rng = np.random.default_rng(6)
+    x, w, a, b = (rng.standard_normal(s).astype(np.float32) for s in ((32, K), (K, N), (K, 12), (12, N)))
+    want = _with_k_cut(ctx, engine, x, w, a, b)
+    for first, rows in ((0, 1), (3, 4), (5, 8), (19, 13), (1, 17)):
+        assert_bits_equal(_with_k_cut(ctx, engine, x[first:first + rows], w, a, b), want[first:first + rows])
